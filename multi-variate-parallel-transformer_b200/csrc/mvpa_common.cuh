@@ -38,7 +38,7 @@ struct BwdArgs {
   int64_t dv_sb, dv_sh, dv_sn;
   float *du, *dvt, *dz, *drt, *drc;
   // workspace carve-up (fp32 elements)
-  float *tbg, *cbg;    // (B*H, N, T), (B*H, N, C) relative scores, base-2 scaled
+  float *tbg, *cbg;    // (B*H, T, N), (B*H, N, C) relative scores, base-2 scaled
   float *dtbg, *dcbg;  // gradients w.r.t. the unscaled relative scores, (B*H, N, slots); the tensor-core
                        // kernels use dtbg as (B*H, T, N) scratch and leave dcbg alone
   float* delta;        // (B*H, N)

@@ -2,9 +2,14 @@
 //
 // These serve element type fp32 (where tensor-core input rounding would break the
 // 1e-4 relative tolerance) and every shape the tcgen05 kernels do not take.  They
-// are tiled through shared memory (32 query rows x 64 keys per step, 256 threads)
-// and deterministic: no floating-point atomics anywhere, cross-tile sums go through
-// per-tile partials.
+// are tiled through shared memory and deterministic: no floating-point atomics
+// anywhere, cross-tile sums go through per-tile partials.
+//
+// What bounds them: short sequences have few row tiles, so the longest CTA sets the time.  Hence sixteen rows per
+// CTA, the column tiles of a row tile shared by four groups of warps, loads in flight under the products, and no
+// CTA-wide barrier in the loop.  Against 32-row CTAs with synchronous loads and five barriers per tile (device time):
+// forward B 1 H 4 T 32 C 16 D 64 71.0 -> 17.4 us; B 1 H 4 Hkv 2 T 24 C 22 D 64 forward 76.5 -> 20.9, query side (with
+// the relative scores and delta, separate launches before) 109 -> 43, key side 208 -> 50, the rest 23 -> 8 us.
 //
 // Math follows the reference forward (`attentions/attn.py:232-333`: base-2 online
 // softmax, window zero-fill, time-block causal mask, L = m + log2 l) and backward
@@ -19,254 +24,407 @@ namespace mvpa {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kBM = 32;   // rows of the register-tiled products
-constexpr int kBN = 64;   // columns
-constexpr int kPLd = kBN + 1;
+constexpr int kMinRows = 16;    // fewest rows a CTA of the query-side backward takes
 constexpr int kDrelSplit = 32;  // split-K factor of the relative-key gradient reduction
-
-// ---- tile helpers (256 threads: ty = tid/16 owns rows 2ty,2ty+1; tx = tid%16) ----
-
-// acc[a][j] += sum_d A[2ty+a][d] * B[tx+16j][d]       (A: 32 x D, B: 64 x D, ld = D+4)
-template <int D>
-__device__ __forceinline__ void tile_nt(const float* __restrict__ As, const float* __restrict__ Bs,
-                                        float (&acc)[2][4]) {
-  constexpr int LD = D + 4;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const float4* a0 = reinterpret_cast<const float4*>(As + (2 * ty) * LD);
-  const float4* a1 = reinterpret_cast<const float4*>(As + (2 * ty + 1) * LD);
-#pragma unroll 4
-  for (int d4 = 0; d4 < D / 4; ++d4) {
-    const float4 x0 = a0[d4], x1 = a1[d4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 y = reinterpret_cast<const float4*>(Bs + (tx + 16 * j) * LD)[d4];
-      acc[0][j] += x0.x * y.x + x0.y * y.y + x0.z * y.z + x0.w * y.w;
-      acc[1][j] += x1.x * y.x + x1.y * y.y + x1.z * y.z + x1.w * y.w;
-    }
-  }
-}
-
-// out[a][e] += sum_c P[2ty+a][c] * B[c][tx+16e]        (P: 32 x 64, ld 65; B: 64 x D)
-template <int D>
-__device__ __forceinline__ void tile_nn(const float* __restrict__ Ps, const float* __restrict__ Bs,
-                                        float (&out)[2][D / 16]) {
-  constexpr int LD = D + 4;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const float* p0 = Ps + (2 * ty) * kPLd;
-  const float* p1 = p0 + kPLd;
-#pragma unroll 4
-  for (int c = 0; c < kBN; ++c) {
-    const float x0 = p0[c], x1 = p1[c];
-#pragma unroll
-    for (int e = 0; e < D / 16; ++e) {
-      const float y = Bs[c * LD + tx + 16 * e];
-      out[0][e] += x0 * y;
-      out[1][e] += x1 * y;
-    }
-  }
-}
-
-// Copy `rows` rows of D elements from global (row stride `sn`, first row `row0`, rows >= n_rows
-// read as zero) to shared (ld = D+4), as (x + bias[d]) * scale in fp32.
-template <typename Tin, int D>
-__device__ __forceinline__ void load_tile(float* __restrict__ dst, const Tin* __restrict__ src,
-                                          int64_t sn, int row0, int n_rows, int rows,
-                                          const Tin* __restrict__ bias, float scale) {
-  constexpr int LD = D + 4;
-  for (int idx = threadIdx.x; idx < rows * D; idx += kThreads) {
-    const int r = idx / D, d = idx % D;
-    const int row = row0 + r;
-    float x = 0.f;
-    if (row < n_rows) {
-      x = to_f32<Tin>(src[(int64_t)row * sn + d]);
-      if (bias != nullptr) x += to_f32<Tin>(bias[d]);
-      x *= scale;
-    }
-    dst[r * LD + d] = x;
-  }
-}
-
-// Relative scores of `rows` query rows held raw in shared memory (ld = D+4):
-//   out_t[r*ldt + s] = c2 * (q_r + vt) . r_time[s],  out_c[r*ldc + e] = c2 * (q_r + z) . r_chan[e]
-// (`attentions/attn.py:1305-1314`, scaled like `:292,307`).  out_* may be shared or global.
-template <typename Tin, int D>
-__device__ __forceinline__ void rel_scores(const float* __restrict__ Qraw, int rows,
-                                           const Tin* __restrict__ vt, const Tin* __restrict__ z,
-                                           const Tin* __restrict__ rt, const Tin* __restrict__ rc,
-                                           int T, int C, float c2, float* out_t, int64_t ldt,
-                                           float* out_c, int64_t ldc, int valid_rows) {
-  constexpr int LD = D + 4;
-  const int total = rows * (T + C);
-  for (int idx = threadIdx.x; idx < total; idx += kThreads) {
-    const int r = idx % rows, s = idx / rows;
-    if (r >= valid_rows) continue;
-    const bool is_t = s < T;
-    const Tin* key = is_t ? rt + (int64_t)s * D : rc + (int64_t)(s - T) * D;
-    const Tin* bias = is_t ? vt : z;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < D; ++d)
-      acc += (Qraw[r * LD + d] + to_f32<Tin>(bias[d])) * to_f32<Tin>(key[d]);
-    acc *= c2;
-    if (is_t) out_t[(int64_t)r * ldt + s] = acc;
-    else out_c[(int64_t)r * ldc + (s - T)] = acc;
-  }
-}
 
 __device__ __forceinline__ bool in_window(int ti, int tk, int T, int window) {
   const int dt = ti - tk;
   return window <= 0 || (dt <= window && dt >= -window) || ti == T - 1;
 }
 
+// ---- building blocks of the tiled kernels --------------------------------------------------------
+//
+// A CTA owns BM = 8 * WPG rows (queries in the forward and the query-side backward, keys in the key-side
+// one) and NG groups of WPG warps share its column tiles: group g takes tiles g, g + NG, ... with its own
+// tile buffers, named barrier and partial results, which are merged once at the end.  A warp owns eight
+// rows; its two half-warps hold four each and their 16 lanes spread over the columns of a tile, so a
+// row's maximum is a four-step shuffle, a row's probabilities never leave the warp, and each product reads
+// (4 + KN / 16) 16-byte words per 16 * KN / 4 multiply-adds.
+
+// Group barrier: the WPG warps of group g.
+template <int WPG>
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(32 * WPG) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = valid ? 16 : 0;  // 0: the destination is zero-filled and nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <typename Tin>
+__device__ __forceinline__ float4 load4(const Tin* p) {
+  if constexpr (sizeof(Tin) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    const uint2 w = *reinterpret_cast<const uint2*>(p);
+    const Tin* e = reinterpret_cast<const Tin*>(&w);
+    return make_float4(to_f32<Tin>(e[0]), to_f32<Tin>(e[1]), to_f32<Tin>(e[2]), to_f32<Tin>(e[3]));
+  }
+}
+
+template <typename Tin>
+__device__ __forceinline__ void store4(Tin* p, float4 v) {
+  if constexpr (sizeof(Tin) == 4) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    uint2 w;
+    Tin* e = reinterpret_cast<Tin*>(&w);
+    e[0] = from_f32<Tin>(v.x); e[1] = from_f32<Tin>(v.y); e[2] = from_f32<Tin>(v.z); e[3] = from_f32<Tin>(v.w);
+    *reinterpret_cast<uint2*>(p) = w;
+  }
+}
+
+// ROWS rows of D elements from global (row stride `sn`, rows at or past n_rows read as zero) to shared memory
+// (fp32, ld = D + 4), by THREADS threads of which this one is number `t`: asynchronous copies for fp32 (the
+// caller commits and waits), converting loads otherwise.  Thread t writes the elements
+// [(i * THREADS + t) * 4, +4) of the row-major tile, the same ones on every call.
+template <typename Tin, int D, int ROWS, int THREADS>
+__device__ __forceinline__ void load_rows(float* dst, const Tin* src, int64_t sn, int row0, int n_rows, int t) {
+  constexpr int LD = D + 4;
+#pragma unroll
+  for (int i = 0; i < (ROWS * D / 4 + THREADS - 1) / THREADS; ++i) {
+    const int idx = i * THREADS + t;
+    if ((ROWS * D / 4) % THREADS != 0 && idx >= ROWS * D / 4) break;
+    const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+    const bool in = row0 + r < n_rows;
+    const Tin* s = src + (int64_t)(in ? row0 + r : 0) * sn + d;
+    if constexpr (sizeof(Tin) == 4)
+      cp_async16(dst + r * LD + d, s, in);
+    else
+      *reinterpret_cast<float4*>(dst + r * LD + d) = in ? load4<Tin>(s) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// acc[a][j] = sum_d A[a][d] * B[tx + 16 j][d]: A points at this half-warp's four rows, both ld = D + 4.
+// Packed multiply-adds over pairs of d (even and odd partial sums): half the instructions of scalar ones,
+// which leaves issue slots for the shared-memory loads.
+template <int D, int KJ>
+__device__ __forceinline__ void product_nt(const float* A, const float* B, int tx, float (&acc)[4][KJ]) {
+  constexpr int LD = D + 4;
+  uint64_t s[4][KJ];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) s[a][j] = 0ull;
+  const float* b0 = B + tx * LD;
+#pragma unroll 4
+  for (int d = 0; d < D; d += 4) {
+    ulonglong2 x[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const ulonglong2*>(A + a * LD + d);
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b0 + 16 * j * LD + d);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) s[a][j] = ffma2(x[a].y, y.y, ffma2(x[a].x, y.x, s[a][j]));
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < KJ; ++j)
+      acc[a][j] = __uint_as_float((uint32_t)s[a][j]) + __uint_as_float((uint32_t)(s[a][j] >> 32));
+}
+
+// Columns of a row that a lane holds: VW = D / 16 of them, in pieces of up to four adjacent ones.
+template <int D>
+struct LaneCols {
+  static constexpr int VW = D / 16;                 // 1, 2, 4, 8
+  static constexpr int PW = VW < 4 ? VW : 4;        // piece width
+  static constexpr int NP = VW / PW;                // pieces
+  __device__ static int col(int tx, int p) { return tx * PW + 16 * PW * p; }
+  __device__ static void load(const float* row, int tx, float (&v)[VW]) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      if constexpr (PW == 4) {
+        const float4 w = *reinterpret_cast<const float4*>(row + col(tx, p));
+        v[4 * p] = w.x; v[4 * p + 1] = w.y; v[4 * p + 2] = w.z; v[4 * p + 3] = w.w;
+      } else if constexpr (PW == 2) {
+        const float2 w = *reinterpret_cast<const float2*>(row + col(tx, p));
+        v[0] = w.x; v[1] = w.y;
+      } else {
+        v[0] = row[col(tx, p)];
+      }
+    }
+  }
+  __device__ static void store(float* row, int tx, const float (&v)[VW]) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      if constexpr (PW == 4) *reinterpret_cast<float4*>(row + col(tx, p)) = make_float4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
+      else if constexpr (PW == 2) *reinterpret_cast<float2*>(row + col(tx, p)) = make_float2(v[0], v[1]);
+      else row[col(tx, p)] = v[0];
+    }
+  }
+};
+
+// out[a][lane's columns] += sum_c P[a][c] * B[c][columns]: P points at this half-warp's four rows (ld = KN + 4).
+template <int D, int KN>
+__device__ __forceinline__ void product_nn(const float* P, const float* B, int tx, float (&out)[4][D / 16]) {
+  constexpr int LD = D + 4, VW = D / 16, LP = KN + 4;
+#pragma unroll 2
+  for (int c = 0; c < KN; c += 4) {
+    float4 x[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const float4*>(P + a * LP + c);
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+      float y[VW];
+      LaneCols<D>::load(B + (c + cc) * LD, tx, y);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float xv = cc == 0 ? x[a].x : cc == 1 ? x[a].y : cc == 2 ? x[a].z : x[a].w;
+#pragma unroll
+        for (int e = 0; e < VW; ++e) out[a][e] = fmaf(xv, y[e], out[a][e]);
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ float half_warp_max(float x) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+__device__ __forceinline__ float half_warp_sum(float x) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// Relative scores of the CTA's rows, all groups together: TB[r][s] = c2 (q_r + vt) . r_time[s] and
+// CB[r][e] = c2 (q_r + z) . r_chan[e]  (`attentions/attn.py:1305-1314`, scaled like `:292,307`), for the
+// `valid` rows that exist, TB with strides tb_r / tb_s.  QT and QC hold the rows with the two biases added; the
+// relative keys pass through the groups' tile buffers `Kg`.
+template <typename Tin, int D, int WPG, int NG, int KN>
+__device__ __forceinline__ void rel_products(const Args& p, int hk, const float* QT, const float* QC, float* Kg,
+                                             int valid, float* TB, int64_t tb_r, int64_t tb_s, float* CB, int g, int tg) {
+  constexpr int LD = D + 4, KJ = KN / 16;
+  const int lane = threadIdx.x & 31, tx = lane & 15, r0 = (tg >> 5) * 8 + (lane >> 4) * 4;
+  const int nt = (p.T + KN - 1) / KN, nc = (p.C + KN - 1) / KN;
+  for (int job = g; job < nt + nc; job += NG) {
+    const bool is_t = job < nt;
+    const int s0 = (is_t ? job : job - nt) * KN, n = is_t ? p.T : p.C;
+    const Tin* src = is_t ? (const Tin*)p.rt + (int64_t)hk * p.T * D : (const Tin*)p.rc + (int64_t)hk * p.C * D;
+    load_rows<Tin, D, KN, 32 * WPG>(Kg, src, D, s0, n, tg);
+    cp_async_commit();
+    cp_async_wait<0>();
+    group_sync<WPG>(g);
+    float acc[4][KJ];
+    product_nt<D, KJ>((is_t ? QT : QC) + r0 * LD, Kg, tx, acc);
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      const int s = s0 + tx + 16 * j;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        if (s < n && r0 + a < valid) {
+          if (is_t) TB[(r0 + a) * tb_r + s * tb_s] = acc[a][j] * p.c2;
+          else CB[(int64_t)(r0 + a) * n + s] = acc[a][j] * p.c2;
+        }
+      }
+    }
+    group_sync<WPG>(g);  // the buffer is free again
+  }
+}
+
 // ------------------------------- forward -------------------------------------
 
-template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_fwd_kernel(Args p) {
-  constexpr int LD = D + 4;
-  constexpr int DV = D / 16;
-  extern __shared__ float smem[];
-  float* Qs = smem;
-  float* Ks = Qs + kBM * LD;
-  float* Vs = Ks + kBN * LD;
-  float* Ps = Vs + kBN * LD;
-  float* TBs = Ps + kBM * kPLd;
-  float* CBs = TBs + kBM * p.T;
-  float* ms = CBs + kBM * p.C;
-  float* ls = ms + kBM;
-  float* alphas = ls + kBM;
+template <int D, int WPG, int NG, int KN>
+constexpr size_t fwd_fixed_floats() {
+  return (size_t)8 * WPG * (D + 4) + (size_t)NG * 2 * KN * (D + 4) + (size_t)NG * WPG * 8 * (KN + 4);
+}
 
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+template <typename Tin, int D, int WPG, int NG, int KN>
+__global__ void __launch_bounds__(32 * WPG * NG) simt_fwd_kernel(Args p) {
+  constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
+  constexpr int GT = 32 * WPG, CT = GT * NG;  // threads of a group, of the CTA
+  static_assert(NG * KN >= 2 * BM, "the V buffers hold two copies of the rows during the prologue");
+  extern __shared__ __align__(16) float smem[];
+  float* Qs = smem;
+  float* Kall = Qs + BM * LD;
+  float* Vall = Kall + NG * KN * LD;
+  float* Pall = Vall + NG * KN * LD;
+  float* TBs = Pall + NG * WPG * 8 * LP;
+  float* CBs = TBs + BM * p.T;
+  float* QT = Vall;  // prologue only
+  float* QC = QT + BM * LD;
+
+  const int tid = threadIdx.x, lane = tid & 31, tx = lane & 15;
+  const int g = tid / GT, tg = tid % GT;
+  const int r0 = (tg >> 5) * 8 + (lane >> 4) * 4;  // first of this half-warp's four rows
+  float* Ks = Kall + g * KN * LD;
+  float* Vs = Vall + g * KN * LD;
+  float* Ps = Pall + (tid >> 5) * 8 * LP + (lane >> 4) * 4 * LP;
+
   const int qt = gridDim.x - 1 - blockIdx.x;  // heaviest (latest) query tiles first
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, hk = h / p.g;
-  const int m0 = qt * kBM;               // first row of the tile inside this call's q / o / lse
+  const int m0 = qt * BM;                // first row of the tile inside this call's q / o / lse
   const int N = p.N, T = p.T, C = p.C;
   const int Nq = p.q_tn * C;             // rows of this call (a query time range, or all of N)
   const int row0 = p.q_t0 * C;           // token index of row 0
   const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
   const Tin* k = (const Tin*)p.k + b * p.k_sb + hk * p.k_sh;
   const Tin* v = (const Tin*)p.v + b * p.v_sb + hk * p.v_sh;
-  const int valid = min(kBM, Nq - m0);
+  const int valid = min(BM, Nq - m0);
 
-  load_tile<Tin, D>(Qs, q, p.q_sn, m0, Nq, kBM, nullptr, 1.f);
-  if (tid < kBM) { ms[tid] = -INFINITY; ls[tid] = 0.f; }
-  __syncthreads();
-  rel_scores<Tin, D>(Qs, kBM, (const Tin*)p.vt + hk * D, (const Tin*)p.z + hk * D,
-                     (const Tin*)p.rt + (int64_t)hk * T * D, (const Tin*)p.rc + (int64_t)hk * C * D,
-                     T, C, p.c2, TBs, T, CBs, C, valid);
-  __syncthreads();
-  {  // Qs <- (q + u) * c2   (`attentions/attn.py:180-183`)
-    const Tin* u = (const Tin*)p.u + hk * D;
-    for (int idx = tid; idx < kBM * D; idx += kThreads) {
-      const int r = idx / D, d = idx % D;
-      Qs[r * LD + d] = (Qs[r * LD + d] + to_f32<Tin>(u[d])) * p.c2;
+  {  // rows with the three biases: QT, QC for the relative scores, Qs = (q + u) c2 (`attentions/attn.py:180-183`)
+    const Tin *u = (const Tin*)p.u + hk * D, *vt = (const Tin*)p.vt + hk * D, *z = (const Tin*)p.z + hk * D;
+    for (int idx = tid; idx < BM * D / 4; idx += CT) {
+      const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+      const float4 x = r < valid ? load4<Tin>(q + (int64_t)(m0 + r) * p.q_sn + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 bu = load4<Tin>(u + d), bt = load4<Tin>(vt + d), bz = load4<Tin>(z + d);
+      *reinterpret_cast<float4*>(Qs + r * LD + d) =
+          make_float4((x.x + bu.x) * p.c2, (x.y + bu.y) * p.c2, (x.z + bu.z) * p.c2, (x.w + bu.w) * p.c2);
+      *reinterpret_cast<float4*>(QT + r * LD + d) = make_float4(x.x + bt.x, x.y + bt.y, x.z + bt.z, x.w + bt.w);
+      *reinterpret_cast<float4*>(QC + r * LD + d) = make_float4(x.x + bz.x, x.y + bz.y, x.z + bz.z, x.w + bz.w);
     }
   }
-  int ti[2], ci[2];
+  __syncthreads();
+  rel_products<Tin, D, WPG, NG, KN>(p, hk, QT, QC, Ks, valid, TBs, T, 1, CBs, g, tg);
+
+  // time step, channel and relative scores of the four rows (rows past the end take the last one's)
+  int ti[4], ci[4];
+  const float *tb[4], *cb[4];  // tb[a][t_k], cb[a][-|c_i - c_k|]
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int i = row0 + min(m0 + 2 * ty + a, Nq - 1);  // token index in the whole sequence
+  for (int a = 0; a < 4; ++a) {
+    const int r = min(r0 + a, valid - 1), i = row0 + m0 + r;  // token index in the whole sequence
     ti[a] = i / C;
     ci[a] = i % C;
+    tb[a] = TBs + r * T + (T - 1 - ti[a]);
+    cb[a] = CBs + r * C + (C - 1);
   }
-  float oacc[2][DV];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int e = 0; e < DV; ++e) oacc[a][e] = 0.f;
-
-  const int t_last = (row0 + m0 + valid - 1) / C;
+  const int t_first = (row0 + m0) / C, t_last = (row0 + m0 + valid - 1) / C;
   const int hi = min(N, (t_last + 1) * C);  // causal bound (`attentions/attn.py:102-104,125-127`)
-  for (int n0 = 0; n0 < hi; n0 += kBN) {
-    __syncthreads();
-    load_tile<Tin, D>(Ks, k, p.k_sn, n0, N, kBN, nullptr, 1.f);
-    load_tile<Tin, D>(Vs, v, p.v_sn, n0, N, kBN, nullptr, 1.f);
-    __syncthreads();
-    float acc[2][4] = {};
-    tile_nt<D>(Qs, Ks, acc);
+  const int n_tiles = (hi + KN - 1) / KN;
+  // every pair of the tile outside the content window: its product with K is not needed
+  auto light = [&](int t) {
+    return p.window > 0 && t_last != T - 1 && t_first - (min(N, (t + 1) * KN) - 1) / C > p.window;
+  };
+  auto fetch_k = [&](int t) {
+    if (t < n_tiles && !light(t)) load_rows<Tin, D, KN, GT>(Ks, k, p.k_sn, t * KN, N, tg);
+    cp_async_commit();
+  };
+  fetch_k(g);  // (the relative scores' last use of the buffer ended with a group barrier)
+  __syncthreads();  // TBs / CBs are complete, QT / QC (the V buffers) are free
+
+  int tk[KJ], ck[KJ];  // time step and channel of this lane's keys, carried from tile to tile
+  const int step_t = NG * KN / C, step_c = NG * KN % C;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = tx + 16 * j, kk = n0 + col;
-      const int tk = kk / C, ck = kk % C;
+  for (int j = 0; j < KJ; ++j) {
+    const int kk = g * KN + tx + 16 * j;
+    tk[j] = kk / C;
+    ck[j] = kk % C;
+  }
+  float m[4], l[4], o[4][VW];
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int r = 2 * ty + a;
-        float s = -INFINITY;
-        if (kk < N && r < valid && tk <= ti[a]) {
-          s = in_window(ti[a], tk, T, p.window) ? acc[a][j] : 0.f;
-          s += TBs[r * T + (T - 1 - (ti[a] - tk))] + CBs[r * C + (C - 1 - abs(ci[a] - ck))];
+  for (int a = 0; a < 4; ++a) {
+    m[a] = -INFINITY;
+    l[a] = 0.f;
+#pragma unroll
+    for (int e = 0; e < VW; ++e) o[a][e] = 0.f;
+  }
+  for (int t = g; t < n_tiles; t += NG) {
+    const int n0 = t * KN;
+    cp_async_wait<0>();
+    group_sync<WPG>(g);  // K has arrived, every warp has left the previous tile's V
+    load_rows<Tin, D, KN, GT>(Vs, v, p.v_sn, n0, N, tg);
+    cp_async_commit();
+    float s[4][KJ];
+    if (light(t)) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) s[a][j] = 0.f;
+    } else {
+      product_nt<D, KJ>(Qs + r0 * LD, Ks, tx, s);
+    }
+    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        float x = -INFINITY;
+        if (tk[j] <= ti[a]) {  // (keys past the end lie past the last time step)
+          x = in_window(ti[a], tk[j], T, p.window) ? s[a][j] : 0.f;
+          x += tb[a][tk[j]] + cb[a][-abs(ci[a] - ck[j])];
         }
-        Ps[r * kPLd + col] = s;
+        s[a][j] = x;
+        mx[a] = fmaxf(mx[a], x);
       }
+      tk[j] += step_t;
+      ck[j] += step_c;
+      if (ck[j] >= C) { ck[j] -= C; ++tk[j]; }
     }
-    __syncthreads();
-    {  // online softmax, one warp per 4 rows (`attentions/attn.py:309-315`)
-      const int w = tid >> 5, lane = tid & 31;
+    // online softmax (`attentions/attn.py:309-315`); l stays a per-lane partial sum until the end
 #pragma unroll
-      for (int rr = 0; rr < 4; ++rr) {
-        const int r = 4 * w + rr;
-        const float s0 = Ps[r * kPLd + lane], s1 = Ps[r * kPLd + lane + 32];
-        float mx = fmaxf(s0, s1);
+    for (int a = 0; a < 4; ++a) {
+      const float m_new = fmaxf(m[a], half_warp_max(mx[a]));
+      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+      const float alpha = exp2f(m[a] - m_use);
+      m[a] = m_new;
+      float sum = 0.f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float m_old = ms[r];
-        const float m_new = fmaxf(m_old, mx);
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        const float alpha = exp2f(m_old - m_use);
-        const float p0 = exp2f(s0 - m_use), p1 = exp2f(s1 - m_use);
-        float sum = p0 + p1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        Ps[r * kPLd + lane] = p0;
-        Ps[r * kPLd + lane + 32] = p1;
-        if (lane == 0) {
-          ls[r] = ls[r] * alpha + sum;
-          ms[r] = m_new;
-          alphas[r] = alpha;
-        }
+      for (int j = 0; j < KJ; ++j) {
+        const float pr = exp2f(s[a][j] - m_use);
+        Ps[a * LP + tx + 16 * j] = pr;
+        sum += pr;
       }
-    }
-    __syncthreads();
+      l[a] = l[a] * alpha + sum;
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      const float al = alphas[2 * ty + a];
-#pragma unroll
-      for (int e = 0; e < DV; ++e) oacc[a][e] *= al;
+      for (int e = 0; e < VW; ++e) o[a][e] *= alpha;
     }
-    tile_nn<D>(Ps, Vs, oacc);
+    cp_async_wait<0>();
+    group_sync<WPG>(g);  // V has arrived, every warp has left K
+    fetch_k(t + NG);
+    product_nn<D, KN>(Ps, Vs, tx, o);
+    __syncwarp();
+  }
+  // merge the groups' partial results
+  __syncthreads();
+  float* Om = Kall;            // [NG][BM][LD]
+  float* ml = Pall;            // [NG][BM][2]
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    LaneCols<D>::store(Om + (g * BM + r0 + a) * LD, tx, o[a]);
+    const float ls = half_warp_sum(l[a]);
+    if (tx == 0) {
+      ml[(g * BM + r0 + a) * 2] = m[a];
+      ml[(g * BM + r0 + a) * 2 + 1] = ls;
+    }
   }
   __syncthreads();
-  Tin* o = (Tin*)p.o + b * p.o_sb + h * p.o_sh;
+  Tin* op = (Tin*)p.o + b * p.o_sb + h * p.o_sh;
+  for (int idx = tid; idx < BM * D / 4; idx += CT) {
+    const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+    if (r >= valid) continue;
+    float mm = -INFINITY, ll = 0.f;
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int r = 2 * ty + a, i = m0 + r;
-    if (r < valid) {
-      const float inv = 1.f / ls[r];
+    for (int gg = 0; gg < NG; ++gg) mm = fmaxf(mm, ml[(gg * BM + r) * 2]);
+    const float m_use = (mm == -INFINITY) ? 0.f : mm;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int e = 0; e < DV; ++e) o[(int64_t)i * p.o_sn + tx + 16 * e] = from_f32<Tin>(oacc[a][e] * inv);
-      if (tx == 0 && p.lse != nullptr) p.lse[(int64_t)bh * Nq + i] = ms[r] + log2f(ls[r]);
+    for (int gg = 0; gg < NG; ++gg) {
+      const float w = exp2f(ml[(gg * BM + r) * 2] - m_use);
+      const float4 y = *reinterpret_cast<const float4*>(Om + (gg * BM + r) * LD + d);
+      ll += ml[(gg * BM + r) * 2 + 1] * w;
+      x.x += y.x * w; x.y += y.y * w; x.z += y.z * w; x.w += y.w * w;
     }
+    const float inv = 1.f / ll;
+    store4<Tin>(op + (int64_t)(m0 + r) * p.o_sn + d, make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv));
+    if (d == 0 && p.lse != nullptr) p.lse[(int64_t)bh * Nq + m0 + r] = mm + log2f(ll);
   }
 }
 
 // ------------------------------- backward ------------------------------------
-
-// Relative scores of every query row to the workspace (the SIMT backward gathers from them).
-template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_rel_kernel(BwdArgs bw) {
-  constexpr int LD = D + 4;
-  const Args& p = bw.a;
-  extern __shared__ float smem[];
-  float* Qs = smem;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, hk = h / p.g;
-  const int m0 = blockIdx.x * kBM, valid = min(kBM, p.N - m0);
-  const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
-  load_tile<Tin, D>(Qs, q, p.q_sn, m0, p.N, kBM, nullptr, 1.f);
-  __syncthreads();
-  rel_scores<Tin, D>(Qs, kBM, (const Tin*)p.vt + hk * D, (const Tin*)p.z + hk * D,
-                     (const Tin*)p.rt + (int64_t)hk * p.T * D, (const Tin*)p.rc + (int64_t)hk * p.C * D,
-                     p.T, p.C, p.c2, bw.tbg + ((int64_t)bh * p.N + m0) * p.T, p.T,
-                     bw.cbg + ((int64_t)bh * p.N + m0) * p.C, p.C, valid);
-}
 
 // delta[bh][i] = sum_d dO[i][d] * O[i][d]   (`attentions/attn.py:1213`).  HBM-bound: a thread reads 16
 // bytes of each tensor at a time, D / VEC threads share a row (VEC = elements per 16 bytes) and
@@ -293,364 +451,574 @@ __global__ void __launch_bounds__(kThreads) simt_delta_kernel(BwdArgs bw) {
   if (part == 0 && rowi < p.N) bw.delta[(int64_t)bh * p.N + rowi] = acc;
 }
 
-// dQ side: one CTA per (32 query rows, b, h).  Walks the causal key tiles, recomputes
-// P = exp2(S2 - L), forms dS, accumulates the content part of dQ and the per-row sums of dS by
-// time slot / channel slot, then finishes dq = dS_w K + dTB r_time + dCB r_chan.
-template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_dq_kernel(BwdArgs bw) {
-  constexpr int LD = D + 4;
-  constexpr int DV = D / 16;
-  const Args& p = bw.a;
-  extern __shared__ float smem[];
-  float* Qs = smem;                 // (q+u)*c2
-  float* Gs = Qs + kBM * LD;        // dO rows
-  float* Ks = Gs + kBM * LD;
-  float* Vs = Ks + kBN * LD;
-  float* Ds = Vs + kBN * LD;        // dS
-  float* Dw = Ds + kBM * kPLd;      // dS * win
-  float* dTBs = Dw + kBM * kPLd;    // 32 x T
-  float* dCBs = dTBs + kBM * p.T;   // 32 x C
-  float* lse_s = dCBs + kBM * p.C;
-  float* dl_s = lse_s + kBM;
-  float* red = dl_s + kBM;          // 16 x D column-sum scratch
 
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+// Query side: one CTA per (BM query rows, b, h); the groups share the causal key tiles.  Recomputes
+// P = exp2(S2 - L), forms dS, accumulates the content part of dQ and the per-row sums of dS by time slot and
+// by key channel, then finishes dq = dS_w K + dTB r_time + dCB r_chan.  On the way it leaves behind what the
+// other kernels need: the relative scores and delta (key side), the gradients of the relative scores
+// (dr_time / dr_chan) and the column sums of the three parts of dq (du / dvt / dz).
+template <int D, int WPG, int NG, int KN>
+constexpr size_t dq_fixed_floats() {
+  return (size_t)2 * 8 * WPG * (D + 4) + (size_t)NG * 2 * KN * (D + 4) + (size_t)NG * WPG * 8 * (KN + 4) + 16 * WPG;
+}
+
+// INS: the relative scores also sit in shared memory; otherwise they are read back from the workspace (long
+// time or channel axes, where the two groups' slot sums fill the shared memory).
+template <typename Tin, int D, int WPG, int NG, int KN, bool INS>
+__global__ void __launch_bounds__(32 * WPG * NG) simt_dq_kernel(BwdArgs bw) {
+  constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
+  constexpr int GT = 32 * WPG, CT = GT * NG;
+  static_assert(NG * KN >= 2 * BM && KN >= BM, "aliased areas");
+  const Args& p = bw.a;
+  extern __shared__ __align__(16) float smem[];
+  float* Qs = smem;                    // (q + u) c2
+  float* Gs = Qs + BM * LD;            // dO rows
+  float* Kall = Gs + BM * LD;
+  float* Vall = Kall + NG * KN * LD;
+  float* Pall = Vall + NG * KN * LD;   // dS, per warp
+  float* lse_s = Pall + NG * WPG * 8 * LP;
+  float* dl_s = lse_s + BM;
+  const int N = p.N, T = p.T, C = p.C, TC = T + C;
+  float* dTall = dl_s + BM;            // [NG][BM][T], by slot
+  float* dCall = dTall + NG * BM * T;  // [NG][BM][C], by key channel
+  float* TBs = dCall + NG * BM * C;    // [BM][T]   (INS)
+  float* CBs = TBs + BM * T;           // [BM][C]   (INS)
+  float* QT = Vall;                    // prologue only
+  float* QC = QT + BM * LD;
+
+  const int tid = threadIdx.x, lane = tid & 31, tx = lane & 15;
+  const int g = tid / GT, tg = tid % GT;
+  const int r0 = (tg >> 5) * 8 + (lane >> 4) * 4;
+  float* Ks = Kall + g * KN * LD;
+  float* Vs = Vall + g * KN * LD;
+  float* Ds = Pall + (tid >> 5) * 8 * LP + (lane >> 4) * 4 * LP;
+  float* dT = dTall + g * BM * T;
+  float* dC = dCall + g * BM * C;
+
   const int qt = gridDim.x - 1 - blockIdx.x;
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, hk = h / p.g;
-  const int m0 = qt * kBM;
-  const int N = p.N, T = p.T, C = p.C;
-  const int valid = min(kBM, N - m0);
+  const int m0 = qt * BM, valid = min(BM, N - m0);
   const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
   const Tin* k = (const Tin*)p.k + b * p.k_sb + hk * p.k_sh;
   const Tin* v = (const Tin*)p.v + b * p.v_sb + hk * p.v_sh;
-  const Tin* g = (const Tin*)bw.d_o + b * bw.do_sb + h * bw.do_sh;
-  const float* tbg = bw.tbg + (int64_t)bh * N * T;
-  const float* cbg = bw.cbg + (int64_t)bh * N * C;
+  const Tin* gp = (const Tin*)bw.d_o + b * bw.do_sb + h * bw.do_sh;
+  const Tin* op = (const Tin*)p.o + b * p.o_sb + h * p.o_sh;
 
-  load_tile<Tin, D>(Qs, q, p.q_sn, m0, N, kBM, (const Tin*)p.u + hk * D, p.c2);
-  load_tile<Tin, D>(Gs, g, bw.do_sn, m0, N, kBM, nullptr, 1.f);
-  for (int idx = tid; idx < kBM * (T + C); idx += kThreads) dTBs[idx] = 0.f;  // dTBs,dCBs adjacent
-  if (tid < kBM) {
-    const int i = min(m0 + tid, N - 1);
-    lse_s[tid] = p.lse[(int64_t)bh * N + i];
-    dl_s[tid] = bw.delta[(int64_t)bh * N + i];
-  }
-  int ti[2], ci[2];
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int i = min(m0 + 2 * ty + a, N - 1);
-    ti[a] = i / C;
-    ci[a] = i % C;
-  }
-  float qacc[2][DV];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int e = 0; e < DV; ++e) qacc[a][e] = 0.f;
-
-  const int t_last = (m0 + valid - 1) / C;
-  const int hi = min(N, (t_last + 1) * C);
-  for (int n0 = 0; n0 < hi; n0 += kBN) {
-    __syncthreads();
-    load_tile<Tin, D>(Ks, k, p.k_sn, n0, N, kBN, nullptr, 1.f);
-    load_tile<Tin, D>(Vs, v, p.v_sn, n0, N, kBN, nullptr, 1.f);
-    __syncthreads();
-    float sacc[2][4] = {}, pacc[2][4] = {};
-    tile_nt<D>(Qs, Ks, sacc);
-    tile_nt<D>(Gs, Vs, pacc);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = tx + 16 * j, kk = n0 + col;
-      const int tk = kk / C, ck = kk % C;
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int r = 2 * ty + a;
-        float ds = 0.f, dsw = 0.f;
-        if (kk < N && r < valid && tk <= ti[a]) {
-          const bool w = in_window(ti[a], tk, T, p.window);
-          const int64_t i = m0 + r;
-          const float s2 = (w ? sacc[a][j] : 0.f) + tbg[i * T + (T - 1 - (ti[a] - tk))] +
-                           cbg[i * C + (C - 1 - abs(ci[a] - ck))];
-          const float pr = exp2f(s2 - lse_s[r]);
-          ds = pr * (pacc[a][j] - dl_s[r]) * p.sm_scale;  // `attentions/attn.py:680`
-          dsw = w ? ds : 0.f;                             // `attentions/attn.py:708-717`
+  {
+    const Tin *u = (const Tin*)p.u + hk * D, *vt = (const Tin*)p.vt + hk * D, *z = (const Tin*)p.z + hk * D;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int idx = tid; idx < BM * D / 4; idx += CT) {
+      const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+      const float4 x = r < valid ? load4<Tin>(q + (int64_t)(m0 + r) * p.q_sn + d) : zero;
+      const float4 bu = load4<Tin>(u + d), bt = load4<Tin>(vt + d), bz = load4<Tin>(z + d);
+      *reinterpret_cast<float4*>(Qs + r * LD + d) =
+          make_float4((x.x + bu.x) * p.c2, (x.y + bu.y) * p.c2, (x.z + bu.z) * p.c2, (x.w + bu.w) * p.c2);
+      *reinterpret_cast<float4*>(QT + r * LD + d) = make_float4(x.x + bt.x, x.y + bt.y, x.z + bt.z, x.w + bt.w);
+      *reinterpret_cast<float4*>(QC + r * LD + d) = make_float4(x.x + bz.x, x.y + bz.y, x.z + bz.z, x.w + bz.w);
+      *reinterpret_cast<float4*>(Gs + r * LD + d) = r < valid ? load4<Tin>(gp + (int64_t)(m0 + r) * bw.do_sn + d) : zero;
+    }
+    // delta = sum_d dO O  (`attentions/attn.py:1213`): one warp per row
+    for (int r = tid >> 5; r < BM; r += CT / 32) {
+      float acc = 0.f;
+      if (r < valid) {
+        for (int d = lane * 4; d < D; d += 128) {
+          const float4 x = load4<Tin>(gp + (int64_t)(m0 + r) * bw.do_sn + d), y = load4<Tin>(op + (int64_t)(m0 + r) * p.o_sn + d);
+          acc += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
         }
-        Ds[r * kPLd + col] = ds;
-        Dw[r * kPLd + col] = dsw;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) {
+        dl_s[r] = acc;
+        lse_s[r] = r < valid ? p.lse[(int64_t)bh * N + m0 + r] : INFINITY;  // P = 0 on rows that do not exist
+        if (r < valid) bw.delta[(int64_t)bh * N + m0 + r] = acc;
       }
     }
-    __syncthreads();
-    {  // row sums of dS per key time step (the reference's dS x csm_time product, `:681-694`)
-      const int tk0 = n0 / C, tk1 = (min(n0 + kBN, N) - 1) / C, nT = tk1 - tk0 + 1;
-      for (int idx = tid; idx < kBM * nT; idx += kThreads) {
-        const int r = idx / nT, tk = tk0 + idx % nT;
-        const int t_i = min(m0 + r, N - 1) / C;
-        if (r >= valid || tk > t_i) continue;
-        const int c_lo = max(n0, tk * C) - n0, c_hi = min(min(n0 + kBN, N), (tk + 1) * C) - n0;
-        float s = 0.f;
-        for (int c = c_lo; c < c_hi; ++c) s += Ds[r * kPLd + c];
-        dTBs[r * T + (T - 1 - (t_i - tk))] += s;
-      }
-      // ... and per channel distance (`:695-707`): slot e collects c_k = c_i - e and c_i + e
-      for (int idx = tid; idx < kBM * C; idx += kThreads) {
-        const int r = idx / C, e = idx % C;
-        if (r >= valid) continue;
-        const int c_i = (m0 + r) % C;
-        float s = 0.f;
-        for (int tk = tk0; tk <= tk1; ++tk) {
-          const int base = tk * C - n0;
-          const int ca = base + c_i - e, cb = base + c_i + e;
-          if (c_i - e >= 0 && ca >= 0 && ca < kBN) s += Ds[r * kPLd + ca];
-          if (e > 0 && c_i + e < C && cb >= 0 && cb < kBN) s += Ds[r * kPLd + cb];
-        }
-        dCBs[r * C + (C - 1 - e)] += s;
-      }
-    }
-    tile_nn<D>(Dw, Ks, qacc);  // dQ += dS_w K   (`attentions/attn.py:719-730`)
+    for (int idx = tid; idx < NG * BM * TC; idx += CT) dTall[idx] = 0.f;  // dTall and dCall are adjacent
   }
   __syncthreads();
-  // Finish dq and the three bias partials (autograd through `_rel_bias`).
+  // the relative scores, time slots row-innermost and channel slots as they are: the key side reads them too
+  float* tbg = bw.tbg + (int64_t)bh * N * T + m0;
+  float* cbg = bw.cbg + ((int64_t)bh * N + m0) * C;
+  if constexpr (INS) rel_products<Tin, D, WPG, NG, KN>(p, hk, QT, QC, Ks, valid, TBs, T, 1, CBs, g, tg);
+  else rel_products<Tin, D, WPG, NG, KN>(p, hk, QT, QC, Ks, valid, tbg, 1, N, cbg, g, tg);
+
+  int ti[4], ci[4];
+  const float *tb[4], *cb[4];  // the scores of the four rows (rows past the end take the last one's)
+  const int64_t tb_s = INS ? 1 : N;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int r = min(r0 + a, valid - 1), i = m0 + r;
+    ti[a] = i / C;
+    ci[a] = i % C;
+    tb[a] = (INS ? TBs + r * T : tbg + r) + (T - 1 - ti[a]) * tb_s;
+    cb[a] = (INS ? CBs : cbg) + (int64_t)r * C + (C - 1);
+  }
+  const int t_first = m0 / C, t_last = (m0 + valid - 1) / C;
+  const int hi = min(N, (t_last + 1) * C);
+  const int n_tiles = (hi + KN - 1) / KN;
+  auto light = [&](int t) {
+    return p.window > 0 && t_last != T - 1 && t_first - (min(N, (t + 1) * KN) - 1) / C > p.window;
+  };
+  auto fetch_k = [&](int t) {
+    if (t < n_tiles && !light(t)) load_rows<Tin, D, KN, GT>(Ks, k, p.k_sn, t * KN, N, tg);
+    cp_async_commit();
+  };
+  auto fetch_v = [&](int t) {
+    if (t < n_tiles) load_rows<Tin, D, KN, GT>(Vs, v, p.v_sn, t * KN, N, tg);
+    cp_async_commit();
+  };
+  __syncthreads();  // TBs / CBs are complete, QT / QC (the V buffers) are free
+  fetch_v(g);
+  fetch_k(g);
+  if constexpr (INS) {
+    for (int idx = tid; idx < BM * T; idx += CT) {
+      const int r = idx % BM, s = idx / BM;
+      if (r < valid) tbg[(int64_t)s * N + r] = TBs[r * T + s];
+    }
+    for (int idx = tid; idx < valid * C; idx += CT) cbg[idx] = CBs[idx];
+  }
+
+  int tk[KJ], ck[KJ];  // time step and channel of this lane's keys, carried from tile to tile
+  const int step_t = NG * KN / C, step_c = NG * KN % C;
+#pragma unroll
+  for (int j = 0; j < KJ; ++j) {
+    const int kk = g * KN + tx + 16 * j;
+    tk[j] = kk / C;
+    ck[j] = kk % C;
+  }
+  float acc[4][VW], lse[4], dl[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    lse[a] = lse_s[r0 + a];
+    dl[a] = dl_s[r0 + a];
+#pragma unroll
+    for (int e = 0; e < VW; ++e) acc[a][e] = 0.f;
+  }
+  for (int t = g; t < n_tiles; t += NG) {
+    const int n0 = t * KN;
+    const bool lt = light(t);
+    cp_async_wait<1>();
+    group_sync<WPG>(g);  // V has arrived
+    float s[4][KJ], dp[4][KJ];
+    product_nt<D, KJ>(Gs + r0 * LD, Vs, tx, dp);
+    cp_async_wait<0>();
+    group_sync<WPG>(g);  // K has arrived, every warp has left V
+    fetch_v(t + NG);
+    if (lt) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) s[a][j] = 0.f;
+    } else {
+      product_nt<D, KJ>(Qs + r0 * LD, Ks, tx, s);
+    }
+    bool w[4][KJ];
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        float ds = 0.f;
+        w[a][j] = in_window(ti[a], tk[j], T, p.window);
+        if (tk[j] <= ti[a]) {  // (keys past the end lie past the last time step)
+          const float s2 = (w[a][j] ? s[a][j] : 0.f) + tb[a][tk[j] * tb_s] + cb[a][-abs(ci[a] - ck[j])];
+          ds = exp2f(s2 - lse[a]) * (dp[a][j] - dl[a]) * p.sm_scale;  // `attentions/attn.py:680`
+        }
+        s[a][j] = ds;
+        Ds[a * LP + tx + 16 * j] = ds;
+      }
+      tk[j] += step_t;
+      ck[j] += step_c;
+      if (ck[j] >= C) { ck[j] -= C; ++tk[j]; }
+    }
+    __syncwarp();
+    {  // sums of dS over the tile, by key time step (the reference's dS x csm_time product, `:681-694`) and by
+       // key channel; this half-warp's lanes take the (row, time step) and (row, channel) pairs of its rows
+      const int last = min(n0 + KN, N) - 1, tk0 = n0 / C, tk1 = last / C, nT = tk1 - tk0 + 1;
+      for (int idx = tx; idx < 4 * nT; idx += 16) {
+        const int a = idx & 3, tk = tk0 + (idx >> 2);
+        const int t_i = min(m0 + r0 + a, N - 1) / C;
+        if (tk <= t_i) {
+          const int lo = max(n0, tk * C) - n0, up = min(last, tk * C + C - 1) - n0;
+          float sum = 0.f;
+          for (int c = lo; c <= up; ++c) sum += Ds[a * LP + c];
+          dT[(r0 + a) * T + (T - 1 - (t_i - tk))] += sum;
+        }
+      }
+      const int c_n = min(C, last - n0 + 1), c_b = n0 - tk0 * C;  // distinct channels of the tile, the first one
+      for (int idx = tx; idx < 4 * c_n; idx += 16) {
+        const int a = idx & 3, off = idx >> 2;
+        float sum = 0.f;
+        for (int c = off; c <= last - n0; c += C) sum += Ds[a * LP + c];
+        int ch = c_b + off;
+        if (ch >= C) ch -= C;
+        dC[(r0 + a) * C + ch] += sum;
+      }
+    }
+    __syncwarp();
+    if (!lt) {  // dQ += dS_w K   (`attentions/attn.py:708-730`)
+#pragma unroll
+      for (int j = 0; j < KJ; ++j)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          if (!w[a][j]) Ds[a * LP + tx + 16 * j] = 0.f;
+      __syncwarp();
+      product_nn<D, KN>(Ds, Ks, tx, acc);
+    }
+    group_sync<WPG>(g);  // every warp has left K
+    fetch_k(t + NG);
+  }
+  __syncthreads();
+  // merge: dq's content part of every group, the slot sums, channel sums folded by |c_i - c_k| (`:695-707`)
+  float* Am = Kall;  // [NG][BM][LD]
+#pragma unroll
+  for (int a = 0; a < 4; ++a) LaneCols<D>::store(Am + (g * BM + r0 + a) * LD, tx, acc[a]);
+  float* dtbg = bw.dtbg + ((int64_t)bh * N + m0) * T;
+  for (int idx = tid; idx < BM * T; idx += CT) {
+    float s = 0.f;
+#pragma unroll
+    for (int gg = 0; gg < NG; ++gg) s += dTall[gg * BM * T + idx];
+    dTall[idx] = s;
+    if (idx < valid * T) dtbg[idx] = s;
+  }
+  float* dcbg = bw.dcbg + ((int64_t)bh * N + m0) * C;
+  for (int idx = tid; idx < BM * C; idx += CT) {
+    const int r = idx / C, e = C - 1 - (idx - r * C), c_i = min(m0 + r, N - 1) % C;
+    float s = 0.f;
+#pragma unroll
+    for (int gg = 0; gg < NG; ++gg) {
+      const float* row = dCall + (gg * BM + r) * C;
+      if (c_i - e >= 0) s += row[c_i - e];
+      if (e > 0 && c_i + e < C) s += row[c_i + e];
+    }
+    if constexpr (INS) CBs[idx] = s;  // (the scores have been used)
+    if (r < valid) dcbg[idx] = s;
+  }
+  __syncthreads();
+  // dq = content + dTB r_time + dCB r_chan (autograd through `_rel_bias`); a thread holds four columns of a row
+  float* parts = Vall;  // [2][BM][LD]: the temporal and the channel part; the content part replaces Am's first copy
   const Tin* rt = (const Tin*)p.rt + (int64_t)hk * T * D;
   const Tin* rc = (const Tin*)p.rc + (int64_t)hk * C * D;
-  float tacc[2][DV] = {}, cacc[2][DV] = {};
-  for (int s = 0; s < T; ++s) {
-    const float x0 = dTBs[(2 * ty) * T + s], x1 = dTBs[(2 * ty + 1) * T + s];
-#pragma unroll
-    for (int e = 0; e < DV; ++e) {
-      const float y = to_f32<Tin>(rt[(int64_t)s * D + tx + 16 * e]);
-      tacc[0][e] += x0 * y;
-      tacc[1][e] += x1 * y;
-    }
-  }
-  for (int s = 0; s < C; ++s) {
-    const float x0 = dCBs[(2 * ty) * C + s], x1 = dCBs[(2 * ty + 1) * C + s];
-#pragma unroll
-    for (int e = 0; e < DV; ++e) {
-      const float y = to_f32<Tin>(rc[(int64_t)s * D + tx + 16 * e]);
-      cacc[0][e] += x0 * y;
-      cacc[1][e] += x1 * y;
-    }
-  }
   Tin* dq = (Tin*)bw.dq + b * bw.dq_sb + h * bw.dq_sh;
+  for (int idx = tid; idx < BM * D / 4; idx += CT) {
+    const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+    float4 x = *reinterpret_cast<const float4*>(Am + r * LD + d);
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int r = 2 * ty + a;
-    if (r < valid) {
-#pragma unroll
-      for (int e = 0; e < DV; ++e)
-        dq[(int64_t)(m0 + r) * bw.dq_sn + tx + 16 * e] = from_f32<Tin>(qacc[a][e] + tacc[a][e] + cacc[a][e]);
+    for (int gg = 1; gg < NG; ++gg) {
+      const float4 y = *reinterpret_cast<const float4*>(Am + (gg * BM + r) * LD + d);
+      x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
     }
+    float4 part[2];
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      const int n = which == 0 ? T : C;
+      const float* f = (which == 0 ? dTall : INS ? CBs : dcbg) + (int64_t)(which == 0 || INS ? r : min(r, valid - 1)) * n;
+      const Tin* key = (which == 0 ? rt : rc) + d;
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (int s = 0; s < (r < valid ? n : 0); ++s) {  // (rows past the end: zero)
+        const float4 kv = load4<Tin>(key + (int64_t)s * D);
+        const float fv = f[s];
+        y.x = fmaf(fv, kv.x, y.x); y.y = fmaf(fv, kv.y, y.y); y.z = fmaf(fv, kv.z, y.z); y.w = fmaf(fv, kv.w, y.w);
+      }
+      part[which] = y;
+      *reinterpret_cast<float4*>(parts + (which * BM + r) * LD + d) = y;
+    }
+    *reinterpret_cast<float4*>(Am + r * LD + d) = x;
+    if (r < valid)
+      store4<Tin>(dq + (int64_t)(m0 + r) * bw.dq_sn + d,
+                  make_float4(x.x + part[0].x + part[1].x, x.y + part[0].y + part[1].y, x.z + part[0].z + part[1].z,
+                              x.w + part[0].w + part[1].w));
   }
-  // rows >= valid contributed zeros everywhere, so plain column sums are exact.
-  float* part = bw.partial + ((int64_t)bh * gridDim.x + qt) * 3 * D;
-  for (int which = 0; which < 3; ++which) {
-    __syncthreads();
+  __syncthreads();
+  // column sums; rows past the end contributed zeros everywhere
+  float* out = bw.partial + ((int64_t)bh * gridDim.x + qt) * 3 * D;
+  for (int idx = tid; idx < 3 * D; idx += CT) {
+    const int which = idx / D, d = idx % D;
+    const float* src = (which == 0 ? Am : parts + (which - 1) * BM * LD) + d;
+    float s = 0.f;
 #pragma unroll
-    for (int e = 0; e < DV; ++e) {
-      const float x = which == 0 ? qacc[0][e] + qacc[1][e]
-                      : which == 1 ? tacc[0][e] + tacc[1][e] : cacc[0][e] + cacc[1][e];
-      red[ty * D + tx + 16 * e] = x;
-    }
-    __syncthreads();
-    for (int d = tid; d < D; d += kThreads) {
-      float s = 0.f;
-      for (int y = 0; y < 16; ++y) s += red[y * D + d];
-      part[which * D + d] = s;
-    }
+    for (int r = 0; r < BM; ++r) s += src[r * LD];
+    out[idx] = s;
   }
-  // gradients of the relative scores, kept for dr_time / dr_chan
-  float* dtbg = bw.dtbg + ((int64_t)bh * N + m0) * T;
-  float* dcbg = bw.dcbg + ((int64_t)bh * N + m0) * C;
-  for (int idx = tid; idx < valid * T; idx += kThreads) dtbg[idx] = dTBs[idx];
-  for (int idx = tid; idx < valid * C; idx += kThreads) dcbg[idx] = dCBs[idx];
 }
 
-// dK / dV side: one CTA per (32 keys, b, kv head); loops over the g query heads of the group and
-// the causal query tiles (64 rows each).  Products are formed transposed (key rows x query cols).
-template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_dkv_kernel(BwdArgs bw) {
-  constexpr int LD = D + 4;
-  constexpr int DV = D / 16;
-  const Args& p = bw.a;
-  extern __shared__ float smem[];
-  float* Ks = smem;               // 32 keys (raw)
-  float* Vs = Ks + kBM * LD;
-  float* Qs = Vs + kBM * LD;      // 64 queries, (q+u)*c2
-  float* Gs = Qs + kBN * LD;      // 64 dO rows
-  float* Ps = Gs + kBN * LD;      // P^T   (32 x 64)
-  float* Dw = Ps + kBM * kPLd;    // dS_w^T
-  float* lse_s = Dw + kBM * kPLd;
-  float* dl_s = lse_s + kBN;
+// Key side: one CTA per (BM keys, b, kv head); the groups share the (query head of the group, causal query
+// tile) items.  Products are formed transposed (key rows x query columns).
+template <int D, int WPG, int NG, int KN>
+constexpr size_t dkv_fixed_floats() {
+  return (size_t)2 * 8 * WPG * (D + 4) + (size_t)NG * 2 * KN * (D + 4) + (size_t)NG * WPG * 16 * (KN + 4) + 2 * NG * KN;
+}
 
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+template <typename Tin, int D, int WPG, int NG, int KN>
+__global__ void __launch_bounds__(32 * WPG * NG) simt_dkv_kernel(BwdArgs bw) {
+  constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
+  constexpr int GT = 32 * WPG, CT = GT * NG;
+  static_assert(KN >= BM, "aliased areas");
+  const Args& p = bw.a;
+  extern __shared__ __align__(16) float smem[];
+  float* Ks = smem;
+  float* Vs = Ks + BM * LD;
+  float* Qall = Vs + BM * LD;
+  float* Gall = Qall + NG * KN * LD;
+  float* Pall = Gall + NG * KN * LD;      // P^T and dS_w^T of each warp's eight key rows
+  float* Lall = Pall + NG * WPG * 16 * LP;  // log-sum-exp and delta of each group's query tile
+
+  const int tid = threadIdx.x, lane = tid & 31, tx = lane & 15;
+  const int g = tid / GT, tg = tid % GT;
+  const int r0 = (tg >> 5) * 8 + (lane >> 4) * 4;
+  float* Qs = Qall + g * KN * LD;
+  float* Gs = Gall + g * KN * LD;
+  float* Ps = Pall + (tid >> 5) * 16 * LP + (lane >> 4) * 4 * LP;
+  float* Dw = Ps + 8 * LP;
+  float* lse_s = Lall + g * 2 * KN;
+  float* dl_s = lse_s + KN;
+
   const int bk = blockIdx.y, b = bk / p.Hkv, hk = bk % p.Hkv;
-  const int n0 = blockIdx.x * kBM;
+  const int n0 = blockIdx.x * BM;  // earliest keys (seen by the most queries) first
   const int N = p.N, T = p.T, C = p.C;
-  const int valid = min(kBM, N - n0);
-  const Tin* k = (const Tin*)p.k + b * p.k_sb + hk * p.k_sh;
-  const Tin* v = (const Tin*)p.v + b * p.v_sb + hk * p.v_sh;
-  load_tile<Tin, D>(Ks, k, p.k_sn, n0, N, kBM, nullptr, 1.f);
-  load_tile<Tin, D>(Vs, v, p.v_sn, n0, N, kBM, nullptr, 1.f);
-  int tk[2], ck[2];
+  const int valid = min(BM, N - n0);
+  load_rows<Tin, D, BM, CT>(Ks, (const Tin*)p.k + b * p.k_sb + hk * p.k_sh, p.k_sn, n0, N, tid);
+  load_rows<Tin, D, BM, CT>(Vs, (const Tin*)p.v + b * p.v_sb + hk * p.v_sh, p.v_sn, n0, N, tid);
+  cp_async_commit();
+  int tk[4], ck[4];
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int kk = min(n0 + 2 * ty + a, N - 1);
+  for (int a = 0; a < 4; ++a) {
+    const int kk = min(n0 + r0 + a, N - 1);
     tk[a] = kk / C;
     ck[a] = kk % C;
   }
-  float kacc[2][DV], vacc[2][DV];
+  const int tk_last = (n0 + valid - 1) / C;
+  const int tile0 = ((n0 / C) * C) / KN, per_head = (N + KN - 1) / KN - tile0;  // first query tile that sees these keys
+  const int items = p.g * per_head;
+  // every pair outside the content window: neither S nor dS_w is needed, only P
+  auto light = [&](int m0) {
+    const int t_hi = (min(N, m0 + KN) - 1) / C;
+    return p.window > 0 && t_hi != T - 1 && m0 / C - tk_last > p.window;
+  };
+  const float4 u4 = load4<Tin>((const Tin*)p.u + hk * D + (tg % (D / 4)) * 4);  // bias of the columns this thread loads
+  static_assert(GT % (D / 4) == 0, "a thread loads the same columns of every row");
+  auto fetch_q = [&](int item) {
+    if (item < items) {
+      const int h = hk * p.g + item / per_head, m0 = (tile0 + item % per_head) * KN;
+      if (!light(m0)) load_rows<Tin, D, KN, GT>(Qs, (const Tin*)p.q + b * p.q_sb + h * p.q_sh, p.q_sn, m0, N, tg);
+    }
+    cp_async_commit();
+  };
+  auto fetch_g = [&](int item) {
+    if (item < items) {
+      const int h = hk * p.g + item / per_head, m0 = (tile0 + item % per_head) * KN;
+      load_rows<Tin, D, KN, GT>(Gs, (const Tin*)bw.d_o + b * bw.do_sb + h * bw.do_sh, bw.do_sn, m0, N, tg);
+    }
+    cp_async_commit();
+  };
+  float kacc[4][VW], vacc[4][VW];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int e = 0; e < DV; ++e) kacc[a][e] = vacc[a][e] = 0.f;
-
-  const int m_first = ((n0 / C) * C) / kBN * kBN;  // first query tile that can see these keys
-  for (int hh = 0; hh < p.g; ++hh) {
-    const int h = hk * p.g + hh, bh = b * p.H + h;
-    const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
-    const Tin* g = (const Tin*)bw.d_o + b * bw.do_sb + h * bw.do_sh;
+    for (int e = 0; e < VW; ++e) kacc[a][e] = vacc[a][e] = 0.f;
+  fetch_q(g);
+  fetch_g(g);
+  cp_async_wait<2>();
+  __syncthreads();  // K and V are in place
+  for (int item = g; item < items; item += NG) {
+    const int h = hk * p.g + item / per_head, bh = b * p.H + h, m0 = (tile0 + item % per_head) * KN;
+    const bool lt = light(m0);
     const float* tbg = bw.tbg + (int64_t)bh * N * T;
     const float* cbg = bw.cbg + (int64_t)bh * N * C;
-    for (int m0 = m_first; m0 < N; m0 += kBN) {
-      __syncthreads();
-      load_tile<Tin, D>(Qs, q, p.q_sn, m0, N, kBN, (const Tin*)p.u + hk * D, p.c2);
-      load_tile<Tin, D>(Gs, g, bw.do_sn, m0, N, kBN, nullptr, 1.f);
-      if (tid < kBN) {
-        const int i = min(m0 + tid, N - 1);
-        lse_s[tid] = p.lse[(int64_t)bh * N + i];
-        dl_s[tid] = bw.delta[(int64_t)bh * N + i];
-      }
-      __syncthreads();
-      float sacc[2][4] = {}, pacc[2][4] = {};
-      tile_nt<D>(Ks, Qs, sacc);  // S^T in base 2 (Qs carries c2)
-      tile_nt<D>(Vs, Gs, pacc);  // dP^T
+    // this tile's relative scores, requested before the products that hide their latency
+    float rel[4][KJ];
+    int ti[KJ];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = tx + 16 * j, i = m0 + col;
-        const int t_i = i / C, c_i = i % C;
+    for (int j = 0; j < KJ; ++j) {
+      const int i = min(m0 + tx + 16 * j, N - 1), t_i = i / C, c_i = i % C;
+      ti[j] = t_i;
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          const int r = 2 * ty + a;
-          float pr = 0.f, dsw = 0.f;
-          if (i < N && r < valid && tk[a] <= t_i) {
-            const bool w = in_window(t_i, tk[a], T, p.window);
-            const float s2 = (w ? sacc[a][j] : 0.f) + tbg[(int64_t)i * T + (T - 1 - (t_i - tk[a]))] +
-                             cbg[(int64_t)i * C + (C - 1 - abs(c_i - ck[a]))];
-            pr = exp2f(s2 - lse_s[col]);
-            const float ds = pr * (pacc[a][j] - dl_s[col]) * p.sm_scale;
-            dsw = w ? ds : 0.f;
-          }
-          Ps[r * kPLd + col] = pr;
-          Dw[r * kPLd + col] = dsw;
-        }
+      for (int a = 0; a < 4; ++a) {
+        const int dt = max(t_i - tk[a], 0);
+        rel[a][j] = tbg[(int64_t)(T - 1 - dt) * N + i] + cbg[(int64_t)i * C + (C - 1 - abs(c_i - ck[a]))];
       }
-      __syncthreads();
-      tile_nn<D>(Ps, Gs, vacc);  // dV += P^T dO        (`attentions/attn.py:671-675`)
-      tile_nn<D>(Dw, Qs, kacc);  // dK += dS_w^T (q+u)  (`attentions/attn.py:718`), times c2
     }
+    for (int c = tg; c < KN; c += GT) {
+      const int i = min(m0 + c, N - 1);
+      lse_s[c] = p.lse[(int64_t)bh * N + i];
+      dl_s[c] = bw.delta[(int64_t)bh * N + i];
+    }
+    cp_async_wait<1>();  // Q: this thread's own pieces
+    if (!lt) {           // Q <- (q + u) c2, rows past the end included (their P is 0)
+#pragma unroll
+      for (int i = 0; i < KN * D / 4 / GT; ++i) {
+        const int idx = i * GT + tg;
+        float4* x = reinterpret_cast<float4*>(Qs + (idx / (D / 4)) * LD + (idx % (D / 4)) * 4);
+        const float4 y = *x;
+        *x = make_float4((y.x + u4.x) * p.c2, (y.y + u4.y) * p.c2, (y.z + u4.z) * p.c2, (y.w + u4.w) * p.c2);
+      }
+    }
+    cp_async_wait<0>();
+    group_sync<WPG>(g);  // Q, dO, lse and delta are in place
+    float s[4][KJ], dp[4][KJ];
+    if (lt) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int j = 0; j < KJ; ++j) s[a][j] = dp[a][j] = 0.f;
+    } else {
+      product_nt<D, KJ>(Ks + r0 * LD, Qs, tx, s);   // S^T in base 2 (Q carries c2)
+      product_nt<D, KJ>(Vs + r0 * LD, Gs, tx, dp);  // dP^T
+    }
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      const int col = tx + 16 * j, i = m0 + col, t_i = ti[j];
+      const float lse = lse_s[col], dl = dl_s[col];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        float pr = 0.f, dsw = 0.f;
+        if (i < N && tk[a] <= t_i) {
+          const bool w = in_window(t_i, tk[a], T, p.window);
+          pr = exp2f((w ? s[a][j] : 0.f) + rel[a][j] - lse);
+          dsw = w ? pr * (dp[a][j] - dl) * p.sm_scale : 0.f;
+        }
+        Ps[a * LP + col] = pr;
+        Dw[a * LP + col] = dsw;
+      }
+    }
+    __syncwarp();
+    if (!lt) product_nn<D, KN>(Dw, Qs, tx, kacc);  // dK += dS_w^T (q + u) c2  (`attentions/attn.py:718`)
+    group_sync<WPG>(g);                            // every warp has left Q, lse and delta
+    fetch_q(item + NG);
+    product_nn<D, KN>(Ps, Gs, tx, vacc);           // dV += P^T dO        (`attentions/attn.py:671-675`)
+    group_sync<WPG>(g);                            // every warp has left dO
+    fetch_g(item + NG);
   }
+  __syncthreads();
+  float *Km = Qall, *Vm = Gall;  // [NG][BM][LD] each
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    LaneCols<D>::store(Km + (g * BM + r0 + a) * LD, tx, kacc[a]);
+    LaneCols<D>::store(Vm + (g * BM + r0 + a) * LD, tx, vacc[a]);
+  }
+  __syncthreads();
   Tin* dk = (Tin*)bw.dk + b * bw.dk_sb + hk * bw.dk_sh;
   Tin* dv = (Tin*)bw.dv + b * bw.dv_sb + hk * bw.dv_sh;
   const float inv_c2 = 1.f / p.c2;
+  for (int idx = tid; idx < 2 * BM * D / 4; idx += CT) {
+    const bool is_k = idx < BM * D / 4;
+    const int rem = is_k ? idx : idx - BM * D / 4;
+    const int r = rem / (D / 4), d = (rem % (D / 4)) * 4;
+    if (r >= valid) continue;
+    const float* src = (is_k ? Km : Vm) + r * LD + d;
+    float4 x = *reinterpret_cast<const float4*>(src);
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int r = 2 * ty + a;
-    if (r < valid) {
-#pragma unroll
-      for (int e = 0; e < DV; ++e) {
-        dk[(int64_t)(n0 + r) * bw.dk_sn + tx + 16 * e] = from_f32<Tin>(kacc[a][e] * inv_c2);
-        dv[(int64_t)(n0 + r) * bw.dv_sn + tx + 16 * e] = from_f32<Tin>(vacc[a][e]);
-      }
+    for (int gg = 1; gg < NG; ++gg) {
+      const float4 y = *reinterpret_cast<const float4*>(src + gg * BM * LD);
+      x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
     }
+    if (is_k)
+      store4<Tin>(dk + (int64_t)(n0 + r) * bw.dk_sn + d, make_float4(x.x * inv_c2, x.y * inv_c2, x.z * inv_c2, x.w * inv_c2));
+    else
+      store4<Tin>(dv + (int64_t)(n0 + r) * bw.dv_sn + d, x);
   }
 }
 
-// dr[hk][slot][d] = sum_{b, h in group, i} dX[b,h,i,slot] * (q[b,h,i,d] + bias[hk][d])
-// One CTA per (32 slots, kv head, split); streams its share of the group's query rows in chunks of 64.
+// dr[hk][slot][d] = sum_{b, h in group, i} dX[b,h,i,slot] * (q[b,h,i,d] + bias[hk][d]), for the T time slots and
+// the C channel slots in one launch.  One CTA per (32 slots, kv head, split); streams its share of the group's
+// query rows in chunks of 64.
+constexpr int kDrelRows = 64, kDrelSlots = 32;
 template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_drel_kernel(BwdArgs bw, int which) {
-  constexpr int LD = D + 4;
-  constexpr int DV = D / 16;
+__global__ void __launch_bounds__(kThreads) simt_drel_kernel(BwdArgs bw) {
+  constexpr int LD = D + 4, VW = D / 16, LX = kDrelSlots + 1;
   const Args& p = bw.a;
-  extern __shared__ float smem[];
-  float* Xs = smem;            // 64 rows x 33
-  float* Qs = Xs + kBN * 33;   // 64 rows x LD
+  extern __shared__ __align__(16) float smem[];
+  float* Qs = smem;                  // 64 rows x LD
+  float* Xs = Qs + kDrelRows * LD;   // 64 rows x 33
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int S = which == 0 ? p.T : p.C;
-  const float* dx = which == 0 ? bw.dtbg : bw.dcbg;
-  const Tin* bias = (const Tin*)(which == 0 ? p.vt : p.z) + blockIdx.y * D;
+  const int t_blocks = (p.T + kDrelSlots - 1) / kDrelSlots;
+  const bool is_t = (int)blockIdx.x < t_blocks;
+  const int S = is_t ? p.T : p.C, s0 = (is_t ? blockIdx.x : blockIdx.x - t_blocks) * kDrelSlots;
+  const float* dx = is_t ? bw.dtbg : bw.dcbg;
+  const int hk = blockIdx.y;
+  const Tin* bias = (const Tin*)(is_t ? p.vt : p.z) + hk * D;
   // split-K over the (batch, head of the group, 64-row chunk) range: gridDim.z partial sums
-  float* out = bw.drel_part + (((int64_t)blockIdx.z * p.Hkv + blockIdx.y) * (p.T + p.C) + (which == 0 ? 0 : p.T)) * D;
-  const int hk = blockIdx.y, s0 = blockIdx.x * 32;
-  const int chunks_per_head = (p.N + kBN - 1) / kBN;
+  float* out = bw.drel_part + (((int64_t)blockIdx.z * p.Hkv + hk) * (p.T + p.C) + (is_t ? 0 : p.T)) * D;
+  const int chunks_per_head = (p.N + kDrelRows - 1) / kDrelRows;
   const int n_chunks = p.B * p.g * chunks_per_head;
   const int per_z = (n_chunks + gridDim.z - 1) / gridDim.z;
   const int c_begin = blockIdx.z * per_z, c_end = min(n_chunks, c_begin + per_z);
-  float acc[2][DV] = {};
+  float acc[2][VW] = {};
   for (int ch = c_begin; ch < c_end; ++ch) {
-    {
-      const int b = ch / (p.g * chunks_per_head), hh = (ch / chunks_per_head) % p.g;
-      const int m0 = (ch % chunks_per_head) * kBN;
-      const int h = hk * p.g + hh, bh = b * p.H + h;
-      const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
-      {
-        __syncthreads();
-        load_tile<Tin, D>(Qs, q, p.q_sn, m0, p.N, kBN, bias, 1.f);
-        for (int idx = tid; idx < kBN * 32; idx += kThreads) {
-          const int r = idx / 32, s = idx % 32;
-          const int i = m0 + r;
-          Xs[r * 33 + s] = (i < p.N && s0 + s < S) ? dx[((int64_t)bh * p.N + i) * S + s0 + s] : 0.f;
-        }
-        __syncthreads();
-        // rows >= N hold bias only in Qs but zero in Xs, so they add nothing
-#pragma unroll 4
-        for (int r = 0; r < kBN; ++r) {
-          const float x0 = Xs[r * 33 + 2 * ty], x1 = Xs[r * 33 + 2 * ty + 1];
+    const int b = ch / (p.g * chunks_per_head), hh = (ch / chunks_per_head) % p.g;
+    const int m0 = (ch % chunks_per_head) * kDrelRows;
+    const int h = hk * p.g + hh, bh = b * p.H + h;
+    const Tin* q = (const Tin*)p.q + b * p.q_sb + h * p.q_sh;
+    __syncthreads();
 #pragma unroll
-          for (int e = 0; e < DV; ++e) {
-            const float y = Qs[r * LD + tx + 16 * e];
-            acc[0][e] += x0 * y;
-            acc[1][e] += x1 * y;
-          }
-        }
+    for (int idx = tid; idx < kDrelRows * D / 4; idx += kThreads) {
+      const int r = idx / (D / 4), d = (idx % (D / 4)) * 4;
+      const float4 bb = load4<Tin>(bias + d);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m0 + r < p.N) x = load4<Tin>(q + (int64_t)(m0 + r) * p.q_sn + d);
+      *reinterpret_cast<float4*>(Qs + r * LD + d) = make_float4(x.x + bb.x, x.y + bb.y, x.z + bb.z, x.w + bb.w);
+    }
+#pragma unroll
+    for (int idx = tid; idx < kDrelRows * kDrelSlots; idx += kThreads) {
+      const int r = idx / kDrelSlots, s = idx % kDrelSlots;
+      const int i = m0 + r;
+      Xs[r * LX + s] = (i < p.N && s0 + s < S) ? dx[((int64_t)bh * p.N + i) * S + s0 + s] : 0.f;
+    }
+    __syncthreads();
+    // rows past the end hold the bias alone in Qs but zero in Xs, so they add nothing
+#pragma unroll 8
+    for (int r = 0; r < kDrelRows; ++r) {
+      const float x0 = Xs[r * LX + 2 * ty], x1 = Xs[r * LX + 2 * ty + 1];
+      float y[VW];
+      LaneCols<D>::load(Qs + r * LD, tx, y);
+#pragma unroll
+      for (int e = 0; e < VW; ++e) {
+        acc[0][e] = fmaf(x0, y[e], acc[0][e]);
+        acc[1][e] = fmaf(x1, y[e], acc[1][e]);
       }
     }
   }
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
     const int s = s0 + 2 * ty + a;
-    if (s < S) {
-#pragma unroll
-      for (int e = 0; e < DV; ++e) out[(int64_t)s * D + tx + 16 * e] = acc[a][e];
+    if (s < S) LaneCols<D>::store(out + (int64_t)s * D, tx, acc[a]);
+  }
+}
+
+// The last sums, in a fixed order (deterministic): dr_time / dr_chan from the split-K partials of
+// simt_drel_kernel (the first n_red blocks), du / dvt / dz from the per-tile partials of simt_dq_kernel (three
+// blocks per kv head).
+__global__ void __launch_bounds__(kThreads) simt_final_kernel(BwdArgs bw, int n_z, int n_qt, int n_red) {
+  const Args& p = bw.a;
+  const int S = p.T + p.C, D = p.D;
+  if ((int)blockIdx.x < n_red) {
+    const int64_t total = (int64_t)p.Hkv * S * D;
+    for (int64_t idx = (int64_t)blockIdx.x * kThreads + threadIdx.x; idx < total; idx += (int64_t)n_red * kThreads) {
+      float sum = 0.f;
+#pragma unroll 8
+      for (int zz = 0; zz < n_z; ++zz) sum += bw.drel_part[(int64_t)zz * total + idx];
+      const int d = idx % D, sl = (idx / D) % S, hk = idx / ((int64_t)D * S);
+      if (sl < p.T) bw.drt[((int64_t)hk * p.T + sl) * D + d] = sum;
+      else bw.drc[((int64_t)hk * p.C + (sl - p.T)) * D + d] = sum;
     }
+    return;
   }
-}
-
-// dr_time / dr_chan = sum of the split-K partials of simt_drel_kernel (fixed order: deterministic).
-__global__ void simt_drel_reduce_kernel(BwdArgs bw, int n_z) {
-  const Args& p = bw.a;
-  const int S = p.T + p.C;
-  const int64_t total = (int64_t)p.Hkv * S * p.D;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-    float sum = 0.f;
-    for (int zz = 0; zz < n_z; ++zz) sum += bw.drel_part[(int64_t)zz * total + idx];
-    const int d = idx % p.D, sl = (idx / p.D) % S, hk = idx / ((int64_t)p.D * S);
-    if (sl < p.T) bw.drt[((int64_t)hk * p.T + sl) * p.D + d] = sum;
-    else bw.drc[((int64_t)hk * p.C + (sl - p.T)) * p.D + d] = sum;
+  __shared__ float s_part[kThreads];
+  const int hk = ((int)blockIdx.x - n_red) / 3, which = ((int)blockIdx.x - n_red) % 3;
+  const int d = threadIdx.x % D, part = threadIdx.x / D, parts = kThreads / D;  // D divides the block size
+  const int per_b = p.g * n_qt, n = p.B * per_b;
+  float s = 0.f;
+#pragma unroll 8
+  for (int it = part; it < n; it += parts) {
+    const int b = it / per_b;
+    const int64_t tile = ((int64_t)b * p.H + hk * p.g) * n_qt + (it - b * per_b);
+    s += bw.partial[(tile * 3 + which) * D + d];
   }
-}
-
-// du/dvt/dz[hk][d] = sum over (b, h in group, query tile) of the per-tile partials.
-__global__ void simt_dbias_kernel(BwdArgs bw, int n_qt) {
-  const Args& p = bw.a;
-  const int hk = blockIdx.x, which = blockIdx.y, D = p.D;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < p.B; ++b)
-      for (int hh = 0; hh < p.g; ++hh) {
-        const int64_t bh = (int64_t)b * p.H + hk * p.g + hh;
-        for (int t = 0; t < n_qt; ++t) s += bw.partial[((bh * n_qt + t) * 3 + which) * D + d];
-      }
+  s_part[threadIdx.x] = s;
+  __syncthreads();
+  if (part == 0) {
+    for (int q = 1; q < parts; ++q) s += s_part[q * D + d];
     float* out = which == 0 ? bw.du : which == 1 ? bw.dvt : bw.dz;
     out[hk * D + d] = s;
   }
@@ -664,18 +1032,65 @@ int set_smem(K kernel, size_t bytes) {
   return MVPA_OK;
 }
 
+constexpr size_t kMaxSmemFloats = 232448 / sizeof(float);
+
+// Rows per CTA and groups: sixteen rows and four groups while that leaves no more than kSmallWaves CTAs per
+// multiprocessor (short sequences: the longest CTA sets the time, so many short ones), thirty-two rows and two
+// groups beyond (every key tile is loaded half as often).
+constexpr int kSmallWaves = 4;
+bool few_rows(int64_t rows, int heads) { return (rows + 15) / 16 * heads <= (int64_t)kSmallWaves * device_sm_count(); }
+
+template <typename Tin, int D, int WPG, int NG, int KN>
+int run_fwd(const Args& a, cudaStream_t s) {
+  constexpr int BM = 8 * WPG;
+  const size_t smem = sizeof(float) * (fwd_fixed_floats<D, WPG, NG, KN>() + (size_t)BM * (a.T + a.C));
+  int rc = set_smem(simt_fwd_kernel<Tin, D, WPG, NG, KN>, smem);
+  if (rc) return rc;
+  simt_fwd_kernel<Tin, D, WPG, NG, KN><<<dim3((a.q_tn * a.C + BM - 1) / BM, a.B * a.H), 32 * WPG * NG, smem, s>>>(a);
+  count_launch();
+  MVPA_CUDA_CHECK(cudaGetLastError());
+  return MVPA_OK;
+}
+
 template <typename Tin, int D>
 int launch_fwd(const Args& a, cudaStream_t s) {
-  const size_t smem = sizeof(float) * ((size_t)kBM * (D + 4) + 2 * kBN * (D + 4) + kBM * kPLd +
-                                       (size_t)kBM * (a.T + a.C) + 3 * kBM);
-  if (smem > 227 * 1024) {
-    set_error("fp32 path: T + C = %d needs %zu bytes of shared memory (max 232448)", a.T + a.C, smem);
+  constexpr int KN = D == 128 ? 32 : 64;
+  // the documented limit on the time and channel slots
+  const size_t limit = sizeof(float) * ((size_t)32 * (D + 4) + 2 * 64 * (D + 4) + 32 * 65 + (size_t)32 * (a.T + a.C) + 3 * 32);
+  if (limit > 227 * 1024) {
+    set_error("fp32 path: T + C = %d needs %zu bytes of shared memory (max 232448)", a.T + a.C, limit);
     return MVPA_ERR_UNSUPPORTED;
   }
-  int rc = set_smem(simt_fwd_kernel<Tin, D>, smem);
+  const size_t tc = (size_t)a.T + a.C;
+  if (few_rows((int64_t)a.q_tn * a.C, a.B * a.H)) {
+    if (fwd_fixed_floats<D, 2, 4, KN>() + 16 * tc <= kMaxSmemFloats) return run_fwd<Tin, D, 2, 4, KN>(a, s);
+  } else if (fwd_fixed_floats<D, 4, 2, KN>() + 32 * tc <= kMaxSmemFloats) {
+    return run_fwd<Tin, D, 4, 2, KN>(a, s);
+  }
+  static_assert(fwd_fixed_floats<D, 2, 2, KN>() + 16 * ((kMaxSmemFloats - 32 * (D + 4)) / 32 - 4 * (D + 4) - 67) <= kMaxSmemFloats,
+                "whatever the limit admits fits");
+  return run_fwd<Tin, D, 2, 2, KN>(a, s);
+}
+
+template <typename Tin, int D, int WPG, int NG, int KN, bool INS>
+int run_dq(const BwdArgs& b, size_t smem_floats, cudaStream_t s) {
+  constexpr int BM = 8 * WPG;
+  int rc = set_smem(simt_dq_kernel<Tin, D, WPG, NG, KN, INS>, smem_floats * sizeof(float));
   if (rc) return rc;
-  dim3 grid((a.q_tn * a.C + kBM - 1) / kBM, a.B * a.H);
-  simt_fwd_kernel<Tin, D><<<grid, kThreads, smem, s>>>(a);
+  simt_dq_kernel<Tin, D, WPG, NG, KN, INS><<<dim3((b.a.N + BM - 1) / BM, b.a.B * b.a.H), 32 * WPG * NG, smem_floats * sizeof(float), s>>>(b);
+  count_launch();
+  MVPA_CUDA_CHECK(cudaGetLastError());
+  return MVPA_OK;
+}
+
+template <typename Tin, int D, int WPG, int NG, int KN>
+int run_dkv(const BwdArgs& b, cudaStream_t s) {
+  constexpr int BM = 8 * WPG;
+  constexpr size_t smem = dkv_fixed_floats<D, WPG, NG, KN>() * sizeof(float);
+  static_assert(smem <= 232448, "shared memory budget");
+  int rc = set_smem(simt_dkv_kernel<Tin, D, WPG, NG, KN>, smem);
+  if (rc) return rc;
+  simt_dkv_kernel<Tin, D, WPG, NG, KN><<<dim3((b.a.N + BM - 1) / BM, b.a.B * b.a.Hkv), 32 * WPG * NG, smem, s>>>(b);
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
@@ -684,61 +1099,54 @@ int launch_fwd(const Args& a, cudaStream_t s) {
 template <typename Tin, int D>
 int launch_bwd(const BwdArgs& b, cudaStream_t s) {
   const Args& a = b.a;
-  constexpr int LD = D + 4;
-  const int n_qt = (a.N + kBM - 1) / kBM;
-  const dim3 grid_q(n_qt, a.B * a.H);
-  if (b.tc_extra == nullptr) {
-    const size_t smem = sizeof(float) * kBM * LD;
-    simt_rel_kernel<Tin, D><<<grid_q, kThreads, smem, s>>>(b);
-    count_launch();
-  }
-  {
-    constexpr int kRowThreads = D / (16 / (int)sizeof(Tin));
-    dim3 grid((a.N * kRowThreads + kThreads - 1) / kThreads, a.B * a.H);
-    simt_delta_kernel<Tin, D><<<grid, kThreads, 0, s>>>(b);
-    count_launch();
-  }
   if (b.tc_extra != nullptr) {
-    // bf16 on the tensor cores: dq, dk, dv and the relative-score gradients
-    if constexpr (D >= 64) {
+    // bf16 on the tensor cores: dq, dk, dv and the relative-key gradients
+    if constexpr (sizeof(Tin) == 2 && D >= 64) {
+      constexpr int kRowThreads = D / (16 / (int)sizeof(Tin));
+      dim3 grid((a.N * kRowThreads + kThreads - 1) / kThreads, a.B * a.H);
+      simt_delta_kernel<Tin, D><<<grid, kThreads, 0, s>>>(b);
+      count_launch();
       int rc = tc_bwd_q(b, b.tc_extra, s);
       if (rc) return rc;
+      return tc_bwd_bias(b, b.tc_extra, s);
     }
+  }
+  constexpr int KN = D == 128 ? 32 : 64;
+  const size_t limit = sizeof(float) * ((size_t)2 * 32 * (D + 4) + 2 * 64 * (D + 4) + 2 * 32 * 65 + (size_t)32 * (a.T + a.C) + 2 * 32 + 16 * D);
+  if (limit > 227 * 1024) {
+    set_error("fp32 backward: T + C = %d needs %zu bytes of shared memory", a.T + a.C, limit);
+    return MVPA_ERR_UNSUPPORTED;
+  }
+  const size_t tc = (size_t)a.T + a.C;
+  const size_t small_f = dq_fixed_floats<D, 2, 4, KN>() + 16 * 5 * tc, large_f = dq_fixed_floats<D, 4, 2, KN>() + 32 * 3 * tc;
+  int rc, bm = 16;
+  if (few_rows(a.N, a.B * a.H) && small_f <= kMaxSmemFloats) {
+    rc = run_dq<Tin, D, 2, 4, KN, true>(b, small_f, s);
+  } else if (!few_rows(a.N, a.B * a.H) && large_f <= kMaxSmemFloats) {
+    rc = run_dq<Tin, D, 4, 2, KN, true>(b, large_f, s);
+    bm = 32;
   } else {
-    const size_t smem = sizeof(float) * ((size_t)2 * kBM * LD + 2 * kBN * LD + 2 * kBM * kPLd +
-                                         (size_t)kBM * (a.T + a.C) + 2 * kBM + 16 * D);
-    if (smem > 227 * 1024) {
-      set_error("fp32 backward: T + C = %d needs %zu bytes of shared memory", a.T + a.C, smem);
-      return MVPA_ERR_UNSUPPORTED;
-    }
-    int rc = set_smem(simt_dq_kernel<Tin, D>, smem);
-    if (rc) return rc;
-    simt_dq_kernel<Tin, D><<<grid_q, kThreads, smem, s>>>(b);
-    count_launch();
+    static_assert(dq_fixed_floats<D, 2, 2, 32>() + 32 * ((kMaxSmemFloats - 64 * (D + 4) - 4224 - 16 * D) / 32 - 4 * (D + 4)) <= kMaxSmemFloats,
+                  "whatever the limit admits fits");
+    rc = run_dq<Tin, D, 2, 2, 32, false>(b, dq_fixed_floats<D, 2, 2, 32>() + 32 * tc, s);
   }
-  if (b.tc_extra == nullptr) {  // (the tensor-core path has produced dK / dV already)
-    const size_t smem = sizeof(float) * ((size_t)2 * kBM * LD + 2 * kBN * LD + 2 * kBM * kPLd + 2 * kBN);
-    int rc = set_smem(simt_dkv_kernel<Tin, D>, smem);
-    if (rc) return rc;
-    dim3 grid(n_qt, a.B * a.Hkv);
-    simt_dkv_kernel<Tin, D><<<grid, kThreads, smem, s>>>(b);
-    count_launch();
-  }
-  if (b.tc_extra != nullptr) {  // the tensor-core kernels have accumulated the relative-key gradients already
-    MVPA_CUDA_CHECK(cudaGetLastError());
-    return tc_bwd_bias(b, b.tc_extra, s);
-  }
+  if (rc) return rc;
+  rc = few_rows(a.N, a.B * a.Hkv) ? run_dkv<Tin, D, 2, 4, KN>(b, s) : run_dkv<Tin, D, 4, 2, KN>(b, s);
+  if (rc) return rc;
+  const int n_qt = (a.N + bm - 1) / bm;
+  const int n_chunks = a.B * a.g * ((a.N + kDrelRows - 1) / kDrelRows);
+  const int n_z = n_chunks < kDrelSplit ? n_chunks : kDrelSplit;
   {
-    const size_t smem = sizeof(float) * ((size_t)kBN * 33 + kBN * LD);
-    int rc = set_smem(simt_drel_kernel<Tin, D>, smem);
+    const size_t smem = sizeof(float) * ((size_t)kDrelRows * (kDrelSlots + 1) + kDrelRows * (D + 4));
+    rc = set_smem(simt_drel_kernel<Tin, D>, smem);
     if (rc) return rc;
-    simt_drel_kernel<Tin, D><<<dim3((a.T + 31) / 32, a.Hkv, kDrelSplit), kThreads, smem, s>>>(b, 0);
-    simt_drel_kernel<Tin, D><<<dim3((a.C + 31) / 32, a.Hkv, kDrelSplit), kThreads, smem, s>>>(b, 1);
-    simt_drel_reduce_kernel<<<148, 256, 0, s>>>(b, kDrelSplit);
-    count_launch(3);
+    const unsigned blocks = (a.T + kDrelSlots - 1) / kDrelSlots + (a.C + kDrelSlots - 1) / kDrelSlots;
+    simt_drel_kernel<Tin, D><<<dim3(blocks, a.Hkv, n_z), kThreads, smem, s>>>(b);
   }
-  simt_dbias_kernel<<<dim3(a.Hkv, 3), 128, 0, s>>>(b, n_qt);
-  count_launch();
+  const int64_t total = (int64_t)a.Hkv * (a.T + a.C) * D;
+  const int n_red = (int)((total + kThreads - 1) / kThreads < 592 ? (total + kThreads - 1) / kThreads : 592);
+  simt_final_kernel<<<n_red + 3 * a.Hkv, kThreads, 0, s>>>(b, n_z, n_qt, n_red);
+  count_launch(2);
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
 }
@@ -795,9 +1203,9 @@ size_t simt_bwd_workspace_floats(const mvpa_problem* p) {
     n = (n + 63) & ~(size_t)63;
     return n + tc_bwd_q_workspace_floats(p);
   }
-  const size_t n_qt = (N + kBM - 1) / kBM;
-  size_t n = 2 * BH * N * (p->T + p->C) + BH * N + BH * n_qt * 3 * p->D +
-             (size_t)kDrelSplit * p->Hkv * (p->T + p->C) * p->D;
+  const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most
+  size_t n = 2 * BH * N * (p->T + p->C) + BH * N + BH * n_qt * 3 * p->D;
+  n = ((n + 3) & ~(size_t)3) + (size_t)kDrelSplit * p->Hkv * (p->T + p->C) * p->D;
   return (n + 63) & ~(size_t)63;
 }
 
@@ -821,14 +1229,15 @@ void simt_bwd_carve(BwdArgs& b, float* ws, int dtype) {
     b.tc_extra = ws + used;
     return;
   }
-  const size_t n_qt = (N + kBM - 1) / kBM;
+  const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most
   b.tbg = ws;
   b.cbg = b.tbg + BH * N * a.T;
   b.dtbg = b.cbg + BH * N * a.C;
   b.dcbg = b.dtbg + BH * N * a.T;
   b.delta = b.dcbg + BH * N * a.C;
   b.partial = b.delta + BH * N;
-  b.drel_part = b.partial + BH * n_qt * 3 * a.D;
+  const size_t used = 2 * BH * N * (a.T + a.C) + BH * N + BH * n_qt * 3 * a.D;
+  b.drel_part = ws + ((used + 3) & ~(size_t)3);  // stored in 16-byte pieces
   b.tc_extra = nullptr;
 }
 

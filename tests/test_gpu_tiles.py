@@ -1,0 +1,47 @@
+"""GPU: the tiled CUDA-core kernels and the training kernels of the block at the edges of their tiles and on both
+sides of each launch rule, against the oracle (operator) and torch in 64 bits (row kernels)."""
+import numpy as np
+import pytest
+import torch
+
+import mvpa_oracle as mo
+from test_gpu_op import BF16_ABS, F16_ABS, F32_REL, GRADS, _np, _op, _oracle_args, _rounded, random_case
+
+pytestmark = pytest.mark.gpu
+
+TOL = {torch.float32: F32_REL, torch.float16: F16_ABS, torch.bfloat16: BF16_ABS}
+
+
+def _check(cuda, g, dtype, window=10):
+    """Forward and all eight gradients against the oracle at the operator tests' tolerances."""
+    gr = g if dtype == torch.float32 else _rounded(g, dtype)
+    o, t = _op(cuda, g, dtype, grads=True, window=window)
+    o.backward(torch.tensor(g["do"], device=cuda, dtype=dtype))
+    ref_o = mo.mvpa_forward(*_oracle_args(gr), float(g["sm_scale"]), window=window)[0]
+    ref = mo.mvpa_backward(*_oracle_args(gr), gr["do"], float(g["sm_scale"]), window=window)
+    pairs = [("o", o, ref_o)] + [(n, t[k].grad, ref[n]) for n, k in zip(
+        GRADS, ("q", "u", "v", "z", "k", "r_time", "r_chan", "val"))]
+    for name, got, want in pairs:
+        err = np.abs(_np(got).reshape(np.shape(want)) - want).max()
+        assert err <= TOL[dtype] * max(1.0, np.abs(want).max()), (name, err)
+
+
+# (B, H, Hkv, T, C, D): fewer rows than a tile, one row and one key past a tile, ragged channels that put a time
+# step's end inside a tile, light tiles (T > window + tile), and every head_dim
+@pytest.mark.parametrize("shape", [(1, 2, 1, 1, 3, 64), (1, 2, 1, 1, 17, 16), (2, 4, 2, 5, 13, 64), (1, 2, 2, 3, 43, 32),
+                                   (1, 2, 1, 24, 11, 128), (1, 1, 1, 45, 3, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_cuda_core_tiles_sixteen_rows(cuda, shape, dtype):
+    _check(cuda, random_case(sum(shape), *shape), dtype)
+
+
+# more sixteen-row tiles than four per multiprocessor: thirty-two rows per CTA, last tile ragged
+@pytest.mark.parametrize("shape", [(2, 16, 16, 15, 21, 16), (1, 32, 16, 17, 19, 32)])
+def test_cuda_core_tiles_thirty_two_rows(cuda, shape):
+    _check(cuda, random_case(sum(shape), *shape), torch.float32)
+
+
+# time / channel axes whose slot sums do not fit beside the four groups' tiles
+@pytest.mark.parametrize("shape", [(1, 1, 1, 2, 400, 64), (1, 1, 1, 300, 2, 128), (1, 2, 1, 2, 440, 32)])
+def test_cuda_core_long_axes(cuda, shape):
+    _check(cuda, random_case(sum(shape), *shape), torch.float32)
