@@ -185,6 +185,25 @@ int mvpa_silu_mul(const void* gate, const void* up, int64_t ld_in, void* out, in
                   int64_t rows, int32_t width, int32_t dtype, void* cuda_stream);
 
 /*
+ * Backward of mvpa_rmsnorm without `add` (what autograd derives from the reference's RMSNorm):
+ * dx (rows, width) and dweight (width), both in the element type; sums over the rows in fp32, in a
+ * fixed order.  The caller provides `workspace` of at least
+ * mvpa_rmsnorm_bwd_workspace_bytes(rows, width) bytes, 16-byte aligned.  Same widths as mvpa_rmsnorm.
+ */
+size_t mvpa_rmsnorm_bwd_workspace_bytes(int64_t rows, int32_t width);
+int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, void* dx, void* dweight,
+                     int64_t rows, int32_t width, float eps, int32_t dtype, void* workspace,
+                     size_t workspace_bytes, void* cuda_stream);
+
+/*
+ * Backward of mvpa_silu_mul: dgate and dup (leading dimension ld_grad) from dout (ld_dout) and the
+ * forward's inputs.
+ */
+int mvpa_silu_mul_bwd(const void* gate, const void* up, int64_t ld_in, const void* dout,
+                      int64_t ld_dout, void* dgate, void* dup, int64_t ld_grad, int64_t rows,
+                      int32_t width, int32_t dtype, void* cuda_stream);
+
+/*
  * Number of coefficients `WaveEncoder` produces for a segment of `segment_len` samples with an
  * 8-tap wavelet in periodic mode (`models/fftencoder.py:69-78`: every level floor((n + 7) / 2),
  * floor(log2(len / 7)) levels, plus the last approximation); 0 if the segment is too short.

@@ -3,8 +3,9 @@
 //   rmsnorm / add_rmsnorm   `ln_1`, `ln_f` and the residual sum of the parallel block
 //                           (`models/mvpformer.py:132-147`: h = x + MLP(ln_1 x) + Attn(ln_1 x)),
 //                           one pass over the hidden state instead of three
+//   rmsnorm_bwd             their backward in training
 //   silu_mul                the SwiGLU gate of the MLP (`LlamaMLP`: down(silu(gate x) * up x)) on a
-//                           strided view of a fused gate|up projection
+//                           strided view of a fused gate|up projection, and its backward
 //   wave_encode             `WaveEncoder.block` + its RMSNorm (`models/fftencoder.py:79-97`): all levels
 //                           of the periodic db4 wavelet transform of one segment in shared memory,
 //                           concatenated coarse-to-fine, normalised, written once in the model's dtype
@@ -151,6 +152,107 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_kernel(const T* __r
   }
 }
 
+// Backward of rmsnorm_kernel without the residual add:  with g = dy w and xh = x rstd,
+//   dx = rstd (g - xh mean(g xh)),   dw = sum_rows dy xh.
+// One warp per row at a time, rows strided over the grid; x and dy are read once, the row stays in registers;
+// each lane keeps the dw of its columns over all its rows, the warps of a CTA meet in shared memory and one
+// fp32 row per CTA goes to `dw_part` (summed in a fixed order by colsum_kernel: deterministic).
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
+                                                                        const T* __restrict__ dy, T* __restrict__ dx,
+                                                                        float* __restrict__ dw_part,
+                                                                        int64_t rows, int E, float eps) {
+  constexpr int N = Vec<T>::N;
+  extern __shared__ __align__(16) float s_dw[];  // [kWarpsPerCta][E]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float acc[NV][N];
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int e = 0; e < N; ++e) acc[i][e] = 0.f;
+  for (int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + warp; row < rows; row += (int64_t)gridDim.x * kWarpsPerCta) {
+    uint4 rx[NV], rg[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = (i * 32 + lane) * N;
+      if (col < E) {
+        rx[i] = *reinterpret_cast<const uint4*>(x + row * E + col);
+        rg[i] = *reinterpret_cast<const uint4*>(dy + row * E + col);
+      }
+    }
+    float ss = 0.f, sg = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = (i * 32 + lane) * N;
+      if (col < E) {
+        float v[N], g[N], wv[N];
+        Vec<T>::unpack(rx[i], v);
+        Vec<T>::unpack(rg[i], g);
+        Vec<T>::load(w + col, wv);
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          ss += v[e] * v[e];
+          sg += g[e] * wv[e] * v[e];
+        }
+      }
+    }
+    const float rstd = rsqrtf(warp_sum(ss) / (float)E + eps);
+    const float c = warp_sum(sg) * rstd / (float)E;  // mean(g xh)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = (i * 32 + lane) * N;
+      if (col < E) {
+        float v[N], g[N], wv[N], r[N];
+        Vec<T>::unpack(rx[i], v);
+        Vec<T>::unpack(rg[i], g);
+        Vec<T>::load(w + col, wv);
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          const float xh = v[e] * rstd;
+          acc[i][e] += g[e] * xh;
+          r[e] = rstd * (g[e] * wv[e] - xh * c);
+        }
+        Vec<T>::store(dx + row * E + col, r);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int col = (i * 32 + lane) * N;
+    if (col < E) {
+#pragma unroll
+      for (int e = 0; e < N; e += 4)
+        *reinterpret_cast<float4*>(s_dw + warp * E + col + e) = make_float4(acc[i][e], acc[i][e + 1], acc[i][e + 2], acc[i][e + 3]);
+    }
+  }
+  __syncthreads();
+  for (int col = threadIdx.x; col < E; col += kWarpsPerCta * 32) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kWarpsPerCta; ++k) s += s_dw[k * E + col];
+    dw_part[(int64_t)blockIdx.x * E + col] = s;
+  }
+}
+
+// out[col] = sum_r part[r][col] in a fixed order: 32 columns per CTA, eight row strides.
+template <typename T>
+__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ part, T* __restrict__ out, int n, int E) {
+  __shared__ float s[8][33];
+  const int col = blockIdx.x * 32 + (threadIdx.x & 31), k = threadIdx.x >> 5;
+  float acc = 0.f;
+  if (col < E) {
+#pragma unroll 8
+    for (int r = k; r < n; r += 8) acc += part[(int64_t)r * E + col];
+  }
+  s[k][threadIdx.x & 31] = acc;
+  __syncthreads();
+  if (k == 0 && col < E) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) acc += s[q][threadIdx.x];
+    out[col] = from_f32<T>(acc);
+  }
+}
+
 // out = silu(gate) * up, elementwise, rows of `width` elements at independent leading dimensions.
 template <typename T>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_t ld_in,
@@ -167,6 +269,36 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gat
 #pragma unroll
     for (int e = 0; e < N; ++e) g[e] = Vec<T>::round(g[e] / (1.f + __expf(-g[e]))) * u[e];
     Vec<T>::store(out + r * ld_out + c, g);
+  }
+}
+
+// Backward of silu_mul_kernel for out = silu(gate) * up: with s = sigmoid(gate),
+//   dgate = dout up s (1 + gate (1 - s)),  dup = dout silu(gate)   (silu rounded to T as in the forward).
+template <typename T>
+__global__ void __launch_bounds__(256) silu_mul_bwd_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_t ld_in,
+                                                           const T* __restrict__ dout, int64_t ld_dout,
+                                                           T* __restrict__ dgate, T* __restrict__ dup, int64_t ld_g,
+                                                           int64_t rows, int width) {
+  constexpr int N = Vec<T>::N;
+  const int vec_per_row = width / N;
+  const int64_t total = rows * vec_per_row;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / vec_per_row;
+    const int c = (int)(i % vec_per_row) * N;
+    float g[N], u[N], d[N];
+    Vec<T>::load(gate + r * ld_in + c, g);
+    Vec<T>::load(up + r * ld_in + c, u);
+    Vec<T>::load(dout + r * ld_dout + c, d);
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const float s = 1.f / (1.f + __expf(-g[e]));
+      const float silu = Vec<T>::round(g[e] / (1.f + __expf(-g[e])));
+      const float du = d[e] * silu;
+      g[e] = d[e] * u[e] * (s * (1.f + g[e] * (1.f - s)));
+      u[e] = du;
+    }
+    Vec<T>::store(dgate + r * ld_g + c, g);
+    Vec<T>::store(dup + r * ld_g + c, u);
   }
 }
 
@@ -422,6 +554,35 @@ int launch_rmsnorm(const void* x, const void* a, const void* w, void* h_out, voi
   return MVPA_OK;
 }
 
+int rmsnorm_bwd_blocks(int64_t rows) {
+  const int64_t want = (rows + kWarpsPerCta - 1) / kWarpsPerCta, most = 2 * (int64_t)device_sm_count();
+  return (int)(want < most ? want : most);
+}
+
+template <typename T, int NV>
+int run_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* ws, int64_t rows, int E,
+                    float eps, cudaStream_t s) {
+  const size_t smem = sizeof(float) * kWarpsPerCta * E;
+  if (smem > 48 * 1024)
+    MVPA_CUDA_CHECK(cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = rmsnorm_bwd_blocks(rows);
+  rmsnorm_bwd_kernel<T, NV><<<grid, kWarpsPerCta * 32, smem, s>>>((const T*)x, (const T*)w, (const T*)dy, (T*)dx, ws, rows, E, eps);
+  colsum_kernel<T><<<(E + 31) / 32, 256, 0, s>>>(ws, (T*)dw, grid, E);
+  count_launch(2);
+  MVPA_CUDA_CHECK(cudaGetLastError());
+  return MVPA_OK;
+}
+
+template <typename T>
+int launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* ws, int64_t rows, int E,
+                       float eps, cudaStream_t s) {
+  const int nv = (E / Vec<T>::N + 31) / 32;
+  if (nv <= 2) return run_rmsnorm_bwd<T, 2>(x, w, dy, dx, dw, ws, rows, E, eps, s);
+  if (nv <= 4) return run_rmsnorm_bwd<T, 4>(x, w, dy, dx, dw, ws, rows, E, eps, s);
+  if (nv <= 8) return run_rmsnorm_bwd<T, 8>(x, w, dy, dx, dw, ws, rows, E, eps, s);
+  return run_rmsnorm_bwd<T, 16>(x, w, dy, dx, dw, ws, rows, E, eps, s);
+}
+
 int check_rows(const char* what, int64_t rows, int width, int dtype, int max_vectors) {
   if (dtype != MVPA_F32 && dtype != MVPA_BF16) {
     set_error("%s: element type must be MVPA_F32 or MVPA_BF16", what);
@@ -482,6 +643,55 @@ int mvpa_silu_mul(const void* gate, const void* up, int64_t ld_in, void* out, in
   else
     silu_mul_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, ld_in,
                                                        (__nv_bfloat16*)out, ld_out, rows, width);
+  count_launch();
+  MVPA_CUDA_CHECK(cudaGetLastError());
+  return MVPA_OK;
+}
+
+size_t mvpa_rmsnorm_bwd_workspace_bytes(int64_t rows, int32_t width) {
+  if (rows <= 0 || width <= 0) return 0;
+  return sizeof(float) * (size_t)rmsnorm_bwd_blocks(rows) * width;
+}
+
+int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, void* dx, void* dweight, int64_t rows,
+                     int32_t width, float eps, int32_t dtype, void* workspace, size_t workspace_bytes, void* cuda_stream) {
+  int rc = check_rows("mvpa_rmsnorm_bwd", rows, width, dtype, 16);
+  if (rc) return rc;
+  if (!aligned16(x) || !aligned16(weight) || !aligned16(dy) || !aligned16(dx) || !aligned16(dweight)) {
+    set_error("mvpa_rmsnorm_bwd: x, weight, dy, dx and dweight must be 16-byte aligned and not NULL");
+    return MVPA_ERR_ALIGNMENT;
+  }
+  if (!aligned16(workspace) || workspace_bytes < mvpa_rmsnorm_bwd_workspace_bytes(rows, width)) {
+    set_error("mvpa_rmsnorm_bwd: 16-byte aligned workspace of %zu bytes required, %zu given",
+              mvpa_rmsnorm_bwd_workspace_bytes(rows, width), workspace_bytes);
+    return MVPA_ERR_WORKSPACE;
+  }
+  cudaStream_t s = (cudaStream_t)cuda_stream;
+  return dtype == MVPA_F32
+             ? launch_rmsnorm_bwd<float>(x, weight, dy, dx, dweight, (float*)workspace, rows, width, eps, s)
+             : launch_rmsnorm_bwd<__nv_bfloat16>(x, weight, dy, dx, dweight, (float*)workspace, rows, width, eps, s);
+}
+
+int mvpa_silu_mul_bwd(const void* gate, const void* up, int64_t ld_in, const void* dout, int64_t ld_dout, void* dgate,
+                      void* dup, int64_t ld_grad, int64_t rows, int32_t width, int32_t dtype, void* cuda_stream) {
+  int rc = check_rows("mvpa_silu_mul_bwd", rows, width, dtype, 0);
+  if (rc) return rc;
+  const int n = dtype == MVPA_F32 ? 4 : 8;
+  if (!aligned16(gate) || !aligned16(up) || !aligned16(dout) || !aligned16(dgate) || !aligned16(dup) || ld_in % n != 0 ||
+      ld_dout % n != 0 || ld_grad % n != 0 || ld_in < width || ld_dout < width || ld_grad < width) {
+    set_error("mvpa_silu_mul_bwd: pointers must be 16-byte aligned, leading dimensions multiples of %d and >= the width", n);
+    return MVPA_ERR_ALIGNMENT;
+  }
+  cudaStream_t s = (cudaStream_t)cuda_stream;
+  const int64_t ctas = (rows * (width / n) + 255) / 256, most = (int64_t)device_sm_count() * 16;
+  const unsigned grid = (unsigned)(ctas < most ? ctas : most);
+  if (dtype == MVPA_F32)
+    silu_mul_bwd_kernel<float><<<grid, 256, 0, s>>>((const float*)gate, (const float*)up, ld_in, (const float*)dout, ld_dout,
+                                                    (float*)dgate, (float*)dup, ld_grad, rows, width);
+  else
+    silu_mul_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, ld_in,
+                                                            (const __nv_bfloat16*)dout, ld_dout, (__nv_bfloat16*)dgate,
+                                                            (__nv_bfloat16*)dup, ld_grad, rows, width);
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;

@@ -115,8 +115,8 @@ class MVPFormerGQAAttention(torch.nn.Module):
         channel_key = self.channel_net(channel_embedding)        # (1,C,Hkv*D)
         # Strided (B, heads, N, D) views of the projection outputs: no copies.
         q4 = query.view(B, N, H, D).permute(0, 2, 1, 3)
-        k4 = kv.view(B, N, 2 * Hkv, D)[:, :, :Hkv].permute(0, 2, 1, 3)
-        v4 = kv.view(B, N, 2 * Hkv, D)[:, :, Hkv:].permute(0, 2, 1, 3)
+        # (split, not slices: autograd then writes the gradient of `kv` with one concatenation)
+        k4, v4 = (t.permute(0, 2, 1, 3) for t in kv.view(B, N, 2 * Hkv, D).split(Hkv, dim=2))
         rt = time_key.view(1, T, Hkv, D).permute(0, 2, 1, 3)     # (1,Hkv,T,D)
         rc = channel_key.view(1, C, Hkv, D).permute(0, 2, 1, 3)  # (1,Hkv,C,D)
         u, v, z = (b.view(1, Hkv, 1, D).to(query.dtype) for b in self.attn_bias.split(self.embed_kv_dim))

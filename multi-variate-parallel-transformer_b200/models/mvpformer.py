@@ -17,8 +17,9 @@ h = x + MLP(ln_1 x) + Attn(ln_1 x)) built for B200:
   * the relative keys of all layers (`position_net`, `channel_net` of the embeddings, which do not depend
     on the input) come from one GEMM each per forward.
 
-With gradients enabled the blocks run the reference's op order through differentiable torch
-expressions and the differentiable `attentions.flashmvpa`.
+With gradients enabled the blocks run the reference's op order through differentiable operations: torch's
+projections, `mvpa_ops.rmsnorm_train` and `mvpa_ops.swiglu` (one kernel each way instead of about ten
+elementwise launches), and `attentions.flashmvpa`.
 """
 from __future__ import annotations
 
@@ -72,8 +73,7 @@ class RMSNorm(torch.nn.Module):
 
     def forward(self, x):
         if torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad):
-            xf = x.float()
-            return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps) * self.weight.float()).to(x.dtype)
+            return mvpa_ops.rmsnorm_train(x, self.weight, self.eps)
         return mvpa_ops.rmsnorm(x.contiguous(), self.weight.detach().to(x.dtype), self.eps)
 
 
@@ -88,7 +88,7 @@ class LlamaMLP(torch.nn.Module):
         self.down_proj = torch.nn.Linear(config.intermediate_size, config.hidden_size, bias=False)
 
     def forward(self, x):
-        return self.down_proj(F.silu(self.gate_proj(x)) * self.up_proj(x))
+        return self.down_proj(mvpa_ops.swiglu(self.gate_proj(x), self.up_proj(x)))
 
 
 class MVPFormerBlock(torch.nn.Module):

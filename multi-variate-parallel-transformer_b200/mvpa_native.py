@@ -93,7 +93,7 @@ EXPORTS = ("mvpa_fwd", "mvpa_bwd", "mvpa_fwd_workspace_bytes", "mvpa_bwd_workspa
            "mvpa_workspace_status", "mvpa_fwd_noalloc", "mvpa_bwd_status", "mvpa_noalloc_status",
            "mvpa_selftest_wait_timeout", "mvpa_rmsnorm", "mvpa_silu_mul", "mvpa_wave_encode_size",
            "mvpa_wave_encode", "mvpa_channel_mean", "mvpa_contrastive_logits", "mvpa_peer_gather", "mvpa_peer_signal",
-           "mvpa_peer_wait")
+           "mvpa_peer_wait", "mvpa_rmsnorm_bwd", "mvpa_rmsnorm_bwd_workspace_bytes", "mvpa_silu_mul_bwd")
 ABI_VERSION = 3   # mvpa_abi_version() of the header this shim was written against
 
 
@@ -138,6 +138,12 @@ def lib() -> ctypes.CDLL:
         L.mvpa_rmsnorm.argtypes = [vp, vp, vp, vp, vp, i64, i32, f32, i32, vp]
         L.mvpa_silu_mul.restype = ctypes.c_int
         L.mvpa_silu_mul.argtypes = [vp, vp, i64, vp, i64, i64, i32, i32, vp]
+        L.mvpa_rmsnorm_bwd_workspace_bytes.restype = ctypes.c_size_t
+        L.mvpa_rmsnorm_bwd_workspace_bytes.argtypes = [i64, i32]
+        L.mvpa_rmsnorm_bwd.restype = ctypes.c_int
+        L.mvpa_rmsnorm_bwd.argtypes = [vp, vp, vp, vp, vp, i64, i32, f32, i32, vp, ctypes.c_size_t, vp]
+        L.mvpa_silu_mul_bwd.restype = ctypes.c_int
+        L.mvpa_silu_mul_bwd.argtypes = [vp, vp, i64, vp, i64, vp, vp, i64, i64, i32, i32, vp]
         L.mvpa_wave_encode_size.restype = i32
         L.mvpa_wave_encode_size.argtypes = [i32, ctypes.POINTER(i32), i32]
         L.mvpa_wave_encode.restype = ctypes.c_int

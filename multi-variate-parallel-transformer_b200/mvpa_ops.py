@@ -1,8 +1,8 @@
 """Torch-tensor front ends of the C-ABI kernels that surround the attention in an MVPFormer block,
 its encoder and its heads (``include/mvpa.h``: mvpa_rmsnorm, mvpa_silu_mul, mvpa_wave_encode,
-mvpa_channel_mean, mvpa_contrastive_logits).  Forward only: these are the inference kernels; the
-modules in ``models/`` fall back to differentiable torch expressions when gradients are required.
-CUDA tensors only, bf16 or fp32.
+mvpa_channel_mean, mvpa_contrastive_logits, and the backwards mvpa_rmsnorm_bwd, mvpa_silu_mul_bwd).
+`rmsnorm_train` and `swiglu` are differentiable and take any tensor (torch expressions serve what the
+kernels do not); the others are forward only, CUDA tensors, bf16 or fp32.
 """
 from __future__ import annotations
 
@@ -62,6 +62,115 @@ def silu_mul(gate, up, out):
                                       width, _code(gate), _stream(gate))
     _nat.check(st, "mvpa_silu_mul")
     return out
+
+
+def rmsnorm_bwd(x, weight, dy, eps):
+    """Gradients (dx, dweight) of `rmsnorm(x, weight, eps)` (no `add`) for the incoming gradient `dy`."""
+    _need_cuda(x, weight, dy)
+    E = x.shape[-1]
+    x2, dy2 = x.reshape(-1, E), dy.reshape(-1, E)
+    assert x2.is_contiguous() and dy2.is_contiguous() and weight.is_contiguous()
+    assert weight.dtype == x.dtype == dy.dtype and dy.shape == x.shape
+    dx, dw = torch.empty_like(x2), torch.empty_like(weight)
+    lib = _nat.lib()
+    nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    with torch.cuda.device(x.device):
+        st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+                                  x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes, _stream(x))
+    _nat.check(st, "mvpa_rmsnorm_bwd")
+    return dx.view(x.shape), dw
+
+
+def silu_mul_bwd(gate, up, dout):
+    """Gradients (dgate, dup) of silu(gate) * up for 2-D tensors with unit inner stride."""
+    _need_cuda(gate, up, dout)
+    rows, width = gate.shape
+    assert up.shape == gate.shape and dout.shape == gate.shape and gate.dtype == up.dtype == dout.dtype
+    assert gate.stride(1) == up.stride(1) == dout.stride(1) == 1 and gate.stride(0) == up.stride(0)
+    dgate, dup = (torch.empty((rows, width), dtype=gate.dtype, device=gate.device) for _ in range(2))
+    with torch.cuda.device(gate.device):
+        st = _nat.lib().mvpa_silu_mul_bwd(gate.data_ptr(), up.data_ptr(), gate.stride(0), dout.data_ptr(), dout.stride(0),
+                                          dgate.data_ptr(), dup.data_ptr(), width, rows, width, _code(gate), _stream(gate))
+    _nat.check(st, "mvpa_silu_mul_bwd")
+    return dgate, dup
+
+
+def _plain(*ts):
+    """Tensors that the kernels can take and that nothing traces: ordinary CUDA tensors of one supported dtype,
+    contiguous, 16-byte aligned, not empty; no forward-mode level, functorch transform or tracer is active
+    (those are served by the differentiable torch expressions)."""
+    t0 = ts[0]
+    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._functorch.peek_interpreter_stack() is not None:
+        return False
+    if torch.autograd.forward_ad._current_level >= 0 or t0.dtype not in (torch.bfloat16, torch.float32):
+        return False
+    # (a backward may run on a thread of the autograd engine, where a transform shows on the tensor alone)
+    if any(torch._C._functorch.is_functorch_wrapped_tensor(t) for t in ts):
+        return False
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == t0.dtype and t.device == t0.device
+               and t.is_contiguous() and t.numel() > 0 and t.data_ptr() % 16 == 0 for t in ts)
+
+
+def _rows_fit(t):
+    """The row kernels' widths: whole 16-byte vectors, at most 512 of them."""
+    nbytes = t.shape[-1] * t.element_size() if t.dim() else 0
+    return nbytes % 16 == 0 and nbytes <= 512 * 16
+
+
+class _RMSNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        ctx.save_for_backward(x, weight)
+        ctx.eps = eps
+        return rmsnorm(x, weight, eps)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight = ctx.saved_tensors
+        if not torch.is_grad_enabled() and _plain(x, weight, dy.contiguous()):
+            return (*rmsnorm_bwd(x, weight, dy.contiguous(), ctx.eps), None)
+        # a graph of the gradient is wanted (or a transform is active): the same formula in torch operations
+        xf, wf, g = x.float(), weight.float(), dy.float()
+        rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + ctx.eps)
+        xh, gw = xf * rstd, g * wf
+        dx = rstd * (gw - xh * (gw * xh).mean(-1, keepdim=True))
+        return dx.to(x.dtype), (g * xh).sum(dim=tuple(range(x.dim() - 1))).to(weight.dtype), None
+
+
+def rmsnorm_train(x, weight, eps):
+    """Differentiable `x * rsqrt(mean(x^2) + eps) * weight` over the last dimension, in fp32, rounded once: one
+    kernel forward and two backward where the kernels apply, torch operations everywhere else."""
+    if _plain(x, weight) and _rows_fit(x) and x.dim() > 0 and weight.shape == x.shape[-1:]:
+        return _RMSNorm.apply(x, weight, eps)
+    xf = x.float()
+    return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * weight.float()).to(x.dtype)
+
+
+class _SwiGLU(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, gate, up):
+        ctx.save_for_backward(gate, up)
+        w = gate.shape[-1]
+        return silu_mul(gate.view(-1, w), up.view(-1, w), torch.empty_like(gate).view(-1, w)).view(gate.shape)
+
+    @staticmethod
+    def backward(ctx, dout):
+        gate, up = ctx.saved_tensors
+        if not torch.is_grad_enabled() and _plain(gate, up, dout.contiguous()):
+            w = gate.shape[-1]
+            dgate, dup = silu_mul_bwd(gate.view(-1, w), up.view(-1, w), dout.contiguous().view(-1, w))
+            return dgate.view(gate.shape), dup.view(gate.shape)
+        gf, d = gate.float(), dout.float()
+        s = torch.sigmoid(gf)
+        return (d * up.float() * (s * (1 + gf * (1 - s)))).to(gate.dtype), (d * (gf * s)).to(up.dtype)
+
+
+def swiglu(gate, up):
+    """Differentiable silu(gate) * up: one kernel each way where the kernels apply, torch operations elsewhere."""
+    if _plain(gate, up) and gate.shape == up.shape and gate.dim() > 0 and gate.shape[-1] * gate.element_size() % 16 == 0:
+        return _SwiGLU.apply(gate, up)
+    return torch.nn.functional.silu(gate) * up
 
 
 @functools.lru_cache(maxsize=None)
