@@ -116,6 +116,8 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* s
 // All 256 softmax threads; only called outside data-dependent control flow.
 __device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
+__device__ __forceinline__ float2 as_float2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
+
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -590,6 +592,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
 
     // sm_scale is folded into the exponent: the loop works with P' = sm_scale * P, so dS = P' (dP - delta)
     const float lscale = log2f(p.sm_scale);
+    const float2 neg_delta = make_float2(-delta_i, -delta_i);
     // The gathered channel scores (fp16, dense tiles) and their exponentials (light tiles) wait in this
     // thread's lane of the dP columns, which no MMA touches before the first dense tile.
     __half2 cbl[NCH / 2];
@@ -628,6 +631,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
       const bool dense = is_dense(s);
       const int J = tile_of(s);
       float offs[TPW], wmul[TPW], dtb_acc[TPW];
+      float2 dtb2[TPW];
       int slot[TPW];
       bool valid[TPW];
 #pragma unroll
@@ -636,7 +640,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         valid[tl] = dt >= 0 && tk_abs < T && row_valid;
         slot[tl] = T - 1 - min(max(dt, 0), T - 1);
         wmul[tl] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
-        dtb_acc[tl] = 0.f;
+        dtb2[tl] = make_float2(0.f, 0.f);
         offs[tl] = valid[tl] ? tb_next[tl] + off_row + lscale : -INFINITY;
       }
       if (s + 1 < n_tiles) {
@@ -664,27 +668,29 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
           for (int jj = 0; jj < 32; jj += 2) {
             const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
             const float2 cb = __half22float2(cbl[k / 2]);
-            const float p0 = ex2(fmaf(__uint_as_float(sv[jj]), wmul[tl], cb.x) + offs[tl]);
-            const float p1 = ex2(fmaf(__uint_as_float(sv[jj + 1]), wmul[tl], cb.y) + offs[tl]);
-            const float ds0 = p0 * (__uint_as_float(dp[jj]) - delta_i);
-            const float ds1 = p1 * (__uint_as_float(dp[jj + 1]) - delta_i);
-            dcb_acc[k] += ds0;
-            dcb_acc[k + 1] += ds1;
-            dtb_acc[tl] += ds0 + ds1;
-            const uint32_t both = pack_bf16(ds0, ds1);
+            const float2 x = fadd2(ffma2(as_float2(sv[jj], sv[jj + 1]), make_float2(wmul[tl], wmul[tl]), cb),
+                                   make_float2(offs[tl], offs[tl]));
+            const float2 ds = fmul2(make_float2(ex2(x.x), ex2(x.y)), fadd2(as_float2(dp[jj], dp[jj + 1]), neg_delta));
+            const float2 ca = fadd2(make_float2(dcb_acc[k], dcb_acc[k + 1]), ds);
+            dcb_acc[k] = ca.x;
+            dcb_acc[k + 1] = ca.y;
+            dtb2[tl] = fadd2(dtb2[tl], ds);
+            const uint32_t both = pack_bf16(ds.x, ds.y);
             pk[jj / 2] = wmul[tl] != 0.f ? both : 0u;  // content term only inside the window
           }
           tmem_st16(s_addr + 16 * half, pk);  // dS_w over this thread's consumed S columns
         }
         tmem_st_wait();
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl) dtb_acc[tl] = dtb2[tl].x + dtb2[tl].y;
       } else {
-        float a[TPW], w0[TPW], w1[TPW];
+        float a[TPW];
+        float2 w2[TPW];
 #pragma unroll
         for (int tl = 0; tl < TPW; ++tl) {
           a[tl] = ex2(offs[tl]);  // 0 where the time step is not visible
           a_sum += a[tl];
-          w0[tl] = 0.f;
-          w1[tl] = 0.f;
+          w2[tl] = make_float2(0.f, 0.f);
         }
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -694,15 +700,15 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
 #pragma unroll
           for (int jj = 0; jj < 32; jj += 2) {
             const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
-            const float d0 = __uint_as_float(dp[jj]), d1 = __uint_as_float(dp[jj + 1]);
-            dcb_acc[k] = fmaf(a[tl], d0, dcb_acc[k]);
-            dcb_acc[k + 1] = fmaf(a[tl], d1, dcb_acc[k + 1]);
-            w0[tl] = fmaf(bcf[k], d0, w0[tl]);
-            w1[tl] = fmaf(bcf[k + 1], d1, w1[tl]);
+            const float2 d = as_float2(dp[jj], dp[jj + 1]);
+            const float2 ca = ffma2(make_float2(a[tl], a[tl]), d, make_float2(dcb_acc[k], dcb_acc[k + 1]));
+            dcb_acc[k] = ca.x;
+            dcb_acc[k + 1] = ca.y;
+            w2[tl] = ffma2(make_float2(bcf[k], bcf[k + 1]), d, w2[tl]);
           }
         }
 #pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) dtb_acc[tl] = a[tl] * (w0[tl] + w1[tl] - delta_i * bc_sum);
+        for (int tl = 0; tl < TPW; ++tl) dtb_acc[tl] = a[tl] * (w2[tl].x + w2[tl].y - delta_i * bc_sum);
         if (s == n_light - 1) {
           // transition: scale the light phase's inner sums, then fetch the scores the dense tiles need
           // (before the report below lets the first dense dP product overwrite where they wait)
@@ -943,7 +949,10 @@ struct BkArgs {
   int* status;
 };
 enum BkBarrier {
-  kKvFull = 0, kQdoFull, kQdoFull1, kBkSdpFull, kPdsFull, kPairDone, kBkAllDone,
+  kKvFull = 0, kBkAllDone,
+  kQFull, kQFull1, kDoFull, kDoFull1,    // dense pairs: Q' / dO loaded, by buffer
+  kSFull, kDpFull, kPFull, kDsFull,      // ... S / dP in TMEM, P / dS_w in shared memory (S / dP consumed)
+  kDvDone, kDvDone1, kDkDone, kDkDone1,  // ... dV / dK product of the pair complete, by pair parity
   kLdoFull, kLdoFull1, kLdoFull2, kLdoFull3, kLdoFree, kLdoFree1, kLdoFree2, kLdoFree3,  // light pairs: four dO buffers
   kLpFull, kLpFull1, kLFree, kLFree1,                                                      // ... and two P buffers
   kBkBars
@@ -954,11 +963,13 @@ struct BkCfg {
   static constexpr int TILE = (D / 64) * 16384;
   static constexpr int SMEM_K = 0, SMEM_V = TILE, SMEM_Q = 2 * TILE, SMEM_DO = 3 * TILE;
   static constexpr int SMEM_P = 4 * TILE, SMEM_DS = 4 * TILE + 32768;
-  // head_dim 64 has room for a second Q' / dO pair: the loads of the next dense pair and its S / dP
-  // products then overlap the softmax work and the dV / dK products of the current one
-  static constexpr int NSET = D == 64 ? 2 : 1;
-  static constexpr int SMEM_QDO1 = 4 * TILE + 65536;
-  static constexpr int SMEM_TAIL = SMEM_QDO1 + (NSET - 1) * 2 * TILE;
+  // Two Q' buffers: the score product of the next dense pair runs while the softmax warps work on this one.
+  // head_dim 64 has room for a second dO buffer as well; at 128 the next dO is loaded as soon as the
+  // dV product has left the buffer, under the dK product and the next pair's probabilities.
+  static constexpr int ND = D == 64 ? 2 : 1;
+  static constexpr int SMEM_Q1 = 4 * TILE + 65536;
+  static constexpr int SMEM_DO1 = SMEM_Q1 + TILE;
+  static constexpr int SMEM_TAIL = SMEM_Q1 + ND * TILE;
   static constexpr int SMEM_BYTES = SMEM_TAIL + kBkBars * 8 + 16 + 1024;
 };
 
@@ -980,9 +991,9 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
   uint8_t* sV = smem + C_::SMEM_V;
   uint8_t* sQ = smem + C_::SMEM_Q;
   uint8_t* sDO = smem + C_::SMEM_DO;
-  constexpr int NSET = C_::NSET;
-  uint8_t* sQ1 = smem + C_::SMEM_QDO1;  // second set (head_dim 64 only)
-  uint8_t* sDO1 = sQ1 + TILE;
+  constexpr int ND = C_::ND;
+  uint8_t* sQ1 = smem + C_::SMEM_Q1;
+  uint8_t* sDO1 = smem + C_::SMEM_DO1;  // (head_dim 64 only)
   uint8_t* sP = smem + C_::SMEM_P;
   uint8_t* sDS = smem + C_::SMEM_DS;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C_::SMEM_TAIL);
@@ -1021,12 +1032,17 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
   // earlier CTA may have given up), warp 9 allocates the tensor memory - all at the same time.
   if (tid == 0) {
     mbar_init(&bars[kKvFull], 1);
-    mbar_init(&bars[kQdoFull], 1);
-    mbar_init(&bars[kQdoFull + 1], 1);
-    mbar_init(&bars[kBkSdpFull], 1);
-    mbar_init(&bars[kPdsFull], kSoftmaxThreads);
-    mbar_init(&bars[kPairDone], 1);
     mbar_init(&bars[kBkAllDone], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars[kQFull + i], 1);
+      mbar_init(&bars[kDoFull + i], 1);
+      mbar_init(&bars[kDvDone + i], 1);
+      mbar_init(&bars[kDkDone + i], 1);
+    }
+    mbar_init(&bars[kSFull], 1);
+    mbar_init(&bars[kDpFull], 1);
+    mbar_init(&bars[kPFull], kSoftmaxThreads);
+    mbar_init(&bars[kDsFull], kSoftmaxThreads);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars[kLdoFull + i], 1);
       mbar_init(&bars[kLdoFree + i], 1);
@@ -1064,26 +1080,26 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
         tma_load_5d(sV + hh * HALF, &maps.v, &bars[kKvFull], hh * 64, 0, J * TPB, hk, b);
       }
       bool ok = true;
+      // (every wait below is for the latest phase its barrier can have reached: a buffer's next use cannot
+      // complete before the load issued here)
       for (int s = 0; ok && s < n_dense; ++s) {
         int h, i;
         dense_pair(s, h, i);
-        const int set = s % NSET;
-        if (s >= NSET) ok = mbar_wait(&bars[kPairDone], (s - NSET) & 1, p.status, 210);  // the set's buffers are free
+        const int qs = s & 1, ds = s % ND;
+        if (s >= 2) ok = mbar_wait(&bars[kDkDone + qs], ((s >> 1) - 1) & 1, p.status, 210);  // Q' buffer free
         if (!ok) break;
-        uint8_t* dq_ = set == 0 ? sQ : sQ1;
-        uint8_t* ddo_ = set == 0 ? sDO : sDO1;
-        mbar_arrive_expect_tx(&bars[kQdoFull + set], 2 * TILE);
-        for (int hh = 0; hh < NH; ++hh) {
-          tma_load_5d(dq_ + hh * HALF, &maps.qp, &bars[kQdoFull + set], hh * 64, 0, i * TPB, h, b);
-          tma_load_5d(ddo_ + hh * HALF, &maps.dout, &bars[kQdoFull + set], hh * 64, 0, i * TPB, h, b);
-        }
+        uint8_t* dq_ = qs == 0 ? sQ : sQ1;
+        mbar_arrive_expect_tx(&bars[kQFull + qs], TILE);
+        for (int hh = 0; hh < NH; ++hh) tma_load_5d(dq_ + hh * HALF, &maps.qp, &bars[kQFull + qs], hh * 64, 0, i * TPB, h, b);
+        if (s >= ND) ok = mbar_wait(&bars[kDvDone + ((s - ND) & 1)], ((s - ND) >> 1) & 1, p.status, 211);  // dO buffer free
+        if (!ok) break;
+        uint8_t* ddo_ = ds == 0 ? sDO : sDO1;
+        mbar_arrive_expect_tx(&bars[kDoFull + ds], TILE);
+        for (int hh = 0; hh < NH; ++hh) tma_load_5d(ddo_ + hh * HALF, &maps.dout, &bars[kDoFull + ds], hh * 64, 0, i * TPB, h, b);
       }
-      // light pairs: dO only, alternately into the dO and the (now idle) Q' area
-      // (a parity wait can only tell the current phase from the one before it: the phases are waited for
-      // one by one, none skipped)
-      if (ok && n_light > 0 && NSET == 2 && n_dense >= 2)
-        ok = mbar_wait(&bars[kPairDone], (n_dense - 2) & 1, p.status, 211);
-      if (ok && n_light > 0) ok = mbar_wait(&bars[kPairDone], (n_dense - 1) & 1, p.status, 211);
+      // light pairs reuse the dense pairs' buffers: every dense product has to be complete (the last dK is
+      // issued after the last dV and after all earlier products)
+      if (ok && n_light > 0) ok = mbar_wait(&bars[kDkDone + ((n_dense - 1) & 1)], ((n_dense - 1) >> 1) & 1, p.status, 213);
       // Four dO buffers in the light phase: the dO, Q', K and V areas (K and V are dead once the dense pairs
       // are done).  The loads run far enough ahead to cover the TMA latency.
       for (int l = 0; ok && l < n_light; ++l) {
@@ -1114,47 +1130,65 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
       const DescHalves dpm = make_desc_halves_sw128(smem_u32(sP), HALF, 1024);
       const DescHalves ddsm = make_desc_halves_sw128(smem_u32(sDS), HALF, 1024);
       bool ok = __all_sync(kFull, mbar_wait(&bars[kKvFull], 0, p.status, 220));
-      const uint32_t set1 = (uint32_t)(C_::SMEM_QDO1 - C_::SMEM_Q) >> 4;  // descriptor distance to the second set
-      auto issue_sdp = [&](int s) {  // S = Q' K^T, dP = dO V^T of dense pair s
-        const int set = s % NSET;
-        ok = __all_sync(kFull, mbar_wait(&bars[kQdoFull + set], (s / NSET) & 1, p.status, 221));
+      constexpr uint32_t q1 = (uint32_t)(C_::SMEM_Q1 - C_::SMEM_Q) >> 4;     // descriptor distance to the second
+      constexpr uint32_t do1 = (uint32_t)(C_::SMEM_DO1 - C_::SMEM_DO) >> 4;  // Q' / dO buffer
+      auto issue_s = [&](int s) {  // S = Q' K^T of dense pair s
+        ok = __all_sync(kFull, mbar_wait(&bars[kQFull + (s & 1)], (s >> 1) & 1, p.status, 221));
         if (!ok) return;
         tc_fence_after();
-        DescHalves a_q = dqk, a_do = ddok;
-        a_q.lo += set * set1;
-        a_do.lo += set * set1;
+        DescHalves a_q = dqk;
+        a_q.lo += (uint32_t)(s & 1) * q1;
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk) {
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           mma_ss_w(el, tm + kColS, a_q, off, dk, off, idesc_s, kk > 0);
         }
+        mma_commit_w(el, smem_u32(&bars[kSFull]));
+      };
+      auto issue_dp = [&](int s) {  // dP = dO V^T
+        ok = __all_sync(kFull, mbar_wait(&bars[kDoFull + s % ND], (s / ND) & 1, p.status, 225));
+        if (!ok) return;
+        tc_fence_after();
+        DescHalves a_do = ddok;
+        a_do.lo += (uint32_t)(s % ND) * do1;
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk) {
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           mma_ss_w(el, tm + kColDP, a_do, off, dv, off, idesc_s, kk > 0);
         }
-        mma_commit_w(el, smem_u32(&bars[kBkSdpFull]));
+        mma_commit_w(el, smem_u32(&bars[kDpFull]));
       };
-      if (ok && n_dense > 0) issue_sdp(0);
+      // Two hand-offs per pair.  Once P is in shared memory (and S consumed): dV and the next pair's S.  Once dS_w is
+      // there (and dP consumed): dK and the next pair's dP.  The softmax warps form the next P from S while dP is
+      // still on its way.  With one dO buffer dV goes first, because the next dO is loaded into the buffer it leaves,
+      // and dK runs under that load; with two the products that the softmax warps wait for go first.
+      if (ok && n_dense > 0) issue_s(0);
+      if (ok && n_dense > 0) issue_dp(0);
       for (int s = 0; ok && s < n_dense; ++s) {
-        const int set = s % NSET;
-        ok = __all_sync(kFull, mbar_wait(&bars[kPdsFull], s & 1, p.status, 222));  // P / dS_w are in shared memory, S / dP consumed
+        const bool next = s + 1 < n_dense;
+        ok = __all_sync(kFull, mbar_wait(&bars[kPFull], s & 1, p.status, 222));
         if (!ok) break;
         tc_fence_after();
-        // with a second buffer set the next pair's S / dP go first: the softmax warps wait for them
-        if (NSET == 2 && s + 1 < n_dense) issue_sdp(s + 1);
+        if (ND == 2 && next) issue_s(s + 1);
         if (!ok) break;
         DescHalves b_do = ddom, b_q = dqm;
-        b_do.lo += set * set1;
-        b_q.lo += set * set1;
+        b_do.lo += (uint32_t)(s % ND) * do1;
+        b_q.lo += (uint32_t)(s & 1) * q1;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dV += P^T dO   (K = 128 query rows, 16 per step)
           mma_ss_w(el, tm + kColDV, dpm, kk * 2048, b_do, kk * 2048, idesc_g, (s > 0 || kk > 0));
+        mma_commit_w(el, smem_u32(&bars[kDvDone + (s & 1)]));
+        if (ND == 1 && next) issue_s(s + 1);
+        if (ok) ok = __all_sync(kFull, mbar_wait(&bars[kDsFull], s & 1, p.status, 226));
+        if (!ok) break;
+        tc_fence_after();
+        if (ND == 2 && next) issue_dp(s + 1);
+        if (!ok) break;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dK += dS_w^T Q'
           mma_ss_w(el, tm + kColDK, ddsm, kk * 2048, b_q, kk * 2048, idesc_g, (s > 0 || kk > 0));
-        mma_commit_w(el, smem_u32(&bars[kPairDone]));
-        if (NSET == 1 && s + 1 < n_dense) issue_sdp(s + 1);
+        mma_commit_w(el, smem_u32(&bars[kDkDone + (s & 1)]));
+        if (ND == 1 && next) issue_dp(s + 1);
       }
       const DescHalves dkm = make_desc_halves_sw128(smem_u32(sK), HALF, 1024);  // K / V areas as dO buffers
       const DescHalves dvm = make_desc_halves_sw128(smem_u32(sV), HALF, 1024);
@@ -1183,32 +1217,42 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
     const int tt_base = (64 * wg) / CP;
     const int ck_base = CP == 128 ? 64 * wg : 0;
     bool ok = true;
+    // Per-row quantities of a query tile, from the query-side kernel's workspace.  Those of pair s+1 are requested
+    // as soon as pair s has formed its P (the channel scores are dead then), under its dS phase.
+    __half2 cbl[NCH / 2];
+    float off_row, delta_next, tb_row[TPW];
+    auto fetch_row = [&](int s) {
+      int h, i;
+      dense_pair(s, h, i);
+      const int ti_abs = i * TPB + ti_loc;
+      const bool row_valid = c_i < C && ti_abs < T;
+      const int N = T * C, n_loc = row_valid ? ti_abs * C + c_i : 0;
+      const int64_t bhq = (int64_t)b * p.H + h;
+      const uint4* src = reinterpret_cast<const uint4*>(p.cblw) + (bhq * (CP / 8) + ck_base / 8) * N + n_loc;
+#pragma unroll
+      for (int m = 0; m < NCH / 8; ++m) {
+        const uint4 w = src[(int64_t)m * N];
+        *reinterpret_cast<uint32_t*>(&cbl[4 * m]) = w.x;
+        *reinterpret_cast<uint32_t*>(&cbl[4 * m + 1]) = w.y;
+        *reinterpret_cast<uint32_t*>(&cbl[4 * m + 2]) = w.z;
+        *reinterpret_cast<uint32_t*>(&cbl[4 * m + 3]) = w.w;
+      }
+      off_row = p.offw[bhq * N + n_loc];
+      delta_next = p.delta[bhq * N + n_loc];
+#pragma unroll
+      for (int tl = 0; tl < TPW; ++tl) {
+        const int dt = min(max(ti_abs - (J * TPB + tt_base + tl), 0), T - 1);
+        tb_row[tl] = row_valid ? p.tbw[(bhq * T + (T - 1 - dt)) * N + n_loc] : 0.f;
+      }
+    };
+    fetch_row(0);
     for (int s = 0; ok && s < n_dense; ++s) {
       int h, i;
       dense_pair(s, h, i);
       const int ti_abs = i * TPB + ti_loc;
       const bool row_valid = c_i < C && ti_abs < T;
-      const int N = T * C, n_loc = ti_abs * C + c_i;
-      const int64_t bhq = (int64_t)b * p.H + h, n_row = bhq * N + n_loc;
-      // per-row quantities of this query tile, from the query-side kernel's workspace
-      __half2 cbl[NCH / 2];
-      float off_row = -INFINITY, delta_i = 0.f;
-      if (row_valid) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.cblw) + (bhq * (CP / 8) + ck_base / 8) * N + n_loc;
-#pragma unroll
-        for (int m = 0; m < NCH / 8; ++m) {
-          const uint4 w = src[(int64_t)m * N];
-          *reinterpret_cast<uint32_t*>(&cbl[4 * m]) = w.x;
-          *reinterpret_cast<uint32_t*>(&cbl[4 * m + 1]) = w.y;
-          *reinterpret_cast<uint32_t*>(&cbl[4 * m + 2]) = w.z;
-          *reinterpret_cast<uint32_t*>(&cbl[4 * m + 3]) = w.w;
-        }
-        off_row = p.offw[n_row];
-        delta_i = p.delta[n_row];
-      } else {
-#pragma unroll
-        for (int k2 = 0; k2 < NCH / 2; ++k2) cbl[k2] = __floats2half2_rn(0.f, 0.f);
-      }
+      const float delta_i = row_valid ? delta_next : 0.f;
+      const float2 neg_delta = make_float2(-delta_i, -delta_i);
       float offs[TPW], wmul[TPW], scw[TPW];
 #pragma unroll
       for (int tl = 0; tl < TPW; ++tl) {
@@ -1216,54 +1260,77 @@ tc_bwd_kv_kernel(const __grid_constant__ BkMaps maps, const BkArgs p) {
         const bool valid = dt >= 0 && tk_abs < T && row_valid;
         wmul[tl] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
         scw[tl] = wmul[tl] * p.sm_scale;  // dS_w = P (dP - delta) sm_scale inside the window, 0 outside
-        offs[tl] = valid ? p.tbw[(bhq * T + (T - 1 - dt)) * N + n_loc] + off_row : -INFINITY;
+        offs[tl] = valid ? tb_row[tl] + off_row : -INFINITY;
       }
-      ok = warp_wait(&bars[kBkSdpFull], s & 1, p.status, 232);
+      // P = exp2(S2 - L) of this thread's 64 keys, from S alone
+      ok = warp_wait(&bars[kSFull], s & 1, p.status, 232);
       if (!ok) break;
       tc_fence_after();
+      float pr[64];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        uint32_t sv[32], dp[32];
+        uint32_t sv[32];
         tmem_ld32(lane_base + kColS + 64 * wg + 32 * half, sv);
-        tmem_ld32(lane_base + kColDP + 64 * wg + 32 * half, dp);
         tmem_ld_wait();
-        uint32_t pp[16], pd[16];
 #pragma unroll
         for (int jj = 0; jj < 32; jj += 2) {
           const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
           const float2 cb = __half22float2(cbl[k / 2]);
-          const float s0 = fmaf(__uint_as_float(sv[jj]), wmul[tl], cb.x);
-          const float s1 = fmaf(__uint_as_float(sv[jj + 1]), wmul[tl], cb.y);
-          const float p0 = ex2(s0 + offs[tl]), p1 = ex2(s1 + offs[tl]);
-          const float ds0 = p0 * (__uint_as_float(dp[jj]) - delta_i) * scw[tl];
-          const float ds1 = p1 * (__uint_as_float(dp[jj + 1]) - delta_i) * scw[tl];
-          pp[jj / 2] = pack_bf16(p0, p1);
-          pd[jj / 2] = pack_bf16(ds0, ds1);
+          const float2 x = fadd2(ffma2(as_float2(sv[jj], sv[jj + 1]), make_float2(wmul[tl], wmul[tl]), cb),
+                                 make_float2(offs[tl], offs[tl]));
+          pr[lc] = ex2(x.x);
+          pr[lc + 1] = ex2(x.y);
         }
-        // (with two buffer sets these warps run ahead of the previous pair's dV / dK products, which
-        // still read the P / dS areas)
-        if (NSET == 2 && half == 0 && s > 0) {
-          ok = warp_wait(&bars[kPairDone], (s - 1) & 1, p.status, 233);
-          if (!ok) break;
+      }
+      // MN-major operand layout: 64-key block = this warpgroup, one 128-byte row per query row,
+      // 16-byte chunks swizzled by (row mod 8).  The previous pair's dV product has to have left the area.
+      if (s > 0) {
+        ok = warp_wait(&bars[kDvDone + ((s - 1) & 1)], ((s - 1) >> 1) & 1, p.status, 233);
+        if (!ok) break;
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t o = wg * HALF + row * 128 + ((c ^ (row & 7)) << 4);
+        *reinterpret_cast<uint4*>(sP + o) = make_uint4(pack_bf16(pr[8 * c], pr[8 * c + 1]), pack_bf16(pr[8 * c + 2], pr[8 * c + 3]),
+                                                       pack_bf16(pr[8 * c + 4], pr[8 * c + 5]), pack_bf16(pr[8 * c + 6], pr[8 * c + 7]));
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      mbar_arrive(&bars[kPFull]);
+      if (s + 1 < n_dense) fetch_row(s + 1);
+      // dS_w = P (dP - delta) sm_scale inside the window
+      ok = warp_wait(&bars[kDpFull], s & 1, p.status, 237);
+      if (ok && s > 0) ok = warp_wait(&bars[kDkDone + ((s - 1) & 1)], ((s - 1) >> 1) & 1, p.status, 238);  // the dS area is free
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t dp[32];
+        tmem_ld32(lane_base + kColDP + 64 * wg + 32 * half, dp);
+        tmem_ld_wait();
+        uint32_t pd[16];
+#pragma unroll
+        for (int jj = 0; jj < 32; jj += 2) {
+          const int lc = 32 * half + jj, tl = lc / CP;
+          const float2 ds = fmul2(fmul2(make_float2(pr[lc], pr[lc + 1]), fadd2(as_float2(dp[jj], dp[jj + 1]), neg_delta)),
+                                  make_float2(scw[tl], scw[tl]));
+          pd[jj / 2] = pack_bf16(ds.x, ds.y);
         }
-        // MN-major operand layout: 64-key block = this warpgroup, one 128-byte row per query row,
-        // 16-byte chunks swizzled by (row mod 8)
 #pragma unroll
         for (int c4 = 0; c4 < 4; ++c4) {
           const int c = 4 * half + c4;
           const uint32_t o = wg * HALF + row * 128 + ((c ^ (row & 7)) << 4);
-          *reinterpret_cast<uint4*>(sP + o) = make_uint4(pp[4 * c4], pp[4 * c4 + 1], pp[4 * c4 + 2], pp[4 * c4 + 3]);
           *reinterpret_cast<uint4*>(sDS + o) = make_uint4(pd[4 * c4], pd[4 * c4 + 1], pd[4 * c4 + 2], pd[4 * c4 + 3]);
         }
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(&bars[kPdsFull]);
+      mbar_arrive(&bars[kDsFull]);
     }
     // ---- light pairs: P[i, k] = a_i[t_k] bc_i[c_k] straight into the operand layout ----
     // The row's data of pair l+1 is requested while pair l is processed: with nothing else to wait for,
     // the latency of these loads would otherwise be the whole cost of a light pair.
-    if (ok && n_light > 0) ok = warp_wait(&bars[kPairDone], (n_dense - 1) & 1, p.status, 235);  // P / dS areas are free
+    if (ok && n_light > 0) ok = warp_wait(&bars[kDkDone + ((n_dense - 1) & 1)], ((n_dense - 1) >> 1) & 1, p.status, 235);  // P / dS areas are free
     // Two register stages: the row's data of pair l+2 is requested while pair l is processed (one pair
     // ahead does not cover the latency of these loads once a pair takes about a thousand cycles).
     struct RowData {

@@ -45,3 +45,12 @@ def test_cuda_core_tiles_thirty_two_rows(cuda, shape):
 @pytest.mark.parametrize("shape", [(1, 1, 1, 2, 400, 64), (1, 1, 1, 300, 2, 128), (1, 2, 1, 2, 440, 32)])
 def test_cuda_core_long_axes(cuda, shape):
     _check(cuda, random_case(sum(shape), *shape), torch.float32)
+
+
+# key-side tensor-core pipeline: one, two and three dense pairs, then the first light pairs, one and two heads a
+# group, both head_dims and each number of channel slots
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 100, 128), (1, 2, 1, 2, 128, 128), (1, 1, 1, 3, 70, 128), (1, 2, 1, 13, 65, 128),
+                                   (1, 2, 1, 27, 33, 128), (1, 1, 1, 45, 20, 128), (1, 1, 1, 2, 100, 64), (1, 2, 1, 14, 100, 64),
+                                   (1, 2, 1, 27, 50, 64), (1, 1, 1, 49, 32, 64)])
+def test_key_side_pipeline_bf16(cuda, shape):
+    _check(cuda, random_case(sum(shape), *shape, scale=0.5), torch.bfloat16)
