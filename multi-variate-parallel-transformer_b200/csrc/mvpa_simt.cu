@@ -426,32 +426,6 @@ __global__ void __launch_bounds__(32 * WPG * NG) simt_fwd_kernel(Args p) {
 
 // ------------------------------- backward ------------------------------------
 
-// delta[bh][i] = sum_d dO[i][d] * O[i][d]   (`attentions/attn.py:1213`).  HBM-bound: a thread reads 16
-// bytes of each tensor at a time, D / VEC threads share a row (VEC = elements per 16 bytes) and
-// combine with shuffles; D is a power of two >= 16, so a row never straddles warps.
-template <typename Tin, int D>
-__global__ void __launch_bounds__(kThreads) simt_delta_kernel(BwdArgs bw) {
-  constexpr int VEC = 16 / sizeof(Tin), TPR = D / VEC;  // threads per row: 4 .. 32
-  const Args& p = bw.a;
-  const int gid = blockIdx.x * kThreads + threadIdx.x;
-  const int rowi = gid / TPR, part = gid % TPR;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
-  float acc = 0.f;
-  if (rowi < p.N) {
-    const Tin* o = (const Tin*)p.o + b * p.o_sb + h * p.o_sh + (int64_t)rowi * p.o_sn + part * VEC;
-    const Tin* g = (const Tin*)bw.d_o + b * bw.do_sb + h * bw.do_sh + (int64_t)rowi * bw.do_sn + part * VEC;
-    const uint4 ov = *reinterpret_cast<const uint4*>(o), gv = *reinterpret_cast<const uint4*>(g);
-    const Tin* oe = reinterpret_cast<const Tin*>(&ov);
-    const Tin* ge = reinterpret_cast<const Tin*>(&gv);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) acc += to_f32<Tin>(oe[e]) * to_f32<Tin>(ge[e]);
-  }
-#pragma unroll
-  for (int s = TPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (part == 0 && rowi < p.N) bw.delta[(int64_t)bh * p.N + rowi] = acc;
-}
-
-
 // Query side: one CTA per (BM query rows, b, h); the groups share the causal key tiles.  Recomputes
 // P = exp2(S2 - L), forms dS, accumulates the content part of dQ and the per-row sums of dS by time slot and
 // by key channel, then finishes dq = dS_w K + dTB r_time + dCB r_chan.  On the way it leaves behind what the
@@ -1102,10 +1076,6 @@ int launch_bwd(const BwdArgs& b, cudaStream_t s) {
   if (b.tc_extra != nullptr) {
     // bf16 on the tensor cores: dq, dk, dv and the relative-key gradients
     if constexpr (sizeof(Tin) == 2 && D >= 64) {
-      constexpr int kRowThreads = D / (16 / (int)sizeof(Tin));
-      dim3 grid((a.N * kRowThreads + kThreads - 1) / kThreads, a.B * a.H);
-      simt_delta_kernel<Tin, D><<<grid, kThreads, 0, s>>>(b);
-      count_launch();
       int rc = tc_bwd_q(b, b.tc_extra, s);
       if (rc) return rc;
       return tc_bwd_bias(b, b.tc_extra, s);
@@ -1194,14 +1164,17 @@ bool tc_path(int dtype, int D, int C, int T) {
   return dtype == MVPA_BF16 && tc_bwd_q_supported(a);
 }
 bool tc_needs_dtb(int D, int C) { return !(D == 64 && C <= 64); }
+size_t round4(size_t n) { return (n + 3) & ~(size_t)3; }
+// delta and, behind it on a 16-byte boundary, the temporal-score gradients
+size_t tc_head_floats(size_t rows, int D, int C, int T) {
+  return (round4(rows) + (tc_needs_dtb(D, C) ? rows * T : 0) + 63) & ~(size_t)63;
+}
 }  // namespace
 
 size_t simt_bwd_workspace_floats(const mvpa_problem* p) {
   const size_t BH = (size_t)p->B * p->H, N = (size_t)p->T * p->C;
   if (tc_path(p->dtype, p->D, p->C, p->T)) {
-    size_t n = BH * N + (tc_needs_dtb(p->D, p->C) ? BH * N * p->T : 0);
-    n = (n + 63) & ~(size_t)63;
-    return n + tc_bwd_q_workspace_floats(p);
+    return tc_head_floats(BH * N, p->D, p->C, p->T) + tc_bwd_q_workspace_floats(p);
   }
   const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most
   size_t n = 2 * BH * N * (p->T + p->C) + BH * N + BH * n_qt * 3 * p->D;
@@ -1212,9 +1185,8 @@ size_t simt_bwd_workspace_floats(const mvpa_problem* p) {
 const int* bwd_status_word(const mvpa_problem* p, const void* workspace) {
   if (!tc_path(p->dtype, p->D, p->C, p->T)) return nullptr;  // the CUDA-core kernels have no device-side waits
   const size_t BH = (size_t)p->B * p->H, N = (size_t)p->T * p->C;
-  size_t used = BH * N + (tc_needs_dtb(p->D, p->C) ? BH * N * p->T : 0);
-  used = (used + 63) & ~(size_t)63;
-  return reinterpret_cast<const int*>(static_cast<const float*>(workspace) + used + tc_bwd_status_offset_floats(p));
+  return reinterpret_cast<const int*>(static_cast<const float*>(workspace) + tc_head_floats(BH * N, p->D, p->C, p->T) +
+                                      tc_bwd_status_offset_floats(p));
 }
 
 void simt_bwd_carve(BwdArgs& b, float* ws, int dtype) {
@@ -1223,10 +1195,8 @@ void simt_bwd_carve(BwdArgs& b, float* ws, int dtype) {
   if (tc_path(dtype, a.D, a.C, a.T)) {
     b.tbg = b.cbg = b.dcbg = b.partial = b.drel_part = nullptr;
     b.delta = ws;
-    b.dtbg = ws + BH * N;  // (B*H, T, N) scratch of the tensor-core kernels, when they need it
-    size_t used = BH * N + (tc_needs_dtb(a.D, a.C) ? BH * N * a.T : 0);
-    used = (used + 63) & ~(size_t)63;
-    b.tc_extra = ws + used;
+    b.dtbg = ws + round4(BH * N);  // (B*H, T, N) scratch of the tensor-core kernels, when they need it
+    b.tc_extra = ws + tc_head_floats(BH * N, a.D, a.C, a.T);
     return;
   }
   const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most

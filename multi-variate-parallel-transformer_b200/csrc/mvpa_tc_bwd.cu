@@ -1527,33 +1527,59 @@ int make_maps(BqMaps& m, const BwdArgs& bw, int CP, const void* qp) {
   return MVPA_OK;
 }
 
-// du / dvt / dz of one kv head: du = sum of the query tiles' content column sums; dvt = (column sums
-// of dTB) r_time, dz = (column sums of dCB) r_chan (`_rel_bias` adds q_btime / q_bchan to every row, so
-// their gradients are the row sums of dq's temporal / channel parts).
-__global__ void __launch_bounds__(1024) tc_dbias_kernel(const float* __restrict__ cs_dq,
-                                                       const unsigned long long* __restrict__ cacc,
-                                                       const __nv_bfloat16* __restrict__ rt,
-                                                       const __nv_bfloat16* __restrict__ rc, float* __restrict__ du,
-                                                       float* __restrict__ dvt, float* __restrict__ dz, int B, int H,
-                                                       int g, int T, int C, int D, int n_qt) {
+// The last sums, in one launch of 1024-thread blocks.
+//   blocks [0, Hkv): du / dvt / dz of one kv head: du = sum of the query tiles' content column sums; dvt = (column
+//   sums of dTB) r_time, dz = (column sums of dCB) r_chan (`_rel_bias` adds q_btime / q_bchan to every row, so their
+//   gradients are the row sums of dq's temporal / channel parts).
+//   the others: dr_time / dr_chan from the accumulators of the query-side kernel, 32 columns of one kv head each:
+//     dr[j, d] = sum_i dX[i, j] (q[i, d] + bias[d]) = R'[j, d] / c2 + colsum[j] (bias[d] - u[d]),   Q' = (q + u) c2,
+//   transposed through shared memory (the accumulators have the slot innermost, the results the column).
+struct FinArgs {
+  const float* cs_dq;
+  const unsigned long long *racc, *cacc;
+  const __nv_bfloat16 *rt, *rc, *u, *vt, *z;
+  float *du, *dvt, *dz, *drt, *drc;
+  int B, H, Hkv, g, T, C, D, n_qt;
+  float inv_c2;
+};
+__global__ void __launch_bounds__(1024) tc_bwd_final_kernel(const FinArgs p) {
   __shared__ float s_cs[256];
   __shared__ float s_part[3][1024];
+  __shared__ float s_t[128][33];
+  const int T = p.T, C = p.C, D = p.D, tid = threadIdx.x;
+  if ((int)blockIdx.x >= p.Hkv) {
+    const int per = 2 * (D / 32), blk = (int)blockIdx.x - p.Hkv;
+    const int hk = blk / per, which = (blk % per) / (D / 32), d0 = (blk % (D / 32)) * 32, S = which == 0 ? T : C;
+    const unsigned long long* acc = p.racc + (((size_t)hk * 2 + which) * D + d0) * 128;
+    const unsigned long long* cs = p.cacc + ((size_t)hk * 2 + which) * 128;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int idx = i * 1024 + tid;
+      s_t[idx & 127][idx >> 7] = fix_read(acc[idx]);
+    }
+    __syncthreads();
+    const int d = tid & 31;
+    const float db = __bfloat162float((which == 0 ? p.vt : p.z)[(size_t)hk * D + d0 + d]) - __bfloat162float(p.u[(size_t)hk * D + d0 + d]);
+    float* out = (which == 0 ? p.drt : p.drc) + (size_t)hk * S * D + d0 + d;
+    for (int j = tid >> 5; j < S; j += 32) out[(size_t)j * D] = s_t[j][d] * p.inv_c2 + fix_read(cs[j]) * db;
+    return;
+  }
   const int hk = blockIdx.x;
-  if (threadIdx.x < 256) s_cs[threadIdx.x] = fix_read(cacc[(size_t)hk * 256 + threadIdx.x]);
+  if (tid < 256) s_cs[tid] = fix_read(p.cacc[(size_t)hk * 256 + tid]);
   __syncthreads();
-  const int d = threadIdx.x % D, part = threadIdx.x / D, parts = blockDim.x / D;
+  const int d = tid % D, part = tid / D, parts = 1024 / D;
   float su = 0.f, st = 0.f, sz = 0.f;
-  const int n_items = n_qt * B * g;
+  const int n_items = p.n_qt * p.B * p.g;
 #pragma unroll 8
   for (int it = part; it < n_items; it += parts) {  // (independent loads: eight in flight per thread)
-    const int tq = it / (B * g), b = (it / g) % B, hh = it % g;
-    su += cs_dq[((size_t)tq * B * H + (size_t)b * H + hk * g + hh) * D + d];
+    const int tq = it / (p.B * p.g), b = (it / p.g) % p.B, hh = it % p.g;
+    su += p.cs_dq[((size_t)tq * p.B * p.H + (size_t)b * p.H + hk * p.g + hh) * D + d];
   }
-  for (int j = part; j < T; j += parts) st += s_cs[j] * __bfloat162float(rt[((size_t)hk * T + j) * D + d]);
-  for (int j = part; j < C; j += parts) sz += s_cs[128 + j] * __bfloat162float(rc[((size_t)hk * C + j) * D + d]);
-  s_part[0][threadIdx.x] = su;
-  s_part[1][threadIdx.x] = st;
-  s_part[2][threadIdx.x] = sz;
+  for (int j = part; j < T; j += parts) st += s_cs[j] * __bfloat162float(p.rt[((size_t)hk * T + j) * D + d]);
+  for (int j = part; j < C; j += parts) sz += s_cs[128 + j] * __bfloat162float(p.rc[((size_t)hk * C + j) * D + d]);
+  s_part[0][tid] = su;
+  s_part[1][tid] = st;
+  s_part[2][tid] = sz;
   __syncthreads();
   if (part == 0) {
     for (int q = 1; q < parts; ++q) {
@@ -1561,30 +1587,60 @@ __global__ void __launch_bounds__(1024) tc_dbias_kernel(const float* __restrict_
       st += s_part[1][q * D + d];
       sz += s_part[2][q * D + d];
     }
-    du[hk * D + d] = su;
-    dvt[hk * D + d] = st;
-    dz[hk * D + d] = sz;
+    p.du[hk * D + d] = su;
+    p.dvt[hk * D + d] = st;
+    p.dz[hk * D + d] = sz;
   }
 }
 
-// dr_time / dr_chan from the accumulators of the query-side kernel:
-//   dr[j, d] = sum_i dX[i, j] (q[i, d] + bias[d]) = R'[j, d] / c2 + colsum[j] (bias[d] - u[d]),   Q' = (q + u) c2.
-__global__ void __launch_bounds__(256) tc_drel_final_kernel(const unsigned long long* __restrict__ racc,
-                                                            const unsigned long long* __restrict__ cacc,
-                                                            const __nv_bfloat16* __restrict__ u,
-                                                            const __nv_bfloat16* __restrict__ vt,
-                                                            const __nv_bfloat16* __restrict__ z, float* __restrict__ drt,
-                                                            float* __restrict__ drc, int T, int C, int D, float inv_c2) {
-  const int hk = blockIdx.x, which = blockIdx.y, S = which == 0 ? T : C;
-  const unsigned long long* acc = racc + ((size_t)hk * 2 + which) * D * 128;
-  const unsigned long long* cs = cacc + ((size_t)hk * 2 + which) * 128;
-  const __nv_bfloat16* bias = (which == 0 ? vt : z) + (size_t)hk * D;
-  float* out = (which == 0 ? drt : drc) + (size_t)hk * S * D;
-  for (int idx = threadIdx.x; idx < S * D; idx += blockDim.x) {
-    const int j = idx / D, d = idx % D;
-    out[idx] = fix_read(acc[(size_t)d * 128 + j]) * inv_c2 +
-               fix_read(cs[j]) * (__bfloat162float(bias[d]) - __bfloat162float(u[(size_t)hk * D + d]));
+// Everything the two main kernels need beforehand, in one launch:
+//   blocks [0, n_delta)           delta[bh][i] = sum_d dO[i][d] O[i][d]  (`attentions/attn.py:1213`), HBM-bound: D / 8
+//                                 threads share a row, one 16-byte load of each tensor per thread
+//   the next Hkv blocks           the relative-product constants of one kv head (rel_const_row)
+//   the remaining blocks          zeros: status words, relative-key accumulators, temporal-score gradients
+constexpr int kPreThreads = 256;
+struct PreArgs {
+  const __nv_bfloat16 *o, *d_o, *vt, *z, *rt, *rc;
+  int64_t o_sb, o_sh, o_sn, do_sb, do_sh, do_sn;
+  float *delta, *relc;
+  uint4* zero[3];
+  int64_t zero_n[3];  // 16-byte units
+  int BH, H, Hkv, N, T, C, n_delta;
+};
+template <int D>
+__global__ void __launch_bounds__(kPreThreads) tc_bwd_pre_kernel(const PreArgs p) {
+  constexpr int TPR = D / 8;  // threads per row: 8 or 16
+  if ((int)blockIdx.x < p.n_delta) {
+    const int64_t gid = (int64_t)blockIdx.x * kPreThreads + threadIdx.x, r = gid / TPR;
+    const int part = (int)(gid % TPR);
+    const bool in = r < (int64_t)p.BH * p.N;
+    float acc = 0.f;
+    if (in) {
+      const int bh = (int)(r / p.N), i = (int)(r - (int64_t)bh * p.N), b = bh / p.H, h = bh % p.H;
+      const uint4 ov = *reinterpret_cast<const uint4*>(p.o + b * p.o_sb + h * p.o_sh + (int64_t)i * p.o_sn + part * 8);
+      const uint4 gv = *reinterpret_cast<const uint4*>(p.d_o + b * p.do_sb + h * p.do_sh + (int64_t)i * p.do_sn + part * 8);
+      const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc += __uint_as_float(ow[e] << 16) * __uint_as_float(gw[e] << 16);
+        acc += __uint_as_float(ow[e] & 0xffff0000u) * __uint_as_float(gw[e] & 0xffff0000u);
+      }
+    }
+#pragma unroll
+    for (int s = TPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (in && part == 0) p.delta[r] = acc;
+    return;
   }
+  const int blk = (int)blockIdx.x - p.n_delta;
+  if (blk < p.Hkv) {
+    rel_const_row<D>(p.vt, p.z, p.rt, p.rc, p.relc, p.T, p.C, blk);
+    return;
+  }
+  const int64_t first = (int64_t)(blk - p.Hkv) * kPreThreads + threadIdx.x;
+  const int64_t step = ((int64_t)gridDim.x - p.n_delta - p.Hkv) * kPreThreads;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    for (int64_t i = first; i < p.zero_n[a]; i += step) p.zero[a][i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int D, int CP>
@@ -1616,12 +1672,26 @@ int launch(const BwdArgs& bw, float* cs_dq, int* status, float* relc, unsigned l
   static_assert(smem <= 232448, "shared memory budget");
   static_assert(Cfg<D>::EARLY >= 2, "the first tile's K and V load while the prologue runs");
   MVPA_CUDA_CHECK(cudaFuncSetAttribute(tc_bwd_q_kernel<D, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  MVPA_CUDA_CHECK(cudaMemsetAsync(status, 0, 256, s));
-  MVPA_CUDA_CHECK(cudaMemsetAsync(racc, 0, sizeof(unsigned long long) * (size_t)a.Hkv * (2 * D * 128 + 256), s));
-  if (!(D == 64 && CP <= 64))  // (the kernel keeps these sums in shared memory otherwise)
-    MVPA_CUDA_CHECK(cudaMemsetAsync(bw.dtbg, 0, sizeof(float) * (size_t)a.B * a.H * a.N * a.T, s));
-  rel_const_kernel<D><<<a.Hkv, 256, 0, s>>>((const __nv_bfloat16*)a.vt, (const __nv_bfloat16*)a.z,
-                                           (const __nv_bfloat16*)a.rt, (const __nv_bfloat16*)a.rc, relc, a.T, a.C, nullptr);
+  {
+    PreArgs pre;
+    pre.o = (const __nv_bfloat16*)a.o; pre.d_o = (const __nv_bfloat16*)bw.d_o;
+    pre.vt = (const __nv_bfloat16*)a.vt; pre.z = (const __nv_bfloat16*)a.z;
+    pre.rt = (const __nv_bfloat16*)a.rt; pre.rc = (const __nv_bfloat16*)a.rc;
+    pre.o_sb = a.o_sb; pre.o_sh = a.o_sh; pre.o_sn = a.o_sn;
+    pre.do_sb = bw.do_sb; pre.do_sh = bw.do_sh; pre.do_sn = bw.do_sn;
+    pre.delta = bw.delta; pre.relc = relc;
+    // (the areas end on 64-float boundaries; the temporal-score gradients may round up into the padding behind them)
+    pre.zero[0] = reinterpret_cast<uint4*>(status); pre.zero_n[0] = 256 / 16;
+    pre.zero[1] = reinterpret_cast<uint4*>(racc); pre.zero_n[1] = (int64_t)a.Hkv * (2 * D * 128 + 256) / 2;
+    // (the query-side kernel keeps these sums in shared memory where one thread owns each)
+    pre.zero[2] = reinterpret_cast<uint4*>(bw.dtbg);
+    pre.zero_n[2] = (D == 64 && CP <= 64) ? 0 : ((int64_t)a.B * a.H * a.N * a.T + 3) / 4;
+    pre.BH = a.B * a.H; pre.H = a.H; pre.Hkv = a.Hkv; pre.N = a.N; pre.T = a.T; pre.C = a.C;
+    pre.n_delta = (int)(((int64_t)pre.BH * a.N * (D / 8) + kPreThreads - 1) / kPreThreads);
+    const int64_t zeros = pre.zero_n[1] + pre.zero_n[2];
+    const int64_t want = (zeros + 4 * kPreThreads - 1) / (4 * kPreThreads), most = 8 * (int64_t)device_sm_count();
+    tc_bwd_pre_kernel<D><<<(unsigned)(pre.n_delta + a.Hkv + (want < most ? want : most)), kPreThreads, 0, s>>>(pre);
+  }
   const unsigned grid = (unsigned)t.n_qt * a.B * a.H;
   tc_bwd_q_kernel<D, CP><<<grid, kThreads, smem, s>>>(maps, t);
   count_launch(2);
@@ -1659,12 +1729,15 @@ int tc_bwd_bias(const BwdArgs& bw, float* extra, cudaStream_t s) {
   const unsigned long long* racc =
       reinterpret_cast<const unsigned long long*>(extra + cs_dq_floats(a.B, a.H, a.T, a.D) + 64 + (size_t)a.Hkv * 256);
   const unsigned long long* cacc = racc + (size_t)a.Hkv * 2 * a.D * 128;
-  tc_dbias_kernel<<<a.Hkv, 1024, 0, s>>>(extra, cacc, (const __nv_bfloat16*)a.rt, (const __nv_bfloat16*)a.rc, bw.du,
-                                       bw.dvt, bw.dz, a.B, a.H, a.g, a.T, a.C, a.D, (a.T + TPB - 1) / TPB);
-  tc_drel_final_kernel<<<dim3(a.Hkv, 2), 256, 0, s>>>(racc, cacc, (const __nv_bfloat16*)a.u,
-                                                     (const __nv_bfloat16*)a.vt, (const __nv_bfloat16*)a.z, bw.drt,
-                                                     bw.drc, a.T, a.C, a.D, 1.f / a.c2);
-  count_launch(2);
+  FinArgs f;
+  f.cs_dq = extra; f.racc = racc; f.cacc = cacc;
+  f.rt = (const __nv_bfloat16*)a.rt; f.rc = (const __nv_bfloat16*)a.rc; f.u = (const __nv_bfloat16*)a.u;
+  f.vt = (const __nv_bfloat16*)a.vt; f.z = (const __nv_bfloat16*)a.z;
+  f.du = bw.du; f.dvt = bw.dvt; f.dz = bw.dz; f.drt = bw.drt; f.drc = bw.drc;
+  f.B = a.B; f.H = a.H; f.Hkv = a.Hkv; f.g = a.g; f.T = a.T; f.C = a.C; f.D = a.D; f.n_qt = (a.T + TPB - 1) / TPB;
+  f.inv_c2 = 1.f / a.c2;
+  tc_bwd_final_kernel<<<a.Hkv * (1 + 2 * (a.D / 32)), 1024, 0, s>>>(f);
+  count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
 }

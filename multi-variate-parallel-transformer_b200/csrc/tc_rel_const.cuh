@@ -12,16 +12,10 @@ namespace mvpa {
 // One thread per column: its key row comes in with 16-byte loads that are all in flight at once (D is 64
 // or 128 on the tensor-core paths: 8 or 16 loads), so the kernel costs one memory round trip, not D / 2.
 template <int D>
-static __global__ void __launch_bounds__(256) rel_const_kernel(const __nv_bfloat16* __restrict__ vt,
-                                                               const __nv_bfloat16* __restrict__ z,
-                                                               const __nv_bfloat16* __restrict__ rt,
-                                                               const __nv_bfloat16* __restrict__ rc,
-                                                               float* __restrict__ relc, int T, int C,
-                                                               int* __restrict__ status_words) {
-  // (also clears the 64 status words of the kernels that follow, where the caller asks for it: one memset
-  // node less in front of them)
-  if (status_words != nullptr && blockIdx.x == 0 && threadIdx.x < 64) status_words[threadIdx.x] = 0;
-  const int hk = blockIdx.x, j = threadIdx.x & 127;
+static __device__ __forceinline__ void rel_const_row(const __nv_bfloat16* __restrict__ vt, const __nv_bfloat16* __restrict__ z,
+                                                      const __nv_bfloat16* __restrict__ rt, const __nv_bfloat16* __restrict__ rc,
+                                                      float* __restrict__ relc, int T, int C, int hk) {
+  const int j = threadIdx.x & 127;  // 256 threads
   const bool is_t = threadIdx.x < 128;
   const int rows = is_t ? T : C;
   float acc = 0.f;
@@ -46,6 +40,18 @@ static __global__ void __launch_bounds__(256) rel_const_kernel(const __nv_bfloat
     }
   }
   relc[hk * 256 + threadIdx.x] = acc;
+}
+
+template <int D>
+static __global__ void __launch_bounds__(256) rel_const_kernel(const __nv_bfloat16* __restrict__ vt,
+                                                               const __nv_bfloat16* __restrict__ z,
+                                                               const __nv_bfloat16* __restrict__ rt,
+                                                               const __nv_bfloat16* __restrict__ rc,
+                                                               float* __restrict__ relc, int T, int C,
+                                                               int* __restrict__ status_words) {
+  // (also clears the 64 status words of the kernels that follow: one memset node less in front of them)
+  if (blockIdx.x == 0 && threadIdx.x < 64) status_words[threadIdx.x] = 0;
+  rel_const_row<D>(vt, z, rt, rc, relc, T, C, blockIdx.x);
 }
 
 }  // namespace mvpa

@@ -85,6 +85,11 @@ inline int encode_bf16_sw128(CUtensorMap* map, const void* base, int rank, const
 
 inline int encode_bf16_sw128_uncached(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                                       const uint64_t* strides_bytes, const uint32_t* box) {
+  // The driver call needs a current context, and a thread's first runtime call is what binds one: make that call here,
+  // whatever the caller has done on this thread so far (autograd runs backwards on threads of its own).
+  int device = 0;
+  MVPA_CUDA_CHECK(cudaGetDevice(&device));
+  MVPA_CUDA_CHECK(cudaSetDevice(device));
   EncodeTiledFn fn = get_encode_tiled();
   if (fn == nullptr) {
     set_error("cuTensorMapEncodeTiled is not available from this driver");
