@@ -34,19 +34,23 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 def _tensor(t: torch.Tensor) -> _nat.Tensor:
-    return _nat.Tensor(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
+    sb, sh, sn, _ = t.stride()
+    return _nat.Tensor(t.data_ptr(), sb, sh, sn)
+
+
+def _aligned(t: torch.Tensor) -> bool:
+    """A contiguous last dimension, 16-byte aligned base and strides: what the kernels read in place."""
+    sb, sh, sn, sd = t.stride()
+    return sd == 1 and not (((sb | sh | sn) * t.element_size() | t.data_ptr()) & 15)
 
 
 def _rows(t: torch.Tensor) -> torch.Tensor:
     """(B,H,N,D) with a contiguous last dim and 16-byte aligned strides, copying only if needed."""
-    es = t.element_size()
-    if t.stride(-1) != 1 or any((s * es) % 16 for s in t.stride()[:-1]) or t.data_ptr() % 16:
-        t = t.contiguous()
-    return t
+    return t if _aligned(t) else t.contiguous()
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream(t: torch.Tensor) -> ctypes.c_void_p:
+    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
 def _problem(q, k, r_time, r_chan, sm_scale, window, q_time=(0, 0)) -> _nat.Problem:
@@ -55,32 +59,43 @@ def _problem(q, k, r_time, r_chan, sm_scale, window, q_time=(0, 0)) -> _nat.Prob
                         _dtype_code(q), float(sm_scale), 0, int(q_time[0]), int(q_time[1]))
 
 
+def _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, want_lse):
+    """One `mvpa_fwd` call on tensors the kernels can read in place.  Returns the log-sum-exp (or None)."""
+    lib = _nat.lib()
+    prob = _problem(q, k, r_time, r_chan, sm_scale, window, q_time)
+    lse = torch.empty((q.shape[0] * q.shape[1], q.shape[2]), device=q.device, dtype=torch.float32) if want_lse else None
+    nbytes = lib.mvpa_fwd_workspace_bytes(ctypes.byref(prob))
+    ws = torch.empty(nbytes, device=q.device, dtype=torch.uint8) if nbytes else None
+    tq, tk, tv, to = _tensor(q), _tensor(k), _tensor(v), _tensor(o)
+    with _nat.on_device(q.device):
+        st = lib.mvpa_fwd(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
+                          u.data_ptr(), vt.data_ptr(), z.data_ptr(), r_time.data_ptr(), r_chan.data_ptr(),
+                          ctypes.byref(to), None if lse is None else lse.data_ptr(), None if ws is None else ws.data_ptr(),
+                          nbytes, _stream(q))
+    _nat.check(st, "mvpa_fwd")
+    if _CHECK_STATUS and nbytes:  # debugging aid: synchronises the stream
+        _nat.check(lib.mvpa_workspace_status(ws.data_ptr(), nbytes, _stream(q)), "mvpa_fwd kernels")
+    return lse
+
+
+def _need_cuda(q):
+    if not q.is_cuda:
+        raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
+
+
 class FlashMVPA(torch.autograd.Function):
     """Autograd wrapper; the counterpart of the reference's `FlashMVPA`
     (`attentions/attn.py:1013-1302`), taking the relative keys themselves instead of
-    pre-multiplied score matrices."""
+    pre-multiplied score matrices.  The small tensors may have any shape with their elements in
+    (kv head, row, D) order, r_time and r_chan with the rows next to last; their gradients take that shape."""
 
     @staticmethod
     def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0)):
-        if not q.is_cuda:
-            raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
-        lib = _nat.lib()
+        _need_cuda(q)
         q, k, v = _rows(q), _rows(k), _rows(v)
         u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
-        prob = _problem(q, k, r_time, r_chan, sm_scale, window, q_time)
         o = torch.empty_like(q)
-        lse = torch.empty((q.shape[0] * q.shape[1], q.shape[2]), device=q.device, dtype=torch.float32)
-        nbytes = lib.mvpa_fwd_workspace_bytes(ctypes.byref(prob))
-        ws = torch.empty(max(nbytes, 16), device=q.device, dtype=torch.uint8)
-        tq, tk, tv, to = _tensor(q), _tensor(k), _tensor(v), _tensor(o)
-        with torch.cuda.device(q.device):
-            st = lib.mvpa_fwd(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                              u.data_ptr(), vt.data_ptr(), z.data_ptr(), r_time.data_ptr(),
-                              r_chan.data_ptr(), ctypes.byref(to), lse.data_ptr(), ws.data_ptr(),
-                              nbytes, _stream())
-        _nat.check(st, "mvpa_fwd")
-        if _CHECK_STATUS and nbytes:  # debugging aid: synchronises the stream
-            _nat.check(lib.mvpa_workspace_status(ws.data_ptr(), nbytes, _stream()), "mvpa_fwd kernels")
+        lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
         ctx.save_for_backward(q, u, vt, z, k, r_time, r_chan, v, o, lse)
         ctx.sm_scale, ctx.window, ctx.q_time = sm_scale, window, q_time
         return o
@@ -94,26 +109,45 @@ class FlashMVPA(torch.autograd.Function):
         do = _rows(do)
         prob = _problem(q, k, r_time, r_chan, ctx.sm_scale, ctx.window)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        # the five small gradients leave the library as fp32: one buffer, so that one cast serves all of them
-        shapes = (u.shape, vt.shape, z.shape, r_time.shape, r_chan.shape)
-        sizes = [(math.prod(sh) + 3) // 4 * 4 for sh in shapes]             # 16-byte aligned pieces
+        # the five small gradients leave the library as fp32: one buffer, so that one cast serves all of them (every
+        # piece is a whole number of rows of D >= 16 elements, hence 16-byte aligned)
+        shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]
+        sizes = [sh.numel() for sh in shapes]
         small = torch.empty(sum(sizes), device=q.device, dtype=torch.float32)
-        du, dvt, dz, drt, drc = (piece[:math.prod(sh)].view(sh) for piece, sh in zip(small.split(sizes), shapes))
+        ptrs, at = [], small.data_ptr()
+        for n in sizes:
+            ptrs.append(at)
+            at += 4 * n
         nbytes = lib.mvpa_bwd_workspace_bytes(ctypes.byref(prob))
         ws = torch.empty(max(nbytes, 16), device=q.device, dtype=torch.uint8)
         T = [_tensor(x) for x in (q, k, v, o, do, dq, dk, dv)]
         r = [ctypes.byref(x) for x in T]
-        with torch.cuda.device(q.device):
+        with _nat.on_device(q.device):
             st = lib.mvpa_bwd(ctypes.byref(prob), r[0], r[1], r[2], u.data_ptr(), vt.data_ptr(),
                               z.data_ptr(), r_time.data_ptr(), r_chan.data_ptr(), r[3], lse.data_ptr(),
-                              r[4], r[5], r[6], r[7], du.data_ptr(), dvt.data_ptr(), dz.data_ptr(),
-                              drt.data_ptr(), drc.data_ptr(), ws.data_ptr(), nbytes, _stream())
+                              r[4], r[5], r[6], r[7], *ptrs, ws.data_ptr(), nbytes, _stream(q))
         _nat.check(st, "mvpa_bwd")
         if _CHECK_STATUS:  # debugging aid: synchronises the stream
-            _nat.check(lib.mvpa_bwd_status(ctypes.byref(prob), ws.data_ptr(), nbytes, _stream()), "mvpa_bwd kernels")
+            _nat.check(lib.mvpa_bwd_status(ctypes.byref(prob), ws.data_ptr(), nbytes, _stream(q)), "mvpa_bwd kernels")
         small = small.to(q.dtype)
-        du, dvt, dz, drt, drc = (piece[:math.prod(sh)].view(sh) for piece, sh in zip(small.split(sizes), shapes))
+        du, dvt, dz, drt, drc = (piece.view(sh) for piece, sh in zip(small.split(sizes), shapes))
         return (dq, du, dvt, dz, dk, drt, drc, dv, None, None, None)
+
+
+def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
+    """FlashMVPA with or without its autograd record.  The record costs about as much host time as everything else
+    of a small call, so an ordinary call that no gradient flows through goes to the kernels directly (and stores no
+    log-sum-exp); whatever traces or transforms the call sees the autograd function."""
+    ts = (q, u, vt, z, k, r_time, r_chan, v)
+    if ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or not _nat.untraced()
+            or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts)):
+        return FlashMVPA.apply(*ts, sm_scale, window, q_time)
+    _need_cuda(q)
+    q, k, v = _rows(q), _rows(k), _rows(v)
+    u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
+    o = torch.empty_like(q)
+    _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, False)
+    return o
 
 
 def flash_mvpa_into(out, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window_size=10, q_time_range=None):
@@ -122,26 +156,13 @@ def flash_mvpa_into(out, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window_siz
     next projection reads).  u, vt, z (Hkv,D); r_time (Hkv,T,D); r_chan (Hkv,C,D).  `q_time_range=(t0, n)`:
     `q` and `out` hold only the tokens of time steps t0..t0+n-1 (see `flash_mvpa`).  No counterpart in the
     reference, whose operator always allocates its output (`attentions/attn.py:1047`)."""
-    if not q.is_cuda:
-        raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
-    lib = _nat.lib()
+    _need_cuda(q)
     q, k, v = _rows(q), _rows(k), _rows(v)
     u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
-    es = out.element_size()
-    if out.stride(-1) != 1 or any((st * es) % 16 for st in out.stride()[:-1]) or out.data_ptr() % 16 or out.shape != q.shape:
+    if not _aligned(out) or out.shape != q.shape:
         raise RuntimeError("flash_mvpa_into: `out` must have q's shape, a contiguous last dimension and 16-byte aligned strides")
     q_time = (0, 0) if q_time_range is None else (int(q_time_range[0]), int(q_time_range[1]))
-    prob = _problem(q, k, r_time, r_chan, sm_scale, window_size, q_time)
-    nbytes = lib.mvpa_fwd_workspace_bytes(ctypes.byref(prob))
-    ws = torch.empty(max(nbytes, 16), device=q.device, dtype=torch.uint8)
-    tq, tk, tv, to = _tensor(q), _tensor(k), _tensor(v), _tensor(out)
-    with torch.cuda.device(q.device):
-        st = lib.mvpa_fwd(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                          u.data_ptr(), vt.data_ptr(), z.data_ptr(), r_time.data_ptr(), r_chan.data_ptr(),
-                          ctypes.byref(to), None, ws.data_ptr(), nbytes, _stream())
-    _nat.check(st, "mvpa_fwd")
-    if _CHECK_STATUS and nbytes:
-        _nat.check(lib.mvpa_workspace_status(ws.data_ptr(), nbytes, _stream()), "mvpa_fwd kernels")
+    _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, out, sm_scale, window_size, q_time, False)
     return out
 
 
@@ -202,9 +223,10 @@ def flash_mvpa(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, causal, s
         time_keep = torch.rand(time_ctx, device=q.device, generator=generator) > p_per_dim
         keep = (time_keep[:, None] & chan_keep[None, :]).reshape(1, 1, n_ctx, 1)
         v = v * keep.to(v.dtype)
-    u, vt, z = (x.reshape(kv_heads, D) for x in (q_bias, q_btime, q_bchan))
-    o = FlashMVPA.apply(q, u, vt, z, k_glob, k_time.reshape(kv_heads, time_ctx, D),
-                        k_chan.reshape(kv_heads, chan_ctx, D), v, sm_scale, window_size, q_time)
+    for x, n in ((q_bias, 1), (q_btime, 1), (q_bchan, 1), (k_time, time_ctx), (k_chan, chan_ctx)):
+        if x.numel() != kv_heads * n * D:
+            raise RuntimeError(f"flash_mvpa: shape {tuple(x.shape)} is invalid for {kv_heads} kv heads x {n} x {D}")
+    o = _attend(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, sm_scale, window_size, q_time)
     if p_drop and p_drop > 0:
         o = (o.float() * (1.0 / (1 - p_drop))).to(o.dtype)
     return o

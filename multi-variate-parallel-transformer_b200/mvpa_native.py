@@ -13,6 +13,9 @@ import os
 import shutil
 import subprocess
 import threading
+from contextlib import nullcontext
+
+import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
@@ -167,6 +170,20 @@ def lib() -> ctypes.CDLL:
                               "rebuild it (python __graft_entry__.py)")
         _lib = L
         return L
+
+
+_SAME_DEVICE = nullcontext()
+
+
+def on_device(device):
+    """Context in which `device` is the current CUDA device; costs nothing when it already is."""
+    return _SAME_DEVICE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def untraced() -> bool:
+    """No forward-mode level, functorch transform, tracer or compiler is watching the current call."""
+    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
 
 
 def last_error() -> str:

@@ -43,7 +43,7 @@ def rmsnorm(x, weight, eps, add=None, sum_out=None, out=None):
     y = torch.empty_like(x2) if out is None else out
     if add is not None:
         assert add.dtype == x.dtype and add.reshape(-1, E).is_contiguous()
-    with torch.cuda.device(x.device):
+    with _nat.on_device(x.device):
         st = _nat.lib().mvpa_rmsnorm(x2.data_ptr(), add.data_ptr() if add is not None else None, weight.data_ptr(),
                                      sum_out.data_ptr() if sum_out is not None else None, y.data_ptr(), x2.shape[0], E,
                                      float(eps), _code(x), _stream(x))
@@ -57,7 +57,7 @@ def silu_mul(gate, up, out):
     rows, width = gate.shape
     assert up.shape == gate.shape and out.shape == gate.shape
     assert gate.stride(1) == up.stride(1) == out.stride(1) == 1 and gate.stride(0) == up.stride(0)
-    with torch.cuda.device(gate.device):
+    with _nat.on_device(gate.device):
         st = _nat.lib().mvpa_silu_mul(gate.data_ptr(), up.data_ptr(), gate.stride(0), out.data_ptr(), out.stride(0), rows,
                                       width, _code(gate), _stream(gate))
     _nat.check(st, "mvpa_silu_mul")
@@ -75,7 +75,7 @@ def rmsnorm_bwd(x, weight, dy, eps):
     lib = _nat.lib()
     nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with _nat.on_device(x.device):
         st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), dx.data_ptr(), dw.data_ptr(),
                                   x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes, _stream(x))
     _nat.check(st, "mvpa_rmsnorm_bwd")
@@ -89,7 +89,7 @@ def silu_mul_bwd(gate, up, dout):
     assert up.shape == gate.shape and dout.shape == gate.shape and gate.dtype == up.dtype == dout.dtype
     assert gate.stride(1) == up.stride(1) == dout.stride(1) == 1 and gate.stride(0) == up.stride(0)
     dgate, dup = (torch.empty((rows, width), dtype=gate.dtype, device=gate.device) for _ in range(2))
-    with torch.cuda.device(gate.device):
+    with _nat.on_device(gate.device):
         st = _nat.lib().mvpa_silu_mul_bwd(gate.data_ptr(), up.data_ptr(), gate.stride(0), dout.data_ptr(), dout.stride(0),
                                           dgate.data_ptr(), dup.data_ptr(), width, rows, width, _code(gate), _stream(gate))
     _nat.check(st, "mvpa_silu_mul_bwd")
@@ -101,9 +101,7 @@ def _plain(*ts):
     contiguous, 16-byte aligned, not empty; no forward-mode level, functorch transform or tracer is active
     (those are served by the differentiable torch expressions)."""
     t0 = ts[0]
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._functorch.peek_interpreter_stack() is not None:
-        return False
-    if torch.autograd.forward_ad._current_level >= 0 or t0.dtype not in (torch.bfloat16, torch.float32):
+    if not _nat.untraced() or t0.dtype not in (torch.bfloat16, torch.float32):
         return False
     # (a backward may run on a thread of the autograd engine, where a transform shows on the tensor alone)
     if any(torch._C._functorch.is_functorch_wrapped_tensor(t) or not torch._C._has_storage(t) for t in ts):
@@ -214,7 +212,7 @@ def wave_encode(x, ln_weight, eps=1e-5, pad_to=None):
     out = torch.empty((rows, ld_out), dtype=ln_weight.dtype, device=x.device)
     lo, hi = db4_filters()
     fp = ctypes.POINTER(ctypes.c_float)
-    with torch.cuda.device(x.device):
+    with _nat.on_device(x.device):
         st = _nat.lib().mvpa_wave_encode(x.data_ptr(), x.stride(0), _code(x), lo.ctypes.data_as(fp), hi.ctypes.data_as(fp),
                                          ln_weight.data_ptr(), out.data_ptr(), ld_out, _code(ln_weight), rows, n,
                                          float(eps), _stream(x))
@@ -228,7 +226,7 @@ def channel_mean(h):
     B, T, C, E = h.shape
     assert h.is_contiguous()
     out = torch.empty((B, E), dtype=h.dtype, device=h.device)
-    with torch.cuda.device(h.device):
+    with _nat.on_device(h.device):
         st = _nat.lib().mvpa_channel_mean(h.data_ptr(), out.data_ptr(), B, T, C, E, _code(h), _stream(h))
     _nat.check(st, "mvpa_channel_mean")
     return out
@@ -242,7 +240,7 @@ def contrastive_logits(pred, enc, negatives, temperature):
     assert enc.shape == pred.shape and pred.is_contiguous() and enc.is_contiguous() and enc.dtype == pred.dtype
     assert negatives.dtype == torch.int32 and negatives.is_contiguous() and negatives.shape[:3] == (B, T, C)
     out = torch.empty((B * (T - 1) * C, K + 1), dtype=torch.float32, device=pred.device)
-    with torch.cuda.device(pred.device):
+    with _nat.on_device(pred.device):
         st = _nat.lib().mvpa_contrastive_logits(pred.data_ptr(), enc.data_ptr(), negatives.data_ptr(), out.data_ptr(), B, T,
                                                 C, E, K, float(temperature), _code(pred), _stream(pred))
     _nat.check(st, "mvpa_contrastive_logits")
