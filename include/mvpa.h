@@ -187,12 +187,13 @@ int mvpa_silu_mul(const void* gate, const void* up, int64_t ld_in, void* out, in
 /*
  * Backward of mvpa_rmsnorm without `add` (what autograd derives from the reference's RMSNorm):
  * dx (rows, width) and dweight (width), both in the element type; sums over the rows in fp32, in a
- * fixed order.  The caller provides `workspace` of at least
+ * fixed order.  `add` (may be NULL) is added to dx before it is rounded: the gradient that reaches x
+ * past the norm, through a residual connection.  The caller provides `workspace` of at least
  * mvpa_rmsnorm_bwd_workspace_bytes(rows, width) bytes, 16-byte aligned.  Same widths as mvpa_rmsnorm.
  */
 size_t mvpa_rmsnorm_bwd_workspace_bytes(int64_t rows, int32_t width);
-int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, void* dx, void* dweight,
-                     int64_t rows, int32_t width, float eps, int32_t dtype, void* workspace,
+int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, const void* add, void* dx,
+                     void* dweight, int64_t rows, int32_t width, float eps, int32_t dtype, void* workspace,
                      size_t workspace_bytes, void* cuda_stream);
 
 /*

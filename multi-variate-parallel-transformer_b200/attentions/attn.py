@@ -78,6 +78,33 @@ def _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, 
     return lse
 
 
+def _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, do, dq, dk, dv, sm_scale, window):
+    """One `mvpa_bwd` call on tensors the kernels can read and write in place (dq, dk, dv are filled).  Returns the
+    gradients of u, vt, z, r_time and r_chan, one after the other, flat, in q's dtype: they leave the library as fp32,
+    and one buffer means that one cast serves all of them (every piece is a whole number of rows of D >= 16 elements,
+    hence 16-byte aligned)."""
+    lib = _nat.lib()
+    prob = _problem(q, k, r_time, r_chan, sm_scale, window)
+    sizes = [x.numel() for x in (u, vt, z, r_time, r_chan)]
+    small = torch.empty(sum(sizes), device=q.device, dtype=torch.float32)
+    ptrs, at = [], small.data_ptr()
+    for n in sizes:
+        ptrs.append(at)
+        at += 4 * n
+    nbytes = lib.mvpa_bwd_workspace_bytes(ctypes.byref(prob))
+    ws = torch.empty(max(nbytes, 16), device=q.device, dtype=torch.uint8)
+    T = [_tensor(x) for x in (q, k, v, o, do, dq, dk, dv)]
+    r = [ctypes.byref(x) for x in T]
+    with _nat.on_device(q.device):
+        st = lib.mvpa_bwd(ctypes.byref(prob), r[0], r[1], r[2], u.data_ptr(), vt.data_ptr(),
+                          z.data_ptr(), r_time.data_ptr(), r_chan.data_ptr(), r[3], lse.data_ptr(),
+                          r[4], r[5], r[6], r[7], *ptrs, ws.data_ptr(), nbytes, _stream(q))
+    _nat.check(st, "mvpa_bwd")
+    if _CHECK_STATUS:  # debugging aid: synchronises the stream
+        _nat.check(lib.mvpa_bwd_status(ctypes.byref(prob), ws.data_ptr(), nbytes, _stream(q)), "mvpa_bwd kernels")
+    return small.to(q.dtype)
+
+
 def _need_cuda(q):
     if not q.is_cuda:
         raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
@@ -105,31 +132,10 @@ class FlashMVPA(torch.autograd.Function):
         q, u, vt, z, k, r_time, r_chan, v, o, lse = ctx.saved_tensors
         if ctx.q_time[1]:
             raise NotImplementedError("flash_mvpa: backward through a query time range is not implemented")
-        lib = _nat.lib()
-        do = _rows(do)
-        prob = _problem(q, k, r_time, r_chan, ctx.sm_scale, ctx.window)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        # the five small gradients leave the library as fp32: one buffer, so that one cast serves all of them (every
-        # piece is a whole number of rows of D >= 16 elements, hence 16-byte aligned)
+        small = _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, _rows(do), dq, dk, dv, ctx.sm_scale, ctx.window)
         shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]
         sizes = [sh.numel() for sh in shapes]
-        small = torch.empty(sum(sizes), device=q.device, dtype=torch.float32)
-        ptrs, at = [], small.data_ptr()
-        for n in sizes:
-            ptrs.append(at)
-            at += 4 * n
-        nbytes = lib.mvpa_bwd_workspace_bytes(ctypes.byref(prob))
-        ws = torch.empty(max(nbytes, 16), device=q.device, dtype=torch.uint8)
-        T = [_tensor(x) for x in (q, k, v, o, do, dq, dk, dv)]
-        r = [ctypes.byref(x) for x in T]
-        with _nat.on_device(q.device):
-            st = lib.mvpa_bwd(ctypes.byref(prob), r[0], r[1], r[2], u.data_ptr(), vt.data_ptr(),
-                              z.data_ptr(), r_time.data_ptr(), r_chan.data_ptr(), r[3], lse.data_ptr(),
-                              r[4], r[5], r[6], r[7], *ptrs, ws.data_ptr(), nbytes, _stream(q))
-        _nat.check(st, "mvpa_bwd")
-        if _CHECK_STATUS:  # debugging aid: synchronises the stream
-            _nat.check(lib.mvpa_bwd_status(ctypes.byref(prob), ws.data_ptr(), nbytes, _stream(q)), "mvpa_bwd kernels")
-        small = small.to(q.dtype)
         du, dvt, dz, drt, drc = (piece.view(sh) for piece, sh in zip(small.split(sizes), shapes))
         return (dq, du, dvt, dz, dk, drt, drc, dv, None, None, None)
 

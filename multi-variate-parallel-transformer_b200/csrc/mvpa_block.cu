@@ -153,14 +153,14 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_kernel(const T* __r
 }
 
 // Backward of rmsnorm_kernel without the residual add:  with g = dy w and xh = x rstd,
-//   dx = rstd (g - xh mean(g xh)),   dw = sum_rows dy xh.
+//   dx = rstd (g - xh mean(g xh)) (+ add),   dw = sum_rows dy xh.
 // One warp per row at a time, rows strided over the grid; x and dy are read once, the row stays in registers;
 // each lane keeps the dw of its columns over all its rows, the warps of a CTA meet in shared memory and one
 // fp32 row per CTA goes to `dw_part` (summed in a fixed order by colsum_kernel: deterministic).
 template <typename T, int NV>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                                        const T* __restrict__ dy, T* __restrict__ dx,
-                                                                        float* __restrict__ dw_part,
+                                                                        const T* __restrict__ dy, const T* __restrict__ add,
+                                                                        T* __restrict__ dx, float* __restrict__ dw_part,
                                                                         int64_t rows, int E, float eps) {
   constexpr int N = Vec<T>::N;
   extern __shared__ __align__(16) float s_dw[];  // [kWarpsPerCta][E]
@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_bwd_kernel(const T*
     for (int i = 0; i < NV; ++i) {
       const int col = (i * 32 + lane) * N;
       if (col < E) {
-        float v[N], g[N], wv[N], r[N];
+        float v[N], g[N], wv[N], r[N] = {};
+        if (add != nullptr) Vec<T>::load(add + row * E + col, r);
         Vec<T>::unpack(rx[i], v);
         Vec<T>::unpack(rg[i], g);
         Vec<T>::load(w + col, wv);
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_bwd_kernel(const T*
         for (int e = 0; e < N; ++e) {
           const float xh = v[e] * rstd;
           acc[i][e] += g[e] * xh;
-          r[e] = rstd * (g[e] * wv[e] - xh * c);
+          r[e] += rstd * (g[e] * wv[e] - xh * c);
         }
         Vec<T>::store(dx + row * E + col, r);
       }
@@ -560,13 +561,13 @@ int rmsnorm_bwd_blocks(int64_t rows) {
 }
 
 template <typename T, int NV>
-int run_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* ws, int64_t rows, int E,
+int run_rmsnorm_bwd(const void* x, const void* w, const void* dy, const void* add, void* dx, void* dw, float* ws, int64_t rows, int E,
                     float eps, cudaStream_t s) {
   const size_t smem = sizeof(float) * kWarpsPerCta * E;
   if (smem > 48 * 1024)
     MVPA_CUDA_CHECK(cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = rmsnorm_bwd_blocks(rows);
-  rmsnorm_bwd_kernel<T, NV><<<grid, kWarpsPerCta * 32, smem, s>>>((const T*)x, (const T*)w, (const T*)dy, (T*)dx, ws, rows, E, eps);
+  rmsnorm_bwd_kernel<T, NV><<<grid, kWarpsPerCta * 32, smem, s>>>((const T*)x, (const T*)w, (const T*)dy, (const T*)add, (T*)dx, ws, rows, E, eps);
   colsum_kernel<T><<<(E + 31) / 32, 256, 0, s>>>(ws, (T*)dw, grid, E);
   count_launch(2);
   MVPA_CUDA_CHECK(cudaGetLastError());
@@ -574,13 +575,13 @@ int run_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void
 }
 
 template <typename T>
-int launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* ws, int64_t rows, int E,
+int launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, const void* add, void* dx, void* dw, float* ws, int64_t rows, int E,
                        float eps, cudaStream_t s) {
   const int nv = (E / Vec<T>::N + 31) / 32;
-  if (nv <= 2) return run_rmsnorm_bwd<T, 2>(x, w, dy, dx, dw, ws, rows, E, eps, s);
-  if (nv <= 4) return run_rmsnorm_bwd<T, 4>(x, w, dy, dx, dw, ws, rows, E, eps, s);
-  if (nv <= 8) return run_rmsnorm_bwd<T, 8>(x, w, dy, dx, dw, ws, rows, E, eps, s);
-  return run_rmsnorm_bwd<T, 16>(x, w, dy, dx, dw, ws, rows, E, eps, s);
+  if (nv <= 2) return run_rmsnorm_bwd<T, 2>(x, w, dy, add, dx, dw, ws, rows, E, eps, s);
+  if (nv <= 4) return run_rmsnorm_bwd<T, 4>(x, w, dy, add, dx, dw, ws, rows, E, eps, s);
+  if (nv <= 8) return run_rmsnorm_bwd<T, 8>(x, w, dy, add, dx, dw, ws, rows, E, eps, s);
+  return run_rmsnorm_bwd<T, 16>(x, w, dy, add, dx, dw, ws, rows, E, eps, s);
 }
 
 int check_rows(const char* what, int64_t rows, int width, int dtype, int max_vectors) {
@@ -653,12 +654,13 @@ size_t mvpa_rmsnorm_bwd_workspace_bytes(int64_t rows, int32_t width) {
   return sizeof(float) * (size_t)rmsnorm_bwd_blocks(rows) * width;
 }
 
-int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, void* dx, void* dweight, int64_t rows,
-                     int32_t width, float eps, int32_t dtype, void* workspace, size_t workspace_bytes, void* cuda_stream) {
+int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, const void* add, void* dx, void* dweight,
+                     int64_t rows, int32_t width, float eps, int32_t dtype, void* workspace, size_t workspace_bytes, void* cuda_stream) {
   int rc = check_rows("mvpa_rmsnorm_bwd", rows, width, dtype, 16);
   if (rc) return rc;
-  if (!aligned16(x) || !aligned16(weight) || !aligned16(dy) || !aligned16(dx) || !aligned16(dweight)) {
-    set_error("mvpa_rmsnorm_bwd: x, weight, dy, dx and dweight must be 16-byte aligned and not NULL");
+  if (!aligned16(x) || !aligned16(weight) || !aligned16(dy) || !aligned16(dx) || !aligned16(dweight) ||
+      (add != nullptr && !aligned16(add))) {
+    set_error("mvpa_rmsnorm_bwd: x, weight, dy, dx, dweight (and add when given) must be 16-byte aligned and not NULL");
     return MVPA_ERR_ALIGNMENT;
   }
   if (!aligned16(workspace) || workspace_bytes < mvpa_rmsnorm_bwd_workspace_bytes(rows, width)) {
@@ -668,8 +670,8 @@ int mvpa_rmsnorm_bwd(const void* x, const void* weight, const void* dy, void* dx
   }
   cudaStream_t s = (cudaStream_t)cuda_stream;
   return dtype == MVPA_F32
-             ? launch_rmsnorm_bwd<float>(x, weight, dy, dx, dweight, (float*)workspace, rows, width, eps, s)
-             : launch_rmsnorm_bwd<__nv_bfloat16>(x, weight, dy, dx, dweight, (float*)workspace, rows, width, eps, s);
+             ? launch_rmsnorm_bwd<float>(x, weight, dy, add, dx, dweight, (float*)workspace, rows, width, eps, s)
+             : launch_rmsnorm_bwd<__nv_bfloat16>(x, weight, dy, add, dx, dweight, (float*)workspace, rows, width, eps, s);
 }
 
 int mvpa_silu_mul_bwd(const void* gate, const void* up, int64_t ld_in, const void* dout, int64_t ld_dout, void* dgate,

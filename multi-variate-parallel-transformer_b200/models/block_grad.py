@@ -1,0 +1,149 @@
+"""Training form of the parallel block (`models/mvpformer.py:132-147`, h = x + MLP(ln_1 x) + Attn(ln_1 x)) as ONE autograd
+function.
+
+The same operations as the modules run, in the same order, but with what lies between them removed: the residual and
+branch sums are accumulated by the output projections (beta = 1 products instead of two additions), the four
+projections' input gradients by their products (instead of three additions), the residual's gradient by the RMSNorm
+backward kernel; the attention backward writes dq, dk, dv straight into the buffers the weight-gradient products read
+(no slices, concatenations or copies), and autograd keeps one node per block instead of about forty.
+"""
+from __future__ import annotations
+
+import torch
+import torch.nn.functional as F
+
+import mvpa_native as _nat
+import mvpa_ops
+from attentions import attn as _attn
+from attentions import flashmvpa
+
+WINDOW = 10
+
+
+def expression(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, eps, heads):
+    """The block in differentiable operations (what a graph of the gradient is built from)."""
+    H, Hkv, D = heads
+    B, T, C, E = x.shape
+    N, KV = T * C, Hkv * D
+    xn = mvpa_ops.rmsnorm_train(x, ln_w, eps)
+    q = F.linear(xn, wq).view(B, N, H, D).permute(0, 2, 1, 3)
+    k, v = (t.permute(0, 2, 1, 3) for t in F.linear(xn, wkv).view(B, N, 2 * Hkv, D).split(Hkv, dim=2))
+    rt = F.linear(pos, wpos).view(1, T, Hkv, D).permute(0, 2, 1, 3)
+    rc = F.linear(chan, wchan).view(1, C, Hkv, D).permute(0, 2, 1, 3)
+    u, vt, z = (b.view(1, Hkv, 1, D) for b in bias.split(KV))
+    o = flashmvpa(q, u, vt, z, k, rt, rc, v, causal=True, sm_scale=1.0 / (D ** 0.5), window_size=WINDOW)
+    mlp = F.linear(mvpa_ops.swiglu(F.linear(xn, wg), F.linear(xn, wu)), wd)
+    return x + mlp + F.linear(o.permute(0, 2, 1, 3).reshape(B, T, C, E), wc)
+
+
+def _heads_view(t, B, N, heads, D):
+    """(B*N, heads*D) columns as the kernels' (B, heads, N, D)."""
+    return t.view(B, N, heads, D).permute(0, 2, 1, 3)
+
+
+def _rel_keys(embeds, w, Hkv, D):
+    return torch.mm(embeds[0], w.t()).view(-1, Hkv, D).transpose(0, 1).contiguous()      # (Hkv, rows, D)
+
+
+class BlockFunction(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, eps, heads):
+        H, Hkv, D = heads
+        B, T, C, E = x.shape
+        N, KV = T * C, Hkv * D
+        x2 = x.view(B * N, E)
+        xn = mvpa_ops.rmsnorm(x2, ln_w, eps)
+        q, kv, g, up = (torch.mm(xn, w.t()) for w in (wq, wkv, wg, wu))
+        rt, rc = _rel_keys(pos, wpos, Hkv, D), _rel_keys(chan, wchan, Hkv, D)
+        o = torch.empty_like(q)
+        lse = _attn._launch_fwd(_heads_view(q, B, N, H, D), *bias.view(3, Hkv, D), _heads_view(kv[:, :KV], B, N, Hkv, D),
+                                rt, rc, _heads_view(kv[:, KV:], B, N, Hkv, D), _heads_view(o, B, N, H, D),
+                                1.0 / (D ** 0.5), WINDOW, (0, 0), True)
+        act = mvpa_ops.silu_mul(g, up, torch.empty_like(g))
+        h = torch.addmm(x2, act, wd.t())
+        h.addmm_(o, wc.t())
+        ctx.save_for_backward(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act)
+        ctx.eps, ctx.heads = eps, heads
+        return h.view(B, T, C, E)
+
+    @staticmethod
+    def backward(ctx, dh):
+        saved = ctx.saved_tensors
+        need = ctx.needs_input_grad[:13]
+        if torch.is_grad_enabled() or not _nat.untraced() or not mvpa_ops._plain(dh.contiguous()):
+            # a graph of the gradient is wanted (or a transform is active): through the differentiable operations
+            with torch.enable_grad():
+                ins = [t if t.requires_grad else t.detach().requires_grad_(n) for t, n in zip(saved[:13], need)]
+                out = expression(*ins, ctx.eps, ctx.heads)
+                got = iter(torch.autograd.grad(out, [t for t, n in zip(ins, need) if n], dh, create_graph=True))
+            return (*(next(got) if n else None for n in need), None, None)
+        x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act = saved
+        H, Hkv, D = ctx.heads
+        B, T, C, E = x.shape
+        N, KV = T * C, Hkv * D
+        dh2 = dh.contiguous().view(B * N, E)
+        grad = [None] * 13
+        weight = lambda i, d, a: grad.__setitem__(i, torch.mm(d.t(), a)) if need[i] else None   # d W = d^T input
+        weight(9, dh2, o)
+        weight(12, dh2, act)
+        dg, dup = mvpa_ops.silu_mul_bwd(g, up, torch.mm(dh2, wd))
+        do = torch.mm(dh2, wc)
+        dq, dkv = torch.empty_like(q), torch.empty_like(kv)
+        view = lambda t, heads: _heads_view(t, B, N, heads, D)
+        small = _attn._launch_bwd(view(q, H), *bias.view(3, Hkv, D), view(kv[:, :KV], Hkv), rt, rc, view(kv[:, KV:], Hkv),
+                                  view(o, H), lse, view(do, H), view(dq, H), view(dkv[:, :KV], Hkv), view(dkv[:, KV:], Hkv),
+                                  1.0 / (D ** 0.5), WINDOW)
+        dbias, drt, drc = small.split((3 * KV, T * KV, C * KV))
+        if need[8]:
+            grad[8] = dbias.view(bias.shape)
+        for d, n, e, i_e, w, i_w in ((drt, T, pos, 1, wpos, 6), (drc, C, chan, 2, wchan, 7)):
+            d = d.view(Hkv, n, D).transpose(0, 1).reshape(n, KV)
+            weight(i_w, d, e[0])
+            if need[i_e]:
+                grad[i_e] = torch.mm(d, w).view(e.shape)
+        for i, d in ((4, dq), (5, dkv), (10, dg), (11, dup)):
+            weight(i, d, xn)
+        if need[0] or need[3]:
+            dxn = torch.mm(dq, wq)
+            for d, w in ((dkv, wkv), (dg, wg), (dup, wu)):
+                dxn.addmm_(d, w)
+            dx, grad[3] = mvpa_ops.rmsnorm_bwd(x.view(B * N, E), ln_w, dxn, ctx.eps, add=dh2)
+            grad[0] = dx.view(x.shape)
+        return (*grad, None, None)
+
+
+def _unhooked(m, cls):
+    return (type(m) is cls and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks
+            and not m._backward_hooks and not m._backward_pre_hooks)
+
+
+def applies(block, x, pos, chan, classes) -> bool:
+    """Whether `block` is exactly the computation above on tensors the kernels take in place: the shipped modules, none of
+    them replaced, hooked or patched, no dropout or autocast, one dtype, contiguous and 16-byte aligned, and nothing
+    tracing the call.  Everything else goes through the modules."""
+    norm_cls, attn_cls, mlp_cls = classes
+    a, m = block.attn, block.mlp
+    linears = (a.q_attn, a.c_attn, a.position_net, a.channel_net, a.c_proj, m.gate_proj, m.up_proj, m.down_proj) \
+        if type(a) is attn_cls and type(m) is mlp_cls else ()
+    if not linears or not _unhooked(block.ln_1, norm_cls) or not _unhooked(a, attn_cls) or not _unhooked(m, mlp_cls):
+        return False
+    if not all(_unhooked(l, torch.nn.Linear) and l.bias is None for l in linears):
+        return False
+    for d in (a.attn_dropout, a.resid_dropout):
+        if not _unhooked(d, torch.nn.Dropout) or (d.training and d.p):
+            return False
+    if a.training and a.attn_dropout.p or torch.nn.modules.module._has_any_global_hook() or torch.is_autocast_enabled("cuda"):
+        return False
+    if x.dim() != 4 or pos.shape != (1, x.shape[1], x.shape[3]) or chan.shape != (1, x.shape[2], x.shape[3]):
+        return False
+    ts = (x, pos, chan, block.ln_1.weight, a.attn_bias, *(l.weight for l in linears))
+    es = x.element_size()
+    return (mvpa_ops._plain(*ts) and mvpa_ops._rows_fit(x) and m.gate_proj.out_features * es % 16 == 0
+            and block.ln_1.weight.shape == x.shape[-1:] and any(t.requires_grad for t in ts))
+
+
+def run(block, x, pos, chan):
+    a, m = block.attn, block.mlp
+    return BlockFunction.apply(x, pos, chan, block.ln_1.weight, a.q_attn.weight, a.c_attn.weight, a.position_net.weight,
+                               a.channel_net.weight, a.attn_bias, a.c_proj.weight, m.gate_proj.weight, m.up_proj.weight,
+                               m.down_proj.weight, block.ln_1.eps, (a.num_heads, a.num_kv_heads, a.head_dim))

@@ -19,7 +19,7 @@ h = x + MLP(ln_1 x) + Attn(ln_1 x)) built for B200:
 
 With gradients enabled the blocks run the reference's op order through differentiable operations: torch's
 projections, `mvpa_ops.rmsnorm_train` and `mvpa_ops.swiglu` (one kernel each way instead of about ten
-elementwise launches), and `attentions.flashmvpa`.
+elementwise launches), and `attentions.flashmvpa`; as one autograd function where the block is unmodified.
 """
 from __future__ import annotations
 
@@ -32,7 +32,7 @@ import torch.nn.functional as F
 import mvpa_ops
 from attentions import flash_mvpa_into
 from layers import MVPFormerGQAFlashAttention
-from models import BrainDecider
+from models import BrainDecider, block_grad
 
 
 class MVPFormerConfig:
@@ -103,7 +103,12 @@ class MVPFormerBlock(torch.nn.Module):
     def forward(self, hidden_states, positional_embedding, channel_embedding, layer_past=None, attention_mask=None,
                 head_mask=None, encoder_hidden_states=None, encoder_attention_mask=None, use_cache=False,
                 output_attentions=False):
-        """The reference's op order (`models/mvpformer.py:132-152`); differentiable."""
+        """The reference's op order (`models/mvpformer.py:132-152`); differentiable.  With gradients, and nothing
+        replaced, hooked or dropped out, the whole block is one autograd function (`block_grad`)."""
+        if (torch.is_grad_enabled() and not use_cache and not output_attentions
+                and block_grad.applies(self, hidden_states, positional_embedding, channel_embedding,
+                                       (RMSNorm, MVPFormerGQAFlashAttention, LlamaMLP))):
+            return (block_grad.run(self, hidden_states, positional_embedding, channel_embedding),)
         residual = hidden_states
         hidden_states = self.ln_1(hidden_states)
         attn_outputs = self.attn(hidden_states, positional_embedding, channel_embedding, layer_past=layer_past,

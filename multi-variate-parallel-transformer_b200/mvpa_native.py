@@ -144,7 +144,7 @@ def lib() -> ctypes.CDLL:
         L.mvpa_rmsnorm_bwd_workspace_bytes.restype = ctypes.c_size_t
         L.mvpa_rmsnorm_bwd_workspace_bytes.argtypes = [i64, i32]
         L.mvpa_rmsnorm_bwd.restype = ctypes.c_int
-        L.mvpa_rmsnorm_bwd.argtypes = [vp, vp, vp, vp, vp, i64, i32, f32, i32, vp, ctypes.c_size_t, vp]
+        L.mvpa_rmsnorm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, i64, i32, f32, i32, vp, ctypes.c_size_t, vp]
         L.mvpa_silu_mul_bwd.restype = ctypes.c_int
         L.mvpa_silu_mul_bwd.argtypes = [vp, vp, i64, vp, i64, vp, vp, i64, i64, i32, i32, vp]
         L.mvpa_wave_encode_size.restype = i32

@@ -64,20 +64,23 @@ def silu_mul(gate, up, out):
     return out
 
 
-def rmsnorm_bwd(x, weight, dy, eps):
-    """Gradients (dx, dweight) of `rmsnorm(x, weight, eps)` (no `add`) for the incoming gradient `dy`."""
-    _need_cuda(x, weight, dy)
+def rmsnorm_bwd(x, weight, dy, eps, add=None):
+    """Gradients (dx, dweight) of `rmsnorm(x, weight, eps)` (no residual) for the incoming gradient `dy`; `add`, the
+    gradient that reaches x on another way (a residual connection), is added to dx."""
+    _need_cuda(x, weight, dy, add)
     E = x.shape[-1]
     x2, dy2 = x.reshape(-1, E), dy.reshape(-1, E)
     assert x2.is_contiguous() and dy2.is_contiguous() and weight.is_contiguous()
     assert weight.dtype == x.dtype == dy.dtype and dy.shape == x.shape
+    if add is not None:
+        assert add.dtype == x.dtype and add.is_contiguous() and add.numel() == x.numel()
     dx, dw = torch.empty_like(x2), torch.empty_like(weight)
     lib = _nat.lib()
     nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     with _nat.on_device(x.device):
-        st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), dx.data_ptr(), dw.data_ptr(),
-                                  x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes, _stream(x))
+        st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(),
+                                  add.data_ptr() if add is not None else None, dx.data_ptr(), dw.data_ptr(), x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes, _stream(x))
     _nat.check(st, "mvpa_rmsnorm_bwd")
     return dx.view(x.shape), dw
 

@@ -82,3 +82,60 @@ def test_second_derivatives_and_transforms(cuda):
     torch.testing.assert_close(mvpa_ops.rmsnorm_train(odd, odd[0], 1e-5), _norm64(odd, odd[0], 1e-5))
     h = torch.randn(4, 16, device=cuda, dtype=torch.float16)
     torch.testing.assert_close(mvpa_ops.swiglu(h, h), torch.nn.functional.silu(h) * h)
+
+
+def _block(cuda, dtype, E=128, H=4, Hkv=2, I=176, T=13, C=10, B=2):
+    import models
+    torch.manual_seed(0)
+    cfg = models.MVPFormerConfig(n_embd=E, n_layer=1, n_head=H, n_head_kv=Hkv, n_inner=I, n_positions=16, n_channels=16,
+                                 attn_pdrop=0.0, resid_pdrop=0.0)
+    block = models.MVPFormerBlock(cfg).to(cuda).to(dtype)
+    for p in block.parameters():
+        torch.nn.init.normal_(p, std=0.1)
+    x, pos, chan = (torch.randn(*s, E, device=cuda).to(dtype).requires_grad_() for s in ((B, T, C), (1, T), (1, C)))
+    return block, x, pos, chan, torch.randn(B, T, C, E, device=cuda).to(dtype)
+
+
+# The one-function block against the modules, which an (empty) hook brings back.  fp32: the same products in another
+# order; bf16: one rounding per intermediate result (2^-9 each, about six on the longest way) on both sides.
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 3e-2)])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_block_function_equals_the_modules(cuda, dtype, tol, frozen):
+    block, x, pos, chan, dy = _block(cuda, dtype)
+    if frozen:
+        for m in (block.attn.q_attn, block.mlp.down_proj, block.ln_1):
+            m.weight.requires_grad_(False)
+        pos.requires_grad_(False)
+    ins = [t for n, t in [("x", x), ("pos", pos), ("chan", chan), *block.named_parameters()]
+           if t.requires_grad and not n.startswith("ln_2")]
+    y = block(x, pos, chan)[0]
+    assert "BlockFunction" in type(y.grad_fn).__name__
+    got = (y,) + torch.autograd.grad(y, ins, dy)
+    handle = block.mlp.register_forward_hook(lambda *a: None)
+    y2 = block(x, pos, chan)[0]
+    assert "BlockFunction" not in type(y2.grad_fn).__name__
+    ref = (y2,) + torch.autograd.grad(y2, ins, dy)
+    handle.remove()
+    for a, b in zip(got, ref):
+        assert a.dtype == b.dtype and a.shape == b.shape and _rel(a, b.double()) <= tol
+
+
+def test_block_function_graph_of_the_gradient_and_other_routes(cuda):
+    block, x, pos, chan, dy = _block(cuda, torch.float32)
+
+    def penalty(out):
+        return torch.autograd.grad(out, x, dy, create_graph=True)[0].pow(2).sum()
+
+    p1 = penalty(block(x, pos, chan)[0])
+    g1 = torch.autograd.grad(p1, block.mlp.up_proj.weight)[0]
+    handle = block.mlp.register_forward_hook(lambda *a: None)
+    p2 = penalty(block(x, pos, chan)[0])
+    g2 = torch.autograd.grad(p2, block.mlp.up_proj.weight)[0]
+    handle.remove()
+    assert _rel(p1, p2.double()) <= 1e-5 and _rel(g1, g2.double()) <= 1e-4
+    block.attn.resid_dropout.p = 0.5
+    assert "BlockFunction" not in type(block(x, pos, chan)[0].grad_fn).__name__
+    block.eval()
+    assert "BlockFunction" in type(block(x, pos, chan)[0].grad_fn).__name__
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert "BlockFunction" not in type(block(x, pos, chan)[0].grad_fn).__name__
