@@ -234,13 +234,13 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       mbar_init(&slot_free[i], 1);
     }
     mbar_fence_init();
-  } else if (tid == 64) {
-    *s_abort = *p.status;
   }
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  griddep_wait();  // nothing above reads memory; the status words and constants come from the pre-kernel
+  if (tid == 64) *s_abort = *p.status;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1075,9 +1075,20 @@ int launch(const Args& a, int* status, cudaStream_t s) {
                                            a.C, status);  // (clears the status words too)
   count_launch();
   const unsigned grid = (unsigned)t.q_tiles * a.B * a.H;
-  tc_fwd_kernel<D, CP><<<grid, kThreads, smem, s>>>(maps, t);
+  // Programmatic dependent launch: the CTAs come up (barriers, tensor memory) while the pre-kernel runs and wait
+  // for it (griddep_wait) before they touch any memory that it or an earlier kernel has written.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  MVPA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tc_fwd_kernel<D, CP>, maps, t));
   count_launch();
-  MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
 }
 

@@ -366,6 +366,11 @@ __device__ __forceinline__ uint32_t sw128_offset(int row, int col) {
   return (uint32_t)(row * 128 + chunk * 16 + (col & 7) * 2);
 }
 
+// Programmatic dependent launch: let the next kernel's CTAs start / wait until the previous grid has completed and
+// its writes are visible (returns at once in a kernel launched without the attribute).
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // packed fp32 arithmetic: two elements per instruction, each rounded like the scalar operation
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   float2 d;

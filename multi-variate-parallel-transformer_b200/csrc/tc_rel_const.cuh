@@ -4,6 +4,8 @@
 
 #include <cuda_bf16.h>
 
+#include "tc_ptx.cuh"
+
 namespace mvpa {
 
 // Per-column constants of the two relative products, once per kv head instead of once per CTA:
@@ -49,6 +51,7 @@ static __global__ void __launch_bounds__(256) rel_const_kernel(const __nv_bfloat
                                                                const __nv_bfloat16* __restrict__ rc,
                                                                float* __restrict__ relc, int T, int C,
                                                                int* __restrict__ status_words) {
+  ptx::griddep_launch();  // the next kernel's CTAs may come up; they wait for this grid's end before reading anything
   // (also clears the 64 status words of the kernels that follow: one memset node less in front of them)
   if (blockIdx.x == 0 && threadIdx.x < 64) status_words[threadIdx.x] = 0;
   rel_const_row<D>(vt, z, rt, rc, relc, T, C, blockIdx.x);
