@@ -39,8 +39,7 @@ struct BwdArgs {
   float *du, *dvt, *dz, *drt, *drc;
   // workspace carve-up (fp32 elements)
   float *tbg, *cbg;    // (B*H, T, N), (B*H, N, C) relative scores, base-2 scaled
-  float *dtbg, *dcbg;  // gradients w.r.t. the unscaled relative scores, (B*H, N, slots); the tensor-core
-                       // kernels use dtbg as (B*H, T, N) scratch and leave dcbg alone
+  float *dtbg, *dcbg;  // gradients w.r.t. the unscaled relative scores, (B*H, N, slots)
   float* delta;        // (B*H, N)
   float* partial;      // (B*H*nQT, 3, D) per-tile column sums for du/dvt/dz
   float* drel_part;    // (split, Hkv, T + C, D) split-K partials of dr_time / dr_chan

@@ -1156,25 +1156,20 @@ int simt_bwd(const BwdArgs& b, int dtype, cudaStream_t s) {
 }
 
 namespace {
-// bf16 problems the tensor-core backward takes need only delta and (when two threads own a temporal
-// slot) the temporal-score gradients from this file's areas; everything else lives in tc_extra.
+// bf16 problems the tensor-core backward takes need only delta from this file's areas; everything else lives in tc_extra.
 bool tc_path(int dtype, int D, int C, int T) {
   Args a{};
   a.D = D; a.C = C; a.T = T;
   return dtype == MVPA_BF16 && tc_bwd_q_supported(a);
 }
-bool tc_needs_dtb(int D, int C) { return !(D == 64 && C <= 64); }
-size_t round4(size_t n) { return (n + 3) & ~(size_t)3; }
-// delta and, behind it on a 16-byte boundary, the temporal-score gradients
-size_t tc_head_floats(size_t rows, int D, int C, int T) {
-  return (round4(rows) + (tc_needs_dtb(D, C) ? rows * T : 0) + 63) & ~(size_t)63;
-}
+// delta, in front of the tensor-core kernels' own workspace
+size_t tc_head_floats(size_t rows) { return (rows + 63) & ~(size_t)63; }
 }  // namespace
 
 size_t simt_bwd_workspace_floats(const mvpa_problem* p) {
   const size_t BH = (size_t)p->B * p->H, N = (size_t)p->T * p->C;
   if (tc_path(p->dtype, p->D, p->C, p->T)) {
-    return tc_head_floats(BH * N, p->D, p->C, p->T) + tc_bwd_q_workspace_floats(p);
+    return tc_head_floats(BH * N) + tc_bwd_q_workspace_floats(p);
   }
   const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most
   size_t n = 2 * BH * N * (p->T + p->C) + BH * N + BH * n_qt * 3 * p->D;
@@ -1185,7 +1180,7 @@ size_t simt_bwd_workspace_floats(const mvpa_problem* p) {
 const int* bwd_status_word(const mvpa_problem* p, const void* workspace) {
   if (!tc_path(p->dtype, p->D, p->C, p->T)) return nullptr;  // the CUDA-core kernels have no device-side waits
   const size_t BH = (size_t)p->B * p->H, N = (size_t)p->T * p->C;
-  return reinterpret_cast<const int*>(static_cast<const float*>(workspace) + tc_head_floats(BH * N, p->D, p->C, p->T) +
+  return reinterpret_cast<const int*>(static_cast<const float*>(workspace) + tc_head_floats(BH * N) +
                                       tc_bwd_status_offset_floats(p));
 }
 
@@ -1193,10 +1188,9 @@ void simt_bwd_carve(BwdArgs& b, float* ws, int dtype) {
   const Args& a = b.a;
   const size_t BH = (size_t)a.B * a.H, N = a.N;
   if (tc_path(dtype, a.D, a.C, a.T)) {
-    b.tbg = b.cbg = b.dcbg = b.partial = b.drel_part = nullptr;
+    b.tbg = b.cbg = b.dtbg = b.dcbg = b.partial = b.drel_part = nullptr;
     b.delta = ws;
-    b.dtbg = ws + round4(BH * N);  // (B*H, T, N) scratch of the tensor-core kernels, when they need it
-    b.tc_extra = ws + tc_head_floats(BH * N, a.D, a.C, a.T);
+    b.tc_extra = ws + tc_head_floats(BH * N);
     return;
   }
   const size_t n_qt = (N + kMinRows - 1) / kMinRows;  // at most

@@ -66,7 +66,6 @@ struct BqArgs {
   float* cs_dq;        // (grid, D) per-CTA column sums of dq (fp32), for du
   // Everything a thread (= query row) reads or writes per row is stored row-innermost, so that the 32
   // rows of a warp touch consecutive addresses.
-  float* dtb;          // (B*H, T, N) zero-initialised; slot T-1-(t_i-t_k)
   // Accumulators over all query-side CTAs of a kv head, zero-initialised, in 64-bit fixed point (see kFix):
   unsigned long long* racc;  // (Hkv, 2, D, 128): sum over query rows of dTB^T Q' / dCB^T Q'
   unsigned long long* cacc;  // (Hkv, 2, 128):    column sums of dTB / dCB (as bf16, like racc)
@@ -85,6 +84,8 @@ struct BqArgs {
 enum BarrierIndex {
   kBarProFull = 0, kBarProMma, kBarProDone, kBarSFull, kBarSFull1, kBarDpFull, kBarDpFull1, kBarDsFull, kBarDsFull1, kBarAllDone,
   kBarFinFull, kBarFinLoaded, kBarFinDone, kBarRelDone,
+  kBarTbPart,                    // 4: the second warpgroup's part of a tile's dTB is in shared memory (CP = 128)
+  kBarTbPartEnd = kBarTbPart + 3,
   kBarSlotFull,  // NS, then slot_free NS
 };
 
@@ -100,14 +101,13 @@ struct Cfg {
   static constexpr int SMEM_DO = TILE;
   static constexpr int SMEM_RING = 2 * TILE;
   static constexpr int SMEM_PRO = SMEM_RING + EARLY * TILE;
-  // head_dim 64 leaves room for the tile's temporal-score gradients, [row][slot] as bf16 in the operand
-  // layout, through the whole main loop (used when every (row, slot) has a single owning thread)
+  // the tile's temporal-score gradients, [row][slot] as bf16 in the operand layout, through the whole main loop
   static constexpr int SMEM_TBT = SMEM_RING + NS * TILE;
-  static constexpr int SMEM_TAIL = SMEM_TBT + (D == 64 ? 32768 : 0);
+  static constexpr int SMEM_TAIL = SMEM_TBT + 32768;
   // tail: u (D f32), vR[128], zC[128], smax[2][128], barriers, tmem slot, abort
   static constexpr int TAIL_FLOATS = D + 128 + 128 + 256;
   static constexpr int TAIL_BYTES = TAIL_FLOATS * 4 + (kBarSlotFull + 2 * NS) * 8 + 16;
-  static constexpr int SMEM_BYTES = SMEM_TAIL + TAIL_BYTES + 1024;
+  static constexpr int SMEM_BYTES = SMEM_TAIL + TAIL_BYTES;  // (the block's shared memory starts on a 1024-byte boundary)
 };
 
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
@@ -145,17 +145,18 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   // the prologue (the scaled scores are re-read from the workspace, tile by tile); the dr_time
   // accumulator of the epilogue takes the second S buffer.
   constexpr uint32_t kQS = 0, kQS1 = 128, kQDP = 256, kQDQ = 384;
-  // With at most 64 channel slots a key time step belongs to one warpgroup, so each (row, slot) sum of
-  // dS has one owner and goes straight into a shared-memory tile; otherwise the two owners add into the
-  // workspace with atomics and the tile is rebuilt from there after the loop.
-  constexpr bool TBS = (D == 64) && (CP <= 64);
+  // Each (row, slot) sum of dS goes into a shared-memory tile.  With at most 64 channel slots a key time step
+  // belongs to one warpgroup; with 128 the second warpgroup hands its part to the first one through shared memory,
+  // which stores the sum one tile later, when the part has long arrived (four buffers: a part's place is written again
+  // four tiles on, and the report of the tile after it lies between).
+  constexpr bool PART = CP == 128;
   // The prologue's scratch rows are padded instead of rotated when that fits (<= 64 channel slots).
   constexpr bool PAD = CP <= 64;
   constexpr int LDP = PAD ? CP + 2 : CP;
   static_assert(CP >= 32 && CP <= 128 && (CP & (CP - 1)) == 0, "CP in {32,64,128}");
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_q[];
+  uint8_t* smem = smem_q;
   uint8_t* sQ = smem + C_::SMEM_Q;
   uint8_t* sDO = smem + C_::SMEM_DO;
   uint8_t* ring = smem + C_::SMEM_RING;
@@ -167,6 +168,8 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   float* s_vr = s_bias + D;
   float* s_zc = s_vr + 128;
   float* s_max = s_zc + 128;  // [2 wg][128]
+  float* s_part = s_bias;     // [4][128], once the prologue is over (s_bias .. s_max are dead by then)
+  static_assert(C_::TAIL_FLOATS >= 512, "four buffers of partial sums");
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_max + 256);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBarSlotFull + 2 * NS);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
@@ -215,6 +218,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     mbar_init(&bars[kBarFinLoaded], 1);
     mbar_init(&bars[kBarFinDone], 1);
     mbar_init(&bars[kBarRelDone], 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&bars[kBarTbPart + i], kSoftmaxThreads / 2);
     for (int i = 0; i < NS; ++i) {
       mbar_init(&slot_full[i], 1);
       mbar_init(&slot_free[i], 1);
@@ -396,7 +400,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
       if (ok) {
         constexpr uint32_t idesc_r = make_idesc_bf16_ab(128, D, 1, 1);
         constexpr uint32_t idesc_1 = make_idesc_bf16_ab(128, 16, 1, 0);
-        const DescHalves dtbt = make_desc_halves_sw128(smem_u32(TBS ? s_tbt_main : ring), HALF, 1024);
+        const DescHalves dtbt = make_desc_halves_sw128(smem_u32(s_tbt_main), HALF, 1024);
         const DescHalves dcbt = make_desc_halves_sw128(smem_u32(D == 128 ? sDO : ring + 98304), HALF, 1024);
         const DescHalves dqm = make_desc_halves_sw128(smem_u32(sQ), HALF, 1024);
         const DescHalves dones = make_desc_halves_sw128(smem_u32(ring + 32768), 16, 1024);
@@ -429,7 +433,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const int tt_base = (64 * wg) / CP;
     const int ck_base = CP == 128 ? 64 * wg : 0;
-    if constexpr (TBS) {  // slots no key tile reaches stay zero
+    {  // slots no key tile reaches stay zero
 #pragma unroll
       for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(s_tbt_main + tid * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -627,6 +631,17 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     }
     tc_fence_before();
     mbar_arrive(&bars[kBarProDone]);  // only now may a dP product overwrite the staged values
+    auto put_tb = [&](int sl, float x) {
+      *reinterpret_cast<__nv_bfloat16*>(s_tbt_main + (sl >> 6) * HALF + row * 128 + ((((sl & 63) >> 3) ^ (row & 7)) << 4) +
+                                        (sl & 7) * 2) = __float2bfloat16_rn(x);
+    };
+    float own_sum = 0.f;  // this warpgroup's part of the previous tile's sum, and its slot (PART, first warpgroup)
+    int own_slot = -1;
+    auto flush_part = [&](int s) -> bool {
+      if (!warp_wait(&bars[kBarTbPart + (s & 3)], (s >> 2) & 1, p.status, 137)) return false;
+      if (own_slot >= 0) put_tb(own_slot, own_sum + s_part[(s & 3) * 128 + row]);
+      return true;
+    };
     for (int s = 0; ok && s < n_tiles; ++s) {
       const bool dense = is_dense(s);
       const int J = tile_of(s);
@@ -719,21 +734,24 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
       }
       tc_fence_before();
       mbar_arrive(&bars[kBarDsFull + (s & 1)]);
-      // row sums per key time step; both warpgroups may own part of a time step (CP = 128)
-#pragma unroll
-      for (int tl = 0; tl < TPW; ++tl) {
-        if (valid[tl]) {
-          if constexpr (TBS) {
-            const int sl = slot[tl];
-            *reinterpret_cast<__nv_bfloat16*>(s_tbt_main + (sl >> 6) * HALF + row * 128 +
-                                              ((((sl & 63) >> 3) ^ (row & 7)) << 4) + (sl & 7) * 2) =
-                __float2bfloat16_rn(dtb_acc[tl]);
-          } else {
-            atomicAdd(&p.dtb[((int64_t)bh * T + slot[tl]) * N + n_loc], dtb_acc[tl]);
-          }
+      // row sums per key time step
+      if constexpr (PART) {
+        if (wg == 1) {
+          s_part[(s & 3) * 128 + row] = dtb_acc[0];
+          mbar_arrive(&bars[kBarTbPart + (s & 3)]);
+        } else {
+          if (s > 0) ok = flush_part(s - 1);
+          if (!ok) break;
+          own_sum = dtb_acc[0];
+          own_slot = valid[0] ? slot[0] : -1;
         }
+      } else {
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl)
+          if (valid[tl]) put_tb(slot[tl], dtb_acc[tl]);
       }
     }
+    if (PART && wg == 0 && ok) ok = flush_part(n_tiles - 1);
     // ------------------------------- epilogue ---------------------------------
     if (ok) ok = warp_wait(&bars[kBarAllDone], 0, p.status, 134);
     // du = sum over rows of dq's content part (`attentions/attn.py:1305-1306`: q + q_bias feeds the content
@@ -815,37 +833,17 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         tmem_st8(lane_base + kQDP + jb / 2 + m0, pkv);
       }
     }
-    if constexpr (!TBS) __threadfence();  // this CTA's atomic row sums in dtb are complete before anyone re-reads them
     softmax_bar();
     if (ok) {
       // dTB of the row (this thread's 64 of the 128 r_time rows) as bf16 pairs: A operand of dQ += dTB r_time
       // in TMEM, and the [row][j] tile in shared memory for the dr_time product
-      if constexpr (TBS) {
-        const uint8_t* my = s_tbt_main + wg * HALF + row * 128;
+      const uint8_t* my = s_tbt_main + wg * HALF + row * 128;
 #pragma unroll
-        for (int m8 = 0; m8 < 32; m8 += 8) {
-          const uint4 w0 = *reinterpret_cast<const uint4*>(my + (((m8 / 4) ^ (row & 7)) << 4));
-          const uint4 w1 = *reinterpret_cast<const uint4*>(my + (((m8 / 4 + 1) ^ (row & 7)) << 4));
-          const uint32_t pk[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-          tmem_st8(lane_base + kQS + 32 * wg + m8, pk);
-        }
-      } else {
-        const float* src = p.dtb + ((int64_t)bh * T + 64 * wg) * N + (row_valid ? n_loc : 0);
-        const float keep = row_valid ? 1.f : 0.f;
-        uint8_t* s_tbt = ring + wg * HALF + row * 128;  // (the scatter area is dead)
-        float a[64];  // every load in flight at once
-#pragma unroll
-        for (int jl = 0; jl < 64; ++jl) a[jl] = (64 * wg + jl < T) ? __ldcg(src + (int64_t)jl * N) : 0.f;
-#pragma unroll
-        for (int m8 = 0; m8 < 32; m8 += 8) {
-          uint32_t pk[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) pk[e] = pack_bf16(a[2 * (m8 + e)] * keep, a[2 * (m8 + e) + 1] * keep);
-          tmem_st8(lane_base + kQS + 32 * wg + m8, pk);
-          const int c0 = m8 / 4;  // 16-byte chunks c0 and c0 + 1 of this row's 128 bytes
-          *reinterpret_cast<uint4*>(s_tbt + (((c0) ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          *reinterpret_cast<uint4*>(s_tbt + (((c0 + 1) ^ (row & 7)) << 4)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        }
+      for (int m8 = 0; m8 < 32; m8 += 8) {
+        const uint4 w0 = *reinterpret_cast<const uint4*>(my + (((m8 / 4) ^ (row & 7)) << 4));
+        const uint4 w1 = *reinterpret_cast<const uint4*>(my + (((m8 / 4 + 1) ^ (row & 7)) << 4));
+        const uint32_t pk[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        tmem_st8(lane_base + kQS + 32 * wg + m8, pk);
       }
       // a [16 x 128] tile of ones (K-major): column sums of dTB / dCB come out of the tensor core too
       *reinterpret_cast<uint4*>(ring + 32768 + tid * 16) = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
@@ -1597,14 +1595,14 @@ __global__ void __launch_bounds__(1024) tc_bwd_final_kernel(const FinArgs p) {
 //   blocks [0, n_delta)           delta[bh][i] = sum_d dO[i][d] O[i][d]  (`attentions/attn.py:1213`), HBM-bound: D / 8
 //                                 threads share a row, one 16-byte load of each tensor per thread
 //   the next Hkv blocks           the relative-product constants of one kv head (rel_const_row)
-//   the remaining blocks          zeros: status words, relative-key accumulators, temporal-score gradients
+//   the remaining blocks          zeros: status words, relative-key accumulators
 constexpr int kPreThreads = 256;
 struct PreArgs {
   const __nv_bfloat16 *o, *d_o, *vt, *z, *rt, *rc;
   int64_t o_sb, o_sh, o_sn, do_sb, do_sh, do_sn;
   float *delta, *relc;
-  uint4* zero[3];
-  int64_t zero_n[3];  // 16-byte units
+  uint4* zero[2];
+  int64_t zero_n[2];  // 16-byte units
   int BH, H, Hkv, N, T, C, n_delta;
 };
 template <int D>
@@ -1639,7 +1637,7 @@ __global__ void __launch_bounds__(kPreThreads) tc_bwd_pre_kernel(const PreArgs p
   const int64_t first = (int64_t)(blk - p.Hkv) * kPreThreads + threadIdx.x;
   const int64_t step = ((int64_t)gridDim.x - p.n_delta - p.Hkv) * kPreThreads;
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int a = 0; a < 2; ++a)
     for (int64_t i = first; i < p.zero_n[a]; i += step) p.zero[a][i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
@@ -1653,7 +1651,7 @@ int launch(const BwdArgs& bw, float* cs_dq, int* status, float* relc, unsigned l
   BqArgs t;
   t.u = (const __nv_bfloat16*)a.u;
   t.relc = relc; t.lse = a.lse; t.delta = bw.delta;
-  t.cs_dq = cs_dq; t.dtb = bw.dtbg;
+  t.cs_dq = cs_dq;
   t.racc = racc; t.cacc = racc + (size_t)a.Hkv * 2 * D * 128;
   {
     const size_t rows = (size_t)a.B * a.H * a.N;
@@ -1680,15 +1678,11 @@ int launch(const BwdArgs& bw, float* cs_dq, int* status, float* relc, unsigned l
     pre.o_sb = a.o_sb; pre.o_sh = a.o_sh; pre.o_sn = a.o_sn;
     pre.do_sb = bw.do_sb; pre.do_sh = bw.do_sh; pre.do_sn = bw.do_sn;
     pre.delta = bw.delta; pre.relc = relc;
-    // (the areas end on 64-float boundaries; the temporal-score gradients may round up into the padding behind them)
     pre.zero[0] = reinterpret_cast<uint4*>(status); pre.zero_n[0] = 256 / 16;
     pre.zero[1] = reinterpret_cast<uint4*>(racc); pre.zero_n[1] = (int64_t)a.Hkv * (2 * D * 128 + 256) / 2;
-    // (the query-side kernel keeps these sums in shared memory where one thread owns each)
-    pre.zero[2] = reinterpret_cast<uint4*>(bw.dtbg);
-    pre.zero_n[2] = (D == 64 && CP <= 64) ? 0 : ((int64_t)a.B * a.H * a.N * a.T + 3) / 4;
     pre.BH = a.B * a.H; pre.H = a.H; pre.Hkv = a.Hkv; pre.N = a.N; pre.T = a.T; pre.C = a.C;
     pre.n_delta = (int)(((int64_t)pre.BH * a.N * (D / 8) + kPreThreads - 1) / kPreThreads);
-    const int64_t zeros = pre.zero_n[1] + pre.zero_n[2];
+    const int64_t zeros = pre.zero_n[1];
     const int64_t want = (zeros + 4 * kPreThreads - 1) / (4 * kPreThreads), most = 8 * (int64_t)device_sm_count();
     tc_bwd_pre_kernel<D><<<(unsigned)(pre.n_delta + a.Hkv + (want < most ? want : most)), kPreThreads, 0, s>>>(pre);
   }
