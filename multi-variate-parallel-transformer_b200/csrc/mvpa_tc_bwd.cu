@@ -150,9 +150,10 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   // which stores the sum one tile later, when the part has long arrived (four buffers: a part's place is written again
   // four tiles on, and the report of the tile after it lies between).
   constexpr bool PART = CP == 128;
-  // The prologue's scratch rows are padded instead of rotated when that fits (<= 64 channel slots).
-  constexpr bool PAD = CP <= 64;
-  constexpr int LDP = PAD ? CP + 2 : CP;
+  // The prologue's scratch rows are padded by two floats: slot C-1-|c_i - c_k| runs up the row for c_k <= c_i and down it
+  // for c_k > c_i, without bank conflicts either way.  (128 slots: the last kilobyte reaches into the tile of temporal
+  // sums, which is cleared once the scratch is dead.)
+  constexpr int LDP = CP + 2;
   static_assert(CP >= 32 && CP <= 128 && (CP & (CP - 1)) == 0, "CP in {32,64,128}");
 
   extern __shared__ __align__(1024) uint8_t smem_q[];
@@ -433,10 +434,6 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const int tt_base = (64 * wg) / CP;
     const int ck_base = CP == 128 ? 64 * wg : 0;
-    {  // slots no key tile reaches stay zero
-#pragma unroll
-      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(s_tbt_main + tid * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
     for (int d = tid; d < D; d += kSoftmaxThreads) s_bias[d] = __bfloat162float(p.u[hk * D + d]);
     s_vr[tid] = p.relc[hk * 256 + tid];  // s_vr and s_zc are adjacent: 256 floats
     // L = +inf on rows that do not exist: their P is 0 everywhere
@@ -465,15 +462,16 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         };
         const int j_tile = max(T - 1 - (I * TPB + TPB - 1), 0) - 64 * wg;  // first slot any row of the tile can see
         const int c_first = j_tile <= 0 ? 0 : (j_tile & ~15);
+        const int c_last = min(64, (T - 64 * wg + 15) & ~15);  // nothing past the last time step
         uint32_t va[8], vb[8];  // the next 8 columns are in flight while 8 are stored
-        if (c_first < 64) tmem_ld8(lane_base + kQDQ + 64 * wg + c_first, va);
+        if (c_first < c_last) tmem_ld8(lane_base + kQDQ + 64 * wg + c_first, va);
 #pragma unroll 1
-        for (int c8 = c_first; c8 < 64; c8 += 16) {
+        for (int c8 = c_first; c8 < c_last; c8 += 16) {
           tmem_ld_wait();
           tmem_ld8(lane_base + kQDQ + 64 * wg + c8 + 8, vb);
           put8(va, c8);
           tmem_ld_wait();
-          if (c8 + 16 < 64) tmem_ld8(lane_base + kQDQ + 64 * wg + c8 + 16, va);
+          if (c8 + 16 < c_last) tmem_ld8(lane_base + kQDQ + 64 * wg + c8 + 16, va);
           put8(vb, c8 + 8);
         }
       }
@@ -486,8 +484,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const float val = p.c2 * (__uint_as_float(v[e]) + s_zc[c8 + e]);
-          if constexpr (PAD) scratch[row * LDP + c8 + e] = val;
-          else scratch[row * CP + ((c8 + e + 2 * row) & (CP - 1))] = val;
+          scratch[row * LDP + c8 + e] = val;
         }
       }
       tc_fence_before();
@@ -497,27 +494,30 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     {
       // gather by key channel slot: g_k = CB[i, C-1-|c_i - c_k|]; first the row maximum, then fp16 values
       // relative to it, staged in this thread's own row of s_cbl (16-byte chunks swizzled by the row)
-      // (up to 64 channel slots: padded rows, slot C-1-|c_i - c_k| runs up through the row for c_k <= c_i
-      // and down for c_k > c_i; positions of channels that do not exist may lie outside the row and
-      // are dropped.  128 slots: rotated rows.)
-      const float* up = scratch + row * LDP + (C - 1 - c_i);
-      const float* down = scratch + row * LDP + (C - 1 + c_i);
-      const int climit = c_i < C ? C : 0;
+      // (positions of channels that do not exist may lie outside the row; their values are dropped)
+      const float* up = scratch + row * LDP + (C - 1 - c_i) + ck_base;
+      const float* down = scratch + row * LDP + (C - 1 + c_i) - ck_base;
+      const int kc = c_i - ck_base, climit = c_i < C ? C - ck_base : 0;
       auto gathered = [&](int k) {
-        if constexpr (PAD) {
-          const float val = ok ? (k <= c_i ? up[k] : down[-k]) : 0.f;
-          return k < climit ? val : -INFINITY;
-        } else {
-          const int ck = ck_base + k;
-          const int jc = min(max(C - 1 - abs(c_i - ck), 0), CP - 1);
-          const float val = ok ? scratch[row * CP + ((jc + 2 * row) & (CP - 1))] : 0.f;
-          return (c_i < C && ck < C) ? val : -INFINITY;
-        }
+        const float* src = k <= kc ? up + k : down - k;
+        return (ok && k < climit) ? *src : -INFINITY;
       };
+      // At 128 slots the values stay in registers (12 -> 9 k cycles for the whole step); below, where the step is shorter, a
+      // second walk in a short loop is the faster form (8.0 against 9.3 k cycles at 32 slots).
+      constexpr bool KEEP = CP == 128;
+      float gv[KEEP ? NCH : 1];
       float mx = -INFINITY;
+      if constexpr (KEEP) {
+#pragma unroll
+        for (int k = 0; k < NCH; ++k) {
+          gv[k] = gathered(k);
+          mx = fmaxf(mx, gv[k]);
+        }
+      } else {
 #pragma unroll 4
-      for (int k = 0; k < NCH; ++k) mx = fmaxf(mx, gathered(k));
-      if constexpr (!PAD) {  // the row maximum spans both warpgroups' columns
+        for (int k = 0; k < NCH; ++k) mx = fmaxf(mx, gathered(k));
+      }
+      if constexpr (CP == 128) {  // the row maximum spans both warpgroups' columns
         s_max[wg * 128 + row] = mx;
         softmax_bar();
         mx = fmaxf(mx, s_max[(wg ^ 1) * 128 + row]);
@@ -525,12 +525,12 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
       mc = (mx == -INFINITY) ? 0.f : mx;
       // fp16 pairs relative to the maximum, staged in this thread's lane of idle TMEM columns so that the
       // loop stays short and the values still end up in registers
-#pragma unroll 1
-      for (int k16 = 0; k16 < NCH; k16 += 16) {
+      auto stage = [&](int k16) {
         uint32_t pk[8], pb[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float x0 = gathered(k16 + 2 * e) - mc, x1 = gathered(k16 + 2 * e + 1) - mc;
+          const float x0 = (KEEP ? gv[KEEP ? k16 + 2 * e : 0] : gathered(k16 + 2 * e)) - mc;
+          const float x1 = (KEEP ? gv[KEEP ? k16 + 2 * e + 1 : 0] : gathered(k16 + 2 * e + 1)) - mc;
           const __half2 hh2 = __floats2half2_rn(x0, x1);
           const __half2 eh2 = __floats2half2_rn(ex2(x0), ex2(x1));
           pk[e] = *reinterpret_cast<const uint32_t*>(&hh2);
@@ -553,7 +553,18 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
           bdst[0] = make_uint4(wb[0], wb[1], wb[2], wb[3]);
           bdst[N] = make_uint4(wb[4], wb[5], wb[6], wb[7]);
         }
+      };
+      if constexpr (KEEP) {
+#pragma unroll
+        for (int k16 = 0; k16 < NCH; k16 += 16) stage(k16);
+      } else {
+#pragma unroll 1
+        for (int k16 = 0; k16 < NCH; k16 += 16) stage(k16);
       }
+      // the tile of temporal sums: slots no key tile reaches stay zero (at 128 channel slots the barrier above stands after
+      // every read of the scratch that reaches into it)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(s_tbt_main + tid * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
       tmem_st_wait();  // the staged values are read back where they are needed (light phase: bc; dense phase: cbl)
       tc_fence_before();
       const bool store_cbl = ok && row_valid && (CP == 128 || wg == 0);
@@ -789,17 +800,28 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     }
     softmax_bar();
     // channel-score gradient: from key-channel slots to |c_i - c_k| slots, through shared memory
-    float* sc = reinterpret_cast<float*>(ring);  // [128][CP]; every TMA load has been consumed by now
-    if (CP == 128 || wg == 0) {
+    // (rows without bank conflicts on either diagonal: padded by two floats up to 64 slots, rotated at 128, where padded
+    // ones would reach into the relative keys that arrive behind)
+    constexpr bool ROT = CP == 128;
+    float* sc = reinterpret_cast<float*>(ring) + row * (ROT ? CP : LDP);  // every TMA load has been consumed by now
+    if constexpr (ROT) {
 #pragma unroll
-      for (int k = 0; k < NCH; ++k) sc[row * CP + ((ck_base + k + 2 * row) & (CP - 1))] = dcb_acc[k];
+      for (int k = 0; k < NCH; ++k) sc[(ck_base + k + 2 * row) & (CP - 1)] = dcb_acc[k];
+    } else if (wg == 0) {
+#pragma unroll
+      for (int k = 0; k < NCH; k += 2) *reinterpret_cast<float2*>(sc + k) = make_float2(dcb_acc[k], dcb_acc[k + 1]);
     }
     softmax_bar();
-    if (CP < 128 && wg == 1) {  // both warpgroups hold sums for the same channel slots (different time steps)
+    if constexpr (!ROT) {  // both warpgroups hold sums for the same channel slots (different time steps)
+      if (wg == 1) {
 #pragma unroll
-      for (int k = 0; k < NCH; ++k) sc[row * CP + ((k + 2 * row) & (CP - 1))] += dcb_acc[k];
+        for (int k = 0; k < NCH; k += 2) {
+          float2* d = reinterpret_cast<float2*>(sc + k);
+          *d = fadd2(*d, make_float2(dcb_acc[k], dcb_acc[k + 1]));
+        }
+      }
+      softmax_bar();
     }
-    softmax_bar();
     // dCB[i, j], j = C-1-e, e = |c_i - c_k|, as bf16 pairs: into TMEM columns kQDP + j/2 (A operand of
     // dQ += dCB r_chan) and into a shared-memory tile [row][j] (A operand, transposed, of the dr_chan product).
     // Each warpgroup takes half of the slots.
@@ -817,11 +839,18 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
 #pragma unroll
           for (int t2 = 0; t2 < 2; ++t2) {
             const int j = jb + 2 * m + t2, e = C - 1 - j;
-            // both candidates are read from wrapped (always valid) positions and masked: no divergence
-            const float lo = sc[row * CP + ((c_i - e + 2 * row) & (CP - 1))];
-            const float hi = sc[row * CP + ((c_i + e + 2 * row) & (CP - 1))];
-            const bool on = row_valid && e >= 0;
-            vv[t2] = ((on && c_i - e >= 0) ? lo : 0.f) + ((on && e > 0 && c_i + e < C) ? hi : 0.f);
+            const bool on = row_valid && e >= 0, on_lo = on && e <= c_i, on_hi = on && e > 0 && c_i + e < C;
+            float lo, hi;
+            if constexpr (ROT) {  // read from wrapped (always valid) positions and masked: no divergence
+              lo = sc[(c_i - e + 2 * row) & (CP - 1)];
+              hi = sc[(c_i + e + 2 * row) & (CP - 1)];
+              lo = on_lo ? lo : 0.f;
+              hi = on_hi ? hi : 0.f;
+            } else {
+              lo = on_lo ? sc[c_i - e] : 0.f;
+              hi = on_hi ? sc[c_i + e] : 0.f;
+            }
+            vv[t2] = lo + hi;
           }
           pkv[mi] = pack_bf16(vv[0], vv[1]);
           const int j = jb + 2 * m;
