@@ -36,6 +36,17 @@ def expression(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, e
     return x + mlp + F.linear(o.permute(0, 2, 1, 3).reshape(B, T, C, E), wc)
 
 
+def through_expression(f, ins, need, grad_out):
+    """Gradients of f(*ins) for `grad_out`, differentiable if gradients are recorded; None where `need` is False.
+    They are taken with respect to aliases of `ins`: an input's own history may lead to another input (a later block's x
+    depends on the embeddings that it also receives), and autograd would follow it and return total derivatives."""
+    create = torch.is_grad_enabled()
+    with torch.enable_grad():
+        local = [t.view_as(t) if t.requires_grad else t.detach().requires_grad_(n) for t, n in zip(ins, need)]
+        got = iter(torch.autograd.grad(f(*local), [t for t, n in zip(local, need) if n], grad_out, create_graph=create))
+    return [next(got) if n else None for n in need]
+
+
 def _heads_view(t, B, N, heads, D):
     """(B*N, heads*D) columns as the kernels' (B, heads, N, D)."""
     return t.view(B, N, heads, D).permute(0, 2, 1, 3)
@@ -72,11 +83,8 @@ class BlockFunction(torch.autograd.Function):
         need = ctx.needs_input_grad[:13]
         if torch.is_grad_enabled() or not _nat.untraced() or not mvpa_ops._plain(dh.contiguous()):
             # a graph of the gradient is wanted (or a transform is active): through the differentiable operations
-            with torch.enable_grad():
-                ins = [t if t.requires_grad else t.detach().requires_grad_(n) for t, n in zip(saved[:13], need)]
-                out = expression(*ins, ctx.eps, ctx.heads)
-                got = iter(torch.autograd.grad(out, [t for t, n in zip(ins, need) if n], dh, create_graph=True))
-            return (*(next(got) if n else None for n in need), None, None)
+            grads = through_expression(lambda *ins: expression(*ins, ctx.eps, ctx.heads), saved[:13], need, dh)
+            return (*grads, None, None)
         x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act = saved
         H, Hkv, D = ctx.heads
         B, T, C, E = x.shape

@@ -5,6 +5,7 @@ import torch
 
 import models
 from eeg_datasets import synthetic_ieeg
+from models import block_grad
 from test_model_oracle import load_model_golden
 
 
@@ -63,3 +64,46 @@ def test_synthetic_ieeg_is_seeded_pink_and_bursty():
     slope = np.log(p[:, hi].mean() / p[:, lo].mean()) / np.log(f[hi].mean() / f[lo].mean())
     assert -1.3 < slope < -0.7                                                   # power ~ 1/f
     assert float(a.abs().max()) > 4.0 > float(quiet.abs().max()) * 0.8           # bursts stand out of the background
+
+
+class _Step(torch.autograd.Function):
+    """A block whose backward always goes through the differentiable expression: x + tanh(x * e) * w."""
+    calls = 0
+
+    @staticmethod
+    def f(x, e, w):
+        return x + torch.tanh(x * e) * w
+
+    @staticmethod
+    def forward(ctx, x, e, w):
+        ctx.save_for_backward(x, e, w)
+        return _Step.f(x, e, w)
+
+    @staticmethod
+    def backward(ctx, dy):
+        _Step.calls += 1
+        return tuple(block_grad.through_expression(_Step.f, ctx.saved_tensors, ctx.needs_input_grad, dy))
+
+
+def test_gradients_through_the_expression_stop_at_the_block():
+    """Stacked blocks that share a non-leaf input: first and second derivatives, one backward call per block."""
+    g = torch.Generator().manual_seed(0)
+    x, w, a = (torch.randn(3, dtype=torch.float64, generator=g, requires_grad=True) for _ in range(3))
+    ins, dy = (x, w, a), torch.randn(3, dtype=torch.float64, generator=g)
+
+    def run(step):
+        e, y = a * 2, x
+        for _ in range(6):
+            y = step(y, e, w)
+        first = torch.autograd.grad(y, ins, dy, create_graph=True)
+        return first, torch.autograd.grad(sum((t * t).sum() for t in first), ins)
+
+    _Step.calls = 0
+    plain = torch.autograd.grad(_Step.apply(x, a * 2, w), ins, dy)
+    assert _Step.calls == 1 and not any(t.requires_grad for t in plain)
+    _Step.calls = 0
+    got = run(_Step.apply)
+    assert _Step.calls <= 6 + 6          # (the second derivative may run each block's graph, never the blocks below it)
+    for p, q in zip(got, run(_Step.f)):
+        for s, t in zip(p, q):
+            torch.testing.assert_close(s, t, rtol=1e-12, atol=1e-12)
