@@ -110,17 +110,24 @@ def _need_cuda(q):
         raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
 
 
+def _lay_out(q, u, vt, z, k, r_time, r_chan, v):
+    """The operands as the kernels read them, copied only where their layout asks for it."""
+    _need_cuda(q)
+    return (_rows(q), u.contiguous(), vt.contiguous(), z.contiguous(), _rows(k), r_time.contiguous(), r_chan.contiguous(),
+            _rows(v))
+
+
 class FlashMVPA(torch.autograd.Function):
     """Autograd wrapper; the counterpart of the reference's `FlashMVPA`
     (`attentions/attn.py:1013-1302`), taking the relative keys themselves instead of
     pre-multiplied score matrices.  The small tensors may have any shape with their elements in
-    (kv head, row, D) order, r_time and r_chan with the rows next to last; their gradients take that shape."""
+    (kv head, row, D) order, r_time and r_chan with the rows next to last; their gradients take that shape.
+    Second derivatives reach the operands that the kernels read in place (`flash_mvpa` lays the others out first)."""
 
     @staticmethod
-    def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0)):
-        _need_cuda(q)
-        q, k, v = _rows(q), _rows(k), _rows(v)
-        u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
+    def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0), laid_out=False):
+        if not laid_out:
+            q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v)
         o = torch.empty_like(q)
         lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
         ctx.save_for_backward(q, u, vt, z, k, r_time, r_chan, v, o, lse)
@@ -129,15 +136,82 @@ class FlashMVPA(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do):
-        q, u, vt, z, k, r_time, r_chan, v, o, lse = ctx.saved_tensors
         if ctx.q_time[1]:
             raise NotImplementedError("flash_mvpa: backward through a query time range is not implemented")
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        small = _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, _rows(do), dq, dk, dv, ctx.sm_scale, ctx.window)
-        shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]
-        sizes = [sh.numel() for sh in shapes]
-        du, dvt, dz, drt, drc = (piece.view(sh) for piece, sh in zip(small.split(sizes), shapes))
-        return (dq, du, dvt, dz, dk, drt, drc, dv, None, None, None)
+        if torch.is_grad_enabled():  # a graph of the gradient is wanted
+            return (*_FlashMVPAGrad.apply(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None, None)
+        return (*_gradients(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None, None)
+
+
+def _gradients(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window):
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    small = _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, _rows(do), dq, dk, dv, sm_scale, window)
+    shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]
+    sizes = [sh.numel() for sh in shapes]
+    du, dvt, dz, drt, drc = (piece.view(sh) for piece, sh in zip(small.split(sizes), shapes))
+    return dq, du, dvt, dz, dk, drt, drc, dv
+
+
+class _FlashMVPAGrad(torch.autograd.Function):
+    """The backward of `FlashMVPA` as a function of its own: the same kernels, and a derivative, taken in 64 bits on the
+    materialised scores of one (sample, kv head) after the other.  Gradient penalties and Hessian products at sizes where
+    (query heads per kv head, N, N) fits; the kernels have no second derivative."""
+
+    @staticmethod
+    def forward(ctx, do, *operands):
+        ctx.save_for_backward(do, *operands[:8])
+        ctx.sm_scale, ctx.window = operands[-2:]
+        return _gradients(do, *operands)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        create = torch.is_grad_enabled()
+        with torch.enable_grad():
+            ins = [t.view_as(t) if t.requires_grad else t for t in ctx.saved_tensors]
+            q, k, T, C = ins[1], ins[5], ins[6].shape[-2], ins[7].shape[-2]
+            (B, H, N, D), Hkv = q.shape, k.shape[1]
+            rows = {0: N, 1: N, 5: N, 6: T, 7: C, 8: N}      # (the three biases: one row)
+
+            def parts(t, i, b, j):   # what kv head j of sample b reads of operand i (or of its gradient), in 64 bits
+                if i in (0, 1):
+                    return t[b, j * (H // Hkv):(j + 1) * (H // Hkv)].double()
+                return (t[b, j] if i in (5, 8) else t.reshape(Hkv, rows.get(i, 1), D)[j]).double()
+
+            out = [[[None] * Hkv for _ in range(B)] for _ in ins]
+            for b in range(B):
+                for j in range(Hkv):
+                    local = [parts(t, i, b, j) for i, t in enumerate(ins)]
+                    local = [t if t.requires_grad else t.requires_grad_() for t in local]
+                    o = _dense_head(*local[1:], ctx.sm_scale, ctx.window)
+                    first = torch.autograd.grad(o, local[1:], local[0], create_graph=True)
+                    inner = sum((f * parts(g, i + 1, b, j)).sum() for i, (f, g) in enumerate(zip(first, grads)))
+                    for i, t in enumerate(torch.autograd.grad(inner, local, create_graph=create)):
+                        out[i][b][j] = t
+            res = []
+            for i, t in enumerate(ins):
+                if i in (0, 1):
+                    whole = torch.stack([torch.cat(per_b) for per_b in out[i]])
+                elif i in (5, 8):
+                    whole = torch.stack([torch.stack(per_b) for per_b in out[i]])
+                else:
+                    whole = torch.stack([sum(per_b[j] for per_b in out[i]) for j in range(Hkv)])
+                res.append(whole.reshape(t.shape).to(t.dtype))
+        return (*res, None, None, None, None)
+
+
+def _dense_head(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window):
+    """The operator for one kv head on materialised scores, in differentiable operations: q (heads, N, D), k, v (N, D)."""
+    T, C = r_time.shape[0], r_chan.shape[0]
+    n = torch.arange(T * C, device=q.device)
+    t, c = n // C, n % C
+    dt = t[:, None] - t[None, :]
+    at = lambda x, index: x.gather(-1, index.expand(*x.shape[:-1], index.shape[-1]))
+    s = (q + u) @ k.t()
+    if window > 0:
+        s = s.masked_fill((dt.abs() > window) & (t[:, None] != T - 1), 0.0)
+    s = s + at((q + vt) @ r_time.t(), (T - 1 - dt).clamp(max=T - 1)) \
+        + at((q + z) @ r_chan.t(), C - 1 - (c[:, None] - c[None, :]).abs())
+    return torch.softmax((s * sm_scale).masked_fill(dt < 0, -math.inf), -1) @ v
 
 
 def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
@@ -145,12 +219,11 @@ def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
     of a small call, so an ordinary call that no gradient flows through goes to the kernels directly (and stores no
     log-sum-exp); whatever traces or transforms the call sees the autograd function."""
     ts = (q, u, vt, z, k, r_time, r_chan, v)
-    if ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or not _nat.untraced()
-            or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts)):
+    if not _nat.untraced() or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts):
         return FlashMVPA.apply(*ts, sm_scale, window, q_time)
-    _need_cuda(q)
-    q, k, v = _rows(q), _rows(k), _rows(v)
-    u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
+    q, u, vt, z, k, r_time, r_chan, v = _lay_out(*ts)
+    if torch.is_grad_enabled() and any(t.requires_grad for t in ts):
+        return FlashMVPA.apply(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time, True)
     o = torch.empty_like(q)
     _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, False)
     return o
@@ -162,9 +235,7 @@ def flash_mvpa_into(out, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window_siz
     next projection reads).  u, vt, z (Hkv,D); r_time (Hkv,T,D); r_chan (Hkv,C,D).  `q_time_range=(t0, n)`:
     `q` and `out` hold only the tokens of time steps t0..t0+n-1 (see `flash_mvpa`).  No counterpart in the
     reference, whose operator always allocates its output (`attentions/attn.py:1047`)."""
-    _need_cuda(q)
-    q, k, v = _rows(q), _rows(k), _rows(v)
-    u, vt, z, r_time, r_chan = (x.contiguous() for x in (u, vt, z, r_time, r_chan))
+    q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v)
     if not _aligned(out) or out.shape != q.shape:
         raise RuntimeError("flash_mvpa_into: `out` must have q's shape, a contiguous last dimension and 16-byte aligned strides")
     q_time = (0, 0) if q_time_range is None else (int(q_time_range[0]), int(q_time_range[1]))

@@ -1,8 +1,12 @@
-"""GPU: the one-function block against the modules where a graph of the gradient is built."""
+"""GPU: gradients of gradients through the operator and the one-function block, against 64-bit dense torch and against the
+modules."""
 import pytest
 import torch
+import torch.nn.functional as F
 
+import attentions
 import models
+import mvpa_port_torch as port
 
 pytestmark = pytest.mark.gpu
 
@@ -41,6 +45,26 @@ class _Stack(torch.nn.Module):
         return [p for n, p in self.named_parameters() if "ln_2" not in n]
 
 
+def _stack64(stack, x):
+    """The same in plain torch at the inputs' precision, dense attention; nothing of the package's arithmetic."""
+    pos, chan = stack.embeddings(x.shape[1], x.shape[2])
+    B, T, C, E = x.shape
+    N = T * C
+    for block in stack.h:
+        a, m = block.attn, block.mlp
+        H, Hkv, D = a.num_heads, a.num_kv_heads, a.head_dim
+        xn = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + block.ln_1.eps) * block.ln_1.weight
+        q = F.linear(xn, a.q_attn.weight).view(B, N, H, D).transpose(1, 2)
+        k, v = (t.transpose(1, 2) for t in F.linear(xn, a.c_attn.weight).view(B, N, 2 * Hkv, D).split(Hkv, dim=2))
+        rt = F.linear(pos, a.position_net.weight).view(T, Hkv, D).transpose(0, 1)
+        rc = F.linear(chan, a.channel_net.weight).view(C, Hkv, D).transpose(0, 1)
+        u, vt, z = (b.view(Hkv, D) for b in a.attn_bias.split(Hkv * D))
+        o = port.rel_attn(q, u, vt, z, k, rt, rc, v, D ** -0.5, 10).transpose(1, 2).reshape(B, T, C, E)
+        mlp = F.linear(F.silu(F.linear(xn, m.gate_proj.weight)) * F.linear(xn, m.up_proj.weight), m.down_proj.weight)
+        x = x + mlp + F.linear(o, a.c_proj.weight)
+    return x
+
+
 def _hook(stack):
     return [b.mlp.register_forward_hook(lambda *a: None) for b in stack.h]
 
@@ -64,3 +88,61 @@ def test_graph_of_the_gradient_stops_at_each_block(cuda):
         h.remove()
     for a, b, c in zip(plain, graphed, ref):
         assert _rel(a, c) <= 1e-5 and _rel(b, c) <= 1e-5
+
+
+# The derivative of a gradient penalty with respect to everything, through two blocks, on both routes.  fp32 against 64 bits:
+# a chain of a few dozen products, each of at most 80 terms rounded to 2^-24 and each condition number of order one.
+@pytest.mark.parametrize("hooked", [False, True])
+def test_gradient_penalty_against_64_bits(cuda, hooked):
+    torch.manual_seed(1)
+    stack = _Stack(2).to(cuda)
+    x = torch.randn(1, 13, 3, 64, device=cuda, requires_grad=True)
+    dy = torch.randn(1, 13, 3, 64, device=cuda)
+
+    def penalty_gradients(f, mod, x, dy):
+        ins = [x, *mod.used()]
+        first = torch.autograd.grad(f(x), ins, dy, create_graph=True)
+        return torch.autograd.grad(sum((g * g).sum() for g in first), ins)
+
+    handles = _hook(stack) if hooked else []
+    got = penalty_gradients(stack, stack, x, dy)
+    for h in handles:
+        h.remove()
+    s64 = _Stack(2).to(cuda).double()
+    s64.load_state_dict({k: v.double() for k, v in stack.state_dict().items()})
+    want = penalty_gradients(lambda t: _stack64(s64, t), s64, x.detach().double().requires_grad_(), dy.double())
+    for a, b in zip(got, want):
+        assert _rel(a, b) <= 2e-5
+
+
+def _operands(B, H, Hkv, T, C, D, dtype, cuda, strided):
+    g = torch.Generator().manual_seed(T * 100 + C)
+    r = lambda *s, std=1.0: (torch.randn(*s, generator=g) * std).to(dtype).to(cuda)
+    N = T * C
+    a = [r(B, H, N, D), r(1, Hkv, 1, D), r(1, Hkv, 1, D), r(1, Hkv, 1, D), r(B, Hkv, N, D), r(1, Hkv, T, D), r(1, Hkv, C, D),
+         r(B, Hkv, N, D)]
+    if strided:   # token-major storage (read in place), and an odd row stride and reversed axes (copied)
+        a[0] = a[0].transpose(1, 2).contiguous().transpose(1, 2)
+        a[4] = torch.cat([a[4], a[4][..., :1]], -1)[..., :D]
+        a[5] = a[5].transpose(1, 2).contiguous().transpose(1, 2)
+    return a, r(B, H, N, D)
+
+
+# One head, several, grouped; one time step, steps beyond the window (masked content), one channel.  16-bit types: the
+# first derivatives are rounded once (2^-8, 2^-11) before they are squared, and the result once more.
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2), (torch.float16, 4e-3)])
+@pytest.mark.parametrize("shape,strided", [((1, 1, 1, 1, 3, 16), False), ((2, 4, 2, 14, 3, 32), True), ((1, 2, 1, 15, 1, 64), False)])
+def test_operator_second_derivative(cuda, dtype, tol, shape, strided):
+    args, do = _operands(*shape, dtype, cuda, strided)
+    D = shape[-1]
+
+    def second(f, args, do):
+        ins = [t.detach().requires_grad_() for t in (*args, do)]
+        first = torch.autograd.grad(f(*ins[:-1]), ins[:-1], ins[-1], create_graph=True)
+        return torch.autograd.grad(sum((g.double() * g).sum() for g in first), ins)
+
+    got = second(lambda *a: attentions.flashmvpa(*a, True, D ** -0.5, window_size=10), args, do)
+    want = second(lambda *a: port.rel_attn(*a, D ** -0.5, 10), [t.double() for t in args], do.double())
+    for a, t, b in zip(got, (*args, do), want):
+        assert a.dtype == dtype and a.shape == t.shape
+        assert (a.double() - b).norm() <= tol * max(b.norm().item(), 1.0)
