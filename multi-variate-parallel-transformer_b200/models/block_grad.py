@@ -12,6 +12,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
+import layers.mvpa as _layer
 import mvpa_native as _nat
 import mvpa_ops
 from attentions import attn as _attn
@@ -120,25 +121,37 @@ class BlockFunction(torch.autograd.Function):
         return (*grad, None, None)
 
 
-def _unhooked(m, cls):
-    return (type(m) is cls and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks
-            and not m._backward_hooks and not m._backward_pre_hooks)
+def shipped(cls):
+    """A module class with the code that it came with; a later replacement of its `forward` shows against it."""
+    return cls, cls.forward
+
+
+_LINEAR, _DROPOUT = shipped(torch.nn.Linear), shipped(torch.nn.Dropout)
+_ATTENTION = _layer.MVPFormerGQAAttention._mvpa_forward
+
+
+def _unhooked(m, code):
+    cls, forward = code
+    return (type(m) is cls and cls.forward is forward and "forward" not in m.__dict__ and not m._forward_hooks
+            and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
 
 
 def applies(block, x, pos, chan, classes) -> bool:
-    """Whether `block` is exactly the computation above on tensors the kernels take in place: the shipped modules, none of
-    them replaced, hooked or patched, no dropout or autocast, one dtype, contiguous and 16-byte aligned, and nothing
-    tracing the call.  Everything else goes through the modules."""
-    norm_cls, attn_cls, mlp_cls = classes
+    """Whether `block` is exactly the computation above on tensors the kernels take in place: the shipped modules (norm,
+    attention and MLP in `classes`, as `shipped` returned them), neither they nor their code replaced, hooked or patched,
+    no dropout or autocast, one dtype, contiguous and 16-byte aligned, and nothing tracing the call.  Everything else goes
+    through the modules."""
+    norm, attn, mlp = classes
     a, m = block.attn, block.mlp
-    linears = (a.q_attn, a.c_attn, a.position_net, a.channel_net, a.c_proj, m.gate_proj, m.up_proj, m.down_proj) \
-        if type(a) is attn_cls and type(m) is mlp_cls else ()
-    if not linears or not _unhooked(block.ln_1, norm_cls) or not _unhooked(a, attn_cls) or not _unhooked(m, mlp_cls):
+    if not (_unhooked(block.ln_1, norm) and _unhooked(a, attn) and _unhooked(m, mlp)):
         return False
-    if not all(_unhooked(l, torch.nn.Linear) and l.bias is None for l in linears):
+    if getattr(a._mvpa_forward, "__func__", None) is not _ATTENTION or _layer.flashmvpa is not flashmvpa:
+        return False
+    linears = (a.q_attn, a.c_attn, a.position_net, a.channel_net, a.c_proj, m.gate_proj, m.up_proj, m.down_proj)
+    if not all(_unhooked(l, _LINEAR) and l.bias is None for l in linears):
         return False
     for d in (a.attn_dropout, a.resid_dropout):
-        if not _unhooked(d, torch.nn.Dropout) or (d.training and d.p):
+        if not _unhooked(d, _DROPOUT) or (d.training and d.p):
             return False
     if a.training and a.attn_dropout.p or torch.nn.modules.module._has_any_global_hook() or torch.is_autocast_enabled("cuda"):
         return False

@@ -91,6 +91,9 @@ class LlamaMLP(torch.nn.Module):
         return self.down_proj(mvpa_ops.swiglu(self.gate_proj(x), self.up_proj(x)))
 
 
+_SHIPPED = tuple(block_grad.shipped(cls) for cls in (RMSNorm, MVPFormerGQAFlashAttention, LlamaMLP))
+
+
 class MVPFormerBlock(torch.nn.Module):
     def __init__(self, config, layer_idx=None):
         super().__init__()
@@ -106,8 +109,7 @@ class MVPFormerBlock(torch.nn.Module):
         """The reference's op order (`models/mvpformer.py:132-152`); differentiable.  With gradients, and nothing
         replaced, hooked or dropped out, the whole block is one autograd function (`block_grad`)."""
         if (torch.is_grad_enabled() and not use_cache and not output_attentions
-                and block_grad.applies(self, hidden_states, positional_embedding, channel_embedding,
-                                       (RMSNorm, MVPFormerGQAFlashAttention, LlamaMLP))):
+                and block_grad.applies(self, hidden_states, positional_embedding, channel_embedding, _SHIPPED)):
             return (block_grad.run(self, hidden_states, positional_embedding, channel_embedding),)
         residual = hidden_states
         hidden_states = self.ln_1(hidden_states)

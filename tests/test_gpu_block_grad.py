@@ -1,12 +1,14 @@
 """GPU: gradients of gradients through the operator and the one-function block, against 64-bit dense torch and against the
-modules."""
+modules, and the blocks that must keep going through their modules."""
 import pytest
 import torch
 import torch.nn.functional as F
 
 import attentions
+import layers.mvpa as layer_module
 import models
 import mvpa_port_torch as port
+from models import mvpformer
 
 pytestmark = pytest.mark.gpu
 
@@ -146,3 +148,35 @@ def test_operator_second_derivative(cuda, dtype, tol, shape, strided):
     for a, t, b in zip(got, (*args, do), want):
         assert a.dtype == dtype and a.shape == t.shape
         assert (a.double() - b).norm() <= tol * max(b.norm().item(), 1.0)
+
+
+def _block(cuda, E=64, H=4, Hkv=2):
+    torch.manual_seed(0)
+    stack = _Stack(1, E=E, H=H, Hkv=Hkv).to(cuda)
+    pos, chan = stack.embeddings(6, 5)
+    return stack.h[0], torch.randn(1, 6, 5, E, device=cuda), pos, chan
+
+
+def test_replaced_code_is_not_bypassed(cuda, monkeypatch):
+    block, x, pos, chan = _block(cuda)
+    assert _one_function(block(x, pos, chan)[0])
+    calls = []
+
+    def seen(f):
+        def g(*a, **k):
+            calls.append(f)
+            return f(*a, **k)
+        return g
+
+    for owner, name in ((mvpformer.RMSNorm, "forward"), (mvpformer.LlamaMLP, "forward"), (torch.nn.Linear, "forward"),
+                        (torch.nn.Dropout, "forward"), (layer_module.MVPFormerGQAFlashAttention, "forward"),
+                        (layer_module.MVPFormerGQAAttention, "_mvpa_forward"), (layer_module, "flashmvpa")):
+        with monkeypatch.context() as m:
+            m.setattr(owner, name, seen(getattr(owner, name)))
+            calls.clear()
+            assert not _one_function(block(x, pos, chan)[0]) and calls, (owner, name)
+    with monkeypatch.context() as m:
+        m.setattr(block.attn, "_mvpa_forward", seen(block.attn._mvpa_forward))
+        calls.clear()
+        assert not _one_function(block(x, pos, chan)[0]) and calls
+    assert _one_function(block(x, pos, chan)[0])
