@@ -16,6 +16,8 @@ import threading
 from contextlib import nullcontext
 
 import torch
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
@@ -181,9 +183,12 @@ def on_device(device):
 
 
 def untraced() -> bool:
-    """No forward-mode level, functorch transform, tracer or compiler is watching the current call."""
+    """No forward-mode level, functorch transform, tracer, compiler or mode that sees each operation is watching the
+    current call.  (A default device is a function mode as well; it only fills in where new tensors live.)"""
     return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and not torch._C._len_torch_dispatch_stack()
+            and (not torch._C._len_torch_function_stack()
+                 or all(isinstance(m, DeviceContext) for m in _get_current_function_mode_stack())))
 
 
 def last_error() -> str:

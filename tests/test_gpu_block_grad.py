@@ -180,3 +180,28 @@ def test_replaced_code_is_not_bypassed(cuda, monkeypatch):
         calls.clear()
         assert not _one_function(block(x, pos, chan)[0]) and calls
     assert _one_function(block(x, pos, chan)[0])
+
+
+def test_recording_modes_see_the_operations(cuda):
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Ops(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Calls(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", str(func)))
+            return func(*args, **(kwargs or {}))
+
+    block, x, pos, chan = _block(cuda)
+    for mode in (Ops, Calls):
+        seen = []
+        with mode():
+            y = block(x, pos, chan)[0]
+        assert not _one_function(y)
+        assert any("silu" in s for s in seen) and any("rsqrt" in s for s in seen) and any("pow" in s for s in seen)
+    with torch.device(cuda):   # a default device is a function mode too, but watches nothing
+        assert _one_function(block(x, pos, chan)[0])
