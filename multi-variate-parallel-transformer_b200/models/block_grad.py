@@ -155,6 +155,8 @@ def applies(block, x, pos, chan, classes) -> bool:
             return False
     if a.training and a.attn_dropout.p or torch.nn.modules.module._has_any_global_hook() or torch.is_autocast_enabled("cuda"):
         return False
+    if a.head_dim not in (16, 32, 64, 128) or a.num_heads % a.num_kv_heads:
+        return False                 # (what the operator refuses is refused by the operator)
     if x.dim() != 4 or pos.shape != (1, x.shape[1], x.shape[3]) or chan.shape != (1, x.shape[2], x.shape[3]):
         return False
     ts = (x, pos, chan, block.ln_1.weight, a.attn_bias, *(l.weight for l in linears))

@@ -205,3 +205,10 @@ def test_recording_modes_see_the_operations(cuda):
         assert any("silu" in s for s in seen) and any("rsqrt" in s for s in seen) and any("pow" in s for s in seen)
     with torch.device(cuda):   # a default device is a function mode too, but watches nothing
         assert _one_function(block(x, pos, chan)[0])
+
+
+@pytest.mark.parametrize("E,H,Hkv", [(96, 2, 1), (96, 6, 4)])   # head_dim 48; query heads that no kv head divides
+def test_refused_heads_are_refused_alike(cuda, E, H, Hkv):
+    block, x, pos, chan = _block(cuda, E=E, H=H, Hkv=Hkv)
+    with pytest.raises(AssertionError):
+        block(x, pos, chan)
