@@ -34,14 +34,14 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 def _tensor(t: torch.Tensor) -> _nat.Tensor:
-    sb, sh, sn, _ = t.stride()
-    return _nat.Tensor(t.data_ptr(), sb, sh, sn)
+    strides = t.stride()
+    return _nat.Tensor(t.data_ptr(), strides[0], strides[1], strides[2])
 
 
 def _aligned(t: torch.Tensor) -> bool:
     """A contiguous last dimension, 16-byte aligned base and strides: what the kernels read in place."""
-    sb, sh, sn, sd = t.stride()
-    return sd == 1 and not (((sb | sh | sn) * t.element_size() | t.data_ptr()) & 15)
+    strides = t.stride()
+    return strides[-1] == 1 and not (((strides[0] | strides[1] | strides[2]) * t.element_size() | t.data_ptr()) & 15)
 
 
 def _rows(t: torch.Tensor) -> torch.Tensor:
@@ -175,7 +175,7 @@ class _FlashMVPAGrad(torch.autograd.Function):
             def parts(t, i, b, j):   # what kv head j of sample b reads of operand i (or of its gradient), in 64 bits
                 if i in (0, 1):
                     return t[b, j * (H // Hkv):(j + 1) * (H // Hkv)].double()
-                return (t[b, j] if i in (5, 8) else t.reshape(Hkv, rows.get(i, 1), D)[j]).double()
+                return (t.reshape(B, Hkv, N, D)[b, j] if i in (5, 8) else t.reshape(Hkv, rows.get(i, 1), D)[j]).double()
 
             out = [[[None] * Hkv for _ in range(B)] for _ in ins]
             for b in range(B):
@@ -303,6 +303,8 @@ def flash_mvpa(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, causal, s
     for x, n in ((q_bias, 1), (q_btime, 1), (q_bchan, 1), (k_time, time_ctx), (k_chan, chan_ctx)):
         if x.numel() != kv_heads * n * D:
             raise RuntimeError(f"flash_mvpa: shape {tuple(x.shape)} is invalid for {kv_heads} kv heads x {n} x {D}")
+    if k_time.dim() != 4 or k_chan.dim() != 4:   # (the kernels' sizes are read off the axis next to the last)
+        k_time, k_chan = k_time.reshape(1, kv_heads, time_ctx, D), k_chan.reshape(1, kv_heads, chan_ctx, D)
     o = _attend(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, sm_scale, window_size, q_time)
     if p_drop and p_drop > 0:
         o = (o.float() * (1.0 / (1 - p_drop))).to(o.dtype)

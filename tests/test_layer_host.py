@@ -66,3 +66,21 @@ def test_operator_refuses_cpu_tensors():
     with pytest.raises(AssertionError):
         attentions.flashmvpa(q, b, b, b, q, torch.zeros(1, 2, 3, 16), torch.zeros(1, 2, 2, 16), q,
                              causal=True, sm_scale=0.25)
+
+
+def test_operands_with_an_axis_of_one_more(monkeypatch):
+    """Relative keys, keys and values may carry a further axis of one: sizes and strides are those of the axes before it."""
+    from attentions import attn
+    seen = []
+    monkeypatch.setattr(attn, "_attend", lambda *a: seen.append(a) or a[0])
+    Hkv, T, C, D = 2, 3, 5, 16
+    q, k = torch.zeros(1, 4, T * C, D), torch.zeros(1, T * C, Hkv, D).transpose(1, 2)
+    bias, rt, rc = torch.zeros(1, Hkv, 1, D), torch.zeros(1, Hkv, T, D), torch.zeros(1, Hkv, C, D)
+    attn.flash_mvpa(q, bias, bias, bias, k.unsqueeze(3), rt.unsqueeze(3), rc.unsqueeze(3), k.unsqueeze(3), True, 1.0)
+    _, _, _, _, k5, rt5, rc5, v5 = seen[0][:8]
+    p = attn._problem(q, k5, rt5, rc5, 1.0, 10)
+    assert (p.B, p.H, p.Hkv, p.T, p.C, p.D) == (1, 4, Hkv, T, C, D)
+    for t in (k5, v5):
+        d = attn._tensor(t)
+        assert attn._aligned(t) and (d.stride_b, d.stride_h, d.stride_n) == k.stride()[:3]
+    assert not attn._aligned(torch.zeros(1, 2, 3, 18)[..., :16]) and not attn._aligned(torch.zeros(1, 2, 16, 3).transpose(2, 3))
