@@ -53,6 +53,42 @@ def test_swiglu_gradients(cuda, dtype, shape):
         assert v.dtype == dtype and _rel(v, ref) <= TOL_SWIGLU[dtype]
 
 
+# fp32, element by element, gates as large as a trained MLP's: an exponential and a division within one unit in the last
+# place each (2^-23 relative), the addition and the products half a unit each: three units for silu(gate) * up.  dgate's
+# factor 1 + gate (1 - s) cancels near gate = -1.28, so it is held in the 2-norm: exp's unit times gate, of size std.
+@pytest.mark.parametrize("std", [1.0, 3.0, 8.0])
+def test_fp32_elementwise_accuracy(cuda, std):
+    g = torch.Generator().manual_seed(3)
+    gate, up, dy = (torch.randn(300, 1028, generator=g).to(cuda) for _ in range(3))
+    gate = (gate * std).requires_grad_()
+    up.requires_grad_()
+    y = mvpa_ops.swiglu(gate, up)
+    dgate, dup = torch.autograd.grad(y, (gate, up), dy)
+    a64, b64 = gate.detach().double().requires_grad_(), up.detach().double().requires_grad_()
+    y64 = torch.nn.functional.silu(a64) * b64
+    dgate64, dup64 = torch.autograd.grad(y64, (a64, b64), dy.double())
+    ulp = 2.0 ** -23
+    worst = lambda v, r: ((v.double() - r).abs() / r.abs().clamp_min(2.0 ** -100)).max().item()
+    assert worst(y, y64) <= 3 * ulp and worst(dup, dup64) <= 3 * ulp
+    assert _rel(dgate, dgate64) <= max(1.0, std / 3) * ulp
+
+
+# The norm's weight gradient sums over the rows; its terms are products of values with about half a unit of error each, and
+# their sum may add no more than that again.
+@pytest.mark.parametrize("rows,width", [(2000, 260), (300, 768), (40, 2048)])
+def test_fp32_norm_accuracy(cuda, rows, width):
+    g = torch.Generator().manual_seed(5)
+    x, dy = (torch.randn(rows, width, generator=g).to(cuda) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(width, generator=g)).to(cuda)
+    ins = [x.requires_grad_(), w.requires_grad_()]
+    y = mvpa_ops.rmsnorm_train(*ins, 1e-5)
+    got = (y, *torch.autograd.grad(y, ins, dy))
+    ins64 = [t.detach().double().requires_grad_() for t in ins]
+    y64 = _norm64(*ins64, 1e-5)
+    for v, r in zip(got, (y64, *torch.autograd.grad(y64, ins64, dy.double()))):
+        assert _rel(v, r) <= 2.0 ** -23
+
+
 def test_second_derivatives_and_transforms(cuda):
     x = torch.randn(6, 64, device=cuda, requires_grad=True)
     w = torch.randn(64, device=cuda, requires_grad=True)
