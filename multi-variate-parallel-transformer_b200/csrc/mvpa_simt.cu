@@ -106,34 +106,44 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
 }
 
 // acc[a][j] = sum_d A[a][d] * B[tx + 16 j][d]: A points at this half-warp's four rows, both ld = D + 4.
-// Packed multiply-adds over pairs of d (even and odd partial sums): half the instructions of scalar ones,
-// which leaves issue slots for the shared-memory loads.
+// Packed multiply-adds over pairs of d: half the instructions of scalar ones, which leaves issue slots for the
+// shared-memory loads.  The two halves of d are summed by themselves, because four chains of D / 4 terms round less than
+// a scalar sum in groups of four does, and two chains of D / 2 more: output and dq at 4 x 4 tokens, D 64, against 64 bits,
+// 1.14e-7 and 2.24e-7 with four chains, 1.21e-7 and 2.28e-7 in groups, 1.28e-7 and 2.49e-7 with two chains (which are 3 %
+// faster in the forward of 32 x 16 tokens: 17.5 against 18.1 us).
 template <int D, int KJ>
 __device__ __forceinline__ void product_nt(const float* A, const float* B, int tx, float (&acc)[4][KJ]) {
   constexpr int LD = D + 4;
-  uint64_t s[4][KJ];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int j = 0; j < KJ; ++j) s[a][j] = 0ull;
   const float* b0 = B + tx * LD;
+  auto half = [&](int d0) {
+    uint64_t s[4][KJ];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) s[a][j] = 0ull;
 #pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
-    ulonglong2 x[4];
+    for (int dd = 0; dd < D / 2; dd += 4) {
+      const int d = d0 + dd;
+      ulonglong2 x[4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const ulonglong2*>(A + a * LD + d);
+      for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const ulonglong2*>(A + a * LD + d);
 #pragma unroll
-    for (int j = 0; j < KJ; ++j) {
-      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b0 + 16 * j * LD + d);
+      for (int j = 0; j < KJ; ++j) {
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b0 + 16 * j * LD + d);
 #pragma unroll
-      for (int a = 0; a < 4; ++a) s[a][j] = ffma2(x[a].y, y.y, ffma2(x[a].x, y.x, s[a][j]));
+        for (int a = 0; a < 4; ++a) s[a][j] = ffma2(x[a].y, y.y, ffma2(x[a].x, y.x, s[a][j]));
+      }
     }
-  }
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int j = 0; j < KJ; ++j)
-      acc[a][j] = __uint_as_float((uint32_t)s[a][j]) + __uint_as_float((uint32_t)(s[a][j] >> 32));
+      for (int j = 0; j < KJ; ++j) {
+        const float v = __uint_as_float((uint32_t)s[a][j]) + __uint_as_float((uint32_t)(s[a][j] >> 32));
+        acc[a][j] = d0 == 0 ? v : acc[a][j] + v;
+      }
+  };
+  half(0);
+  half(D / 2);
 }
 
 // Columns of a row that a lane holds: VW = D / 16 of them, in pieces of up to four adjacent ones.
@@ -236,6 +246,13 @@ __device__ __forceinline__ void rel_products(const Args& p, int hk, const float*
   }
 }
 
+// CTAs that a multiprocessor holds as far as shared memory goes, with room for `slots` floats of time and channel slots:
+// two where they fit, which the compiler has to be told (at most 128 registers a thread), or it takes 160 and one CTA stays
+// out: forward B 2 H 8 T 48 C 32 D 32 165 against 136 us, query side 352 against 258.
+constexpr int resident_ctas(size_t fixed_floats, size_t slots) {
+  return 2 * (fixed_floats + slots) * sizeof(float) + 2 * 1024 <= 233472 ? 2 : 1;
+}
+
 // ------------------------------- forward -------------------------------------
 
 template <int D, int WPG, int NG, int KN>
@@ -244,7 +261,8 @@ constexpr size_t fwd_fixed_floats() {
 }
 
 template <typename Tin, int D, int WPG, int NG, int KN>
-__global__ void __launch_bounds__(32 * WPG * NG) simt_fwd_kernel(Args p) {
+__global__ void __launch_bounds__(32 * WPG * NG, resident_ctas(fwd_fixed_floats<D, WPG, NG, KN>(), 8 * WPG * 64))
+simt_fwd_kernel(Args p) {
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;  // threads of a group, of the CTA
   static_assert(NG * KN >= 2 * BM, "the V buffers hold two copies of the rows during the prologue");
@@ -439,7 +457,8 @@ constexpr size_t dq_fixed_floats() {
 // INS: the relative scores also sit in shared memory; otherwise they are read back from the workspace (long
 // time or channel axes, where the two groups' slot sums fill the shared memory).
 template <typename Tin, int D, int WPG, int NG, int KN, bool INS>
-__global__ void __launch_bounds__(32 * WPG * NG) simt_dq_kernel(BwdArgs bw) {
+__global__ void __launch_bounds__(32 * WPG * NG, resident_ctas(dq_fixed_floats<D, WPG, NG, KN>(), 8 * WPG * (NG + INS) * 64))
+simt_dq_kernel(BwdArgs bw) {
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;
   static_assert(NG * KN >= 2 * BM && KN >= BM, "aliased areas");
@@ -724,8 +743,10 @@ constexpr size_t dkv_fixed_floats() {
   return (size_t)2 * 8 * WPG * (D + 4) + (size_t)NG * 2 * KN * (D + 4) + (size_t)NG * WPG * 16 * (KN + 4) + 2 * NG * KN;
 }
 
+// (two CTAs a multiprocessor at D 16: 159 against 185 us at B 2 H 8 T 48 C 32; from D 32 on the 128 registers that leaves
+// a thread spill: 387 against 232 us)
 template <typename Tin, int D, int WPG, int NG, int KN>
-__global__ void __launch_bounds__(32 * WPG * NG) simt_dkv_kernel(BwdArgs bw) {
+__global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kernel(BwdArgs bw) {
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;
   static_assert(KN >= BM, "aliased areas");

@@ -4,7 +4,9 @@ import numpy as np
 import pytest
 import torch
 
+import attentions
 import mvpa_oracle as mo
+import mvpa_port_torch as mp
 from test_gpu_op import BF16_ABS, F16_ABS, F32_REL, GRADS, _np, _op, _oracle_args, _rounded, random_case
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +56,25 @@ def test_cuda_core_long_axes(cuda, shape):
                                    (1, 2, 1, 27, 50, 64), (1, 1, 1, 49, 32, 64)])
 def test_key_side_pipeline_bf16(cuda, shape):
     _check(cuda, random_case(sum(shape), *shape, scale=0.5), torch.bfloat16)
+
+
+# fp32 sums at the smallest sizes, where the score products' rounding is all there is: root mean square over fifty draws of
+# the relative error against 64 bits.  A product of 64 terms in four chains measures 1.14e-7 (output) and 2.24e-7 (dq), in
+# groups of four terms 1.21e-7 and 2.28e-7, in two chains 1.28e-7 and 2.49e-7: the limits lie above the second.
+def test_fp32_scores_round_no_more_than_a_sum_in_groups(cuda):
+    B, H, Hkv, T, C, D = 1, 2, 1, 4, 4, 64
+    errors = []
+    for seed in range(50):
+        gen = torch.Generator().manual_seed(seed)
+        r = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(cuda)
+        a = [r(B, H, T * C, D), r(1, Hkv, 1, D, std=0.1), r(1, Hkv, 1, D, std=0.1), r(1, Hkv, 1, D, std=0.1), r(B, Hkv, T * C, D),
+             r(1, Hkv, T, D, std=0.3), r(1, Hkv, C, D, std=0.3), r(B, Hkv, T * C, D)]
+        do = r(B, H, T * C, D)
+        q = a[0].requires_grad_()
+        o = attentions.flashmvpa(*a, True, D ** -0.5, window_size=10)
+        q64 = q.detach().double().requires_grad_()
+        o64 = mp.rel_attn(q64, *(t.double() for t in a[1:]), D ** -0.5, 10)
+        pairs = (o, o64), (torch.autograd.grad(o, q, do)[0], torch.autograd.grad(o64, q64, do.double())[0])
+        errors.append([((x.double() - y).norm() / y.norm()).item() ** 2 for x, y in pairs])
+    rms_o, rms_dq = np.sqrt(np.mean(errors, axis=0))
+    assert rms_o <= 1.23e-7 and rms_dq <= 2.33e-7
