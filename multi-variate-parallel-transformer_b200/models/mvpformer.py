@@ -88,7 +88,12 @@ class LlamaMLP(torch.nn.Module):
         self.down_proj = torch.nn.Linear(config.intermediate_size, config.hidden_size, bias=False)
 
     def forward(self, x):
-        return self.down_proj(mvpa_ops.swiglu(self.gate_proj(x), self.up_proj(x)))
+        gate, up = self.gate_proj(x), self.up_proj(x)
+        if torch.jit.is_scripting():
+            act = F.silu(gate) * up
+        else:
+            act = mvpa_ops.swiglu(gate, up)
+        return self.down_proj(act)
 
 
 _SHIPPED = tuple(block_grad.shipped(cls) for cls in (RMSNorm, MVPFormerGQAFlashAttention, LlamaMLP))

@@ -104,12 +104,14 @@ def _plain(*ts):
     contiguous, 16-byte aligned, not empty; no forward-mode level, functorch transform or tracer is active
     (those are served by the differentiable torch expressions)."""
     t0 = ts[0]
-    if not _nat.untraced() or t0.dtype not in (torch.bfloat16, torch.float32):
+    # (types first: a symbolic value answers no question about itself)
+    if not all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts) or not _nat.untraced() \
+            or t0.dtype not in (torch.bfloat16, torch.float32):
         return False
     # (a backward may run on a thread of the autograd engine, where a transform shows on the tensor alone)
     if any(torch._C._functorch.is_functorch_wrapped_tensor(t) or not torch._C._has_storage(t) for t in ts):
         return False
-    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == t0.dtype and t.device == t0.device
+    return all(t.is_cuda and t.dtype == t0.dtype and t.device == t0.device
                and t.is_contiguous() and t.numel() > 0 and t.data_ptr() % 16 == 0 for t in ts)
 
 

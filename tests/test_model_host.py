@@ -107,3 +107,12 @@ def test_gradients_through_the_expression_stop_at_the_block():
     for p, q in zip(got, run(_Step.f)):
         for s, t in zip(p, q):
             torch.testing.assert_close(s, t, rtol=1e-12, atol=1e-12)
+
+
+def test_mlp_can_be_traced_scripted_and_compiled():
+    m = models.mvpformer.LlamaMLP(models.MVPFormerConfig(n_embd=8, n_inner=16))
+    x = torch.randn(3, 8)
+    want = m.down_proj(torch.nn.functional.silu(m.gate_proj(x)) * m.up_proj(x))
+    for form in (m, torch.fx.symbolic_trace(m), torch.jit.script(m), torch.jit.trace(m, x),
+                 torch.compile(m, backend="eager", fullgraph=True), torch.export.export(m, (x,)).module(), torch.vmap(m)):
+        torch.testing.assert_close(form(x), want)
