@@ -18,8 +18,9 @@ h = x + MLP(ln_1 x) + Attn(ln_1 x)) built for B200:
     on the input) come from one GEMM each per forward.
 
 With gradients enabled the blocks run the reference's op order through differentiable operations: torch's
-projections, `mvpa_ops.rmsnorm_train` and `mvpa_ops.swiglu` (one kernel each way instead of about ten
-elementwise launches), and `attentions.flashmvpa`; as one autograd function where the block is unmodified.
+projections, `mvpa_ops.rmsnorm_train` (one kernel forward and two backward instead of about ten elementwise
+launches), `mvpa_ops.swiglu` where the gate is large, and `attentions.flashmvpa`; as one autograd function where the
+block is unmodified.
 """
 from __future__ import annotations
 
@@ -77,6 +78,22 @@ class RMSNorm(torch.nn.Module):
         return mvpa_ops.rmsnorm(x.contiguous(), self.weight.detach().to(x.dtype), self.eps)
 
 
+# From this size of its operands on, the fused gate is the faster one; below, its host path costs more than the torch
+# launches that it saves.  The MLP in us, torch against fused, bf16, without gradients / with: 1600 rows of 768 x 1728
+# (5 MiB) 51 / 84 and 240 / 338; 6400 rows (21 MiB) 81 / 83 and 245 / 354; 3200 rows of 2048 x 5632 (34 MiB) 188 / 176 and
+# 647 / 594; 12800 rows of 768 x 1728 (42 MiB) 136 / 116 and 425 / 397; 16384 rows of 2048 x 5632 (176 MiB) 1041 / 958 and
+# 3217 / 2961.
+GATE_BYTES = 32 << 20
+
+
+def _gate(gate, up):
+    # (a compiler or tracer would take the size for a condition of the program)
+    if (type(gate) is torch.Tensor and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and gate.nbytes >= GATE_BYTES):
+        return mvpa_ops.swiglu(gate, up)
+    return F.silu(gate) * up
+
+
 class LlamaMLP(torch.nn.Module):
     """SwiGLU MLP with the parameter names of `transformers`' `LlamaMLP`, which the reference block uses
     (`models/mvpformer.py:34, 114`): down_proj(silu(gate_proj(x)) * up_proj(x)), no biases."""
@@ -92,7 +109,7 @@ class LlamaMLP(torch.nn.Module):
         if torch.jit.is_scripting():
             act = F.silu(gate) * up
         else:
-            act = mvpa_ops.swiglu(gate, up)
+            act = _gate(gate, up)
         return self.down_proj(act)
 
 

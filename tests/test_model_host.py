@@ -116,3 +116,16 @@ def test_mlp_can_be_traced_scripted_and_compiled():
     for form in (m, torch.fx.symbolic_trace(m), torch.jit.script(m), torch.jit.trace(m, x),
                  torch.compile(m, backend="eager", fullgraph=True), torch.export.export(m, (x,)).module(), torch.vmap(m)):
         torch.testing.assert_close(form(x), want)
+
+
+def test_the_fused_gate_starts_at_its_size(monkeypatch):
+    calls = []
+    monkeypatch.setattr(models.mvpformer.mvpa_ops, "swiglu",
+                        lambda g, u: calls.append(g.shape) or torch.nn.functional.silu(g) * u)
+    m = models.mvpformer.LlamaMLP(models.MVPFormerConfig(n_embd=8, n_inner=16))
+    m(torch.randn(300, 8))
+    assert not calls                                   # far below the line: torch's two launches
+    monkeypatch.setattr(models.mvpformer, "GATE_BYTES", 300 * 16 * 4)
+    m(torch.randn(299, 8))
+    m(torch.randn(300, 8))
+    assert calls == [(300, 16)]
