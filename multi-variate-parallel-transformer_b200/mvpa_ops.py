@@ -76,11 +76,12 @@ def rmsnorm_bwd(x, weight, dy, eps, add=None):
         assert add.dtype == x.dtype and add.is_contiguous() and add.numel() == x.numel()
     dx, dw = torch.empty_like(x2), torch.empty_like(weight)
     lib = _nat.lib()
-    nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-    with _nat.on_device(x.device):
-        st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(),
-                                  add.data_ptr() if add is not None else None, dx.data_ptr(), dw.data_ptr(), x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes, _stream(x))
+    with _nat.on_device(x.device):   # (the size depends on the device's multiprocessors)
+        nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+        st = lib.mvpa_rmsnorm_bwd(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), add.data_ptr() if add is not None else None,
+                                  dx.data_ptr(), dw.data_ptr(), x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes,
+                                  _stream(x))
     _nat.check(st, "mvpa_rmsnorm_bwd")
     return dx.view(x.shape), dw
 

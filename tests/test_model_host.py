@@ -129,3 +129,33 @@ def test_the_fused_gate_starts_at_its_size(monkeypatch):
     m(torch.randn(299, 8))
     m(torch.randn(300, 8))
     assert calls == [(300, 16)]
+
+
+def test_scratch_sizes_are_asked_for_on_the_tensors_device(monkeypatch):
+    """The norm's backward sizes its scratch by the multiprocessors of the current device: that has to be x's."""
+    from contextlib import contextmanager
+    import mvpa_ops
+    current, asked = ["another"], []
+
+    @contextmanager
+    def on_device(device):
+        current.append(device)
+        yield
+        current.pop()
+
+    class Lib:
+        def mvpa_rmsnorm_bwd_workspace_bytes(self, rows, width):
+            asked.append(current[-1])
+            return 16
+
+        def mvpa_rmsnorm_bwd(self, *args):
+            asked.append(current[-1])
+            return 0
+
+    monkeypatch.setattr(mvpa_ops._nat, "lib", Lib)
+    monkeypatch.setattr(mvpa_ops._nat, "on_device", on_device)
+    monkeypatch.setattr(mvpa_ops, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(mvpa_ops, "_stream", lambda t: None)
+    x = torch.zeros(3, 8)
+    mvpa_ops.rmsnorm_bwd(x, x[0], x, 1e-5)
+    assert asked == [x.device, x.device]
