@@ -132,6 +132,12 @@ def lib() -> ctypes.CDLL:
             L = ctypes.CDLL(LIB_PATH)
         except OSError as e:  # no silent fallback: the CUDA library is the product
             raise ImportError(f"cannot load {LIB_PATH}: {e}") from e
+        # a stale binary, kept because the rebuild failed: another version, or one from before an entry point was added
+        version = L.mvpa_abi_version() if hasattr(L, "mvpa_abi_version") else None
+        missing = [name for name in EXPORTS if not hasattr(L, name)]
+        if version != ABI_VERSION or missing:
+            raise ImportError(f"{LIB_PATH} has ABI version {version}, this shim needs {ABI_VERSION}"
+                              + (f" with {', '.join(missing)}" if missing else "") + ": rebuild it (python __graft_entry__.py)")
         P, Tn, vp = ctypes.POINTER(Problem), ctypes.POINTER(Tensor), ctypes.c_void_p
         L.mvpa_fwd_workspace_bytes.restype = ctypes.c_size_t
         L.mvpa_fwd_workspace_bytes.argtypes = [P]
@@ -180,10 +186,6 @@ def lib() -> ctypes.CDLL:
         L.mvpa_contrastive_logits.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp]
         L.mvpa_last_error_string.restype = ctypes.c_char_p
         L.mvpa_launch_count.restype = ctypes.c_uint64
-        L.mvpa_abi_version.restype = ctypes.c_int
-        if L.mvpa_abi_version() != ABI_VERSION:  # e.g. a stale binary kept because the rebuild failed
-            raise ImportError(f"{LIB_PATH} has ABI version {L.mvpa_abi_version()}, this shim needs {ABI_VERSION}: "
-                              "rebuild it (python __graft_entry__.py)")
         _lib = L
         return L
 

@@ -3,6 +3,9 @@ rejects bad arguments with the documented codes before touching a device."""
 import ctypes
 import os
 import re
+import subprocess
+
+import pytest
 
 import mvpa_native as nat
 from conftest import ROOT
@@ -23,6 +26,19 @@ def test_library_exports_every_declared_symbol():
         assert hasattr(lib, n), n
     assert set(nat.EXPORTS) <= set(names)
     assert lib.mvpa_abi_version() == nat.ABI_VERSION
+
+
+@pytest.mark.parametrize("version,names", [(nat.ABI_VERSION, nat.EXPORTS[:-3]), (nat.ABI_VERSION + 1, nat.EXPORTS), (None, ["f"])])
+def test_a_stale_binary_is_refused_with_instructions(monkeypatch, tmp_path, version, names):
+    """Entry points that are missing, another version, no version at all: one ImportError that says what to do."""
+    src = "".join(f"int {n}(void) {{ return {version or 0}; }}\n" for n in names)
+    (tmp_path / "old.c").write_text(src)
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "old.c"), "-o", str(tmp_path / "old.so")], check=True)
+    monkeypatch.setattr(nat, "LIB_PATH", str(tmp_path / "old.so"))
+    monkeypatch.setattr(nat, "_lib", None)
+    monkeypatch.setattr(nat, "_stale", lambda: False)
+    with pytest.raises(ImportError, match="rebuild it"):
+        nat.lib()
 
 
 def _prob(**kw):
