@@ -161,7 +161,7 @@ class _FlashMVPAGrad(torch.autograd.Function):
     def forward(ctx, do, *operands):
         ctx.save_for_backward(do, *operands[:8])
         ctx.sm_scale, ctx.window = operands[-2:]
-        return _gradients(do, *operands)
+        return tuple(t.clone() if t._is_view() else t for t in _gradients(do, *operands))
 
     @staticmethod
     def backward(ctx, *grads):

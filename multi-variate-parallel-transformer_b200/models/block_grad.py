@@ -72,11 +72,11 @@ class BlockFunction(torch.autograd.Function):
                                 rt, rc, _heads_view(kv[:, KV:], B, N, Hkv, D), _heads_view(o, B, N, H, D),
                                 1.0 / (D ** 0.5), WINDOW, (0, 0), True)
         act = mvpa_ops.silu_mul(g, up, torch.empty_like(g))
-        h = torch.addmm(x2, act, wd.t())
-        h.addmm_(o, wc.t())
+        h = torch.empty_like(x)          # (not a view of a matrix: the caller may change it in place)
+        torch.addmm(x2, act, wd.t(), out=h.view(B * N, E)).addmm_(o, wc.t())
         ctx.save_for_backward(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act)
         ctx.eps, ctx.heads = eps, heads
-        return h.view(B, T, C, E)
+        return h
 
     @staticmethod
     def backward(ctx, dh):
@@ -116,8 +116,7 @@ class BlockFunction(torch.autograd.Function):
             dxn = torch.mm(dq, wq)
             for d, w in ((dkv, wkv), (dg, wg), (dup, wu)):
                 dxn.addmm_(d, w)
-            dx, grad[3] = mvpa_ops.rmsnorm_bwd(x.view(B * N, E), ln_w, dxn, ctx.eps, add=dh2)
-            grad[0] = dx.view(x.shape)
+            grad[0], grad[3] = mvpa_ops.rmsnorm_bwd(x, ln_w, dxn.view(x.shape), ctx.eps, add=dh2)
         return (*grad, None, None)
 
 

@@ -74,7 +74,7 @@ def rmsnorm_bwd(x, weight, dy, eps, add=None):
     assert weight.dtype == x.dtype == dy.dtype and dy.shape == x.shape
     if add is not None:
         assert add.dtype == x.dtype and add.is_contiguous() and add.numel() == x.numel()
-    dx, dw = torch.empty_like(x2), torch.empty_like(weight)
+    dx, dw = torch.empty(x.shape, dtype=x.dtype, device=x.device), torch.empty_like(weight)
     lib = _nat.lib()
     with _nat.on_device(x.device):   # (the size depends on the device's multiprocessors)
         nbytes = lib.mvpa_rmsnorm_bwd_workspace_bytes(x2.shape[0], E)
@@ -83,7 +83,7 @@ def rmsnorm_bwd(x, weight, dy, eps, add=None):
                                   dx.data_ptr(), dw.data_ptr(), x2.shape[0], E, float(eps), _code(x), ws.data_ptr(), nbytes,
                                   _stream(x))
     _nat.check(st, "mvpa_rmsnorm_bwd")
-    return dx.view(x.shape), dw
+    return dx, dw
 
 
 def silu_mul_bwd(gate, up, dout):
@@ -127,7 +127,9 @@ class _RMSNorm(torch.autograd.Function):
     def forward(ctx, x, weight, eps):
         ctx.save_for_backward(x, weight)
         ctx.eps = eps
-        return rmsnorm(x, weight, eps)
+        y = torch.empty_like(x)          # (not a view of one: the caller may change it in place)
+        rmsnorm(x, weight, eps, out=y)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
@@ -156,7 +158,9 @@ class _SwiGLU(torch.autograd.Function):
     def forward(ctx, gate, up):
         ctx.save_for_backward(gate, up)
         w = gate.shape[-1]
-        return silu_mul(gate.view(-1, w), up.view(-1, w), torch.empty_like(gate).view(-1, w)).view(gate.shape)
+        out = torch.empty_like(gate)     # (not a view of one, as above)
+        silu_mul(gate.view(-1, w), up.view(-1, w), out.view(-1, w))
+        return out
 
     @staticmethod
     def backward(ctx, dout):

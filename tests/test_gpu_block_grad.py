@@ -212,3 +212,24 @@ def test_refused_heads_are_refused_alike(cuda, E, H, Hkv):
     block, x, pos, chan = _block(cuda, E=E, H=H, Hkv=Hkv)
     with pytest.raises(AssertionError):
         block(x, pos, chan)
+
+
+def test_outputs_and_gradients_may_be_changed_in_place(cuda):
+    import mvpa_ops
+    block, x, pos, chan = _block(cuda)
+    w = block.ln_1.weight
+    for f in (lambda t: block(t, pos, chan)[0], block.ln_1, lambda t: mvpa_ops.swiglu(t, t + 1)):
+        y, z = f(x.requires_grad_()), f(x)
+        y.mul_(2).add_(x.detach())
+        y.view(-1)[3] = 0
+        z = (z * 2 + x.detach()) * (torch.arange(z.numel(), device=cuda) != 3).view(z.shape)
+        assert torch.equal(y, z)
+        for a, b in zip(torch.autograd.grad(y.sum(), (x, w), allow_unused=True), torch.autograd.grad(z.sum(), (x, w), allow_unused=True)):
+            assert (a is None and b is None) or torch.equal(a, b)
+    args, do = _operands(1, 2, 1, 5, 3, 16, torch.float32, cuda, False)
+    ins = [t.requires_grad_() for t in args]
+    o = attentions.flashmvpa(*ins, True, 0.25, window_size=10)
+    for t, g in zip(ins, torch.autograd.grad(o, ins, do, create_graph=True)):
+        assert g.mul_(2).shape == t.shape
+    for g in torch.autograd.grad(block(x, pos, chan)[0].sum(), (x, w)):
+        g.mul_(w.sum())
