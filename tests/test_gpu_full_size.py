@@ -66,7 +66,7 @@ def test_causality_and_batch_independence(cuda, cfg):
 @pytest.mark.parametrize("cfg", [CFG2, CFG3, LONG])
 def test_tensor_core_path_vs_fp32_path_on_a_slice(cuda, cfg):
     """One (batch, kv-group) slice: bf16 tensor-core result vs the fp32 CUDA-core kernels fed the
-    same bf16-rounded values (the fp32 path itself is pinned to the oracle in test_gpu_op)."""
+    same bf16-rounded values (the fp32 kernels of either tile size are pinned to the oracle in test_gpu_tiles)."""
     B, H, Hkv, T, C, D = cfg
     g = H // Hkv
     t = make(cuda, 3, *cfg)
@@ -173,7 +173,7 @@ BWD_CASES = [(1, 16, 16, 128, 32, 64),   # config 3's shape, one batch element: 
 def test_backward_tensor_core_vs_fp32_path_full_size(cuda, cfg):
     """Backward at the benchmark shapes (many key tiles outside the content window, more CTAs than SMs):
     all eight gradients of the bf16 tensor-core kernels against the fp32 CUDA-core kernels fed the same
-    bf16-rounded values; the latter are pinned to the oracle at small sizes in test_gpu_op.
+    bf16-rounded values; the latter are pinned to the oracle at small sizes of either tile size in test_gpu_tiles.
     Tolerance: 3e-2 of the largest magnitude of each gradient (bf16 operands, fp32 accumulation)."""
     t = make(cuda, 5, *cfg)
     gout = torch.randn(t["q"].shape, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(cuda)

@@ -37,8 +37,10 @@ def test_cuda_core_tiles_sixteen_rows(cuda, shape, dtype):
     _check(cuda, random_case(sum(shape), *shape), dtype)
 
 
-# more sixteen-row tiles than four per multiprocessor: thirty-two rows per CTA, last tile ragged
-@pytest.mark.parametrize("shape", [(2, 16, 16, 15, 21, 16), (1, 32, 16, 17, 19, 32)])
+# more sixteen-row tiles than four per multiprocessor: thirty-two rows per CTA, last tile ragged; at D 64 and 128 light
+# tiles too (T > window + tile), and at the last two the key side stays below the line, with query heads above it
+@pytest.mark.parametrize("shape", [(2, 16, 16, 15, 21, 16), (1, 32, 16, 17, 19, 32), (2, 16, 16, 24, 13, 64), (2, 16, 16, 24, 13, 128),
+                                   (1, 64, 8, 24, 13, 64), (1, 64, 8, 24, 13, 128)])
 def test_cuda_core_tiles_thirty_two_rows(cuda, shape):
     _check(cuda, random_case(sum(shape), *shape), torch.float32)
 
