@@ -121,16 +121,17 @@ class FlashMVPA(torch.autograd.Function):
     """Autograd wrapper; the counterpart of the reference's `FlashMVPA`
     (`attentions/attn.py:1013-1302`), taking the relative keys themselves instead of
     pre-multiplied score matrices.  The small tensors may have any shape with their elements in
-    (kv head, row, D) order, r_time and r_chan with the rows next to last; their gradients take that shape.
-    Second derivatives reach the operands that the kernels read in place (`flash_mvpa` lays the others out first)."""
+    (kv head, row, D) order, r_time and r_chan with the rows next to last; their gradients take that shape."""
 
     @staticmethod
-    def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0), laid_out=False):
-        if not laid_out:
-            q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v)
+    def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0)):
+        given = (q, u, vt, z, k, r_time, r_chan, v)
+        q, u, vt, z, k, r_time, r_chan, v = read = _lay_out(*given)
         o = torch.empty_like(q)
         lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
-        ctx.save_for_backward(q, u, vt, z, k, r_time, r_chan, v, o, lse)
+        ctx.save_for_backward(*read, o, lse)
+        # what was copied, for second derivatives alone: the copy belongs to no graph
+        ctx.copied = [(i, t, t._version) for i, (t, r) in enumerate(zip(given, read)) if r is not t]
         ctx.sm_scale, ctx.window, ctx.q_time = sm_scale, window, q_time
         return o
 
@@ -139,8 +140,15 @@ class FlashMVPA(torch.autograd.Function):
         if ctx.q_time[1]:
             raise NotImplementedError("flash_mvpa: backward through a query time range is not implemented")
         if torch.is_grad_enabled():  # a graph of the gradient is wanted
-            return (*_FlashMVPAGrad.apply(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None, None)
-        return (*_gradients(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None, None)
+            read = list(ctx.saved_tensors)
+            for i, t, version in ctx.copied:
+                if t.requires_grad:
+                    if t._version != version:
+                        raise RuntimeError("flash_mvpa: an operand has been modified in place since the forward; its second "
+                                           "derivative cannot be formed")
+                    read[i] = t.contiguous()
+            return (*_FlashMVPAGrad.apply(do, *read, ctx.sm_scale, ctx.window), None, None, None)
+        return (*_gradients(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None)
 
 
 def _gradients(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window):
@@ -219,11 +227,10 @@ def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
     of a small call, so an ordinary call that no gradient flows through goes to the kernels directly (and stores no
     log-sum-exp); whatever traces or transforms the call sees the autograd function."""
     ts = (q, u, vt, z, k, r_time, r_chan, v)
-    if not _nat.untraced() or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts):
+    if ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or not _nat.untraced()
+            or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts)):
         return FlashMVPA.apply(*ts, sm_scale, window, q_time)
     q, u, vt, z, k, r_time, r_chan, v = _lay_out(*ts)
-    if torch.is_grad_enabled() and any(t.requires_grad for t in ts):
-        return FlashMVPA.apply(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time, True)
     o = torch.empty_like(q)
     _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, False)
     return o
