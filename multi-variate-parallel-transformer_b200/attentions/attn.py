@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+from operator import is_
 
 import torch
 
@@ -131,7 +132,7 @@ class FlashMVPA(torch.autograd.Function):
         lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
         ctx.save_for_backward(*read, o, lse)
         # what was copied, for second derivatives alone: the copy belongs to no graph
-        ctx.copied = [(i, t, t._version) for i, (t, r) in enumerate(zip(given, read)) if r is not t]
+        ctx.copied = () if all(map(is_, given, read)) else [(i, t, t._version) for i, t in enumerate(given) if t is not read[i]]
         ctx.sm_scale, ctx.window, ctx.q_time = sm_scale, window, q_time
         return o
 
@@ -139,16 +140,17 @@ class FlashMVPA(torch.autograd.Function):
     def backward(ctx, do):
         if ctx.q_time[1]:
             raise NotImplementedError("flash_mvpa: backward through a query time range is not implemented")
-        if torch.is_grad_enabled():  # a graph of the gradient is wanted
-            read = list(ctx.saved_tensors)
-            for i, t, version in ctx.copied:
-                if t.requires_grad:
-                    if t._version != version:
-                        raise RuntimeError("flash_mvpa: an operand has been modified in place since the forward; its second "
-                                           "derivative cannot be formed")
-                    read[i] = t.contiguous()
-            return (*_FlashMVPAGrad.apply(do, *read, ctx.sm_scale, ctx.window), None, None, None)
-        return (*_gradients(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window), None, None, None)
+        if not torch.is_grad_enabled():
+            return _gradients(do, *ctx.saved_tensors, ctx.sm_scale, ctx.window) + (None, None, None)
+        # a graph of the gradient is wanted
+        read = list(ctx.saved_tensors)
+        for i, t, version in ctx.copied:
+            if t.requires_grad:
+                if t._version != version:
+                    raise RuntimeError("flash_mvpa: an operand has been modified in place since the forward; its second "
+                                       "derivative cannot be formed")
+                read[i] = t.contiguous()
+        return _FlashMVPAGrad.apply(do, *read, ctx.sm_scale, ctx.window) + (None, None, None)
 
 
 def _gradients(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window):
