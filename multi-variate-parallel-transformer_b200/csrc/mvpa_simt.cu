@@ -6,10 +6,11 @@
 // anywhere, cross-tile sums go through per-tile partials.
 //
 // What bounds them: short sequences have few row tiles, so the longest CTA sets the time.  Hence sixteen rows per
-// CTA, the column tiles of a row tile shared by four groups of warps, loads in flight under the products, and no
-// CTA-wide barrier in the loop.  Against 32-row CTAs with synchronous loads and five barriers per tile (device time):
-// forward B 1 H 4 T 32 C 16 D 64 71.0 -> 17.4 us; B 1 H 4 Hkv 2 T 24 C 22 D 64 forward 76.5 -> 20.9, query side (with
-// the relative scores and delta, separate launches before) 109 -> 43, key side 208 -> 50, the rest 23 -> 8 us.
+// CTA, the column tiles of a row tile shared by four groups of warps, loads in flight under the products (fp32; the
+// 16-bit types convert on the way and load in place), and no CTA-wide barrier in the loop.  fp32, against 32-row CTAs
+// with synchronous loads and five barriers per tile (device time): forward B 1 H 4 T 32 C 16 D 64 18.1 against 71.0 us;
+// B 1 H 4 Hkv 2 T 24 C 22 D 64 forward 21.4 / 76.5, query side with the relative scores and delta 41 / 109, key side
+// 50 / 208, the rest 8 / 23 us.
 //
 // Math follows the reference forward (`attentions/attn.py:232-333`: base-2 online
 // softmax, window zero-fill, time-block causal mask, L = m + log2 l) and backward

@@ -1561,7 +1561,8 @@ int make_maps(BqMaps& m, const BwdArgs& bw, int CP, const void* qp) {
 //   the others: dr_time / dr_chan from the accumulators of the query-side kernel, 32 columns of one kv head each:
 //     dr[j, d] = sum_i dX[i, j] (q[i, d] + bias[d]) = R'[j, d] / c2 + colsum[j] (bias[d] - u[d]),   Q' = (q + u) c2,
 //   transposed through shared memory (the accumulators have the slot innermost, the results the column).
-// 21 us at 4 x 25 x 100 tokens, head_dim 128, where two kernels took 18 + 18: what remains is the column sums' walk.
+// One launch for both: 21 us at 4 x 25 x 100 tokens, head_dim 128, against 18 + 18 as two; what remains is the column
+// sums' walk.
 struct FinArgs {
   const float* cs_dq;
   const unsigned long long *racc, *cacc;
@@ -1626,7 +1627,7 @@ __global__ void __launch_bounds__(1024) tc_bwd_final_kernel(const FinArgs p) {
 //                                 threads share a row, one 16-byte load of each tensor per thread
 //   the next Hkv blocks           the relative-product constants of one kv head (rel_const_row)
 //   the remaining blocks          zeros: status words, relative-key accumulators
-// (16k tokens, head_dim 128: 20-29 us where the separate kernels and memsets took 56; most of it reads O and dO, 134 MB)
+// (16k tokens, head_dim 128: 20-29 us against 56 as separate kernels and memsets; most of it reads O and dO, 134 MB)
 constexpr int kPreThreads = 256;
 struct PreArgs {
   const __nv_bfloat16 *o, *d_o, *vt, *z, *rt, *rc;
