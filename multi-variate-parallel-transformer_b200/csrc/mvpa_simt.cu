@@ -1034,12 +1034,14 @@ constexpr size_t kMaxSmemFloats = 232448 / sizeof(float);
 // multiprocessor (short sequences: the longest CTA sets the time, so many short ones), thirty-two rows and two
 // groups beyond (every key tile is loaded half as often).  Measured, fp32, sixteen against thirty-two rows, us:
 //   CTAs of sixteen rows per multiprocessor     forward          query side       key side (its own count)
-//   0.9  (B 1 H 4 Hkv 2, 24 x 22, D 64)         20.7 / 32.6      43.4 / 65.1      49.5 / 87.4  (0.4)
-//   3.6  (B 2 H 8 Hkv 4, 24 x 22, D 64)         54.4 / 57.7      125 / 116        84.7 / 89.2  (1.8)
-//   6.9  (B 2 H 8 Hkv 4, 32 x 32, D 64)         125.9 / 126.5    289 / 262        168 / 200    (3.5)
-//   10.4 (B 2 H 8 Hkv 8, 48 x 32, D 64)         226.8 / 227.3    523 / 471        310 / 302    (10.4)
-//   10.4 (B 2 H 8 Hkv 4, 48 x 32, D 128)        378 / 336        856 / 816        465 / 508    (5.2)
-// The three cross at different counts; one line at four lies between them.
+//   0.9  (B 1 H 4 Hkv 2, 24 x 22, D 64)         21.4 / 35.3      40.8 / 63.0      49.2 / 88.3  (0.4)
+//   3.6  (B 2 H 8 Hkv 4, 24 x 22, D 64)         55.9 / 55.0      120 / 114        86.0 / 90.1  (1.8)
+//   6.9  (B 2 H 8 Hkv 4, 32 x 32, D 64)         128.8 / 119.6    276 / 256        170 / 199    (3.5)
+//   10.4 (B 2 H 8 Hkv 8, 48 x 32, D 64)         232.5 / 200.5    504 / 465        313 / 297    (10.4)
+//   10.4 (B 2 H 8 Hkv 4, 48 x 32, D 128)        369 / 355        822 / 795        466 / 488    (5.2)
+//   10.4 (B 2 H 8 Hkv 4, 48 x 32, D 32)         129 / 136        409 / 254        204 / 224    (5.2)
+// The three cross at different counts (the query side below three, the key side between five and ten); one line at four
+// lies between them.
 constexpr int kSmallWaves = 4;
 bool few_rows(int64_t rows, int heads) { return (rows + 15) / 16 * heads <= (int64_t)kSmallWaves * device_sm_count(); }
 
