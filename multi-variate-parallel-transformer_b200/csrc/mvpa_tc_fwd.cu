@@ -70,7 +70,8 @@ enum BarrierIndex {
   kBarSFull,                     // 2
   kBarPFull = kBarSFull + 2,     // 2
   kBarPlFull = kBarPFull + 2,    // 4: P of the light tiles (four buffers, 64 TMEM columns each)
-  kBarSlotFull = kBarPlFull + 4,  // NS, then slot_free NS
+  kBarMax = kBarPlFull + 4,      // 2: running maximum after a dense tile, by the warpgroup that took it (alternating path)
+  kBarSlotFull = kBarMax + 2,    // NS, then slot_free NS
 };
 
 template <int D>
@@ -156,9 +157,11 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
   constexpr int KSTEPS = D / 16;
   constexpr int DW = D / 2;                    // O columns each warpgroup rescales / stores
   // Alternating dense tiles (head_dim 64, at most 64 channel slots): each softmax warpgroup takes every
-  // other dense tile with whole rows and its own O accumulator, so the two warps that share a
-  // scheduler are in different phases (one in its exponentials, the other loading or reducing)
-  // and no barrier is needed inside a tile; the accumulators are merged before the light tiles.
+  // other dense tile with whole rows, so the two warps that share a scheduler are in different phases (one in
+  // its exponentials, the other loading or reducing); the running maximum goes from one to the other between
+  // their two passes.  Tiles are visited light-first (one maximum, known beforehand, for the whole phase) and summed in one
+  // accumulator in the order, with the partial row sums and from the same values as in tc_fwd_two_kernel: which of the two
+  // kernels takes a call does not show in its result.
   constexpr bool ALT = (D == 64) && (CP <= 64);
   // Split accumulators (head_dim 64 with 128 channel slots): both warpgroups work on every dense tile, each
   // on its 64 key columns with its OWN running maximum, row sum and O accumulator (O_0 / O_1, 2 x 64 TMEM
@@ -185,7 +188,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
   float* s_zc = s_vr + 128;                     // z  . r_chan[j]
   float* s_max = s_zc + 128;                    // [2 slots][2 wg][128 rows]
   float* s_lsum = s_max + 512;                  // [2 wg][128]
-  float* s_merge = s_lsum + 256;                // [m, l][2 wg][128]: accumulator merge of the alternating path
+  float* s_merge = s_lsum + 256;                // [m, l][2 wg][128]: accumulator merge (split), running maxima (alternating)
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_merge + 512);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBarSlotFull + 2 * NS);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
@@ -209,11 +212,15 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
   const int n_tiles = I + 1;
   const int n_light = light_tiles(I, TPB, p.window, p.n_qt);
   const int n_dense = n_tiles - n_light;
-  // visit order: dense tiles n_light..I, then light tiles 0..n_light-1
-  auto tile_of = [&](int s) { return s < n_dense ? n_light + s : s - n_dense; };
+  // visit order: dense tiles n_light..I, then light tiles 0..n_light-1; on the alternating path the light ones first
+  auto tile_of = [&](int s) { return ALT ? s : s < n_dense ? n_light + s : s - n_dense; };
+  auto is_dense = [&](int s) { return ALT ? s >= n_light : s < n_dense; };
   // position of a tile's K / V in the load sequence; slot = q % NS, use count = q / NS
-  auto q_of_k = [&](int s) { return 2 * s; };
-  auto q_of_v = [&](int s) { return s < n_dense ? 2 * s + 1 : n_dense + s; };
+  auto q_of_k = [&](int s) { return ALT ? 2 * s - n_light : 2 * s; };
+  auto q_of_v = [&](int s) {
+    if (ALT) return s < n_light ? s : 2 * s - n_light + 1;
+    return s < n_dense ? 2 * s + 1 : n_dense + s;
+  };
   const int T = p.T, C = p.C;
 
   // One barrier at entry: thread 0 initialises the mbarriers, another warp fetches the status word (an
@@ -229,6 +236,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       mbar_init(&bars[kBarPFull + i], ALT ? kSoftmaxThreads / 2 : kSoftmaxThreads);
     }
     for (int i = 0; i < 4; ++i) mbar_init(&bars[kBarPlFull + i], kSoftmaxThreads);
+    for (int i = 0; i < 2; ++i) mbar_init(&bars[kBarMax + i], kSoftmaxThreads / 2);
     for (int i = 0; i < NS; ++i) {
       mbar_init(&slot_full[i], 1);
       mbar_init(&slot_free[i], 1);
@@ -280,7 +288,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       };
       for (int s = 0; ok && s < n_tiles; ++s) {
         const int J = tile_of(s);
-        if (s < n_dense) load_slot(&maps.k, q_of_k(s), J);
+        if (is_dense(s)) load_slot(&maps.k, q_of_k(s), J);
         if (ok) load_slot(&maps.v, q_of_v(s), J);
       }
     }
@@ -324,6 +332,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       const uint32_t a_plfull = smem_u32(&bars[kBarPlFull]);
       // ring cursor of the next slot to be consumed (K and V slots are consumed in load order)
       uint32_t k_sl = 0, k_par = 0;  // slot / parity of the next K (dense tiles only)
+      if (ALT) { k_sl = n_light % NS; k_par = (n_light / NS) & 1; }
       auto advance = [&](uint32_t& sl, uint32_t& par, int by) {
         sl += by;
         if (sl >= (uint32_t)NS) { sl -= NS; par ^= 1; }
@@ -346,15 +355,16 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         mma_commit_w(el, a_free + 8 * k_sl);
         advance(k_sl, k_par, 2);
       };
-      if (ok && n_dense > 0) issue_qk(0);
+      if (!ALT && ok && n_dense > 0) issue_qk(0);
       // The completion of PV_s is signalled on the free-barrier of the V slot it read: the producer
       // waits there to refill the slot, the softmax warps to reuse P columns / rescale O / finish.
-      uint32_t v_sl = 1 % NS, v_par = 0;  // slot / parity of V_s (V_0 is load 1)
+      uint32_t v_sl = ALT && n_light > 0 ? 0 : 1 % NS, v_par = 0;  // slot / parity of V_s (V_0 is load 1, a light tile's load 0)
       auto advance_v = [&](int by) {
         v_sl += by;
         if (v_sl >= (uint32_t)NS) { v_sl -= NS; v_par ^= 1; }
       };
       // ---- dense tiles ----
+      auto dense_tiles = [&]() {
       for (int s = 0; ok && s < n_dense; ++s) {
         if (s + 1 < n_dense) issue_qk(s + 1);  // S of the next tile first: its softmax is the long pole
         if (ok) ok = __all_sync(kFull, mbar_wait_a(a_full + 8 * v_sl, v_par, p.status, 24));
@@ -365,16 +375,18 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         const uint32_t a0 = tm + kColS + 128 * (s & 1);
         const uint32_t b_lo = dv0.lo + v_sl * (TILE >> 4);
         const bool dn = s + 1 < n_dense;
-        // alternating path: P_s is one contiguous 64-column block, O of even / odd tiles are separate
-        const uint32_t d_o = ALT ? tm + kColO + 64 * (s & 1) : tm + kColO;
-        const uint32_t acc0 = ALT ? (uint32_t)(s > 1) : (uint32_t)(s > 0);
+        // (alternating path: P_s is one contiguous 64-column block)
+        const uint32_t d_o = tm + kColO;
+        const uint32_t acc0 = (uint32_t)(s > 0 || (ALT && n_light > 0));
         mma_ts_x4_w(el, d_o, a0, b_lo, dv0.hi, 2048 >> 4, idesc_o, acc0);
         mma_ts_x4_w(el, SPLIT ? d_o + 64 : d_o, a0 + (ALT ? 32 : 64), b_lo + 4 * (2048 >> 4), dv0.hi, 2048 >> 4, idesc_o,
                     SPLIT ? acc0 : 1u);
         mma_commit_w(el, a_free + 8 * v_sl);
         advance_v(dn ? 2 : 1);  // a dense successor's V is two loads on, a light successor's one
       }
+      };
       // ---- light tiles: P in four contiguous 64-column buffers ----
+      auto light_tiles_pv = [&]() {
       uint32_t pb = 0, pb_par = 0;
       for (int l = 0; ok && l < n_light; ++l) {
         ok = __all_sync(kFull, mbar_wait_a(a_full + 8 * v_sl, v_par, p.status, 24));
@@ -385,10 +397,19 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         const uint32_t b_lo = dv0.lo + v_sl * (TILE >> 4);
         pb = (pb + 1) & 3;
         if (pb == 0) pb_par ^= 1;
-        mma_ts_x4_w(el, tm + kColO, a0, b_lo, dv0.hi, 2048 >> 4, idesc_o, 1u);
+        mma_ts_x4_w(el, tm + kColO, a0, b_lo, dv0.hi, 2048 >> 4, idesc_o, (uint32_t)(!ALT || l > 0));
         mma_ts_x4_w(el, tm + kColO, a0 + 32, b_lo + 4 * (2048 >> 4), dv0.hi, 2048 >> 4, idesc_o, 1u);
         mma_commit_w(el, a_free + 8 * v_sl);
-        advance_v(1);
+        advance_v(ALT && l + 1 == n_light ? 2 : 1);  // (the next tile's V, past its K if it is dense)
+      }
+      };
+      if constexpr (ALT) {
+        light_tiles_pv();
+        if (ok) issue_qk(0);
+        dense_tiles();
+      } else {
+        dense_tiles();
+        light_tiles_pv();
       }
     }
   }
@@ -546,15 +567,151 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       for (int tt = 0; tt < TPB; ++tt) tb_all[tt] = p.c2 * (__uint_as_float(raw[tt]) + s_vr[colj[tt]]) + mc;
     };
 
+    // ------------------------------ light tiles ------------------------------
+    // P[i,k] = a_i[t_k] * bc_i[c_k]: one exponential per (row, key time step), packed bf16
+    // multiplies for the rest.  Four P buffers of 64 TMEM columns (the idle S columns) let these
+    // warps run ahead of the PV products.
+    auto light_phase = [&]() {
+    if (!ALT && ok && n_light > 0) {
+      // the buffers overlap S0 / S1: the last dense PV products must be done with them (and with O)
+      const int q1 = q_of_v(n_dense - 1);
+      ok = warp_wait(&slot_free[q1 % NS], (q1 / NS) & 1, p.status, 37);
+      tc_fence_after();
+    }
+    // Every light tile's score is its temporal score alone (the channel maximum is folded into bc), and
+    // the temporal scores of the row sit in TMEM: one pass finds the maximum over all light tiles, one
+    // rescale of O covers the whole phase, and the loop below carries no maximum.
+    // Key step tk of the light tiles (0 <= tk < n_light * TPB) is temporal column col0 + tk.
+    const int col0 = T - 1 - ti_abs;
+    uint32_t bc[NCH / 2];  // exp2(channel score - its maximum), bf16 pairs
+    float sum_bc = 0.f;
+#pragma unroll
+    for (int k2 = 0; k2 < NCH / 2; ++k2) {
+      bc[k2] = pack_bf16(ex2(cbf[2 * k2]), ex2(cbf[2 * k2 + 1]));
+      sum_bc += __uint_as_float(bc[k2] << 16) + __uint_as_float(bc[k2] & 0xffff0000u);
+    }
+    if (ok && n_light > 0) {
+      const int col1 = col0 + n_light * TPB;
+      float m_light = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (32 * c + 32 <= col0 || 32 * c >= col1) continue;  // (warp-uniform)
+        uint32_t v[32];
+        tmem_ld32(lane_base + kColTB + 32 * c, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int jj = 0; jj < 32; ++jj) {
+          const int col = 32 * c + jj;
+          const float tb = p.c2 * (__uint_as_float(v[jj]) + s_vr[col]) + mc;
+          if (col >= col0 && col < col1) m_light = fmaxf(m_light, tb);
+        }
+      }
+      const bool need = m_light > m_used + kRescaleThreshold;
+      if (ALT) {
+        m_used = m_light;  // (nothing has been summed yet)
+      } else if (__any_sync(0xffffffffu, need)) {
+        const float alpha = need ? ex2(m_used - m_light) : 1.f;
+#pragma unroll
+        for (int c0 = 0; c0 < DW; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32(lane_base + kColO + wg * DW + c0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
+          tmem_st32(lane_base + kColO + wg * DW + c0, v);
+        }
+        tmem_st_wait();
+        l_sum *= alpha;
+        if (need) m_used = m_light;
+      }
+    }
+    // Two tiles per turn: one round trip for the temporal scores and one look at the barriers serve both,
+    // and the second tile's products are formed while the first tile's stores are in flight.  (The scores
+    // of the next pair are fetched meanwhile; with an odd count the last fetch reads the column after the
+    // light tiles, still inside the temporal columns, and drops it.)
+    uint32_t tb_next[2 * TPB];
+    auto tb_fetch = [&](int l) {
+#pragma unroll
+      for (int j = 0; j < 2 * TPB; ++j) tmem_ld1(lane_base + kColTB + col0 + l * TPB + j, tb_next[j]);
+    };
+    auto p_regs = [&](float (&a_t)[TPW], uint32_t (&lo)[16], uint32_t (&hi)[16], bool count) {
+#pragma unroll
+      for (int tl = 0; tl < TPW; ++tl) {
+        const uint32_t a2 = pack_bf16(a_t[tl], a_t[tl]);
+        if (count) l_sum += __uint_as_float(a2 << 16) * sum_bc;
+#pragma unroll
+        for (int k2 = 0; k2 < NCH / 2; ++k2) {
+          const int idx = tl * (NCH / 2) + k2;
+          if (idx < 16) lo[idx] = hmul2_bf16(a2, bc[k2]);
+          else hi[idx - 16] = hmul2_bf16(a2, bc[k2]);
+        }
+      }
+    };
+    if (ok && n_light > 0) tb_fetch(0);
+    for (int l = 0; ok && l < n_light; l += 2) {
+      const int s = ALT ? l : n_dense + l;
+      const bool two = l + 1 < n_light;
+      float a_t[2][TPW];  // exp2(temporal score - m) of this thread's key steps, both tiles
+      tmem_ld_wait();
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl) {
+          const int tt = tt_base + tl;
+          uint32_t raw = 0;
+#pragma unroll
+          for (int q = 0; q < TPB; ++q)
+            if (q == tt) raw = tb_next[u * TPB + q];
+          const float tb = p.c2 * (__uint_as_float(raw) + s_vr[col0 + (l + u) * TPB + tt]) + mc;
+          a_t[u][tl] = ex2(tb - m_used);
+        }
+      }
+      if (l + 2 < n_light) tb_fetch(l + 2);
+      if (l >= 4) {
+        // these buffers last held P of light tiles l-4 and l-3: a PV product frees the V slot it read
+        const int q = q_of_v(s - 4);
+        ok = warp_wait(&slot_free[q % NS], (q / NS) & 1, p.status, 35);
+        if (ok && two) ok = warp_wait(&slot_free[(q + 1) % NS], ((q + 1) / NS) & 1, p.status, 35);
+        if (!ok) break;
+        tc_fence_after();
+      }
+      uint32_t lo0[16], hi0[16], lo1[16], hi1[16];
+      const uint32_t p_addr0 = lane_base + kColS + 64 * (l & 3) + 32 * wg;
+      const uint32_t p_addr1 = lane_base + kColS + 64 * ((l + 1) & 3) + 32 * wg;
+      p_regs(a_t[0], lo0, hi0, true);
+      tmem_st16(p_addr0, lo0);
+      tmem_st16(p_addr0 + 16, hi0);
+      p_regs(a_t[1], lo1, hi1, two);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&bars[kBarPlFull + (l & 3)]);
+      if (two) {
+        tmem_st16(p_addr1, lo1);
+        tmem_st16(p_addr1 + 16, hi1);
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&bars[kBarPlFull + ((l + 1) & 3)]);
+      }
+    }
+    };
+
     // ------------------------------ dense tiles ------------------------------
     // Abort protocol: this loop contains a named barrier, which must never lose a participant.
     // A warp whose bounded wait runs out raises s_giveup, stops touching TMEM, and keeps walking
     // to the next named barrier; there every warp sees the flag and all leave together.
     if constexpr (ALT) {
       const uint32_t s_addr = lane_base + kColS + 128 * wg;  // this warpgroup's tiles use S buffer `wg`
-      const uint32_t o_addr = lane_base + kColO + 64 * wg;
+      // The running maximum of tile s - 1 comes from the other warpgroup; the row sums of both follow every change of it.
+      auto take_max = [&](int s) -> bool {
+        if (!warp_wait(&bars[kBarMax + (s & 1)], (s >> 1) & 1, p.status, 36)) return false;
+        const float m = s_merge[(s & 1) * 128 + row];
+        l_sum *= ex2(m_used - m);
+        m_used = m;
+        return true;
+      };
+      light_phase();
       for (int s = wg; ok && s < n_dense; s += 2) {
-        const int J = tile_of(s);
+        const int J = n_light + s;
         float tb_all[TPB], wmul[TPB];
         bool valid_all[TPB];
         {
@@ -603,27 +760,35 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         tmem_ld_wait();
         tmem_ld32(s_addr, va);  // first chunk of pass 2
         max_chunk(vb, 3);
-        if (s == wg) {
+        if (s > 0) {
+          ok = take_max(s - 1);
+          if (!ok) break;
+        }
+        if (s == 0 && n_light == 0) {
           m_used = (m_tile == -INFINITY) ? 0.f : m_tile;
+          s_merge[wg * 128 + row] = m_used;
+          mbar_arrive(&bars[kBarMax + wg]);
         } else {
           const bool need = m_tile > m_used + kRescaleThreshold;
+          const float alpha = need ? ex2(m_used - m_tile) : 1.f;
+          if (need) m_used = m_tile;
+          s_merge[wg * 128 + row] = m_used;
+          mbar_arrive(&bars[kBarMax + wg]);
           if (__any_sync(0xffffffffu, need)) {
-            const int qp = q_of_v(s - 2);  // this accumulator's previous product
+            const int qp = q_of_v(n_light + s - 1);  // the previous product: O is complete up to this tile
             if (!warp_wait(&slot_free[qp % NS], (qp / NS) & 1, p.status, 33)) { ok = false; break; }
             tc_fence_after();
-            const float alpha = need ? ex2(m_used - m_tile) : 1.f;
-#pragma unroll
-            for (int c0 = 0; c0 < D; c0 += 32) {
-              uint32_t v[32];
-              tmem_ld32(o_addr + c0, v);
+#pragma unroll 1
+            for (int c0 = 0; c0 < D; c0 += 8) {
+              uint32_t v[8];
+              tmem_ld8(lane_base + kColO + c0, v);
               tmem_ld_wait();
 #pragma unroll
-              for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-              tmem_st32(o_addr + c0, v);
+              for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
+              tmem_st8(lane_base + kColO + c0, v);
             }
             tmem_st_wait();
             l_sum *= alpha;
-            if (need) m_used = m_tile;
           }
         }
         // pass 2: P = exp2(S2 - m) as bf16 over the consumed S columns (chunk c lands in columns 16c..16c+15,
@@ -661,41 +826,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         tc_fence_before();
         mbar_arrive(&bars[kBarPFull + wg]);
       }
-      // ---- merge the two accumulators: O_even <- O_even 2^(m_e - m) + O_odd 2^(m_o - m) ----
-      s_merge[wg * 128 + row] = m_used;
-      s_merge[256 + wg * 128 + row] = l_sum;
-      if (!ok) *s_giveup = 1;
-      softmax_bar();
-      if (*s_giveup != 0) ok = false;
-      if (ok) {
-        const float m_other = s_merge[(wg ^ 1) * 128 + row], l_other = s_merge[256 + (wg ^ 1) * 128 + row];
-        if (n_dense >= 2) {
-          const float m_new = fmaxf(m_used, m_other);
-          const float a_self = ex2(m_used - m_new), a_oth = ex2(m_other - m_new);
-          const int q1 = q_of_v(n_dense - 1), q2 = q_of_v(n_dense - 2);
-          ok = warp_wait(&slot_free[q1 % NS], (q1 / NS) & 1, p.status, 36);
-          if (ok) ok = warp_wait(&slot_free[q2 % NS], (q2 / NS) & 1, p.status, 36);
-          if (ok) {
-            tc_fence_after();
-            const float a_e = wg == 0 ? a_self : a_oth, a_o = wg == 0 ? a_oth : a_self;
-            uint32_t ve[32], vo[32];
-            tmem_ld32(lane_base + kColO + wg * DW, ve);
-            tmem_ld32(lane_base + kColO + 64 + wg * DW, vo);
-            tmem_ld_wait();
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              ve[jj] = __float_as_uint(__uint_as_float(ve[jj]) * a_e + __uint_as_float(vo[jj]) * a_o);
-            tmem_st32(lane_base + kColO + wg * DW, ve);
-            tmem_st_wait();
-            tc_fence_before();
-          }
-          l_sum = wg == 0 ? l_sum * a_self + l_other * a_oth : 0.f;
-          m_used = m_new;
-        } else if (wg == 1) {  // a single dense tile: the second warpgroup adopts the first one's maximum
-          m_used = m_other;
-          l_sum = 0.f;
-        }
-      }
+      // the warpgroup that did not take the last tile follows its maximum
+      if (ok && ((n_dense - 1) & 1) != wg) ok = take_max(n_dense - 1);
     } else {
     for (int s = 0; s < n_dense; ++s) {
       const int buf = s & 1;
@@ -829,131 +961,9 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       // warpgroups' arrival, so it cannot start before both halves are merged)
     }
 
+    light_phase();
     }  // !ALT
 
-    // ------------------------------ light tiles ------------------------------
-    // P[i,k] = a_i[t_k] * bc_i[c_k]: one exponential per (row, key time step), packed bf16
-    // multiplies for the rest.  Four P buffers of 64 TMEM columns (the idle S columns) let these
-    // warps run ahead of the PV products.
-    if (ok && n_light > 0) {
-      // the buffers overlap S0 / S1: the last dense PV products must be done with them (and with O)
-      const int q1 = q_of_v(n_dense - 1);
-      ok = warp_wait(&slot_free[q1 % NS], (q1 / NS) & 1, p.status, 37);
-      tc_fence_after();
-    }
-    // Every light tile's score is its temporal score alone (the channel maximum is folded into bc), and
-    // the temporal scores of the row sit in TMEM: one pass finds the maximum over all light tiles, one
-    // rescale of O covers the whole phase, and the loop below carries no maximum.
-    // Key step tk of the light tiles (0 <= tk < n_light * TPB) is temporal column col0 + tk.
-    const int col0 = T - 1 - ti_abs;
-    uint32_t bc[NCH / 2];  // exp2(channel score - its maximum), bf16 pairs
-    float sum_bc = 0.f;
-#pragma unroll
-    for (int k2 = 0; k2 < NCH / 2; ++k2) {
-      bc[k2] = pack_bf16(ex2(cbf[2 * k2]), ex2(cbf[2 * k2 + 1]));
-      sum_bc += __uint_as_float(bc[k2] << 16) + __uint_as_float(bc[k2] & 0xffff0000u);
-    }
-    if (ok && n_light > 0) {
-      const int col1 = col0 + n_light * TPB;
-      float m_light = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (32 * c + 32 <= col0 || 32 * c >= col1) continue;  // (warp-uniform)
-        uint32_t v[32];
-        tmem_ld32(lane_base + kColTB + 32 * c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int col = 32 * c + jj;
-          const float tb = p.c2 * (__uint_as_float(v[jj]) + s_vr[col]) + mc;
-          if (col >= col0 && col < col1) m_light = fmaxf(m_light, tb);
-        }
-      }
-      const bool need = m_light > m_used + kRescaleThreshold;
-      if (__any_sync(0xffffffffu, need)) {
-        const float alpha = need ? ex2(m_used - m_light) : 1.f;
-#pragma unroll
-        for (int c0 = 0; c0 < DW; c0 += 32) {
-          uint32_t v[32];
-          tmem_ld32(lane_base + kColO + wg * DW + c0, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-          tmem_st32(lane_base + kColO + wg * DW + c0, v);
-        }
-        tmem_st_wait();
-        l_sum *= alpha;
-        if (need) m_used = m_light;
-      }
-    }
-    // Two tiles per turn: one round trip for the temporal scores and one look at the barriers serve both,
-    // and the second tile's products are formed while the first tile's stores are in flight.  (The scores
-    // of the next pair are fetched meanwhile; with an odd count the last fetch reads the column after the
-    // light tiles, still inside the temporal columns, and drops it.)
-    uint32_t tb_next[2 * TPB];
-    auto tb_fetch = [&](int l) {
-#pragma unroll
-      for (int j = 0; j < 2 * TPB; ++j) tmem_ld1(lane_base + kColTB + col0 + l * TPB + j, tb_next[j]);
-    };
-    auto p_regs = [&](float (&a_t)[TPW], uint32_t (&lo)[16], uint32_t (&hi)[16], bool count) {
-#pragma unroll
-      for (int tl = 0; tl < TPW; ++tl) {
-        const uint32_t a2 = pack_bf16(a_t[tl], a_t[tl]);
-        if (count) l_sum += __uint_as_float(a2 << 16) * sum_bc;
-#pragma unroll
-        for (int k2 = 0; k2 < NCH / 2; ++k2) {
-          const int idx = tl * (NCH / 2) + k2;
-          if (idx < 16) lo[idx] = hmul2_bf16(a2, bc[k2]);
-          else hi[idx - 16] = hmul2_bf16(a2, bc[k2]);
-        }
-      }
-    };
-    if (ok && n_light > 0) tb_fetch(0);
-    for (int l = 0; ok && l < n_light; l += 2) {
-      const int s = n_dense + l;
-      const bool two = l + 1 < n_light;
-      float a_t[2][TPW];  // exp2(temporal score - m) of this thread's key steps, both tiles
-      tmem_ld_wait();
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-#pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) {
-          const int tt = tt_base + tl;
-          uint32_t raw = 0;
-#pragma unroll
-          for (int q = 0; q < TPB; ++q)
-            if (q == tt) raw = tb_next[u * TPB + q];
-          const float tb = p.c2 * (__uint_as_float(raw) + s_vr[col0 + (l + u) * TPB + tt]) + mc;
-          a_t[u][tl] = ex2(tb - m_used);
-        }
-      }
-      if (l + 2 < n_light) tb_fetch(l + 2);
-      if (l >= 4) {
-        // these buffers last held P of light tiles l-4 and l-3: a PV product frees the V slot it read
-        const int q = q_of_v(s - 4);
-        ok = warp_wait(&slot_free[q % NS], (q / NS) & 1, p.status, 35);
-        if (ok && two) ok = warp_wait(&slot_free[(q + 1) % NS], ((q + 1) / NS) & 1, p.status, 35);
-        if (!ok) break;
-        tc_fence_after();
-      }
-      uint32_t lo0[16], hi0[16], lo1[16], hi1[16];
-      const uint32_t p_addr0 = lane_base + kColS + 64 * (l & 3) + 32 * wg;
-      const uint32_t p_addr1 = lane_base + kColS + 64 * ((l + 1) & 3) + 32 * wg;
-      p_regs(a_t[0], lo0, hi0, true);
-      tmem_st16(p_addr0, lo0);
-      tmem_st16(p_addr0 + 16, hi0);
-      p_regs(a_t[1], lo1, hi1, two);
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars[kBarPlFull + (l & 3)]);
-      if (two) {
-        tmem_st16(p_addr1, lo1);
-        tmem_st16(p_addr1 + 16, hi1);
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&bars[kBarPlFull + ((l + 1) & 3)]);
-      }
-    }
     // ------------------------------- epilogue ---------------------------------
     if (ok) {
       const int ql = q_of_v(n_tiles - 1);
@@ -1002,6 +1012,14 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     tmem_dealloc(tmem, kTmemCols);
   }
 }
+
+}  // namespace
+}  // namespace mvpa
+
+#include "tc_fwd_two.cuh"
+
+namespace mvpa {
+namespace {
 
 int make_maps(TcMaps& m, const Args& a, int CP) {
   const int TPB = 128 / CP;
@@ -1067,19 +1085,28 @@ int launch(const Args& a, int* status, cudaStream_t s) {
   t.status = status;
   float* relc = reinterpret_cast<float*>(status) + 64;  // workspace + 256 bytes
   t.relc = relc;
-  constexpr int smem = Cfg<D>::SMEM_BYTES;
-  static_assert(smem <= 232448, "shared memory budget");
+  const unsigned grid = (unsigned)t.q_tiles * a.B * a.H;
+  void (*kernel)(TcMaps, TcArgs) = tc_fwd_kernel<D, CP>;
+  int smem = Cfg<D>::SMEM_BYTES, threads = kThreads;
+  static_assert(Cfg<D>::SMEM_BYTES <= 232448, "shared memory budget");
   static_assert(Cfg<D>::EARLY >= 2, "the first tile's K and V load while the prologue runs");
-  MVPA_CUDA_CHECK(cudaFuncSetAttribute(tc_fwd_kernel<D, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if constexpr (D == 64 && CP <= 64) {
+    if (two::applies(a.window, CP, t.n_qt, grid)) {
+      kernel = two::tc_fwd_two_kernel<CP>;
+      smem = two::kSmemBytes;
+      threads = two::kThreads2;
+      MVPA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    }
+  }
+  MVPA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   rel_const_kernel<D><<<a.Hkv, 256, 0, s>>>(t.vt, t.z, (const __nv_bfloat16*)a.rt, (const __nv_bfloat16*)a.rc, relc, a.T,
                                            a.C, status);  // (clears the status words too)
   count_launch();
-  const unsigned grid = (unsigned)t.q_tiles * a.B * a.H;
   // Programmatic dependent launch: the CTAs come up (barriers, tensor memory) while the pre-kernel runs and wait
   // for it (griddep_wait) before they touch any memory that it or an earlier kernel has written.
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr;
@@ -1087,7 +1114,7 @@ int launch(const Args& a, int* status, cudaStream_t s) {
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  MVPA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tc_fwd_kernel<D, CP>, maps, t));
+  MVPA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, maps, t));
   count_launch();
   return MVPA_OK;
 }
