@@ -17,6 +17,7 @@ from operator import is_
 
 import torch
 
+import mvpa_host as _host
 import mvpa_native as _nat
 
 
@@ -127,13 +128,18 @@ class FlashMVPA(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time=(0, 0)):
         given = (q, u, vt, z, k, r_time, r_chan, v)
+        ctx.sm_scale, ctx.window, ctx.q_time = sm_scale, window, q_time
+        native = _host.module().forward(*given, sm_scale, window, *q_time, _CHECK_STATUS) if _host.usable(q) else None
+        if native is not None:
+            ctx.save_for_backward(*given, *native)
+            ctx.copied = ()
+            return native[0]
         q, u, vt, z, k, r_time, r_chan, v = read = _lay_out(*given)
         o = torch.empty_like(q)
         lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
         ctx.save_for_backward(*read, o, lse)
         # what was copied, for second derivatives alone: the copy belongs to no graph
         ctx.copied = () if all(map(is_, given, read)) else [(i, t, t._version) for i, t in enumerate(given) if t is not read[i]]
-        ctx.sm_scale, ctx.window, ctx.q_time = sm_scale, window, q_time
         return o
 
     @staticmethod
@@ -154,6 +160,10 @@ class FlashMVPA(torch.autograd.Function):
 
 
 def _gradients(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window):
+    if _host.usable(q):
+        native = _host.module().backward(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window, _CHECK_STATUS)
+        if native is not None:
+            return native
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     small = _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, _rows(do), dq, dk, dv, sm_scale, window)
     shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]
@@ -225,9 +235,9 @@ def _dense_head(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window):
 
 
 def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
-    """FlashMVPA with or without its autograd record.  The record costs about as much host time as everything else
-    of a small call, so an ordinary call that no gradient flows through goes to the kernels directly (and stores no
-    log-sum-exp); whatever traces or transforms the call sees the autograd function."""
+    """FlashMVPA with or without its autograd record: a call that no gradient flows through goes to the kernels directly (and
+    stores no log-sum-exp); whatever traces or transforms the call sees the autograd function.  (Most calls without a gradient
+    never come here: see the start of `flash_mvpa`.)"""
     ts = (q, u, vt, z, k, r_time, r_chan, v)
     if ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or not _nat.untraced()
             or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts)):
@@ -271,6 +281,11 @@ def flash_mvpa(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, causal, s
     [t0, t0+n) while the keys, values and relative keys describe the whole sequence — what one
     rank computes when a long sample is sharded by query time blocks (`mvpa_shard`).
     """
+    if rel_bias_time and rel_bias_chan and not p_drop and q_time_range is None and _host.usable(q):
+        # an ordinary call that no gradient flows through, with nothing to refuse, copy or trace: one native call
+        o = _host.module().attend(q, q_bias, q_btime, q_bchan, k_glob, k_time, k_chan, v, sm_scale, window_size, _CHECK_STATUS)
+        if o is not None:
+            return o
     if not (rel_bias_time or rel_bias_chan):
         raise NotImplementedError("flash_mvpa: at least one relative term is required (without them the "
                                   "reference runs a plain windowed attention, which these kernels are not)")

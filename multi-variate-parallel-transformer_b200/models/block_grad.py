@@ -13,6 +13,7 @@ import torch
 import torch.nn.functional as F
 
 import layers.mvpa as _layer
+import mvpa_host as _host
 import mvpa_native as _nat
 import mvpa_ops
 from attentions import attn as _attn
@@ -48,76 +49,31 @@ def through_expression(f, ins, need, grad_out):
     return [next(got) if n else None for n in need]
 
 
-def _heads_view(t, B, N, heads, D):
-    """(B*N, heads*D) columns as the kernels' (B, heads, N, D)."""
-    return t.view(B, N, heads, D).permute(0, 2, 1, 3)
-
-
-def _rel_keys(embeds, w, Hkv, D):
-    return torch.mm(embeds[0], w.t()).view(-1, Hkv, D).transpose(0, 1).contiguous()      # (Hkv, rows, D)
-
-
 class BlockFunction(torch.autograd.Function):
+    """Forward and backward are one native call each (`csrc_host/mvpa_host.cpp`: block_forward, block_backward)."""
+
     @staticmethod
     def forward(ctx, x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, eps, heads):
-        H, Hkv, D = heads
-        B, T, C, E = x.shape
-        N, KV = T * C, Hkv * D
-        x2 = x.view(B * N, E)
-        xn = mvpa_ops.rmsnorm(x2, ln_w, eps)
-        q, kv, g, up = (torch.mm(xn, w.t()) for w in (wq, wkv, wg, wu))
-        rt, rc = _rel_keys(pos, wpos, Hkv, D), _rel_keys(chan, wchan, Hkv, D)
-        o = torch.empty_like(q)
-        lse = _attn._launch_fwd(_heads_view(q, B, N, H, D), *bias.view(3, Hkv, D), _heads_view(kv[:, :KV], B, N, Hkv, D),
-                                rt, rc, _heads_view(kv[:, KV:], B, N, Hkv, D), _heads_view(o, B, N, H, D),
-                                1.0 / (D ** 0.5), WINDOW, (0, 0), True)
-        act = mvpa_ops.silu_mul(g, up, torch.empty_like(g))
-        h = torch.empty_like(x)          # (not a view of a matrix: the caller may change it in place)
-        torch.addmm(x2, act, wd.t(), out=h.view(B * N, E)).addmm_(o, wc.t())
-        ctx.save_for_backward(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act)
+        given = (x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd)
+        got = _host.module().block_forward(*given, eps, WINDOW, *heads, _attn._CHECK_STATUS)
+        if got is None:
+            raise RuntimeError("block: tensors that the kernels cannot take in place")   # (`applies` has looked at them)
+        ctx.save_for_backward(*given, *got[1:])      # ... xn, q, kv, g, up, rt, rc, o, lse, act
         ctx.eps, ctx.heads = eps, heads
-        return h
+        return got[0]
 
     @staticmethod
     def backward(ctx, dh):
         saved = ctx.saved_tensors
         need = ctx.needs_input_grad[:13]
-        if torch.is_grad_enabled() or not _nat.untraced() or not mvpa_ops._plain(dh.contiguous()):
-            # a graph of the gradient is wanted (or a transform is active): through the differentiable operations
-            grads = through_expression(lambda *ins: expression(*ins, ctx.eps, ctx.heads), saved[:13], need, dh)
-            return (*grads, None, None)
-        x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, xn, q, kv, g, up, rt, rc, o, lse, act = saved
-        H, Hkv, D = ctx.heads
-        B, T, C, E = x.shape
-        N, KV = T * C, Hkv * D
-        dh2 = dh.contiguous().view(B * N, E)
-        grad = [None] * 13
-        weight = lambda i, d, a: grad.__setitem__(i, torch.mm(d.t(), a)) if need[i] else None   # d W = d^T input
-        weight(9, dh2, o)
-        weight(12, dh2, act)
-        dg, dup = mvpa_ops.silu_mul_bwd(g, up, torch.mm(dh2, wd))
-        do = torch.mm(dh2, wc)
-        dq, dkv = torch.empty_like(q), torch.empty_like(kv)
-        view = lambda t, heads: _heads_view(t, B, N, heads, D)
-        small = _attn._launch_bwd(view(q, H), *bias.view(3, Hkv, D), view(kv[:, :KV], Hkv), rt, rc, view(kv[:, KV:], Hkv),
-                                  view(o, H), lse, view(do, H), view(dq, H), view(dkv[:, :KV], Hkv), view(dkv[:, KV:], Hkv),
-                                  1.0 / (D ** 0.5), WINDOW)
-        dbias, drt, drc = small.split((3 * KV, T * KV, C * KV))
-        if need[8]:
-            grad[8] = dbias.view(bias.shape)
-        for d, n, e, i_e, w, i_w in ((drt, T, pos, 1, wpos, 6), (drc, C, chan, 2, wchan, 7)):
-            d = d.view(Hkv, n, D).transpose(0, 1).reshape(n, KV)
-            weight(i_w, d, e[0])
-            if need[i_e]:
-                grad[i_e] = torch.mm(d, w).view(e.shape)
-        for i, d in ((4, dq), (5, dkv), (10, dg), (11, dup)):
-            weight(i, d, xn)
-        if need[0] or need[3]:
-            dxn = torch.mm(dq, wq)
-            for d, w in ((dkv, wkv), (dg, wg), (dup, wu)):
-                dxn.addmm_(d, w)
-            grad[0], grad[3] = mvpa_ops.rmsnorm_bwd(x, ln_w, dxn.view(x.shape), ctx.eps, add=dh2)
-        return (*grad, None, None)
+        if not torch.is_grad_enabled() and _nat.untraced() and mvpa_ops._plain(dh.contiguous()):
+            mask = sum(n << i for i, n in enumerate(need))
+            grads = _host.module().block_backward(dh, *saved, mask, ctx.eps, WINDOW, *ctx.heads, _attn._CHECK_STATUS)
+            if grads is not None:
+                return (*grads, None, None)
+        # a graph of the gradient is wanted (or a transform is active): through the differentiable operations
+        grads = through_expression(lambda *ins: expression(*ins, ctx.eps, ctx.heads), saved[:13], need, dh)
+        return (*grads, None, None)
 
 
 def shipped(cls):

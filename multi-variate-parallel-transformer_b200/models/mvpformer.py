@@ -30,8 +30,9 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
+import mvpa_host
 import mvpa_ops
-from attentions import flash_mvpa_into
+from attentions import attn as attn_mod, flash_mvpa_into
 from layers import MVPFormerGQAFlashAttention
 from models import BrainDecider, block_grad
 
@@ -162,6 +163,11 @@ class MVPFormerBlock(torch.nn.Module):
         I = self.mlp.gate_proj.out_features
         N, KV = T * C, Hkv * D
         w_in, w_out = self.fused_weights()
+        if mvpa_host.usable(x):
+            out = mvpa_host.module().branches(x, w_in, w_out, a.attn_bias.detach().to(x.dtype), r_time, r_chan, 10, B, T, C, H, Hkv, D,
+                                              attn_mod._CHECK_STATUS)
+            if out is not None:
+                return out
         big = F.linear(x, w_in)                                          # (M, E + 2 KV + 2 I)
         q4 = big[:, :E].view(B, N, H, D).permute(0, 2, 1, 3)
         k4 = big[:, E:E + KV].view(B, N, Hkv, D).permute(0, 2, 1, 3)
@@ -321,7 +327,6 @@ class MVPFormerModel(torch.nn.Module):
         r_chan = F.linear(channel_embeds.to(embeds_local.dtype), w_chan).view(C, L, Hkv, D).permute(1, 2, 0, 3).contiguous()
         h = embeds_local.contiguous().clone()                             # the residual stream is updated in place
         branches = None
-        import attentions.attn as attn_mod
         check = attn_mod._CHECK_STATUS
         attn_mod._CHECK_STATUS = False      # reading a status word back after every launch would stall the overlap
         try:
@@ -348,7 +353,6 @@ class MVPFormerModel(torch.nn.Module):
 
     @torch.no_grad()
     def _graphed_forward(self, hidden, position_ids, channel_ids):
-        import attentions.attn as attn_mod
         key = (tuple(hidden.shape), hidden.dtype, hidden.device.index, tuple(position_ids.shape), tuple(channel_ids.shape))
         entry = self._graphs.get(key)
         if entry is None:

@@ -12,6 +12,7 @@ import functools
 import numpy as np
 import torch
 
+import mvpa_host as _host
 import mvpa_native as _nat
 
 
@@ -105,7 +106,11 @@ def _plain(*ts):
     contiguous, 16-byte aligned, not empty; no forward-mode level, functorch transform or tracer is active
     (those are served by the differentiable torch expressions)."""
     t0 = ts[0]
-    # (types first: a symbolic value answers no question about itself)
+    if _host.usable(t0):
+        answer = _host.module().plain(*ts)
+        if answer >= 0:
+            return answer == 1
+    # (a function mode is active, or the first tensor is none of ours; types first: a symbolic value answers no question about itself)
     if not all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts) or not _nat.untraced() \
             or t0.dtype not in (torch.bfloat16, torch.float32):
         return False
