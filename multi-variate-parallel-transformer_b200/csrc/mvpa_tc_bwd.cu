@@ -84,8 +84,9 @@ struct BqArgs {
 enum BarrierIndex {
   kBarProFull = 0, kBarProMma, kBarProDone, kBarSFull, kBarSFull1, kBarDpFull, kBarDpFull1, kBarDsFull, kBarDsFull1, kBarAllDone,
   kBarFinFull, kBarFinLoaded, kBarFinDone, kBarRelDone,
-  kBarTbPart,                    // 4: the second warpgroup's part of a tile's dTB is in shared memory (CP = 128)
-  kBarTbPartEnd = kBarTbPart + 3,
+  kBarTbPart,                    // 4: one warpgroup's part of a dense tile's dTB is in shared memory (CP = 128)
+  kBarLtPart = kBarTbPart + 4,   // 2: both warpgroups' parts of sixteen light tiles' dTB are in tensor memory (CP = 128)
+  kBarLtPartEnd = kBarLtPart + 1,
   kBarSlotFull,  // NS, then slot_free NS
 };
 
@@ -141,14 +142,16 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   constexpr int KSTEPS = D / 16;
   constexpr int DW = D / 2;
   // TMEM columns: S / dS double-buffered, so that the score product of the next tile runs while the
-  // softmax warps work on this one.  The raw temporal products only pass through the dQ columns during
-  // the prologue (the scaled scores are re-read from the workspace, tile by tile); the dr_time
-  // accumulator of the epilogue takes the second S buffer.
+  // softmax warps work on this one.  The raw temporal products wait in the dQ columns until the first dense
+  // tile (the light tiles read them there; the dense tiles re-read the scaled scores from the workspace); the
+  // dr_time accumulator of the epilogue takes the second S buffer.
   constexpr uint32_t kQS = 0, kQS1 = 128, kQDP = 256, kQDQ = 384;
   // Each (row, slot) sum of dS goes into a shared-memory tile.  With at most 64 channel slots a key time step
-  // belongs to one warpgroup; with 128 the second warpgroup hands its part to the first one through shared memory,
-  // which stores the sum one tile later, when the part has long arrived (four buffers: a part's place is written again
-  // four tiles on, and the report of the tile after it lies between).
+  // belongs to one warpgroup; with 128 each warpgroup has a part of it.  Light tiles: the parts collect in idle
+  // tensor-memory columns (a thread's lane is its row in both warpgroups) and are added sixteen tiles at a time.
+  // Dense tiles: the warpgroups take turns; one hands its part to the other through shared memory, which stores
+  // the sum one tile later, when the part has long arrived (four buffers: a part's place is written again four
+  // tiles on, and the report of the tile after it lies between).
   constexpr bool PART = CP == 128;
   // The prologue's scratch rows are padded by two floats: slot C-1-|c_i - c_k| runs up the row for c_k <= c_i and down it
   // for c_k > c_i, without bank conflicts either way.  (128 slots: the last kilobyte reaches into the tile of temporal
@@ -220,6 +223,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     mbar_init(&bars[kBarFinDone], 1);
     mbar_init(&bars[kBarRelDone], 1);
     for (int i = 0; i < 4; ++i) mbar_init(&bars[kBarTbPart + i], kSoftmaxThreads / 2);
+    for (int i = 0; i < 2; ++i) mbar_init(&bars[kBarLtPart + i], kSoftmaxThreads);
     for (int i = 0; i < NS; ++i) {
       mbar_init(&slot_full[i], 1);
       mbar_init(&slot_free[i], 1);
@@ -242,7 +246,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   }
 
   if (warp >= 8) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
@@ -304,12 +308,12 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         tc_fence_after();
         const DescHalves dr = make_desc_halves_sw128(smem_u32(sR), 16, 1024);
         const DescHalves dc = make_desc_halves_sw128(smem_u32(sC), 16, 1024);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           mma_ss_w(el, tm + kQDQ, dq, off, dr, off, idesc_s, kk > 0);
         }
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {
           const uint32_t offa = (kk / 4) * HALF + (kk % 4) * 32;
           const uint32_t offb = (kk / 4) * (CP * 128) + (kk % 4) * 32;
@@ -332,7 +336,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         tc_fence_after();
         DescHalves dk = dkm0;
         dk.lo += (uint32_t)ksl * (TILE >> 4);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {  // S = Q' K^T
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           mma_ss_w(el, tm + kQS + 128 * (s & 1), dq, off, dk, off, idesc_s, kk > 0);
@@ -346,7 +350,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         tc_fence_after();
         DescHalves dv = dkm0;
         dv.lo += (uint32_t)vsl * (TILE >> 4);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {  // dP = dO V^T  (V rows = keys, D contiguous: K-major operand)
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           // a light tile has no score product: its dP takes the idle S buffer, so two are in flight
@@ -389,7 +393,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         const DescHalves dfc = make_desc_halves_sw128(smem_u32(ring + 65536 + TILE), CP * 128, 1024);
         mma_ts_x4_w(el, tm + kQDQ, tm + kQS, dfr.lo, dfr.hi, 2048 >> 4, idesc_q, 1u);
         mma_ts_x4_w(el, tm + kQDQ, tm + kQS + 32, dfr.lo + 4 * (2048 >> 4), dfr.hi, 2048 >> 4, idesc_q, 1u);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < CP / 16; ++kk) mma_ts_w(el, tm + kQDQ, tm + kQDP + kk * 8, dfc, kk * 2048, idesc_q, 1u);
       }
       mma_commit_w(el, smem_u32(&bars[kBarFinDone]));
@@ -405,11 +409,11 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         const DescHalves dcbt = make_desc_halves_sw128(smem_u32(D == 128 ? sDO : ring + 98304), HALF, 1024);
         const DescHalves dqm = make_desc_halves_sw128(smem_u32(sQ), HALF, 1024);
         const DescHalves dones = make_desc_halves_sw128(smem_u32(ring + 32768), 16, 1024);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < 8; ++kk) mma_ss_w(el, tm + kQS1, dtbt, kk * 2048, dqm, kk * 2048, idesc_r, kk > 0);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < 8; ++kk) mma_ss_w(el, tm + kQS, dcbt, kk * 2048, dqm, kk * 2048, idesc_r, kk > 0);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t offb = (kk / 4) * 2048 + (kk % 4) * 32;
           mma_ss_w(el, tm + kQDP, dtbt, kk * 2048, dones, offb, idesc_1, kk > 0);
@@ -421,7 +425,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     }
   }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ------------------------------ softmax warps ------------------------------
     const int row = tid & 127;
     const int wg = tid >> 7;
@@ -444,35 +448,28 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     if (ok) {
       tc_fence_after();
       // The prologue and the epilogue run once per CTA, so their instructions come from memory rather
-      // than the instruction cache: they are written as short loops, not unrolled.
+      // than the instruction cache: short loops where registers need not be indexed (the products too are issued from loops).
       // temporal scores of the row, for the key-side kernel (each warpgroup dumps half of the columns)
       {
         float* dst = p.tbw + ((int64_t)bh * T + 64 * wg) * N + (row_valid ? n_loc : 0);
         // Only the slots of keys a row can see (t_k <= t_i: slot >= T-1-t_i) are ever read, by this
         // kernel's loop and by the key-side kernel: early query tiles skip most of the dump.
         const int j_row = T - 1 - min(ti_abs, T - 1);
-        auto put8 = [&](const uint32_t (&v)[8], int c8) {
-          if (row_valid) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const int j = 64 * wg + c8 + e;
-              if (j >= j_row && j < T) dst[(int64_t)(c8 + e) * N] = p.c2 * (__uint_as_float(v[e]) + s_vr[j]);
-            }
-          }
-        };
         const int j_tile = max(T - 1 - (I * TPB + TPB - 1), 0) - 64 * wg;  // first slot any row of the tile can see
-        const int c_first = j_tile <= 0 ? 0 : (j_tile & ~15);
-        const int c_last = min(64, (T - 64 * wg + 15) & ~15);  // nothing past the last time step
-        uint32_t va[8], vb[8];  // the next 8 columns are in flight while 8 are stored
-        if (c_first < c_last) tmem_ld8(lane_base + kQDQ + 64 * wg + c_first, va);
+        const int c_first = j_tile <= 0 ? 0 : (j_tile & ~7);
+        const int c_last = min(64, T - 64 * wg);  // nothing past the last time step
+        float* d = dst + (int64_t)c_first * N;
 #pragma unroll 1
-        for (int c8 = c_first; c8 < c_last; c8 += 16) {
+        for (int c8 = c_first; c8 < c_last; c8 += 8) {
+          uint32_t v[8];
+          tmem_ld8(lane_base + kQDQ + 64 * wg + c8, v);
           tmem_ld_wait();
-          tmem_ld8(lane_base + kQDQ + 64 * wg + c8 + 8, vb);
-          put8(va, c8);
-          tmem_ld_wait();
-          if (c8 + 16 < c_last) tmem_ld8(lane_base + kQDQ + 64 * wg + c8 + 16, va);
-          put8(vb, c8 + 8);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int j = 64 * wg + c8 + e;
+            if (row_valid && j >= j_row && j < T) *d = p.c2 * (__uint_as_float(v[e]) + s_vr[j]);
+            d += N;
+          }
         }
       }
       // channel scores by |c_i - c_k| slot to shared memory (8-column chunks alternate between the warpgroups)
@@ -502,20 +499,15 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         const float* src = k <= kc ? up + k : down - k;
         return (ok && k < climit) ? *src : -INFINITY;
       };
-      // At 128 slots the values stay in registers (12 -> 9 k cycles for the whole step); below, where the step is shorter, a
-      // second walk in a short loop is the faster form (8.0 against 9.3 k cycles at 32 slots).
-      constexpr bool KEEP = CP == 128;
-      float gv[KEEP ? NCH : 1];
+      // The values stay in registers between the maximum and their use.  (A second walk in a short loop was the faster form at up
+      // to 64 slots while the kernel's instructions did not fit the caches; now it costs 8 x 128 x 32 tokens 759 against 712 us,
+      // 4 x 25 x 64 122 against 105.)
+      float gv[NCH];
       float mx = -INFINITY;
-      if constexpr (KEEP) {
 #pragma unroll
-        for (int k = 0; k < NCH; ++k) {
-          gv[k] = gathered(k);
-          mx = fmaxf(mx, gv[k]);
-        }
-      } else {
-#pragma unroll 4
-        for (int k = 0; k < NCH; ++k) mx = fmaxf(mx, gathered(k));
+      for (int k = 0; k < NCH; ++k) {
+        gv[k] = gathered(k);
+        mx = fmaxf(mx, gv[k]);
       }
       if constexpr (CP == 128) {  // the row maximum spans both warpgroups' columns
         s_max[wg * 128 + row] = mx;
@@ -529,8 +521,7 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         uint32_t pk[8], pb[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float x0 = (KEEP ? gv[KEEP ? k16 + 2 * e : 0] : gathered(k16 + 2 * e)) - mc;
-          const float x1 = (KEEP ? gv[KEEP ? k16 + 2 * e + 1 : 0] : gathered(k16 + 2 * e + 1)) - mc;
+          const float x0 = gv[k16 + 2 * e] - mc, x1 = gv[k16 + 2 * e + 1] - mc;
           const __half2 hh2 = __floats2half2_rn(x0, x1);
           const __half2 eh2 = __floats2half2_rn(ex2(x0), ex2(x1));
           pk[e] = *reinterpret_cast<const uint32_t*>(&hh2);
@@ -554,13 +545,8 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
           bdst[N] = make_uint4(wb[4], wb[5], wb[6], wb[7]);
         }
       };
-      if constexpr (KEEP) {
 #pragma unroll
-        for (int k16 = 0; k16 < NCH; k16 += 16) stage(k16);
-      } else {
-#pragma unroll 1
-        for (int k16 = 0; k16 < NCH; k16 += 16) stage(k16);
-      }
+      for (int k16 = 0; k16 < NCH; k16 += 16) stage(k16);
       // the tile of temporal sums: slots no key tile reaches stay zero (at 128 channel slots the barrier above stands after
       // every read of the scratch that reaches into it)
 #pragma unroll
@@ -594,17 +580,6 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
     for (int k = 0; k < NCH; ++k) dcb_acc[k] = 0.f;
     const float off_row = mc - L_i;  // every exponent carries +mc (cbl is relative to it) and -L
 
-    // Temporal scores of the row come back from the workspace (this CTA wrote them in the prologue; the
-    // barriers since then order the accesses): TPW values per tile, fetched one tile ahead.
-    const float* tb_src = p.tbw + (int64_t)bh * T * N + (row_valid ? n_loc : 0);
-    auto tb_slot = [&](int s, int tl) {
-      const int tk_abs = tile_of(s) * TPB + tt_base + tl;
-      return T - 1 - min(max(ti_abs - tk_abs, 0), T - 1);
-    };
-    float tb_next[TPW];
-#pragma unroll
-    for (int tl = 0; tl < TPW; ++tl) tb_next[tl] = ok ? __ldcg(tb_src + (int64_t)tb_slot(0, tl) * N) : 0.f;
-
     // sm_scale is folded into the exponent: the loop works with P' = sm_scale * P, so dS = P' (dP - delta)
     const float lscale = log2f(p.sm_scale);
     const float2 neg_delta = make_float2(-delta_i, -delta_i);
@@ -618,151 +593,225 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
 #pragma unroll
       for (int k2 = 0; k2 < NCH / 2; ++k2) *reinterpret_cast<uint32_t*>(&cbl[k2]) = w[k2];
     };
-    // Light tiles: P'[i,k] = a[t_k] bc[c_k] with a = exp2(temporal score + max - L + log2 sm_scale), so
-    //   sum_t dS = bc[c_k] (sum_t a[t] dP[t, c_k] - delta sum_t a[t])        -> two FMAs per element:
-    //   sum_c dS = a[t] (sum_c bc[c] dP[t, c] - delta sum_c bc[c])
-    // dcb_acc holds the inner sums until the transition below scales them.
-    float bcf[NCH];
-    float a_sum = 0.f, bc_sum = 0.f;
-    if (n_light > 0) {
-      uint32_t w[32];
-      tmem_ld32(lane_base + kQDP + 64 + 32 * wg, w);
-      tmem_ld_wait();
-#pragma unroll
-      for (int k2 = 0; k2 < NCH / 2; ++k2) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k2]));
-        bcf[2 * k2] = f.x;
-        bcf[2 * k2 + 1] = f.y;
-        bc_sum += f.x + f.y;
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < NCH; ++k) bcf[k] = 0.f;
-      load_cbl();
-    }
-    tc_fence_before();
-    mbar_arrive(&bars[kBarProDone]);  // only now may a dP product overwrite the staged values
     auto put_tb = [&](int sl, float x) {
       *reinterpret_cast<__nv_bfloat16*>(s_tbt_main + (sl >> 6) * HALF + row * 128 + ((((sl & 63) >> 3) ^ (row & 7)) << 4) +
                                         (sl & 7) * 2) = __float2bfloat16_rn(x);
     };
-    float own_sum = 0.f;  // this warpgroup's part of the previous tile's sum, and its slot (PART, first warpgroup)
+    // The dense tiles' temporal scores come from the workspace (this CTA wrote them in the prologue; the barriers since then
+    // order the accesses): TPW values per tile, requested two tiles ahead, those of the first two before the light tiles.
+    const float* tb_src = p.tbw + (int64_t)bh * T * N + (row_valid ? n_loc : 0);
+    auto tb_load = [&](int s, float (&dst)[TPW]) {
+#pragma unroll
+      for (int tl = 0; tl < TPW; ++tl) {
+        const int dt = ti_abs - (s * TPB + tt_base + tl), slot = T - 1 - min(max(dt, 0), T - 1);
+        dst[tl] = __ldcg(tb_src + (int64_t)slot * N);
+      }
+    };
+    float tb0[TPW], tb1[TPW];  // scores of the next tile and of the one after it
+#pragma unroll
+    for (int tl = 0; tl < TPW; ++tl) tb0[tl] = tb1[tl] = 0.f;
+    if (ok) {
+      tb_load(n_light, tb0);
+      if (n_light + 1 < n_tiles) tb_load(n_light + 1, tb1);
+    }
+    // ---- light tiles ----
+    // P'[i,k] = a[t_k] bc[c_k] with a = exp2(temporal score + max - L + log2 sm_scale), so
+    //   sum_t dS = bc[c_k] (sum_t a[t] dP[t, c_k] - delta sum_t a[t])        -> two FMAs per element:
+    //   sum_c dS = a[t] (sum_c bc[c] dP[t, c] - delta sum_c bc[c])
+    // dcb_acc holds the inner sums until the transition below scales them.
+    // Per tile: the temporal scores from tensor memory (asked for one tile ahead), dP by quarters, each one's load under
+    // the sums of the one before.  The tile is reported as soon as its last value sits in a register, so that
+    // the product of the tile after next runs under the sums.
+    // (Per tile at 16k tokens, D 128: 2.4 k cycles while the scores came from the workspace, the report stood behind
+    // the sums and the parts of dTB were handed over tile by tile, 1.3 k now, most of it hand-over latency.)
+    if (n_light > 0) {
+      float bcf[NCH];
+      float a_sum = 0.f, bc_sum = 0.f;
+      {
+        uint32_t w[32];
+        tmem_ld32(lane_base + kQDP + 64 + 32 * wg, w);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k2 = 0; k2 < NCH / 2; ++k2) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k2]));
+          bcf[2 * k2] = f.x;
+          bcf[2 * k2 + 1] = f.y;
+          bc_sum += f.x + f.y;
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&bars[kBarProDone]);
+      const int tcol0 = T - 1 - ti_abs + tt_base;  // temporal column of this thread's first key step of tile 0
+      uint32_t tb_raw[TPW];
+      auto tb_fetch = [&](int l) {
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl) tmem_ld1(lane_base + kQDQ + tcol0 + l * TPB + tl, tb_raw[tl]);
+      };
+      if (ok) tb_fetch(0);
+      for (int l = 0; ok && l < n_light; ++l) {
+        float a[TPW], dtb[TPW];
+        constexpr int CHAINS = PART ? 2 : 1;
+        float2 w2[TPW][CHAINS];
+        tmem_ld_wait();
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl) {
+          a[tl] = ex2(p.c2 * (__uint_as_float(tb_raw[tl]) + s_vr[tcol0 + l * TPB + tl]) + off_row + lscale);  // (rows that do not exist: 0)
+          a_sum += a[tl];
+#pragma unroll
+          for (int x = 0; x < CHAINS; ++x) w2[tl][x] = make_float2(0.f, 0.f);
+        }
+        auto sums = [&](const uint32_t (&dp)[16], int quarter) {
+#pragma unroll
+          for (int jj = 0; jj < 16; jj += 2) {
+            const int lc = 16 * quarter + jj, tl = lc / CP, k = lc % NCH, x = (jj >> 1) % CHAINS;
+            const float2 d = as_float2(dp[jj], dp[jj + 1]);
+            const float2 ca = ffma2(make_float2(a[tl], a[tl]), d, make_float2(dcb_acc[k], dcb_acc[k + 1]));
+            dcb_acc[k] = ca.x;
+            dcb_acc[k + 1] = ca.y;
+            w2[tl][x] = ffma2(make_float2(bcf[k], bcf[k + 1]), d, w2[tl][x]);
+          }
+        };
+        ok = warp_wait(&bars[kBarDpFull + (l & 1)], (l >> 1) & 1, p.status, 133);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t dp_addr = lane_base + kQS + 128 * (l & 1) + 64 * wg;
+        uint32_t dp0[16], dp1[16];
+        tmem_ld16(dp_addr, dp0);
+        tmem_ld_wait();
+        tmem_ld16(dp_addr + 16, dp1);
+        sums(dp0, 0);
+        tmem_ld_wait();
+        tmem_ld16(dp_addr + 32, dp0);
+        sums(dp1, 1);
+        tmem_ld_wait();
+        tmem_ld16(dp_addr + 48, dp1);
+        if (l + 1 < n_light) tb_fetch(l + 1);
+        sums(dp0, 2);
+        tmem_ld_wait();
+        tc_fence_before();
+        if (l + 1 < n_light) mbar_arrive(&bars[kBarDsFull + (l & 1)]);
+        sums(dp1, 3);
+#pragma unroll
+        for (int tl = 0; tl < TPW; ++tl) {
+          const float2 w = CHAINS == 2 ? fadd2(w2[tl][0], w2[tl][CHAINS - 1]) : w2[tl][0];
+          dtb[tl] = a[tl] * (w.x + w.y - delta_i * bc_sum);
+        }
+        if constexpr (PART) {
+          // columns of the exponentials, which sit in registers by now: [warpgroup][2 buffers][16 tiles]
+          const int n = l >> 4;  // (a buffer is written again two hand-overs later, and everyone has read it by the next one)
+          const uint32_t parts = kQDP + 64 + 16 * (n & 1);
+          tmem_st1(lane_base + parts + 32 * wg + (l & 15), __float_as_uint(dtb[0]));
+          if ((l & 15) == 15 || l + 1 == n_light) {
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(&bars[kBarLtPart + (n & 1)]);
+            ok = warp_wait(&bars[kBarLtPart + (n & 1)], (n >> 1) & 1, p.status, 138);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t p0[8], p1[8];  // each warpgroup adds and stores eight tiles
+            tmem_ld8(lane_base + parts + 8 * wg, p0);
+            tmem_ld8(lane_base + parts + 32 + 8 * wg, p1);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int lj = 16 * n + 8 * wg + j;
+              if (lj < n_light) put_tb(T - 1 - ti_abs + lj, __uint_as_float(p0[j]) + __uint_as_float(p1[j]));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int tl = 0; tl < TPW; ++tl) put_tb(tcol0 + l * TPB + tl, dtb[tl]);
+        }
+      }
+      // transition: scale the light phase's inner sums
+#pragma unroll
+      for (int k = 0; k < NCH; ++k) dcb_acc[k] = bcf[k] * (dcb_acc[k] - delta_i * a_sum);
+    }
+    // The scores the dense tiles need are fetched before the last light tile's report (without light tiles: the
+    // prologue's) lets the first dense dP product overwrite where they, and the parts above, wait.
+    load_cbl();
+    tc_fence_before();
+    if (n_light == 0) mbar_arrive(&bars[kBarProDone]);
+    else if (ok) mbar_arrive(&bars[kBarDsFull + ((n_light - 1) & 1)]);
+
+    // ---- dense tiles ----
+    float own_sum = 0.f;  // this warpgroup's part of the previous tile's sum, and its slot (PART)
     int own_slot = -1;
-    auto flush_part = [&](int s) -> bool {
-      if (!warp_wait(&bars[kBarTbPart + (s & 3)], (s >> 2) & 1, p.status, 137)) return false;
-      if (own_slot >= 0) put_tb(own_slot, own_sum + s_part[(s & 3) * 128 + row]);
+    auto flush_part = [&](int e) -> bool {
+      if (!warp_wait(&bars[kBarTbPart + (e & 3)], (e >> 2) & 1, p.status, 137)) return false;
+      if (own_slot >= 0) put_tb(own_slot, own_sum + s_part[(e & 3) * 128 + row]);
       return true;
     };
-    for (int s = 0; ok && s < n_tiles; ++s) {
-      const bool dense = is_dense(s);
-      const int J = tile_of(s);
-      float offs[TPW], wmul[TPW], dtb_acc[TPW];
+    for (int s = n_light; ok && s < n_tiles; ++s) {
+      const int e = s - n_light;
+      float offs[TPW], wmul[TPW];
       float2 dtb2[TPW];
       int slot[TPW];
       bool valid[TPW];
 #pragma unroll
       for (int tl = 0; tl < TPW; ++tl) {
-        const int tk_abs = J * TPB + tt_base + tl, dt = ti_abs - tk_abs;
+        const int tk_abs = s * TPB + tt_base + tl, dt = ti_abs - tk_abs;
         valid[tl] = dt >= 0 && tk_abs < T && row_valid;
         slot[tl] = T - 1 - min(max(dt, 0), T - 1);
         wmul[tl] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
         dtb2[tl] = make_float2(0.f, 0.f);
-        offs[tl] = valid[tl] ? tb_next[tl] + off_row + lscale : -INFINITY;
+        offs[tl] = valid[tl] ? tb0[tl] + off_row + lscale : -INFINITY;
+        tb0[tl] = tb1[tl];
       }
-      if (s + 1 < n_tiles) {
-#pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) tb_next[tl] = __ldcg(tb_src + (int64_t)tb_slot(s + 1, tl) * N);
-      }
-      if (dense) {
-        ok = warp_wait(&bars[kBarSFull + (s & 1)], ((s - n_light) >> 1) & 1, p.status, 132);
-        if (!ok) break;
-      }
+      if (s + 2 < n_tiles) tb_load(s + 2, tb1);
+      ok = warp_wait(&bars[kBarSFull + (s & 1)], (e >> 1) & 1, p.status, 132);
+      if (!ok) break;
       ok = warp_wait(&bars[kBarDpFull + (s & 1)], (s >> 1) & 1, p.status, 133);
       if (!ok) break;
       tc_fence_after();
-      if (dense) {
-        // P' = exp2(S2 - L + log2 sm_scale), dS = P' (dP - delta)   (`attentions/attn.py:680`)
-        const uint32_t s_addr = lane_base + kQS + 128 * (s & 1) + 64 * wg;
+      // P' = exp2(S2 - L + log2 sm_scale), dS = P' (dP - delta)   (`attentions/attn.py:680`)
+      const uint32_t s_addr = lane_base + kQS + 128 * (s & 1) + 64 * wg;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t sv[32], dp[32];
-          tmem_ld32(s_addr + 32 * half, sv);
-          tmem_ld32(lane_base + kQDP + 64 * wg + 32 * half, dp);
-          tmem_ld_wait();
-          uint32_t pk[16];
+      for (int half = 0; half < 2; ++half) {
+        uint32_t sv[32], dp[32];
+        tmem_ld32(s_addr + 32 * half, sv);
+        tmem_ld32(lane_base + kQDP + 64 * wg + 32 * half, dp);
+        tmem_ld_wait();
+        uint32_t pk[16];
 #pragma unroll
-          for (int jj = 0; jj < 32; jj += 2) {
-            const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
-            const float2 cb = __half22float2(cbl[k / 2]);
-            const float2 x = fadd2(ffma2(as_float2(sv[jj], sv[jj + 1]), make_float2(wmul[tl], wmul[tl]), cb),
-                                   make_float2(offs[tl], offs[tl]));
-            const float2 ds = fmul2(make_float2(ex2(x.x), ex2(x.y)), fadd2(as_float2(dp[jj], dp[jj + 1]), neg_delta));
-            const float2 ca = fadd2(make_float2(dcb_acc[k], dcb_acc[k + 1]), ds);
-            dcb_acc[k] = ca.x;
-            dcb_acc[k + 1] = ca.y;
-            dtb2[tl] = fadd2(dtb2[tl], ds);
-            const uint32_t both = pack_bf16(ds.x, ds.y);
-            pk[jj / 2] = wmul[tl] != 0.f ? both : 0u;  // content term only inside the window
-          }
-          tmem_st16(s_addr + 16 * half, pk);  // dS_w over this thread's consumed S columns
+        for (int jj = 0; jj < 32; jj += 2) {
+          const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
+          const float2 cb = __half22float2(cbl[k / 2]);
+          const float2 x = fadd2(ffma2(as_float2(sv[jj], sv[jj + 1]), make_float2(wmul[tl], wmul[tl]), cb),
+                                 make_float2(offs[tl], offs[tl]));
+          const float2 ds = fmul2(make_float2(ex2(x.x), ex2(x.y)), fadd2(as_float2(dp[jj], dp[jj + 1]), neg_delta));
+          const float2 ca = fadd2(make_float2(dcb_acc[k], dcb_acc[k + 1]), ds);
+          dcb_acc[k] = ca.x;
+          dcb_acc[k + 1] = ca.y;
+          dtb2[tl] = fadd2(dtb2[tl], ds);
+          const uint32_t both = pack_bf16(ds.x, ds.y);
+          pk[jj / 2] = wmul[tl] != 0.f ? both : 0u;  // content term only inside the window
         }
-        tmem_st_wait();
-#pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) dtb_acc[tl] = dtb2[tl].x + dtb2[tl].y;
-      } else {
-        float a[TPW];
-        float2 w2[TPW];
-#pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) {
-          a[tl] = ex2(offs[tl]);  // 0 where the time step is not visible
-          a_sum += a[tl];
-          w2[tl] = make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t dp[32];
-          tmem_ld32(lane_base + kQS + 128 * (s & 1) + 64 * wg + 32 * half, dp);
-          tmem_ld_wait();
-#pragma unroll
-          for (int jj = 0; jj < 32; jj += 2) {
-            const int lc = 32 * half + jj, tl = lc / CP, k = lc % NCH;
-            const float2 d = as_float2(dp[jj], dp[jj + 1]);
-            const float2 ca = ffma2(make_float2(a[tl], a[tl]), d, make_float2(dcb_acc[k], dcb_acc[k + 1]));
-            dcb_acc[k] = ca.x;
-            dcb_acc[k + 1] = ca.y;
-            w2[tl] = ffma2(make_float2(bcf[k], bcf[k + 1]), d, w2[tl]);
-          }
-        }
-#pragma unroll
-        for (int tl = 0; tl < TPW; ++tl) dtb_acc[tl] = a[tl] * (w2[tl].x + w2[tl].y - delta_i * bc_sum);
-        if (s == n_light - 1) {
-          // transition: scale the light phase's inner sums, then fetch the scores the dense tiles need
-          // (before the report below lets the first dense dP product overwrite where they wait)
-#pragma unroll
-          for (int k = 0; k < NCH; ++k) dcb_acc[k] = bcf[k] * (dcb_acc[k] - delta_i * a_sum);
-          load_cbl();
-        }
+        tmem_st16(s_addr + 16 * half, pk);  // dS_w over this thread's consumed S columns
       }
+      tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars[kBarDsFull + (s & 1)]);
       // row sums per key time step
       if constexpr (PART) {
-        if (wg == 1) {
-          s_part[(s & 3) * 128 + row] = dtb_acc[0];
-          mbar_arrive(&bars[kBarTbPart + (s & 3)]);
-        } else {
-          if (s > 0) ok = flush_part(s - 1);
+        // (tile e's sum is stored by warpgroup e mod 2: one part and one stored sum per two tiles for each)
+        const float sum = dtb2[0].x + dtb2[0].y;
+        if ((e & 1) != wg) {
+          s_part[(e & 3) * 128 + row] = sum;
+          mbar_arrive(&bars[kBarTbPart + (e & 3)]);
+          if (e > 0) ok = flush_part(e - 1);
           if (!ok) break;
-          own_sum = dtb_acc[0];
+        } else {
+          own_sum = sum;
           own_slot = valid[0] ? slot[0] : -1;
         }
       } else {
 #pragma unroll
         for (int tl = 0; tl < TPW; ++tl)
-          if (valid[tl]) put_tb(slot[tl], dtb_acc[tl]);
+          if (valid[tl]) put_tb(slot[tl], dtb2[tl].x + dtb2[tl].y);
       }
     }
-    if (PART && wg == 0 && ok) ok = flush_part(n_tiles - 1);
+    if (PART && ok && ((n_tiles - n_light - 1) & 1) == wg) ok = flush_part(n_tiles - n_light - 1);
     // ------------------------------- epilogue ---------------------------------
     if (ok) ok = warp_wait(&bars[kBarAllDone], 0, p.status, 134);
     // du = sum over rows of dq's content part (`attentions/attn.py:1305-1306`: q + q_bias feeds the content
