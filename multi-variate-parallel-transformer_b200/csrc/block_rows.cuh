@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 
 #include "mvpa_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace mvpa {
 namespace {
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) rmsnorm_kernel(const T* __r
                                                                     const T* __restrict__ w, T* __restrict__ h_out,
                                                                     T* __restrict__ y, int64_t rows, int E, float eps) {
   constexpr int N = Vec<T>::N;
+  ptx::griddep_wait();
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ p
 template <typename T>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_t ld_in,
                                                        T* __restrict__ out, int64_t ld_out, int64_t rows, int width) {
+  ptx::griddep_wait();
   constexpr int N = Vec<T>::N;
   const int vec_per_row = width / N;
   const int64_t total = rows * vec_per_row;
@@ -338,8 +341,8 @@ int launch_rmsnorm(const void* x, const void* a, const void* w, void* h_out, voi
   const unsigned grid = (unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta);
   const int nv = (E / N + 31) / 32;
 #define MVPA_RMS(NV)                                                                                             \
-  rmsnorm_kernel<T, NV><<<grid, kWarpsPerCta * 32, 0, s>>>((const T*)x, (const T*)a, (const T*)w, (T*)h_out, (T*)y, \
-                                                            rows, E, eps)
+  MVPA_CUDA_CHECK(launch_dependent(1, rmsnorm_kernel<T, NV>, grid, kWarpsPerCta * 32, 0, s, (const T*)x, (const T*)a, (const T*)w, \
+                                   (T*)h_out, (T*)y, rows, E, eps))
   if (nv <= 2) MVPA_RMS(2);
   else if (nv <= 4) MVPA_RMS(4);
   else if (nv <= 8) MVPA_RMS(8);
@@ -383,8 +386,8 @@ template <typename T>
 int launch_silu_mul(const void* gate, const void* up, int64_t ld_in, void* out, int64_t ld_out, int64_t rows, int width,
                     cudaStream_t s) {
   const int64_t ctas = (rows * (width / Vec<T>::N) + 255) / 256, most = (int64_t)device_sm_count() * 16;
-  silu_mul_kernel<T><<<(unsigned)(ctas < most ? ctas : most), 256, 0, s>>>((const T*)gate, (const T*)up, ld_in, (T*)out, ld_out,
-                                                                           rows, width);
+  MVPA_CUDA_CHECK(launch_dependent(1, silu_mul_kernel<T>, (unsigned)(ctas < most ? ctas : most), 256, 0, s, (const T*)gate, (const T*)up,
+                                   ld_in, (T*)out, ld_out, rows, width));
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;

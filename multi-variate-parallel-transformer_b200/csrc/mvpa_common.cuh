@@ -46,6 +46,27 @@ struct BwdArgs {
   float* tc_extra;     // workspace of the tensor-core query-side kernel (bf16 problems it supports)
 };
 
+// A launch whose CTAs may come up while the kernel before it in the stream runs out: the kernel starts with griddep_wait()
+// (tc_ptx.cuh), before it touches memory that an earlier kernel may have written.  Saves part of the gap between two
+// dependent kernels.  `cluster_z`: CTAs of a cluster along the grid's z.
+template <typename... P>
+inline cudaError_t launch_dependent(unsigned cluster_z, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, P... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = cluster_z;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster_z > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 void set_error(const char* fmt, ...);
 void count_launch(int n = 1);
 

@@ -14,11 +14,11 @@ namespace mvpa {
 // One thread per column: its key row comes in with 16-byte loads that are all in flight at once (D is 64
 // or 128 on the tensor-core paths: 8 or 16 loads), so the kernel costs one memory round trip, not D / 2.
 template <int D>
-static __device__ __forceinline__ void rel_const_row(const __nv_bfloat16* __restrict__ vt, const __nv_bfloat16* __restrict__ z,
-                                                      const __nv_bfloat16* __restrict__ rt, const __nv_bfloat16* __restrict__ rc,
-                                                      float* __restrict__ relc, int T, int C, int hk) {
-  const int j = threadIdx.x & 127;  // 256 threads
-  const bool is_t = threadIdx.x < 128;
+static __device__ __forceinline__ float rel_const(const __nv_bfloat16* __restrict__ vt, const __nv_bfloat16* __restrict__ z,
+                                                   const __nv_bfloat16* __restrict__ rt, const __nv_bfloat16* __restrict__ rc,
+                                                   int T, int C, int hk, int column) {
+  const int j = column & 127;
+  const bool is_t = column < 128;
   const int rows = is_t ? T : C;
   float acc = 0.f;
   if (j < rows) {
@@ -41,7 +41,13 @@ static __device__ __forceinline__ void rel_const_row(const __nv_bfloat16* __rest
       }
     }
   }
-  relc[hk * 256 + threadIdx.x] = acc;
+  return acc;
+}
+template <int D>
+static __device__ __forceinline__ void rel_const_row(const __nv_bfloat16* __restrict__ vt, const __nv_bfloat16* __restrict__ z,
+                                                      const __nv_bfloat16* __restrict__ rt, const __nv_bfloat16* __restrict__ rc,
+                                                      float* __restrict__ relc, int T, int C, int hk) {  // 256 threads
+  relc[hk * 256 + threadIdx.x] = rel_const<D>(vt, z, rt, rc, T, C, hk, threadIdx.x);
 }
 
 template <int D>
