@@ -19,7 +19,10 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <cooperative_groups.h>
+
 #include "mvpa_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace mvpa {
 namespace {
@@ -264,6 +267,7 @@ constexpr size_t fwd_fixed_floats() {
 template <typename Tin, int D, int WPG, int NG, int KN>
 __global__ void __launch_bounds__(32 * WPG * NG, resident_ctas(fwd_fixed_floats<D, WPG, NG, KN>(), 8 * WPG * 64))
 simt_fwd_kernel(Args p) {
+  ptx::griddep_wait();
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;  // threads of a group, of the CTA
   static_assert(NG * KN >= 2 * BM, "the V buffers hold two copies of the rows during the prologue");
@@ -460,6 +464,7 @@ constexpr size_t dq_fixed_floats() {
 template <typename Tin, int D, int WPG, int NG, int KN, bool INS>
 __global__ void __launch_bounds__(32 * WPG * NG, resident_ctas(dq_fixed_floats<D, WPG, NG, KN>(), 8 * WPG * (NG + INS) * 64))
 simt_dq_kernel(BwdArgs bw) {
+  ptx::griddep_wait();
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;
   static_assert(NG * KN >= 2 * BM && KN >= BM, "aliased areas");
@@ -748,6 +753,7 @@ constexpr size_t dkv_fixed_floats() {
 // a thread spill: 387 against 232 us)
 template <typename Tin, int D, int WPG, int NG, int KN>
 __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kernel(BwdArgs bw) {
+  ptx::griddep_wait();
   constexpr int LD = D + 4, KJ = KN / 16, BM = 8 * WPG, LP = KN + 4, VW = D / 16;
   constexpr int GT = 32 * WPG, CT = GT * NG;
   static_assert(KN >= BM, "aliased areas");
@@ -787,6 +793,8 @@ __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kerne
   const int tk_last = (n0 + valid - 1) / C;
   const int tile0 = ((n0 / C) * C) / KN, per_head = (N + KN - 1) / KN - tile0;  // first query tile that sees these keys
   const int items = p.g * per_head;
+  // The CTAs of a cluster (gridDim.z of them own the same keys) and their groups take the items in turn.
+  const int part = blockIdx.z, parts = gridDim.z, first = part * NG + g, stride = parts * NG;
   // every pair outside the content window: neither S nor dS_w is needed, only P
   auto light = [&](int m0) {
     const int t_hi = (min(N, m0 + KN) - 1) / C;
@@ -813,11 +821,11 @@ __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kerne
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int e = 0; e < VW; ++e) kacc[a][e] = vacc[a][e] = 0.f;
-  fetch_q(g);
-  fetch_g(g);
+  fetch_q(first);
+  fetch_g(first);
   cp_async_wait<2>();
   __syncthreads();  // K and V are in place
-  for (int item = g; item < items; item += NG) {
+  for (int item = first; item < items; item += stride) {
     const int h = hk * p.g + item / per_head, bh = b * p.H + h, m0 = (tile0 + item % per_head) * KN;
     const bool lt = light(m0);
     const float* tbg = bw.tbg + (int64_t)bh * N * T;
@@ -881,10 +889,10 @@ __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kerne
     __syncwarp();
     if (!lt) product_nn<D, KN>(Dw, Qs, tx, kacc);  // dK += dS_w^T (q + u) c2  (`attentions/attn.py:718`)
     group_sync<WPG>(g);                            // every warp has left Q, lse and delta
-    fetch_q(item + NG);
+    fetch_q(item + stride);
     product_nn<D, KN>(Ps, Gs, tx, vacc);           // dV += P^T dO        (`attentions/attn.py:671-675`)
     group_sync<WPG>(g);                            // every warp has left dO
-    fetch_g(item + NG);
+    fetch_g(item + stride);
   }
   __syncthreads();
   float *Km = Qall, *Vm = Gall;  // [NG][BM][LD] each
@@ -897,23 +905,32 @@ __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kerne
   Tin* dk = (Tin*)bw.dk + b * bw.dk_sb + hk * bw.dk_sh;
   Tin* dv = (Tin*)bw.dv + b * bw.dv_sb + hk * bw.dv_sh;
   const float inv_c2 = 1.f / p.c2;
-  for (int idx = tid; idx < 2 * BM * D / 4; idx += CT) {
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  if (parts > 1) cluster.sync();  // every CTA's sums are in its shared memory
+  for (int idx = part * CT + tid; idx < 2 * BM * D / 4; idx += parts * CT) {
     const bool is_k = idx < BM * D / 4;
     const int rem = is_k ? idx : idx - BM * D / 4;
     const int r = rem / (D / 4), d = (rem % (D / 4)) * 4;
     if (r >= valid) continue;
-    const float* src = (is_k ? Km : Vm) + r * LD + d;
-    float4 x = *reinterpret_cast<const float4*>(src);
+    float* own = (is_k ? Km : Vm) + r * LD + d;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < parts; ++q) {
+      const float* src = parts > 1 ? cluster.map_shared_rank(own, q) : own;
+      float4 z = *reinterpret_cast<const float4*>(src);
 #pragma unroll
-    for (int gg = 1; gg < NG; ++gg) {
-      const float4 y = *reinterpret_cast<const float4*>(src + gg * BM * LD);
-      x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+      for (int gg = 1; gg < NG; ++gg) {
+        const float4 y = *reinterpret_cast<const float4*>(src + gg * BM * LD);
+        z.x += y.x; z.y += y.y; z.z += y.z; z.w += y.w;
+      }
+      if (q == 0) x = z;
+      else { x.x += z.x; x.y += z.y; x.z += z.z; x.w += z.w; }
     }
     if (is_k)
       store4<Tin>(dk + (int64_t)(n0 + r) * bw.dk_sn + d, make_float4(x.x * inv_c2, x.y * inv_c2, x.z * inv_c2, x.w * inv_c2));
     else
       store4<Tin>(dv + (int64_t)(n0 + r) * bw.dv_sn + d, x);
   }
+  if (parts > 1) cluster.sync();  // nobody leaves while its sums are still being read
 }
 
 // dr[hk][slot][d] = sum_{b, h in group, i} dX[b,h,i,slot] * (q[b,h,i,d] + bias[hk][d]), for the T time slots and
@@ -922,6 +939,7 @@ __global__ void __launch_bounds__(32 * WPG * NG, D == 16 ? 2 : 1) simt_dkv_kerne
 constexpr int kDrelRows = 64, kDrelSlots = 32;
 template <typename Tin, int D>
 __global__ void __launch_bounds__(kThreads) simt_drel_kernel(BwdArgs bw) {
+  ptx::griddep_wait();
   constexpr int LD = D + 4, VW = D / 16, LX = kDrelSlots + 1;
   const Args& p = bw.a;
   extern __shared__ __align__(16) float smem[];
@@ -986,6 +1004,7 @@ __global__ void __launch_bounds__(kThreads) simt_drel_kernel(BwdArgs bw) {
 // simt_drel_kernel (the first n_red blocks), du / dvt / dz from the per-tile partials of simt_dq_kernel (three
 // blocks per kv head).
 __global__ void __launch_bounds__(kThreads) simt_final_kernel(BwdArgs bw, int n_z, int n_qt, int n_red) {
+  ptx::griddep_wait();
   const Args& p = bw.a;
   const int S = p.T + p.C, D = p.D;
   if ((int)blockIdx.x < n_red) {
@@ -1051,7 +1070,8 @@ int run_fwd(const Args& a, cudaStream_t s) {
   const size_t smem = sizeof(float) * (fwd_fixed_floats<D, WPG, NG, KN>() + (size_t)BM * (a.T + a.C));
   int rc = set_smem(simt_fwd_kernel<Tin, D, WPG, NG, KN>, smem);
   if (rc) return rc;
-  simt_fwd_kernel<Tin, D, WPG, NG, KN><<<dim3((a.q_tn * a.C + BM - 1) / BM, a.B * a.H), 32 * WPG * NG, smem, s>>>(a);
+  MVPA_CUDA_CHECK(launch_dependent(1, simt_fwd_kernel<Tin, D, WPG, NG, KN>, dim3((a.q_tn * a.C + BM - 1) / BM, a.B * a.H), 32 * WPG * NG,
+                                   smem, s, a));
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
@@ -1082,7 +1102,8 @@ int run_dq(const BwdArgs& b, size_t smem_floats, cudaStream_t s) {
   constexpr int BM = 8 * WPG;
   int rc = set_smem(simt_dq_kernel<Tin, D, WPG, NG, KN, INS>, smem_floats * sizeof(float));
   if (rc) return rc;
-  simt_dq_kernel<Tin, D, WPG, NG, KN, INS><<<dim3((b.a.N + BM - 1) / BM, b.a.B * b.a.H), 32 * WPG * NG, smem_floats * sizeof(float), s>>>(b);
+  MVPA_CUDA_CHECK(launch_dependent(1, simt_dq_kernel<Tin, D, WPG, NG, KN, INS>, dim3((b.a.N + BM - 1) / BM, b.a.B * b.a.H),
+                                   32 * WPG * NG, smem_floats * sizeof(float), s, b));
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
@@ -1095,7 +1116,14 @@ int run_dkv(const BwdArgs& b, cudaStream_t s) {
   static_assert(smem <= 232448, "shared memory budget");
   int rc = set_smem(simt_dkv_kernel<Tin, D, WPG, NG, KN>, smem);
   if (rc) return rc;
-  simt_dkv_kernel<Tin, D, WPG, NG, KN><<<dim3((b.a.N + BM - 1) / BM, b.a.B * b.a.Hkv), 32 * WPG * NG, smem, s>>>(b);
+  // Few CTAs whose groups have more than one item each: a cluster of two CTAs shares the (head, query tile) items of the same
+  // keys, and each adds up half of the rows out of the other's shared memory.  us at head_dim 64, alone / in pairs: 66 CTAs
+  // (B 1 H 4 Hkv 2 T 24 C 22) 50.5 / 35.7, 96 CTAs 44.2 / 35.2, 132 CTAs 51.1 / 58.2 (more than one round of CTAs); clusters of four
+  // at 66 CTAs 39.8; one item a group (12 x 8 tokens) 9.8 / 11.7.
+  const unsigned tiles = (unsigned)((b.a.N + BM - 1) / BM), heads = (unsigned)(b.a.B * b.a.Hkv);
+  const bool shared_items = b.a.g * ((b.a.N + KN - 1) / KN) > NG && 3 * (int64_t)tiles * heads <= 2 * (int64_t)device_sm_count();
+  const unsigned parts = shared_items ? 2 : 1;
+  MVPA_CUDA_CHECK(launch_dependent(parts, simt_dkv_kernel<Tin, D, WPG, NG, KN>, dim3(tiles, heads, parts), 32 * WPG * NG, smem, s, b));
   count_launch();
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;
@@ -1142,11 +1170,11 @@ int launch_bwd(const BwdArgs& b, cudaStream_t s) {
     rc = set_smem(simt_drel_kernel<Tin, D>, smem);
     if (rc) return rc;
     const unsigned blocks = (a.T + kDrelSlots - 1) / kDrelSlots + (a.C + kDrelSlots - 1) / kDrelSlots;
-    simt_drel_kernel<Tin, D><<<dim3(blocks, a.Hkv, n_z), kThreads, smem, s>>>(b);
+    MVPA_CUDA_CHECK(launch_dependent(1, simt_drel_kernel<Tin, D>, dim3(blocks, a.Hkv, n_z), kThreads, smem, s, b));
   }
   const int64_t total = (int64_t)a.Hkv * (a.T + a.C) * D;
   const int n_red = (int)((total + kThreads - 1) / kThreads < 592 ? (total + kThreads - 1) / kThreads : 592);
-  simt_final_kernel<<<n_red + 3 * a.Hkv, kThreads, 0, s>>>(b, n_z, n_qt, n_red);
+  MVPA_CUDA_CHECK(launch_dependent(1, simt_final_kernel, n_red + 3 * a.Hkv, kThreads, 0, s, b, n_z, n_qt, n_red));
   count_launch(2);
   MVPA_CUDA_CHECK(cudaGetLastError());
   return MVPA_OK;

@@ -45,6 +45,14 @@ def test_cuda_core_tiles_thirty_two_rows(cuda, shape):
     _check(cuda, random_case(sum(shape), *shape), torch.float32)
 
 
+# key side in clusters of two CTAs: an odd number of items, the last of a ragged tile, one item more than a CTA's groups, light
+# items, two heads a group, and each head_dim
+@pytest.mark.parametrize("shape", [(1, 2, 1, 9, 17, 16), (1, 5, 1, 5, 12, 32), (1, 4, 2, 24, 11, 64), (1, 1, 1, 45, 11, 64), (2, 2, 1, 13, 17, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_cuda_core_key_side_in_pairs(cuda, shape, dtype):
+    _check(cuda, random_case(sum(shape), *shape), dtype)
+
+
 # time / channel axes whose slot sums do not fit beside the four groups' tiles
 @pytest.mark.parametrize("shape", [(1, 1, 1, 2, 400, 64), (1, 1, 1, 300, 2, 128), (1, 2, 1, 2, 440, 32)])
 def test_cuda_core_long_axes(cuda, shape):
