@@ -314,12 +314,12 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         const DescHalves dq = make_desc_halves_sw128(smem_u32(sQ), 16, 1024);
         const DescHalves dr = make_desc_halves_sw128(smem_u32(sR), 16, 1024);
         const DescHalves dc = make_desc_halves_sw128(smem_u32(sC), 16, 1024);
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {  // raw temporal products, all 128 columns at once
           const uint32_t off = (kk / 4) * HALF + (kk % 4) * 32;
           mma_ss_w(el, tm + kColTB, dq, off, dr, off, idesc_s, kk > 0);
         }
-#pragma unroll
+#pragma unroll 1
         for (int kk = 0; kk < KSTEPS; ++kk) {  // raw channel products -> S0 columns [0, CP)
           const uint32_t offa = (kk / 4) * HALF + (kk % 4) * 32;
           const uint32_t offb = (kk / 4) * (CP * 128) + (kk % 4) * 32;
@@ -430,7 +430,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     const int ck_base = CP == 128 ? 64 * wg : 0;  // first channel slot of this thread's columns
     for (int d = tid; d < D; d += kSoftmaxThreads) s_bias[d] = __bfloat162float(p.u[hk * D + d]);
     // (s_vr and s_zc are adjacent: 256 floats)
-    s_vr[tid] = p.relc != nullptr ? p.relc[hk * 256 + tid] : rel_const<D>(p.vt, p.z, p.rt, p.rc, T, C, hk, tid);
+    s_vr[tid] = p.relc != nullptr ? p.relc[hk * 256 + tid] : rel_const<D, 8>(p.vt, p.z, p.rt, p.rc, T, C, hk, tid);
     softmax_bar();
     bool ok = warp_wait(&bars[kBarProFull], 0, p.status, 30);
     if (ok) ok = warp_wait(&bars[kBarProMma], 0, p.status, 31);
@@ -541,14 +541,14 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       const float alpha = need ? ex2(m_used - m_tile) : 1.f;
       // (split accumulators: all D columns of this warpgroup's own O; otherwise its half of the one O)
       constexpr int own0 = SPLIT ? 64 : DW, own_n = SPLIT ? D : DW;
-#pragma unroll
-      for (int c0 = 0; c0 < own_n; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld32(lane_base + kColO + wg * own0 + c0, v);
+#pragma unroll 1
+      for (int c0 = 0; c0 < own_n; c0 += 8) {
+        uint32_t v[8];
+        tmem_ld8(lane_base + kColO + wg * own0 + c0, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-        tmem_st32(lane_base + kColO + wg * own0 + c0, v);
+        for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
+        tmem_st8(lane_base + kColO + wg * own0 + c0, v);
       }
       tmem_st_wait();
       l_sum *= alpha;
@@ -598,15 +598,14 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     if (ok && n_light > 0) {
       const int col1 = col0 + n_light * TPB;
       float m_light = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (32 * c + 32 <= col0 || 32 * c >= col1) continue;  // (warp-uniform)
-        uint32_t v[32];
-        tmem_ld32(lane_base + kColTB + 32 * c, v);
+#pragma unroll 1
+      for (int c = col0 & ~15; c < col1; c += 16) {  // (warp-uniform; a short loop, as everything that runs once per CTA)
+        uint32_t v[16];
+        tmem_ld16(lane_base + kColTB + c, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int col = 32 * c + jj;
+        for (int jj = 0; jj < 16; ++jj) {
+          const int col = c + jj;
           const float tb = p.c2 * (__uint_as_float(v[jj]) + s_vr[col]) + mc;
           if (col >= col0 && col < col1) m_light = fmaxf(m_light, tb);
         }
@@ -616,14 +615,14 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         m_used = m_light;  // (nothing has been summed yet)
       } else if (__any_sync(0xffffffffu, need)) {
         const float alpha = need ? ex2(m_used - m_light) : 1.f;
-#pragma unroll
-        for (int c0 = 0; c0 < DW; c0 += 32) {
-          uint32_t v[32];
-          tmem_ld32(lane_base + kColO + wg * DW + c0, v);
+#pragma unroll 1
+        for (int c0 = 0; c0 < DW; c0 += 8) {
+          uint32_t v[8];
+          tmem_ld8(lane_base + kColO + wg * DW + c0, v);
           tmem_ld_wait();
 #pragma unroll
-          for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-          tmem_st32(lane_base + kColO + wg * DW + c0, v);
+          for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
+          tmem_st8(lane_base + kColO + wg * DW + c0, v);
         }
         tmem_st_wait();
         l_sum *= alpha;
@@ -983,7 +982,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       const int64_t n = (int64_t)(ti_abs - p.q_t0) * C + c_i;  // row inside this call's q / o / lse
       // O / l as bf16 into the Q tile's place (laid out like it: 128-byte swizzled rows), then one TMA
       // store per 64-column half; rows and channels outside the tensor are not written.
-#pragma unroll
+#pragma unroll 1
       for (int c0 = 0; c0 < DW; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(lane_base + kColO + wg * DW + c0, v);

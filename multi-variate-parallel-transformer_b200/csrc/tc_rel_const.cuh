@@ -13,7 +13,8 @@ namespace mvpa {
 // (the bias halves of `_rel_bias`, `attentions/attn.py:1308-1313`).
 // One thread per column: its key row comes in with 16-byte loads that are all in flight at once (D is 64
 // or 128 on the tensor-core paths: 8 or 16 loads), so the kernel costs one memory round trip, not D / 2.
-template <int D>
+// (`FLIGHT` of the row's 16-byte loads in flight at once; a kernel that is much else beside takes a few, for its size)
+template <int D, int FLIGHT = D / 8>
 static __device__ __forceinline__ float rel_const(const __nv_bfloat16* __restrict__ vt, const __nv_bfloat16* __restrict__ z,
                                                    const __nv_bfloat16* __restrict__ rt, const __nv_bfloat16* __restrict__ rc,
                                                    int T, int C, int hk, int column) {
@@ -24,20 +25,23 @@ static __device__ __forceinline__ float rel_const(const __nv_bfloat16* __restric
   if (j < rows) {
     const uint4* key = reinterpret_cast<const uint4*>((is_t ? rt : rc) + ((size_t)hk * rows + j) * D);
     const uint4* bias = reinterpret_cast<const uint4*>((is_t ? vt : z) + (size_t)hk * D);
-    uint4 k[D / 8], b[D / 8];
+#pragma unroll 1
+    for (int i0 = 0; i0 < D / 8; i0 += FLIGHT) {
+      uint4 k[FLIGHT], b[FLIGHT];
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      k[i] = key[i];
-      b[i] = bias[i];
-    }
+      for (int i = 0; i < FLIGHT; ++i) {
+        k[i] = key[i0 + i];
+        b[i] = bias[i0 + i];
+      }
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      const uint32_t kw[4] = {k[i].x, k[i].y, k[i].z, k[i].w}, bw[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+      for (int i = 0; i < FLIGHT; ++i) {
+        const uint32_t kw[4] = {k[i].x, k[i].y, k[i].z, k[i].w}, bw[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {  // the same pairs in the same order as a two-element walk over d
-        const float ax = __uint_as_float(kw[e] << 16), ay = __uint_as_float(kw[e] & 0xffff0000u);
-        const float bx = __uint_as_float(bw[e] << 16), by = __uint_as_float(bw[e] & 0xffff0000u);
-        acc += ax * bx + ay * by;
+        for (int e = 0; e < 4; ++e) {  // the same pairs in the same order as a two-element walk over d
+          const float ax = __uint_as_float(kw[e] << 16), ay = __uint_as_float(kw[e] & 0xffff0000u);
+          const float bx = __uint_as_float(bw[e] << 16), by = __uint_as_float(bw[e] & 0xffff0000u);
+          acc += ax * bx + ay * by;
+        }
       }
     }
   }
