@@ -51,7 +51,7 @@ WORKLOADS = {
 WORKLOAD, NAME = WORKLOADS["cfg2"]
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the forward kernel, from the ncu
 # captures summarised under profiles/ (bytes)
-NCU_DRAM_BYTES = {"cfg2": 137.2e6, "16k": 208.2e6}
+NCU_DRAM_BYTES = {"cfg2": 138.3e6, "16k": 208.2e6}
 METRIC = "flash_mvpa_fwd_tflops"
 UNIT = "TFLOP/s (F_alg)"
 
@@ -891,7 +891,7 @@ def main():
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": None if train else NCU_DRAM_BYTES.get(args.workload), "peak_source": peak_src,
                          "kernel": ("whole step (tc_fwd_kernel, tc_bwd_q_kernel, tc_bwd_kv_kernel, simt_drel_kernel)"
-                                    if train else "tc_fwd_kernel<%d,%d>" %
+                                    if train else ("two CTAs per multiprocessor: tc_fwd_two_kernel, D %d, %d channel slots" if w["D"] == 64 and w["C"] <= 64 else "tc_fwd_kernel<%d,%d>") %
                                     (w["D"], 32 if w["C"] <= 32 else 64 if w["C"] <= 64 else 128)),
                          "flops_per_launch": f["f_alg"],
                          "achieved_dense_convention": f["f_dense"] / (kernel_ms * 1e-3) / 1e12},
