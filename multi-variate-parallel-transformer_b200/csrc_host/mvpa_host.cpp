@@ -310,6 +310,16 @@ Dims block_dims(const Tensor& x, PyObject* const* heads) {
   return d;
 }
 
+// What the body of a block's call runs under.  No autocast: a backward may run inside a region that the forward was outside of, and
+// the kernels read every product as the type that the forward had.
+struct Body {
+  pybind11::gil_scoped_release nogil;
+  c10::cuda::CUDAGuard guard;
+  c10::NoGradGuard no_grad;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::autocast_dispatch_keyset};
+  explicit Body(const Tensor& t) : guard(t.device()) {}
+};
+
 const char* part(const Tensor& t, int64_t elements) { return static_cast<const char*>(t.const_data_ptr()) + elements * t.element_size(); }
 
 // block_forward(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, eps, window, H, Hkv, D, status)
@@ -333,9 +343,7 @@ PyObject* block_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Dims d = block_dims(x, a + 15);
   Tensor h, xn, q, kv, g, up, rt, rc, o, lse, act;
   {
-    pybind11::gil_scoped_release nogil;
-    c10::cuda::CUDAGuard guard(x.device());
-    c10::NoGradGuard no_grad;
+    const Body body(x);
     const int dt = dtype_code(x);
     const Tensor x2 = x.view({d.rows, d.E});
     xn = at::empty_like(x2);
@@ -389,9 +397,7 @@ PyObject* block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Dims d = block_dims(x, a + 27);
   std::vector<Tensor> grad(13);
   {
-    pybind11::gil_scoped_release nogil;
-    c10::cuda::CUDAGuard guard(x.device());
-    c10::NoGradGuard no_grad;
+    const Body body(x);
     const int dt = dtype_code(x);
     const auto needs = [&](int i) { return (need >> i & 1) != 0; };
     const auto weight = [&](int i, const Tensor& dy, const Tensor& y) {  // d W = d^T input

@@ -71,8 +71,9 @@ class BlockFunction(torch.autograd.Function):
             grads = _host.module().block_backward(dh, *saved, mask, ctx.eps, WINDOW, *ctx.heads, _attn._CHECK_STATUS)
             if grads is not None:
                 return (*grads, None, None)
-        # a graph of the gradient is wanted (or a transform is active): through the differentiable operations
-        grads = through_expression(lambda *ins: expression(*ins, ctx.eps, ctx.heads), saved[:13], need, dh)
+        # a graph of the gradient is wanted (or a transform is active): through the differentiable operations, in the forward's types
+        with torch.autocast("cuda", enabled=False):
+            grads = through_expression(lambda *ins: expression(*ins, ctx.eps, ctx.heads), saved[:13], need, dh)
         return (*grads, None, None)
 
 
