@@ -292,7 +292,7 @@ PyObject* plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 struct Dims {
-  int64_t B, T, C, E, H, Hkv, D, N, KV, rows;
+  int64_t B, T, C, E, H, Hkv, D, I, N, KV, rows;
   mvpa_problem problem(int dtype, double scale, int window) const {
     mvpa_problem p = {};
     p.B = (int32_t)B; p.H = (int32_t)H; p.Hkv = (int32_t)Hkv; p.T = (int32_t)T; p.C = (int32_t)C; p.D = (int32_t)D;
@@ -301,13 +301,28 @@ struct Dims {
   }
 };
 
-Dims block_dims(const Tensor& x, PyObject* const* heads) {
-  Dims d;
-  d.B = x.size(0); d.T = x.size(1); d.C = x.size(2); d.E = x.size(3);
+// What the kernels read of a block through pointers: one type and device, contiguous, 16-byte aligned, of the given sizes.
+bool fits(const Tensor& t, const Tensor& like, at::ScalarType type, at::IntArrayRef sizes) {
+  return ordinary(t) && t.scalar_type() == type && t.device() == like.device() && t.is_contiguous() && t.sizes() == sizes &&
+         aligned16(t.const_data_ptr());
+}
+
+// The sizes of a block's call; false where an input (x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd) is not of them.
+bool block_dims(const Tensor* in, PyObject* const* heads, Dims& d) {
+  const Tensor &x = in[0], &bias = in[8], &wg = in[10];
   d.H = PyLong_AsLongLong(heads[0]); d.Hkv = PyLong_AsLongLong(heads[1]); d.D = PyLong_AsLongLong(heads[2]);
   if (PyErr_Occurred()) throw python_error();
+  if (!ordinary(x) || x.dim() != 4 || x.numel() == 0 || dtype_code(x) < 0 || !ordinary(wg) || wg.dim() != 2 || !ordinary(bias) ||
+      d.H <= 0 || d.Hkv <= 0 || d.D <= 0)
+    return false;
+  d.B = x.size(0); d.T = x.size(1); d.C = x.size(2); d.E = x.size(3); d.I = wg.size(0);
   d.N = d.T * d.C; d.KV = d.Hkv * d.D; d.rows = d.B * d.N;
-  return d;
+  const int64_t Q = d.H * d.D;
+  const std::vector<int64_t> sizes[13] = {x.sizes().vec(), {1, d.T, d.E}, {1, d.C, d.E}, {d.E}, {Q, d.E}, {2 * d.KV, d.E}, {d.KV, d.E},
+                                          {d.KV, d.E}, bias.sizes().vec(), {d.E, Q}, {d.I, d.E}, {d.I, d.E}, {d.E, d.I}};
+  for (int i = 0; i < 13; ++i)
+    if (!fits(in[i], x, x.scalar_type(), sizes[i])) return false;
+  return bias.numel() == 3 * d.KV && d.I > 0 && d.I * x.element_size() % 16 == 0;
 }
 
 // What the body of a block's call runs under.  No autocast: a backward may run inside a region that the forward was outside of, and
@@ -323,7 +338,7 @@ struct Body {
 const char* part(const Tensor& t, int64_t elements) { return static_cast<const char*>(t.const_data_ptr()) + elements * t.element_size(); }
 
 // block_forward(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, eps, window, H, Hkv, D, status)
-//   -> (h, xn, q, kv, g, up, rt, rc, o, lse, act): `block_grad.BlockFunction.forward` on tensors that `applies` has looked at
+//   -> (h, xn, q, kv, g, up, rt, rc, o, lse, act): `block_grad.BlockFunction.forward`, or None
 PyObject* block_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arguments(n, 19)) return nullptr;
@@ -332,15 +347,14 @@ PyObject* block_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 0; i < 13; ++i) {
     if (!THPVariable_CheckExact(a[i])) Py_RETURN_NONE;
     in[i] = THPVariable_Unpack(a[i]);
-    if (!ordinary(in[i]) || !in[i].is_contiguous()) Py_RETURN_NONE;
   }
-  if (watched()) Py_RETURN_NONE;
+  Dims d;
+  if (watched() || !block_dims(in, a + 15, d)) Py_RETURN_NONE;
   const Tensor &x = in[0], &pos = in[1], &chan = in[2], &ln_w = in[3], &wq = in[4], &wkv = in[5], &wpos = in[6], &wchan = in[7],
                &bias = in[8], &wc = in[9], &wg = in[10], &wu = in[11], &wd = in[12];
   const double eps = PyFloat_AsDouble(a[13]);
   const int64_t window = PyLong_AsLongLong(a[14]);
   if (PyErr_Occurred()) return nullptr;
-  const Dims d = block_dims(x, a + 15);
   Tensor h, xn, q, kv, g, up, rt, rc, o, lse, act;
   {
     const Body body(x);
@@ -385,16 +399,22 @@ PyObject* block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 0; i < 24; ++i) {
     if (!THPVariable_CheckExact(a[i])) Py_RETURN_NONE;
     in[i] = THPVariable_Unpack(a[i]);
-    if (!ordinary(in[i])) Py_RETURN_NONE;
   }
-  if (watched()) Py_RETURN_NONE;
+  Dims d;
+  if (watched() || !block_dims(in + 1, a + 27, d) || !ordinary(in[0]) || in[0].device() != in[1].device() ||
+      in[0].scalar_type() != in[1].scalar_type() || in[0].sizes() != in[1].sizes())
+    Py_RETURN_NONE;
+  // (a saved-tensor hook may have brought anything back)
+  const std::vector<int64_t> saved[10] = {{d.rows, d.E}, {d.rows, d.H * d.D}, {d.rows, 2 * d.KV}, {d.rows, d.I}, {d.rows, d.I},
+                                          {d.Hkv, d.T, d.D}, {d.Hkv, d.C, d.D}, {d.rows, d.H * d.D}, {d.B * d.H, d.N}, {d.rows, d.I}};
+  for (int i = 0; i < 10; ++i)
+    if (!fits(in[14 + i], in[1], i == 8 ? at::kFloat : in[1].scalar_type(), saved[i])) Py_RETURN_NONE;
   const Tensor &x = in[1], &pos = in[2], &chan = in[3], &ln_w = in[4], &wq = in[5], &wkv = in[6], &wpos = in[7], &wchan = in[8],
                &bias = in[9], &wc = in[10], &wg = in[11], &wu = in[12], &wd = in[13], &xn = in[14], &q = in[15], &kv = in[16],
                &g = in[17], &up = in[18], &rt = in[19], &rc = in[20], &o = in[21], &lse = in[22], &act = in[23];
   const int64_t need = PyLong_AsLongLong(a[24]), window = PyLong_AsLongLong(a[26]);
   const double eps = PyFloat_AsDouble(a[25]);
   if (PyErr_Occurred()) return nullptr;
-  const Dims d = block_dims(x, a + 27);
   std::vector<Tensor> grad(13);
   {
     const Body body(x);

@@ -32,10 +32,10 @@ def expression(x, pos, chan, ln_w, wq, wkv, wpos, wchan, bias, wc, wg, wu, wd, e
     k, v = (t.permute(0, 2, 1, 3) for t in F.linear(xn, wkv).view(B, N, 2 * Hkv, D).split(Hkv, dim=2))
     rt = F.linear(pos, wpos).view(1, T, Hkv, D).permute(0, 2, 1, 3)
     rc = F.linear(chan, wchan).view(1, C, Hkv, D).permute(0, 2, 1, 3)
-    u, vt, z = (b.view(1, Hkv, 1, D) for b in bias.split(KV))
+    u, vt, z = (b.view(1, Hkv, 1, D) for b in bias.clone().split(KV))    # (what a saved-tensor hook brought back may lie anywhere)
     o = flashmvpa(q, u, vt, z, k, rt, rc, v, causal=True, sm_scale=1.0 / (D ** 0.5), window_size=WINDOW)
     mlp = F.linear(mvpa_ops.swiglu(F.linear(xn, wg), F.linear(xn, wu)), wd)
-    return x + mlp + F.linear(o.permute(0, 2, 1, 3).reshape(B, T, C, E), wc)
+    return x + mlp + F.linear(o.permute(0, 2, 1, 3).reshape(B, T, C, H * D), wc)
 
 
 def through_expression(f, ins, need, grad_out):
@@ -95,7 +95,8 @@ def _unhooked(m, code):
 def applies(block, x, pos, chan, classes) -> bool:
     """Whether `block` is exactly the computation above on tensors the kernels take in place: the shipped modules (norm,
     attention and MLP in `classes`, as `shipped` returned them), neither they nor their code replaced, hooked or patched,
-    no dropout or autocast, one dtype, contiguous and 16-byte aligned, and nothing tracing the call.  Everything else goes
+    no dropout or autocast, weights of the sizes that go together, one dtype, contiguous and 16-byte aligned, and nothing
+    tracing the call.  Everything else goes
     through the modules."""
     norm, attn, mlp = classes
     a, m = block.attn, block.mlp
@@ -115,10 +116,15 @@ def applies(block, x, pos, chan, classes) -> bool:
         return False                 # (what the operator refuses is refused by the operator)
     if x.dim() != 4 or pos.shape != (1, x.shape[1], x.shape[3]) or chan.shape != (1, x.shape[2], x.shape[3]):
         return False
-    ts = (x, pos, chan, block.ln_1.weight, a.attn_bias, *(l.weight for l in linears))
-    es = x.element_size()
-    return (mvpa_ops._plain(*ts) and mvpa_ops._rows_fit(x) and m.gate_proj.out_features * es % 16 == 0
-            and block.ln_1.weight.shape == x.shape[-1:] and any(t.requires_grad for t in ts))
+    # (weights of other sizes than the module was made with: a pruned head, a replaced projection)
+    weights = [l.weight for l in linears]
+    E, Q, KV, I = x.shape[3], a.num_heads * a.head_dim, a.num_kv_heads * a.head_dim, weights[5].shape[0]
+    if ([w.shape for w in weights] != [(Q, E), (2 * KV, E), (KV, E), (KV, E), (E, Q), (I, E), (I, E), (E, I)]
+            or block.ln_1.weight.shape != (E,) or a.attn_bias.numel() != 3 * KV):
+        return False
+    ts = (x, pos, chan, block.ln_1.weight, a.attn_bias, *weights)
+    return (mvpa_ops._plain(*ts) and mvpa_ops._rows_fit(x) and I * x.element_size() % 16 == 0
+            and any(t.requires_grad for t in ts))
 
 
 def run(block, x, pos, chan):

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import models
+from models import block_grad
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,57 @@ def test_backward_inside_autocast(cuda, dtype, region):
         got_graphed = torch.autograd.grad(y, ins, dy, create_graph=True)
     for a, b, c, d in zip(want, got, graphed, got_graphed):
         assert a.dtype == b.dtype and torch.equal(a, b) and torch.equal(c, d)
+
+
+def _resized(p, dim, by):
+    shape = list(p.shape)
+    shape[dim] += by
+    return torch.nn.Parameter(torch.randn(shape, device=p.device).to(p.dtype))
+
+
+# weights of other sizes than the block was made with, each alone: refused by the modules, and by the native call
+@pytest.mark.parametrize("path, dim, by", [
+    ("attn.q_attn.weight", 0, -32), ("attn.q_attn.weight", 0, 32), ("attn.c_attn.weight", 0, -32), ("attn.c_attn.weight", 0, 32),
+    ("attn.position_net.weight", 0, -32), ("attn.channel_net.weight", 0, 32), ("attn.attn_bias", 0, -64), ("attn.attn_bias", 0, 32),
+    ("attn.c_proj.weight", 1, -32), ("attn.c_proj.weight", 0, -32), ("mlp.gate_proj.weight", 0, 32), ("mlp.up_proj.weight", 0, -32),
+    ("mlp.up_proj.weight", 0, 32), ("mlp.down_proj.weight", 1, -32), ("ln_1.weight", 0, -32)])
+def test_resized_weights_are_refused(cuda, path, dim, by):
+    block, x, pos, chan = _block(cuda)
+    *way, last = path.split(".")
+    owner = block.get_submodule(".".join(way))
+    setattr(owner, last, _resized(getattr(owner, last), dim, by))
+    with pytest.raises((RuntimeError, ValueError, AssertionError)):
+        block(x, pos, chan)
+    with pytest.raises(RuntimeError):
+        block_grad.run(block, x, pos, chan)
+
+
+# heads taken out of every projection that holds them, and of the counts: a smaller block, as before
+def test_pruned_heads(cuda):
+    block, x, pos, chan = _block(cuda)
+    a = block.attn
+    a.num_heads = 2
+    a.q_attn.weight = torch.nn.Parameter(a.q_attn.weight[:64].clone())
+    a.c_proj.weight = torch.nn.Parameter(a.c_proj.weight[:, :64].clone())
+    y = block(x, pos, chan)[0]
+    assert "BlockFunction" in type(y.grad_fn).__name__
+    args = (x, pos, chan, block.ln_1.weight, a.q_attn.weight, a.c_attn.weight, a.position_net.weight, a.channel_net.weight, a.attn_bias,
+            a.c_proj.weight, block.mlp.gate_proj.weight, block.mlp.up_proj.weight, block.mlp.down_proj.weight)
+    want = block_grad.expression(*args, block.ln_1.eps, (2, 2, 32))
+    assert (y - want).norm() <= 1e-5 * want.norm()
+
+
+# what a saved-tensor hook brings back need not lie in memory as the kernels read it
+@pytest.mark.parametrize("form", [lambda t: torch.nn.functional.pad(t, (0, 1))[..., :-1], lambda t: t.clone(),
+                                  lambda t: torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape)])
+def test_backward_of_rearranged_saved_tensors(cuda, form):
+    block, x, pos, chan = _block(cuda)
+    ins = _inputs(block, x, pos, chan)
+    y = block(x, pos, chan)[0]
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, ins, dy)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), form):
+        y = block(x, pos, chan)[0]
+        assert "BlockFunction" in type(y.grad_fn).__name__
+    for a, b in zip(torch.autograd.grad(y, ins, dy), want):
+        assert (a - b).norm() <= 1e-5 * b.norm()
