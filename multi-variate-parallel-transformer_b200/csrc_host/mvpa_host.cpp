@@ -487,7 +487,8 @@ PyObject* branches(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.N = d.T * d.C; d.KV = d.Hkv * d.D; d.rows = d.B * d.N; d.E = d.H * d.D;
   const int dt = dtype_code(x);
   const int64_t I = x.dim() == 2 && w_in.dim() == 2 ? (w_in.size(0) - d.E - 2 * d.KV) / 2 : 0, es = x.element_size();
-  if (I <= 0 || (dt != MVPA_BF16 && dt != MVPA_F32) || x.size(0) != d.rows || x.size(1) != d.E || I * es % 16 != 0 || bias.numel() != 3 * d.KV ||
+  if (I <= 0 || w_in.size(0) != d.E + 2 * (d.KV + I) || w_out.dim() != 2 || w_out.size(1) != d.E + I || d.KV <= 0 || d.rows <= 0 ||
+      (dt != MVPA_BF16 && dt != MVPA_F32) || x.size(0) != d.rows || x.size(1) != d.E || I * es % 16 != 0 || bias.numel() != 3 * d.KV ||
       d.D * es % 16 != 0 || rt.numel() != d.T * d.KV || rc.numel() != d.C * d.KV || rt.size(-2) != d.T || rc.size(-2) != d.C ||
       function_modes() || watched())
     Py_RETURN_NONE;
@@ -497,15 +498,18 @@ PyObject* branches(PyObject*, PyObject* const* a, Py_ssize_t n) {
     c10::cuda::CUDAGuard guard(x.device());
     c10::NoGradGuard no_grad;
     const Tensor big = at::linear(x, w_in);  // (rows, E + 2 KV + 2 I)
-    const Tensor cat = at::empty({d.rows, d.E + I}, x.options().requires_grad(false));
-    launch_fwd(d.problem(dt, 1.0 / std::sqrt((double)d.D), (int)v[0]), columns(big, 0, d.N, d.D), columns(big, d.E, d.N, d.D),
-               columns(big, d.E + d.KV, d.N, d.D), part(bias, 0), part(bias, d.KV), part(bias, 2 * d.KV), rt, rc,
-               columns(cat, 0, d.N, d.D), nullptr, status);
-    const int64_t g0 = d.E + 2 * d.KV;
-    check(api.silu_mul(part(big, g0), part(big, g0 + I), big.stride(0), const_cast<char*>(part(cat, d.E)), cat.stride(0), d.rows, (int32_t)I,
-                       dt, stream_of(x)), "mvpa_silu_mul");
-    out = at::linear(cat, w_out);
+    if (big.scalar_type() == x.scalar_type()) {  // (autocast may have formed it in another type: Python's path follows that)
+      const Tensor cat = at::empty({d.rows, d.E + I}, x.options().requires_grad(false));
+      launch_fwd(d.problem(dt, 1.0 / std::sqrt((double)d.D), (int)v[0]), columns(big, 0, d.N, d.D), columns(big, d.E, d.N, d.D),
+                 columns(big, d.E + d.KV, d.N, d.D), part(bias, 0), part(bias, d.KV), part(bias, 2 * d.KV), rt, rc,
+                 columns(cat, 0, d.N, d.D), nullptr, status);
+      const int64_t g0 = d.E + 2 * d.KV;
+      check(api.silu_mul(part(big, g0), part(big, g0 + I), big.stride(0), const_cast<char*>(part(cat, d.E)), cat.stride(0), d.rows, (int32_t)I,
+                         dt, stream_of(x)), "mvpa_silu_mul");
+      out = at::linear(cat, w_out);
+    }
   }
+  if (!out.defined()) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }

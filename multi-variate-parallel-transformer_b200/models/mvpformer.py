@@ -168,14 +168,14 @@ class MVPFormerBlock(torch.nn.Module):
                                               attn_mod._CHECK_STATUS)
             if out is not None:
                 return out
-        big = F.linear(x, w_in)                                          # (M, E + 2 KV + 2 I)
+        big = F.linear(x, w_in)                                          # (M, E + 2 KV + 2 I); under autocast in its type
         q4 = big[:, :E].view(B, N, H, D).permute(0, 2, 1, 3)
         k4 = big[:, E:E + KV].view(B, N, Hkv, D).permute(0, 2, 1, 3)
         v4 = big[:, E + KV:E + 2 * KV].view(B, N, Hkv, D).permute(0, 2, 1, 3)
-        cat = torch.empty((x.shape[0], E + I), dtype=x.dtype, device=x.device)
-        u, vt, z = (b.view(Hkv, D).to(x.dtype) for b in a.attn_bias.detach().split(KV))
-        flash_mvpa_into(cat[:, :E].view(B, N, H, D).permute(0, 2, 1, 3), q4, u, vt, z, k4, r_time, r_chan, v4,
-                        1.0 / (D ** 0.5), 10)
+        cat = torch.empty((x.shape[0], E + I), dtype=big.dtype, device=x.device)
+        u, vt, z = (b.view(Hkv, D).to(big.dtype) for b in a.attn_bias.detach().split(KV))
+        flash_mvpa_into(cat[:, :E].view(B, N, H, D).permute(0, 2, 1, 3), q4, u, vt, z, k4, r_time.to(big.dtype),
+                        r_chan.to(big.dtype), v4, 1.0 / (D ** 0.5), 10)
         g0 = E + 2 * KV
         mvpa_ops.silu_mul(big[:, g0:g0 + I], big[:, g0 + I:g0 + 2 * I], cat[:, E:])
         return F.linear(cat, w_out)
@@ -194,8 +194,9 @@ class MVPFormerBlock(torch.nn.Module):
         KV = Hkv * D
         w_in, w_out = self.fused_weights()
         big = F.linear(x, w_in)                                          # (rows of this rank, E + 2 KV + 2 I)
-        cat = torch.empty((x.shape[0], E + I), dtype=x.dtype, device=x.device)
-        u, vt, z = (b.view(Hkv, D).to(x.dtype) for b in a.attn_bias.detach().split(KV))
+        cat = torch.empty((x.shape[0], E + I), dtype=big.dtype, device=x.device)
+        u, vt, z = (b.view(Hkv, D).to(big.dtype) for b in a.attn_bias.detach().split(KV))
+        r_time, r_chan = r_time.to(big.dtype), r_chan.to(big.dtype)
         bounds = [(0, rows[0]), (rows[0], rows[0] + rows[1])]
         part = lambda lo, hi, c0, heads: big[lo:hi, c0:c0 + heads * D].view(1, hi - lo, heads, D) if hi > lo else None
         q_loc = [part(lo, hi, 0, H) for lo, hi in bounds]

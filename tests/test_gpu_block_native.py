@@ -89,3 +89,16 @@ def test_backward_of_rearranged_saved_tensors(cuda, form):
         assert "BlockFunction" in type(y.grad_fn).__name__
     for a, b in zip(torch.autograd.grad(y, ins, dy), want):
         assert (a - b).norm() <= 1e-5 * b.norm()
+
+
+# the inference block inside autocast computes in the region's type throughout
+def test_fused_branches_inside_autocast(cuda):
+    block, x, _, _ = _block(cuda, B=2, T=13, C=5)
+    x = x.detach().view(-1, 128)
+    rt, rc = torch.randn(2, 13, 32, device=cuda), torch.randn(2, 5, 32, device=cuda)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        got = [block.fused_branches(x, a, b, 2, 13, 5) for a, b in ((rt, rc), (rt.bfloat16(), rc.bfloat16()))]
+        again = block.fused_branches(x.bfloat16(), rt.bfloat16(), rc.bfloat16(), 2, 13, 5)
+    want = block.bfloat16().fused_branches(x.bfloat16(), rt.bfloat16(), rc.bfloat16(), 2, 13, 5)
+    for y in (*got, again):
+        assert y.dtype == torch.bfloat16 and torch.equal(y, want)
