@@ -42,10 +42,7 @@ def _source_hash() -> str:
 
 
 def _stale() -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(HASH_PATH)):
-        return True
-    with open(HASH_PATH) as f:
-        return f.read().strip() != _source_hash()
+    return _nat.is_stale(LIB_PATH, HASH_PATH, _source_hash)
 
 
 def build(force: bool = False) -> str:
@@ -57,14 +54,19 @@ def build(force: bool = False) -> str:
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     includes = [os.path.dirname(_HEADER), sysconfig.get_paths()["include"], os.path.join(root, "include"),
                 os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
-    tmp = LIB_PATH + ".tmp"
-    res = subprocess.run([compiler, *FLAGS, *(f"-I{i}" for i in includes), _SOURCE, f"-L{os.path.join(root, 'lib')}",
-                          *(f"-l{name}" for name in LIBS), "-o", tmp], capture_output=True, text=True)
-    if res.returncode != 0:
-        raise ImportError(f"building {_NAME}.so failed:\n" + res.stdout + res.stderr)
-    os.replace(tmp, LIB_PATH)
-    with open(HASH_PATH, "w") as f:
-        f.write(_source_hash())
+
+    def link(path):
+        res = subprocess.run([compiler, *FLAGS, *(f"-I{i}" for i in includes), _SOURCE, f"-L{os.path.join(root, 'lib')}",
+                              *(f"-l{name}" for name in LIBS), "-o", path], capture_output=True, text=True)
+        if res.returncode != 0:
+            raise ImportError(f"building {_NAME}.so failed:\n" + res.stdout + res.stderr)
+
+    try:
+        with _nat.one_builder(LIB_PATH):
+            if force or _stale():
+                _nat.publish(link, LIB_PATH, HASH_PATH, _source_hash())
+    except OSError as e:   # no compiler, or a folder that cannot be written to
+        raise ImportError(f"building {_NAME}.so failed: {e}") from e
     return LIB_PATH
 
 

@@ -8,6 +8,7 @@ callers get an ``ImportError``.
 from __future__ import annotations
 
 import ctypes
+import fcntl
 import hashlib
 import os
 import shutil
@@ -15,7 +16,7 @@ import subprocess
 import tempfile
 import threading
 from concurrent.futures import ThreadPoolExecutor
-from contextlib import nullcontext
+from contextlib import contextmanager, nullcontext
 
 import torch
 from torch.overrides import _get_current_function_mode_stack
@@ -56,10 +57,40 @@ def _source_hash() -> str:
 
 
 def _stale() -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(HASH_PATH)):
+    return is_stale(LIB_PATH, HASH_PATH, _source_hash)
+
+
+def is_stale(lib_path, hash_path, digest) -> bool:
+    if not (os.path.exists(lib_path) and os.path.exists(hash_path)):
         return True
-    with open(HASH_PATH) as f:
-        return f.read().strip() != _source_hash()
+    with open(hash_path) as f:
+        return f.read().strip() != digest()
+
+
+@contextmanager
+def one_builder(lib_path):
+    """Processes that start together on a fresh checkout build one after the other (and all but the first find it done).
+    The lock is on the folder: nothing is left behind.  Where a file system has none, what `publish` does is still whole."""
+    fd = os.open(os.path.dirname(lib_path), os.O_RDONLY)
+    try:
+        try:
+            fcntl.flock(fd, fcntl.LOCK_EX)
+        except OSError:
+            pass
+        yield
+    finally:
+        os.close(fd)
+
+
+def publish(link, lib_path, hash_path, digest: str) -> None:
+    """Put the library that `link(path)` writes, and then its digest, in place; nobody ever sees half of either."""
+    with tempfile.TemporaryDirectory(dir=os.path.dirname(lib_path), prefix=".build") as place:
+        new, new_hash = os.path.join(place, "lib"), os.path.join(place, "hash")
+        link(new)
+        with open(new_hash, "w") as f:
+            f.write(digest)
+        os.replace(new, lib_path)
+        os.replace(new_hash, hash_path)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -83,12 +114,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         run([*fast, *(["-Xptxas=-v"] if verbose else []), "-I", _INCLUDE, "-I", _CSRC, "-c", src, "-o", obj])
         return obj
 
-    tmp = LIB_PATH + ".tmp"
-    with tempfile.TemporaryDirectory() as objects, ThreadPoolExecutor() as pool:
-        run(["-shared", *pool.map(compile_one, sources()), "-o", tmp])
-    os.replace(tmp, LIB_PATH)
-    with open(HASH_PATH, "w") as f:
-        f.write(_source_hash())
+    try:
+        with one_builder(LIB_PATH), tempfile.TemporaryDirectory() as objects, ThreadPoolExecutor() as pool:
+            if force or _stale():
+                digest = _source_hash()      # (of what is compiled, whatever happens to the sources meanwhile)
+                publish(lambda path: run(["-shared", *pool.map(compile_one, sources()), "-o", path]), LIB_PATH, HASH_PATH, digest)
+    except OSError as e:   # a folder that cannot be written to
+        raise ImportError(f"building libmvpa_b200.so failed: {e}") from e
     if verbose:
         print("".join(messages))
     return LIB_PATH
