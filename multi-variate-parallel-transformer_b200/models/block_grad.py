@@ -114,6 +114,8 @@ def applies(block, x, pos, chan, classes) -> bool:
         return False
     if a.head_dim not in (16, 32, 64, 128) or a.num_heads % a.num_kv_heads:
         return False                 # (what the operator refuses is refused by the operator)
+    if not _host.usable(x):
+        return False                 # (without the extension there is no function, but the modules)
     if x.dim() != 4 or pos.shape != (1, x.shape[1], x.shape[3]) or chan.shape != (1, x.shape[2], x.shape[3]):
         return False
     # (weights of other sizes than the module was made with: a pruned head, a replaced projection)

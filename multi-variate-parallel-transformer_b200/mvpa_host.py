@@ -15,6 +15,7 @@ import subprocess
 import sys
 import sysconfig
 import threading
+import warnings
 
 import torch
 
@@ -31,6 +32,7 @@ LIBS = ["c10", "c10_cuda", "torch_cpu", "torch_cuda", "torch_python"]
 
 _lock = threading.Lock()
 _module = None
+_refused = False      # the extension cannot be built or loaded here
 
 
 def _source_hash() -> str:
@@ -71,8 +73,8 @@ def build(force: bool = False) -> str:
 
 
 def module():
-    """The loaded extension; builds it first when its sources are newer than the binary.  (No fallback: a binary built for
-    another torch is refused.)"""
+    """The loaded extension; builds it first when its sources are newer than the binary.  (A binary built for another torch is
+    refused.)"""
     global _module
     if _module is None:
         with _lock:
@@ -87,8 +89,22 @@ def module():
     return _module
 
 
+def available() -> bool:
+    """Whether there is an extension.  A box without a C++ compiler or torch's headers can use a CUDA library that came ready
+    built: the Python paths around the same kernels serve it, with a warning."""
+    global _refused
+    if _module is None and not _refused:
+        _nat.lib()                      # (without the CUDA library nothing works: that error is its own)
+        try:
+            module()
+        except ImportError as e:
+            _refused = True
+            warnings.warn(f"{e}\nCalls go through Python instead: the same kernels and results, more host time.", RuntimeWarning)
+    return _module is not None
+
+
 def usable(t) -> bool:
     """Whether a call on `t` may go to the extension at all: an ordinary CUDA tensor, no compiler looking on, no forward-mode
     level.  (The extension itself sees modes, transforms, tracers and every tensor's layout.)"""
     return ((type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and not torch.compiler.is_compiling()
-            and torch.autograd.forward_ad._current_level < 0 and t.is_cuda)
+            and torch.autograd.forward_ad._current_level < 0 and t.is_cuda and (_module is not None or available()))

@@ -3,6 +3,7 @@ GPU, no real compiler: a stand-in writes the library in two halves)."""
 import os
 import subprocess
 import sys
+import warnings
 
 import pytest
 
@@ -47,3 +48,20 @@ def test_no_compiler_is_an_import_error(tmp_path, monkeypatch):
     with pytest.raises(ImportError):
         mvpa_host.build()
     assert not os.listdir(tmp_path)
+
+
+def test_without_the_extension_python_serves(monkeypatch):
+    sys.path.insert(0, PKG)
+    import mvpa_host
+
+    def refuse(force=False):
+        raise ImportError("no compiler")
+
+    monkeypatch.setattr(mvpa_host, "_module", None)
+    monkeypatch.setattr(mvpa_host, "_refused", False)
+    monkeypatch.setattr(mvpa_host, "build", refuse)
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        assert not mvpa_host.available()
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert not mvpa_host.available()           # (once)

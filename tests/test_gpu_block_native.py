@@ -102,3 +102,29 @@ def test_fused_branches_inside_autocast(cuda):
     want = block.bfloat16().fused_branches(x.bfloat16(), rt.bfloat16(), rc.bfloat16(), 2, 13, 5)
     for y in (*got, again):
         assert y.dtype == torch.bfloat16 and torch.equal(y, want)
+
+
+def test_without_the_extension(cuda, monkeypatch):
+    import attentions
+    import mvpa_host
+    block, x, pos, chan = _block(cuda)
+    ins = _inputs(block, x, pos, chan)
+    gen = torch.Generator().manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=gen).to(cuda)
+    a = [r(2, 4, 30, 64), r(1, 2, 1, 64), r(1, 2, 1, 64), r(1, 2, 1, 64), r(2, 2, 30, 64), r(1, 2, 5, 64), r(1, 2, 6, 64), r(2, 2, 30, 64)]
+    y = block(x, pos, chan)[0]
+    dy = torch.randn_like(y)
+    want, o = torch.autograd.grad(y, ins, dy), attentions.flashmvpa(*a, True, 0.125, window_size=10)
+
+    def refuse(force=False):
+        raise ImportError("no compiler")
+
+    monkeypatch.setattr(mvpa_host, "_module", None)
+    monkeypatch.setattr(mvpa_host, "_refused", False)
+    monkeypatch.setattr(mvpa_host, "build", refuse)
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        assert torch.equal(attentions.flashmvpa(*a, True, 0.125, window_size=10), o)
+    y2 = block(x, pos, chan)[0]
+    assert "BlockFunction" not in type(y2.grad_fn).__name__ and (y2 - y).norm() <= 1e-5 * y.norm()
+    for g, w in zip(torch.autograd.grad(y2, ins, dy), want):
+        assert (g - w).norm() <= 1e-5 * w.norm()
