@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
@@ -44,6 +45,8 @@ struct Api {
   decltype(&mvpa_last_error_string) last_error;
 } api;
 
+PyObject* device_mode = nullptr;  // torch.utils._device.DeviceContext
+
 void check(int status, const char* what) {
   if (status != 0)
     throw std::runtime_error(std::string(what) + " failed (status " + std::to_string(status) + "): " + api.last_error());
@@ -58,7 +61,15 @@ bool watched() {
   return c10::impl::TorchDispatchModeTLS::any_modes_set() || !(c10::impl::tls_local_dispatch_key_set().included_ & keys).empty() ||
          torch::jit::tracer::isTracing();
 }
-bool function_modes() { return at::impl::PythonTorchFunctionTLS::stack_len() > 0; }
+// (A default device is a function mode as well; it only fills in where new tensors live.)
+bool function_modes() {
+  for (int64_t i = 0, n = at::impl::PythonTorchFunctionTLS::stack_len(); i < n; ++i) {
+    const int device = PyObject_IsInstance(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter()), device_mode);
+    if (device < 0) throw python_error();
+    if (device == 0) return true;
+  }
+  return false;
+}
 
 bool ordinary(const Tensor& t) {  // a strided CUDA tensor with storage and no wrapper or lazy bit
   using c10::DispatchKey;
@@ -514,9 +525,13 @@ PyObject* branches(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-PyObject* init(PyObject*, PyObject* path) {  // init(path of libmvpa_b200.so), which is already loaded
-  const char* p = PyUnicode_AsUTF8(path);
+// init(path of libmvpa_b200.so, which is already loaded; the class of the mode that a default device is)
+PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (!arguments(n, 2)) return nullptr;
+  const char* p = PyUnicode_AsUTF8(a[0]);
   if (!p) return nullptr;
+  Py_INCREF(a[1]);
+  device_mode = a[1];
   void* so = dlopen(p, RTLD_NOW);
   if (!so) { PyErr_SetString(PyExc_ImportError, dlerror()); return nullptr; }
   const char* missing = nullptr;
@@ -536,7 +551,7 @@ PyObject* init(PyObject*, PyObject* path) {  // init(path of libmvpa_b200.so), w
 }
 
 #define FAST(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {{"init", init, METH_O, nullptr}, FAST(attend), FAST(forward), FAST(backward), FAST(plain), FAST(block_forward),
+PyMethodDef methods[] = {FAST(init), FAST(attend), FAST(forward), FAST(backward), FAST(plain), FAST(block_forward),
                          FAST(block_backward), FAST(branches), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "mvpa_host_b200", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

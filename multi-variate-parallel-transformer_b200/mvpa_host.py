@@ -18,6 +18,7 @@ import threading
 import warnings
 
 import torch
+from torch.utils._device import DeviceContext
 
 import mvpa_native as _nat
 
@@ -84,7 +85,7 @@ def module():
                 loader = importlib.machinery.ExtensionFileLoader(_NAME, LIB_PATH)
                 loaded = importlib.util.module_from_spec(importlib.util.spec_from_file_location(_NAME, LIB_PATH, loader=loader))
                 loader.exec_module(loaded)
-                loaded.init(_nat.LIB_PATH)
+                loaded.init(_nat.LIB_PATH, DeviceContext)
                 _module = loaded
     return _module
 
