@@ -112,9 +112,19 @@ def _need_cuda(q):
         raise RuntimeError("flash_mvpa: tensors must be on a CUDA device (no CPU path)")
 
 
-def _lay_out(q, u, vt, z, k, r_time, r_chan, v):
-    """The operands as the kernels read them, copied only where their layout asks for it."""
+def _lay_out(q, u, vt, z, k, r_time, r_chan, v, q_time):
+    """The operands as the kernels read them, copied only where their layout asks for it.  (They read through pointers: what
+    does not go together is refused here.)"""
     _need_cuda(q)
+    Hkv, N, D = k.shape[1:]
+    T, C = r_time.shape[-2], r_chan.shape[-2]
+    if (k.shape != v.shape or k.shape[0] != q.shape[0] or q.shape[3] != D or T * C != N or q.shape[2] != (q_time[1] or T) * C
+            or any(t.numel() != Hkv * n * D for t, n in ((u, 1), (vt, 1), (z, 1), (r_time, T), (r_chan, C)))):
+        raise RuntimeError("flash_mvpa: the operands' shapes do not go together: "
+                           + ", ".join(str(tuple(t.shape)) for t in (q, u, vt, z, k, r_time, r_chan, v)))
+    for t in (u, vt, z, k, r_time, r_chan, v):
+        if t.dtype != q.dtype or t.device != q.device:
+            raise RuntimeError(f"flash_mvpa: an operand is {t.dtype} on {t.device}, q is {q.dtype} on {q.device}")
     return (_rows(q), u.contiguous(), vt.contiguous(), z.contiguous(), _rows(k), r_time.contiguous(), r_chan.contiguous(),
             _rows(v))
 
@@ -134,7 +144,7 @@ class FlashMVPA(torch.autograd.Function):
             ctx.save_for_backward(*given, *native)
             ctx.copied = ()
             return native[0]
-        q, u, vt, z, k, r_time, r_chan, v = read = _lay_out(*given)
+        q, u, vt, z, k, r_time, r_chan, v = read = _lay_out(*given, q_time)
         o = torch.empty_like(q)
         lse = _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, True)
         ctx.save_for_backward(*read, o, lse)
@@ -242,7 +252,7 @@ def _attend(q, u, vt, z, k, r_time, r_chan, v, sm_scale, window, q_time):
     if ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or not _nat.untraced()
             or not all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts)):
         return FlashMVPA.apply(*ts, sm_scale, window, q_time)
-    q, u, vt, z, k, r_time, r_chan, v = _lay_out(*ts)
+    q, u, vt, z, k, r_time, r_chan, v = _lay_out(*ts, q_time)
     o = torch.empty_like(q)
     _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, o, sm_scale, window, q_time, False)
     return o
@@ -254,10 +264,10 @@ def flash_mvpa_into(out, q, u, vt, z, k, r_time, r_chan, v, sm_scale, window_siz
     next projection reads).  u, vt, z (Hkv,D); r_time (Hkv,T,D); r_chan (Hkv,C,D).  `q_time_range=(t0, n)`:
     `q` and `out` hold only the tokens of time steps t0..t0+n-1 (see `flash_mvpa`).  No counterpart in the
     reference, whose operator always allocates its output (`attentions/attn.py:1047`)."""
-    q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v)
-    if not _aligned(out) or out.shape != q.shape:
-        raise RuntimeError("flash_mvpa_into: `out` must have q's shape, a contiguous last dimension and 16-byte aligned strides")
     q_time = (0, 0) if q_time_range is None else (int(q_time_range[0]), int(q_time_range[1]))
+    q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v, q_time)
+    if not _aligned(out) or out.shape != q.shape or out.dtype != q.dtype or out.device != q.device:
+        raise RuntimeError("flash_mvpa_into: `out` must have q's shape, type and device, a contiguous last dimension and 16-byte aligned strides")
     _launch_fwd(q, u, vt, z, k, r_time, r_chan, v, out, sm_scale, window_size, q_time, False)
     return out
 

@@ -107,7 +107,7 @@ void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.devi
 
 struct Ops {  // q, u, vt, z, k, r_time, r_chan, v
   Tensor t[8];
-  bool take(PyObject* const* a) {
+  bool take(PyObject* const* a, int64_t steps = 0) {  // `steps` time steps of queries, 0 for all
     for (int i = 0; i < 8; ++i) {
       if (!THPVariable_CheckExact(a[i])) return false;
       t[i] = THPVariable_Unpack(a[i]);
@@ -116,7 +116,10 @@ struct Ops {  // q, u, vt, z, k, r_time, r_chan, v
     if (dtype_code(t[0]) < 0 || !rows_fit(t[0]) || !rows_fit(t[4]) || !rows_fit(t[7]) || t[5].dim() < 2 || t[6].dim() < 2) return false;
     for (int i : {1, 2, 3, 5, 6})
       if (!t[i].is_contiguous()) return false;
-    return true;
+    const int64_t Hkv = t[4].size(1), N = t[4].size(2), D = t[4].size(3), T = t[5].size(-2), C = t[6].size(-2);
+    return t[4].sizes() == t[7].sizes() && t[0].size(0) == t[4].size(0) && t[0].size(3) == D && T * C == N &&
+           t[0].size(2) == (steps ? steps : T) * C && t[1].numel() == Hkv * D && t[2].numel() == Hkv * D && t[3].numel() == Hkv * D &&
+           t[5].numel() == Hkv * T * D && t[6].numel() == Hkv * C * D;
   }
   mvpa_problem problem(double scale, int64_t window, int64_t t0, int64_t tn) const {
     mvpa_problem p = {};
@@ -192,14 +195,11 @@ PyObject* attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int64_t window;
   if (!numbers(a[8], a[9], &scale, &window) || function_modes() || watched() || !x.take(a)) Py_RETURN_NONE;
   const Tensor &q = x.t[0], &k = x.t[4], &rt = x.t[5], &rc = x.t[6];
-  const int64_t Hkv = k.size(1), D = q.size(3), N = q.size(2);
+  const int64_t D = q.size(3);
   if (c10::GradMode::is_enabled())
     for (const Tensor& t : x.t)
       if (t.requires_grad()) Py_RETURN_NONE;
-  if (k.sizes() != x.t[7].sizes() || k.size(0) != q.size(0) || k.size(2) != N || k.size(3) != D || q.size(1) % Hkv != 0 ||
-      (D != 16 && D != 32 && D != 64 && D != 128) || rt.dim() != 4 || rc.dim() != 4 || rt.size(2) * rc.size(2) != N ||
-      rt.numel() != Hkv * rt.size(2) * D || rc.numel() != Hkv * rc.size(2) * D || x.t[1].numel() != Hkv * D ||
-      x.t[2].numel() != Hkv * D || x.t[3].numel() != Hkv * D)
+  if (q.size(1) % k.size(1) != 0 || (D != 16 && D != 32 && D != 64 && D != 128) || rt.dim() != 4 || rc.dim() != 4)
     Py_RETURN_NONE;
   Tensor o;
   {
@@ -223,10 +223,11 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   double scale;
   int64_t window;
   if (!numbers(a[8], a[9], &scale, &window) || !PyLong_CheckExact(a[10]) || !PyLong_CheckExact(a[11]) || function_modes() ||
-      watched() || !x.take(a))
+      watched())
     Py_RETURN_NONE;
   const int64_t t0 = PyLong_AsLongLong(a[10]), tn = PyLong_AsLongLong(a[11]);
   if (PyErr_Occurred()) return nullptr;
+  if (!x.take(a, tn)) Py_RETURN_NONE;
   const Tensor& q = x.t[0];
   Tensor o, lse;
   {
@@ -258,7 +259,9 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor &q = x.t[0], &k = x.t[4], &v = x.t[7];
   for (const Tensor& t : {d_o, o})
     if (!ordinary(t) || t.device() != q.device() || t.scalar_type() != q.scalar_type() || t.sizes() != q.sizes()) Py_RETURN_NONE;
-  if (!ordinary(lse) || lse.scalar_type() != at::kFloat || !lse.is_contiguous() || !rows_fit(o)) Py_RETURN_NONE;
+  if (!ordinary(lse) || lse.scalar_type() != at::kFloat || lse.device() != q.device() || !lse.is_contiguous() ||
+      lse.numel() != q.size(0) * q.size(1) * q.size(2) || !rows_fit(o))
+    Py_RETURN_NONE;
   std::vector<Tensor> g(8);
   {
     pybind11::gil_scoped_release nogil;

@@ -3,6 +3,7 @@ result, which a comparison of results does not show)."""
 import pytest
 import torch
 
+import attentions
 import models
 import mvpa_host
 from test_gpu_host_path import FORMS, _operands
@@ -71,3 +72,28 @@ def test_default_device(cuda):
                 assert not any(taken())
         with _Functions(), torch.device(device):
             assert not any(taken())
+
+
+# operands that do not go together are refused before a kernel reads them, on every way to the kernels
+@pytest.mark.parametrize("change", [lambda a: (4, a[4][:1]), lambda a: (7, a[7][:1]), lambda a: (7, a[7][:, :, :-1]), lambda a: (4, a[4][:, :1]),
+                                    lambda a: (4, a[4].float()), lambda a: (1, a[1].float()), lambda a: (5, a[5].half()), lambda a: (7, a[7].cpu()),
+                                    lambda a: (2, a[2].cpu())])
+@pytest.mark.parametrize("grad", [False, True])
+def test_operands_that_do_not_go_together(cuda, change, grad):
+    a = _operands(cuda, torch.bfloat16)
+    i, t = change(a)
+    a[i] = t
+    if grad:
+        a[0].requires_grad_()
+    with pytest.raises((RuntimeError, AssertionError)):
+        attentions.flashmvpa(*a, True, 0.125, window_size=10)
+    small = [x[0] if j in (1, 2, 3, 5, 6) else x for j, x in enumerate(a)]
+    with pytest.raises((RuntimeError, AssertionError)), torch.no_grad():
+        attentions.flash_mvpa_into(torch.empty_like(a[0]), *small, 0.125, 10)
+
+
+def test_output_of_another_type(cuda):
+    a = _operands(cuda, torch.bfloat16)
+    small = [x[0] if j in (1, 2, 3, 5, 6) else x for j, x in enumerate(a)]
+    with pytest.raises(RuntimeError):
+        attentions.flash_mvpa_into(torch.empty_like(a[0], dtype=torch.float32), *small, 0.125, 10)
