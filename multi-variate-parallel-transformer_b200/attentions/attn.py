@@ -174,6 +174,9 @@ def _gradients(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window):
         native = _host.module().backward(do, q, u, vt, z, k, r_time, r_chan, v, o, lse, sm_scale, window, _CHECK_STATUS)
         if native is not None:
             return native
+    # (a saved-tensor hook may have brought back any layout)
+    q, u, vt, z, k, r_time, r_chan, v = _lay_out(q, u, vt, z, k, r_time, r_chan, v, (0, 0))
+    o, lse = _rows(o), lse.contiguous()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     small = _launch_bwd(q, u, vt, z, k, r_time, r_chan, v, o, lse, _rows(do), dq, dk, dv, sm_scale, window)
     shapes = [x.shape for x in (u, vt, z, r_time, r_chan)]

@@ -97,3 +97,17 @@ def test_output_of_another_type(cuda):
     small = [x[0] if j in (1, 2, 3, 5, 6) else x for j, x in enumerate(a)]
     with pytest.raises(RuntimeError):
         attentions.flash_mvpa_into(torch.empty_like(a[0], dtype=torch.float32), *small, 0.125, 10)
+
+
+# saved tensors that a hook brings back in another layout, on both ways to the kernels
+@pytest.mark.parametrize("form", [lambda t: t.clone(), lambda t: torch.nn.functional.pad(t, (0, 1))[..., :-1],
+                                  lambda t: t.transpose(-1, -2).contiguous().transpose(-1, -2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_backward_of_rearranged_saved_tensors(cuda, dtype, form):
+    a = [t.requires_grad_() for t in _operands(cuda, dtype)]
+    d_o = torch.ones_like(a[0])
+    want = torch.autograd.grad(attentions.flashmvpa(*a, True, 0.125, window_size=2), a, d_o)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), form):
+        o = attentions.flashmvpa(*a, True, 0.125, window_size=2)
+    for g, w in zip(torch.autograd.grad(o, a, d_o), want):
+        assert torch.equal(g, w)
