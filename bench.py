@@ -25,6 +25,7 @@ reference's Triton operator staged under baseline/_ref/ (what `extra.triton_refe
 import argparse
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -740,6 +741,16 @@ def triton_point(args, device_index):
         return {"impl": "triton", "error": "child process exceeded 600 s (compile or run); not retried"}
 
 
+def kernels_of_a_call(torch, attentions, t, w, flush, gout) -> str:
+    """The library's kernels of one timed call, as the profiler names them (after everything that is timed)."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        time_kernel(torch, attentions, t, w, 1, 0, flush, gout)
+        torch.cuda.synchronize()
+    names = [n for e in prof.events() for n in re.findall(r"\b(?:tc|simt|rel)_\w+_kernel(?:<[\w, ]*>)?", e.name)]
+    return ", ".join(dict.fromkeys(names))
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -890,9 +901,7 @@ def main():
             "clocks": clk.summary(),
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": None if train else NCU_DRAM_BYTES.get(args.workload), "peak_source": peak_src,
-                         "kernel": ("whole step (tc_fwd_kernel, tc_bwd_q_kernel, tc_bwd_kv_kernel, simt_drel_kernel)"
-                                    if train else ("two CTAs per multiprocessor: tc_fwd_two_kernel, D %d, %d channel slots" if w["D"] == 64 and w["C"] <= 64 else "tc_fwd_kernel<%d,%d>") %
-                                    (w["D"], 32 if w["C"] <= 32 else 64 if w["C"] <= 64 else 128)),
+                         "kernel": None,   # (named below)
                          "flops_per_launch": f["f_alg"],
                          "achieved_dense_convention": f["f_dense"] / (kernel_ms * 1e-3) / 1e12},
         }
@@ -945,6 +954,7 @@ def main():
             out["cpu_baseline"] = {"value": flops(**sample)["f_alg"] / sec / 1e12, "unit": UNIT, "cores": cores,
                                    "kind": kind, "sample": "1 of the 4 batch elements (16 heads, 4096 tokens), fp32, median of 10 passes",
                                    "seconds": sec}
+        out["roofline"]["kernel"] = ("whole step: " if train else "") + kernels_of_a_call(torch, attentions, t, w, flush, gout)
         print(json.dumps(out))
     if world > 1:
         dist.barrier()
