@@ -12,7 +12,7 @@
 //
 // Same CTA shape as the forward (mvpa_tc_fwd.cu): 128 query rows of one (b,h); two softmax
 // warpgroups (thread = TMEM lane = query row, 64 key columns each), one TMA producer lane, one MMA
-// issuer warp (convergent code, the tcgen05 instructions guarded by the elected lane); dense tiles (inside the content window) first, then light tiles.  Per dense tile
+// issuer warp (convergent code, the tcgen05 instructions guarded by the elected lane); light tiles (outside the content window) first, then dense ones.  Per dense tile
 // three products: S = Q'K^T, dP = dO V^T, dQ += dS_w K (dS_w as bf16 in TMEM, K as MN-major
 // operand); a light tile needs dP only: its content term is zero-filled, so it contributes to the
 // relative-score gradients but not to dQ's content part, and P is the outer product of the forward.
@@ -172,7 +172,9 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   float* s_vr = s_bias + D;
   float* s_zc = s_vr + 128;
   float* s_max = s_zc + 128;  // [2 wg][128]
-  float* s_part = s_bias;     // [4][128], once the prologue is over (s_bias .. s_max are dead by then)
+  // [4][128], from the first dense tile on.  The light tiles read s_vr, which it covers: a fast warp's first part cannot land on it
+  // before a slow warp's last light tile, because the first dense dP product waits for every thread's report of that tile.
+  float* s_part = s_bias;
   static_assert(C_::TAIL_FLOATS >= 512, "four buffers of partial sums");
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_max + 256);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBarSlotFull + 2 * NS);
@@ -198,7 +200,6 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
   // Visit order: the light tiles 0 .. n_light-1 first, then the dense ones (natural key order).  In the
   // light phase the channel-score gradient is accumulated unscaled (see the softmax warps) and folded
   // into the ordinary accumulators at the transition, so it must come first.
-  auto tile_of = [&](int s) { return s; };
   auto is_dense = [&](int s) { return s >= n_light; };
   // position of a tile's K / V in the load sequence (a light tile loads V only)
   auto q_of_k = [&](int s) { return n_light + 2 * (s - n_light); };
@@ -273,9 +274,8 @@ tc_bwd_q_kernel(const __grid_constant__ BqMaps maps, const BqArgs p) {
         for (int hh = 0; hh < NH; ++hh) tma_load_5d(dst + hh * HALF, map, &slot_full[sl], hh * 64, 0, J * TPB, hk, b);
       };
       for (int s = 0; ok && s < n_tiles; ++s) {
-        const int J = tile_of(s);
-        if (is_dense(s)) load_slot(&maps.k, q_of_k(s), J);
-        if (ok) load_slot(&maps.v, q_of_v(s), J);
+        if (is_dense(s)) load_slot(&maps.k, q_of_k(s), s);
+        if (ok) load_slot(&maps.v, q_of_v(s), s);
       }
       // finish: the relative keys once more (the ring is idle once every product has completed)
       if (ok) ok = mbar_wait(&bars[kBarAllDone], 0, p.status, 112);

@@ -14,8 +14,8 @@
 //            allocates / frees TMEM.  The whole warp runs the issue loop in convergent code and
 //            the elected lane's predicate guards the tcgen05 instructions themselves.
 //
-// Key tiles are visited dense-first: the tiles that overlap the content window (and the
-// diagonal), then the "light" tiles that lie wholly outside it.  The reference zero-fills the
+// Key tiles are visited dense-first (light-first on the alternating path, below): the tiles that overlap the content window
+// (and the diagonal), then the "light" tiles that lie wholly outside it.  The reference zero-fills the
 // content term there (`attentions/attn.py:261-271`) but still computes it; here a light tile
 // loads no K, issues no QK^T and computes no exponential per pair: its probabilities are the
 // outer product  exp2(tb_i[t_k] - m) x exp2(cb_i[c_k])  of a per-time-step scalar and the row's
@@ -67,7 +67,7 @@ struct TcArgs {
 };
 
 enum BarrierIndex {
-  kBarProFull = 0, kBarProMma, kBarProDone, kBarXchg,
+  kBarProFull = 0, kBarProMma, kBarProDone,
   kBarSFull,                     // 2
   kBarPFull = kBarSFull + 2,     // 2
   kBarPlFull = kBarPFull + 2,    // 4: P of the light tiles (four buffers, 64 TMEM columns each)
@@ -231,7 +231,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     mbar_init(&bars[kBarProFull], 1);
     mbar_init(&bars[kBarProMma], 1);
     mbar_init(&bars[kBarProDone], kSoftmaxThreads);
-    mbar_init(&bars[kBarXchg], kSoftmaxThreads);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[kBarSFull + i], 1);
       mbar_init(&bars[kBarPFull + i], ALT ? kSoftmaxThreads / 2 : kSoftmaxThreads);
@@ -261,8 +260,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     if (warp == 9) tmem_dealloc(tmem, kTmemCols);
     return;
   }
-  // Register re-balancing between warpgroups: the producer / MMA warpgroup keeps 40 registers
-  // per thread, the two softmax warpgroups grow to 232.
+  // Register re-balancing between warpgroups: the producer / MMA warpgroup keeps 56 registers a thread, the two softmax
+  // warpgroups grow to 224 (64512 in all, what the CTA was launched with).
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 8) {

@@ -539,10 +539,14 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
 // Whether a call takes this kernel.
 //   * Enough CTAs: a single CTA is faster with two softmax warpgroups on a multiprocessor of its own, so the longest one (the
 //     last query tile, n_qt dense tiles: 6.5 + 1.5 n_qt us here) has to be shorter than the whole call in the other kernel.
-//     That is where the CTAs outnumber the multiprocessors 1.15 + n_qt / 20 times.  Measured, us, this kernel / the other
-//     (12 heads): n_qt 2: 144 CTAs 9.9 / 8.7, 192 10.1 / 15.1;  6: 144 15.7 / 14.0, 216 17.9 / 20.4;  13: 156 25.1 / 21.0,
-//     312 29.2 / 33.9;  32: 384 57.0 / 50.0, 768 70.4 / 93.6;  64: 768 112 / 121.  Large calls: 4 x 64 x 64 tokens, 16 heads
-//     179 / 242, 8 x 128 x 64, 12 heads 735 / 957, 8 x 128 x 32, 16 heads 311 / 437.
+//     That is where the CTAs outnumber the multiprocessors 1.15 + n_qt / 20 times.  Measured, us, this kernel / the other as it
+//     is now (calls back to back, pre-kernel included; 64 channels, 12 heads):  n_qt 2: 144 CTAs 12.4 / 9.9, 168 12.5 / 17.1, 192
+//     12.7 / 17.6;  6: 144 17.1 / 13.6, 216 18.3 / 20.5;  13: 156 26.2 / 21.7, 312 29.4 / 33.3;  32: 384 59.1 / 48.6, 768 69.0 / 88.1;
+//     64: 768 110 / 114, 1536 171 / 216.  Large calls: 4 x 64 x 64 tokens, 16 heads 170 / 228, 8 x 128 x 64, 12 heads 664 / 841,
+//     8 x 128 x 32, 16 heads 302 / 407.  (At 32 slots a CTA's tiles are the shorter ones and the line lies a little early: 1 x 128 x 32,
+//     16 heads, 512 CTAs 62 / 56; 2 x 40 x 22, 12 heads, 240 CTAs 24 / 22 stays with the other.)
+//     Large calls that the other kernel keeps for their window: 4 x 64 x 64 tokens, window 15 248, 40 302; 8 x 128 x 64, 12 heads, window 15
+//     925, 40 1182; 8 x 128 x 32, window 13 423, 40 499.
 //   * A content window whose dense key steps fit s_td (every shipped window, 10, does; a window past the last key step, or
 //     none, leaves no light tiles and needs no s_td).
 inline bool applies(int window, int CP, int n_qt, unsigned grid) {
