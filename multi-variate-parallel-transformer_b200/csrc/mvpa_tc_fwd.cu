@@ -628,6 +628,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         if (need) m_used = m_light;
       }
     }
+    const float m_ref = m_used == -INFINITY ? 0.f : m_used;  // (light tiles first, and no light pair counts: every factor is 0)
     // Two tiles per turn: one round trip for the temporal scores and one look at the barriers serve both,
     // and the second tile's products are formed while the first tile's stores are in flight.  (The scores
     // of the next pair are fetched meanwhile; with an odd count the last fetch reads the column after the
@@ -666,7 +667,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           for (int q = 0; q < TPB; ++q)
             if (q == tt) raw = tb_next[u * TPB + q];
           const float tb = p.c2 * (__uint_as_float(raw) + s_vr[col0 + (l + u) * TPB + tt]) + mc;
-          a_t[u][tl] = ex2(tb - m_used);
+          a_t[u][tl] = ex2(tb - m_ref);
         }
       }
       if (l + 2 < n_light) tb_fetch(l + 2);
@@ -775,6 +776,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           const bool need = m_tile > m_used + kRescaleThreshold;
           const float alpha = need ? ex2(m_used - m_tile) : 1.f;
           if (need) m_used = m_tile;
+          if (s == 0 && m_used == -INFINITY) m_used = 0.f;  // (nothing counted so far)
           s_merge[wg * 128 + row] = m_used;
           mbar_arrive(&bars[kBarMax + wg]);
           if (__any_sync(0xffffffffu, need)) {

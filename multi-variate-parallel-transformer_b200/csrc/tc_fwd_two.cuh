@@ -314,6 +314,7 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         for (int jj = 0; jj < 16; ++jj)
           if (c + jj < light_steps) m_used = fmaxf(m_used, score(v[jj / 8][jj % 8], col0 + c + jj));
       }
+      const float m_ref = m_used == -INFINITY ? 0.f : m_used;  // (no light pair counts: every factor is 0)
 #pragma unroll 1
       for (int c = 0; c < light_steps; c += 16) {
         uint32_t v[2][8], w[8];
@@ -322,8 +323,8 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         tmem_ld_wait();
 #pragma unroll
         for (int jj = 0; jj < 16; jj += 2)
-          w[jj / 2] = pack_bf16(ex2(score(v[jj / 8][jj % 8], col0 + c + jj) - m_used),
-                                ex2(score(v[jj / 8][jj % 8 + 1], col0 + c + jj + 1) - m_used));
+          w[jj / 2] = pack_bf16(ex2(score(v[jj / 8][jj % 8], col0 + c + jj) - m_ref),
+                                ex2(score(v[jj / 8][jj % 8 + 1], col0 + c + jj + 1) - m_ref));
         tmem_st8(lane_base + kX + c / 2, w);
       }
     }
@@ -435,7 +436,7 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       tmem_ld32(s_addr, va);  // first chunk of pass 2
       max_chunk(vb, 3);
       if (e == 0 && n_light == 0) {
-        m_used = (m_tile == -INFINITY) ? 0.f : m_tile;
+        m_used = m_tile;
       } else {
         // O and l follow the maximum only when it moved by more than 2^8 (every PV product so far is complete: the
         // score product that has just been waited for was issued behind them)
@@ -457,6 +458,7 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           if (need) m_used = m_tile;
         }
       }
+      if (e == 0 && m_used == -INFINITY) m_used = 0.f;  // (nothing counted so far)
       // pass 2: P = exp2(S2 - m) as bf16 over the consumed S columns (chunk c lands in columns 16c..16c+15,
       // always behind the columns still to be read)
       float2 psum2 = make_float2(0.f, 0.f);
