@@ -139,6 +139,98 @@ __device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
   return d;
 }
 
+// ---- a dense tile by whole rows (head_dim 64, at most 64 channel slots): thread = query row, all 128 key columns ----
+// Shared by the alternating path below and by tc_fwd_two_kernel, whose results are the same bits.
+template <int CP>
+struct DenseTile {
+  static constexpr int TPB = 128 / CP;
+  float tb[TPB], wmul[TPB];  // per key step: temporal score plus the channel maximum; 0 outside the content window, else 1
+  bool valid[TPB];
+};
+// Pass 1: the row's maximum over the tile.  The TMEM load of the next 32 columns is always in flight while the current
+// ones are processed (two register buffers); the first chunk of pass 2 is on its way into `va` at the end.
+template <int CP>
+__device__ __forceinline__ float dense_max(uint32_t s_addr, const DenseTile<CP>& t, const float (&cbf)[CP], uint32_t (&va)[32]) {
+  float m_tile = -INFINITY;
+  uint32_t vb[32];
+  auto chunk = [&](const uint32_t (&v)[32], int c) {
+    const int tt = (32 * c) / CP;
+    const float2 w2 = make_float2(t.wmul[tt], t.wmul[tt]);
+    float g0 = -INFINITY, g1 = -INFINITY;
+#pragma unroll
+    for (int jj = 0; jj < 32; jj += 4) {
+      const int k = (32 * c + jj) % CP;
+      const float2 t0 = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
+      const float2 t1 = ffma2(make_float2(__uint_as_float(v[jj + 2]), __uint_as_float(v[jj + 3])), w2, make_float2(cbf[k + 2], cbf[k + 3]));
+      g0 = fmax3(g0, t0.x, t0.y);
+      g1 = fmax3(g1, t1.x, t1.y);
+    }
+    if (t.valid[tt]) m_tile = fmaxf(m_tile, fmaxf(g0, g1) + t.tb[tt]);
+  };
+  tmem_ld32(s_addr, va);
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 32, vb);
+  chunk(va, 0);
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 64, va);
+  chunk(vb, 1);
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 96, vb);
+  chunk(va, 2);
+  tmem_ld_wait();
+  tmem_ld32(s_addr, va);
+  chunk(vb, 3);
+  return m_tile;
+}
+// Pass 2: P = exp2(S2 - m) as bf16 over the consumed S columns (chunk c lands in columns 16c..16c+15, always behind the
+// columns still to be read).  Returns the row's sum; the stores are in flight.
+template <int CP>
+__device__ __forceinline__ float dense_exp(uint32_t s_addr, const DenseTile<CP>& t, const float (&cbf)[CP], float m_used, uint32_t (&va)[32]) {
+  float2 psum2 = make_float2(0.f, 0.f);
+  uint32_t vb[32];
+  auto chunk = [&](const uint32_t (&v)[32], int c) {
+    const int tt = (32 * c) / CP;
+    const float negmu = t.valid[tt] ? t.tb[tt] - m_used : -INFINITY;
+    const float2 w2 = make_float2(t.wmul[tt], t.wmul[tt]), n2 = make_float2(negmu, negmu);
+    uint32_t pk[16];
+#pragma unroll
+    for (int jj = 0; jj < 32; jj += 2) {
+      const int k = (32 * c + jj) % CP;
+      float2 x = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
+      x = fadd2(x, n2);
+      const float2 e = poly_pair(jj / 2) ? ex2_poly2(x) : make_float2(ex2(x.x), ex2(x.y));
+      psum2 = fadd2(psum2, e);
+      pk[jj / 2] = pack_bf16(e.x, e.y);
+    }
+    tmem_st16(s_addr + 16 * c, pk);
+  };
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 32, vb);
+  chunk(va, 0);
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 64, va);
+  chunk(vb, 1);
+  tmem_ld_wait();
+  tmem_ld32(s_addr + 96, vb);
+  chunk(va, 2);
+  tmem_ld_wait();
+  chunk(vb, 3);
+  return psum2.x + psum2.y;
+}
+// `n` TMEM columns of the row times alpha (a short loop: it runs when the maximum has moved far, which is rare)
+__device__ __forceinline__ void rescale_columns(uint32_t addr, int n, float alpha) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < n; c0 += 8) {
+    uint32_t v[8];
+    tmem_ld8(addr + c0, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
+    tmem_st8(addr + c0, v);
+  }
+  tmem_st_wait();
+}
+
 // Number of leading key tiles of query tile I that are "light": every pair outside the content
 // window, i.e.  I*TPB - (J*TPB + TPB - 1) > window.  Light-ness is monotone in J.
 __device__ __forceinline__ int light_tiles(int I, int TPB, int window, int n_qt) {
@@ -540,16 +632,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       const float alpha = need ? ex2(m_used - m_tile) : 1.f;
       // (split accumulators: all D columns of this warpgroup's own O; otherwise its half of the one O)
       constexpr int own0 = SPLIT ? 64 : DW, own_n = SPLIT ? D : DW;
-#pragma unroll 1
-      for (int c0 = 0; c0 < own_n; c0 += 8) {
-        uint32_t v[8];
-        tmem_ld8(lane_base + kColO + wg * own0 + c0, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-        tmem_st8(lane_base + kColO + wg * own0 + c0, v);
-      }
-      tmem_st_wait();
+      rescale_columns(lane_base + kColO + wg * own0, own_n, alpha);
       l_sum *= alpha;
       if (need) m_used = m_tile;
       return true;
@@ -614,16 +697,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         m_used = m_light;  // (nothing has been summed yet)
       } else if (__any_sync(0xffffffffu, need)) {
         const float alpha = need ? ex2(m_used - m_light) : 1.f;
-#pragma unroll 1
-        for (int c0 = 0; c0 < DW; c0 += 8) {
-          uint32_t v[8];
-          tmem_ld8(lane_base + kColO + wg * DW + c0, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-          tmem_st8(lane_base + kColO + wg * DW + c0, v);
-        }
-        tmem_st_wait();
+        rescale_columns(lane_base + kColO + wg * DW, DW, alpha);
         l_sum *= alpha;
         if (need) m_used = m_light;
       }
@@ -716,54 +790,24 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       light_phase();
       for (int s = wg; ok && s < n_dense; s += 2) {
         const int J = n_light + s;
-        float tb_all[TPB], wmul[TPB];
-        bool valid_all[TPB];
+        DenseTile<CP> t;
         {
           uint32_t tb_raw[TPB];
           int tb_col[TPB];
-          tb_issue(J, tb_raw, tb_col, valid_all);
+          tb_issue(J, tb_raw, tb_col, t.valid);
           ok = warp_wait(&bars[kBarSFull + wg], (s >> 1) & 1, p.status, 32);
           tmem_ld_wait();
           if (!ok) break;
           tc_fence_after();
-          tb_finish(tb_raw, tb_col, tb_all);
+          tb_finish(tb_raw, tb_col, t.tb);
         }
 #pragma unroll
         for (int tt = 0; tt < TPB; ++tt) {
           const int dt = ti_abs - (J * TPB + tt);
-          wmul[tt] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
+          t.wmul[tt] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
         }
-        // pass 1: the row's maximum over the tile.  The TMEM load of the next 32 columns is always in
-        // flight while the current ones are processed (two register buffers).
-        float m_tile = -INFINITY;
-        uint32_t va[32], vb[32];
-        auto max_chunk = [&](const uint32_t (&v)[32], int c) {
-          const int tt = (32 * c) / CP;
-          const float2 w2 = make_float2(wmul[tt], wmul[tt]);
-          float g0 = -INFINITY, g1 = -INFINITY;
-#pragma unroll
-          for (int jj = 0; jj < 32; jj += 4) {
-            const int k = (32 * c + jj) % CP;
-            const float2 t0 = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
-            const float2 t1 = ffma2(make_float2(__uint_as_float(v[jj + 2]), __uint_as_float(v[jj + 3])), w2, make_float2(cbf[k + 2], cbf[k + 3]));
-            g0 = fmax3(g0, t0.x, t0.y);
-            g1 = fmax3(g1, t1.x, t1.y);
-          }
-          if (valid_all[tt]) m_tile = fmaxf(m_tile, fmaxf(g0, g1) + tb_all[tt]);
-        };
-        tmem_ld32(s_addr, va);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 32, vb);
-        max_chunk(va, 0);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 64, va);
-        max_chunk(vb, 1);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 96, vb);
-        max_chunk(va, 2);
-        tmem_ld_wait();
-        tmem_ld32(s_addr, va);  // first chunk of pass 2
-        max_chunk(vb, 3);
+        uint32_t va[32];
+        const float m_tile = dense_max<CP>(s_addr, t, cbf, va);
         if (s > 0) {
           ok = take_max(s - 1);
           if (!ok) break;
@@ -783,50 +827,11 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
             const int qp = q_of_v(n_light + s - 1);  // the previous product: O is complete up to this tile
             if (!warp_wait(&slot_free[qp % NS], (qp / NS) & 1, p.status, 33)) { ok = false; break; }
             tc_fence_after();
-#pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 8) {
-              uint32_t v[8];
-              tmem_ld8(lane_base + kColO + c0, v);
-              tmem_ld_wait();
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-              tmem_st8(lane_base + kColO + c0, v);
-            }
-            tmem_st_wait();
+            rescale_columns(lane_base + kColO, D, alpha);
             l_sum *= alpha;
           }
         }
-        // pass 2: P = exp2(S2 - m) as bf16 over the consumed S columns (chunk c lands in columns 16c..16c+15,
-        // always behind the columns still to be read)
-        float2 psum2 = make_float2(0.f, 0.f);
-        auto exp_chunk = [&](const uint32_t (&v)[32], int c) {
-          const int tt = (32 * c) / CP;
-          const float negmu = valid_all[tt] ? tb_all[tt] - m_used : -INFINITY;
-          const float2 w2 = make_float2(wmul[tt], wmul[tt]), n2 = make_float2(negmu, negmu);
-          uint32_t pk[16];
-#pragma unroll
-          for (int jj = 0; jj < 32; jj += 2) {
-            const int k = (32 * c + jj) % CP;
-            float2 t = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
-            t = fadd2(t, n2);
-            const float2 e = poly_pair(jj / 2) ? ex2_poly2(t) : make_float2(ex2(t.x), ex2(t.y));
-            psum2 = fadd2(psum2, e);
-            pk[jj / 2] = pack_bf16(e.x, e.y);
-          }
-          tmem_st16(s_addr + 16 * c, pk);
-        };
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 32, vb);
-        exp_chunk(va, 0);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 64, va);
-        exp_chunk(vb, 1);
-        tmem_ld_wait();
-        tmem_ld32(s_addr + 96, vb);
-        exp_chunk(va, 2);
-        tmem_ld_wait();
-        exp_chunk(vb, 3);
-        l_sum += psum2.x + psum2.y;
+        l_sum += dense_exp<CP>(s_addr, t, cbf, m_used, va);
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&bars[kBarPFull + wg]);

@@ -383,58 +383,29 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     const uint32_t s_addr = lane_base + kS;
     for (int e = 0; ok && e < n_dense; ++e) {
       const int J = n_light + e;
-      float tb_all[TPB], wmul[TPB];
-      bool valid_all[TPB];
+      DenseTile<CP> t;
 #pragma unroll
       for (int tt = 0; tt < TPB; ++tt) {
         const int tk_abs = J * TPB + tt, dt = ti_abs - tk_abs;
-        valid_all[tt] = dt >= 0 && tk_abs < T;
-        wmul[tt] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
+        t.valid[tt] = dt >= 0 && tk_abs < T;
+        t.wmul[tt] = (p.window > 0 && dt > p.window && ti_abs != T - 1) ? 0.f : 1.f;
         const int slot = T - 1 - min(max(dt, 0), T - 1);  // (uniform in a warp)
         if (n_light > 0) {
-          tb_all[tt] = s_td[(e * TPB + tt) * 128 + row];
+          t.tb[tt] = s_td[(e * TPB + tt) * 128 + row];
         } else if (slot >= near0) {
           uint32_t raw;
           tmem_ld1(lane_base + kX + slot - near0, raw);
           tmem_ld_wait();
-          tb_all[tt] = __uint_as_float(raw);
+          t.tb[tt] = __uint_as_float(raw);
         } else {
-          tb_all[tt] = s_far[slot * 128 + row];
+          t.tb[tt] = s_far[slot * 128 + row];
         }
       }
       ok = warp_wait(&bars[kSFull], e & 1, p.status, 32);
       if (!ok) break;
       tc_fence_after();
-      // pass 1: the row's maximum over the tile, the next 32 columns in flight while the current ones are processed
-      float m_tile = -INFINITY;
-      uint32_t va[32], vb[32];
-      auto max_chunk = [&](const uint32_t (&v)[32], int c) {
-        const int tt = (32 * c) / CP;
-        const float2 w2 = make_float2(wmul[tt], wmul[tt]);
-        float g0 = -INFINITY, g1 = -INFINITY;
-#pragma unroll
-        for (int jj = 0; jj < 32; jj += 4) {
-          const int k = (32 * c + jj) % CP;
-          const float2 t0 = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
-          const float2 t1 = ffma2(make_float2(__uint_as_float(v[jj + 2]), __uint_as_float(v[jj + 3])), w2, make_float2(cbf[k + 2], cbf[k + 3]));
-          g0 = fmax3(g0, t0.x, t0.y);
-          g1 = fmax3(g1, t1.x, t1.y);
-        }
-        if (valid_all[tt]) m_tile = fmaxf(m_tile, fmaxf(g0, g1) + tb_all[tt]);
-      };
-      tmem_ld32(s_addr, va);
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 32, vb);
-      max_chunk(va, 0);
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 64, va);
-      max_chunk(vb, 1);
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 96, vb);
-      max_chunk(va, 2);
-      tmem_ld_wait();
-      tmem_ld32(s_addr, va);  // first chunk of pass 2
-      max_chunk(vb, 3);
+      uint32_t va[32];
+      const float m_tile = dense_max<CP>(s_addr, t, cbf, va);
       if (e == 0 && n_light == 0) {
         m_used = m_tile;
       } else {
@@ -443,54 +414,16 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         const bool need = m_tile > m_used + kRescaleThreshold;
         if (__any_sync(0xffffffffu, need)) {
           const float alpha = need ? ex2(m_used - m_tile) : 1.f;
-#pragma unroll 1
-          for (int c0 = 0; c0 < D; c0 += 8) {
-            uint32_t v[8];
-            tmem_ld8(lane_base + kO + c0, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int jj = 0; jj < 8; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * alpha);
-            tmem_st8(lane_base + kO + c0, v);
-          }
-          tmem_st_wait();
+          rescale_columns(lane_base + kO, D, alpha);
           l_sum[0] *= alpha;
           l_sum[1] *= alpha;
           if (need) m_used = m_tile;
         }
       }
       if (e == 0 && m_used == -INFINITY) m_used = 0.f;  // (nothing counted so far)
-      // pass 2: P = exp2(S2 - m) as bf16 over the consumed S columns (chunk c lands in columns 16c..16c+15,
-      // always behind the columns still to be read)
-      float2 psum2 = make_float2(0.f, 0.f);
-      auto exp_chunk = [&](const uint32_t (&v)[32], int c) {
-        const int tt = (32 * c) / CP;
-        const float negmu = valid_all[tt] ? tb_all[tt] - m_used : -INFINITY;
-        const float2 w2 = make_float2(wmul[tt], wmul[tt]), n2 = make_float2(negmu, negmu);
-        uint32_t pk[16];
-#pragma unroll
-        for (int jj = 0; jj < 32; jj += 2) {
-          const int k = (32 * c + jj) % CP;
-          float2 t = ffma2(make_float2(__uint_as_float(v[jj]), __uint_as_float(v[jj + 1])), w2, make_float2(cbf[k], cbf[k + 1]));
-          t = fadd2(t, n2);
-          const float2 ex = poly_pair(jj / 2) ? ex2_poly2(t) : make_float2(ex2(t.x), ex2(t.y));
-          psum2 = fadd2(psum2, ex);
-          pk[jj / 2] = pack_bf16(ex.x, ex.y);
-        }
-        tmem_st16(s_addr + 16 * c, pk);
-      };
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 32, vb);
-      exp_chunk(va, 0);
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 64, va);
-      exp_chunk(vb, 1);
-      tmem_ld_wait();
-      tmem_ld32(s_addr + 96, vb);
-      exp_chunk(va, 2);
-      tmem_ld_wait();
-      exp_chunk(vb, 3);
-      if (e & 1) l_sum[1] += psum2.x + psum2.y;
-      else l_sum[0] += psum2.x + psum2.y;
+      const float psum = dense_exp<CP>(s_addr, t, cbf, m_used, va);
+      if (e & 1) l_sum[1] += psum;
+      else l_sum[0] += psum;
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars[kPFull]);
