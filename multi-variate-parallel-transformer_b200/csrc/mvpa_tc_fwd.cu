@@ -46,6 +46,9 @@ constexpr uint32_t kColS = 0;  // + 128 * buf
 constexpr uint32_t kColO = 256;
 constexpr uint32_t kColTB = 384;
 constexpr float kRescaleThreshold = 8.f;  // log2 units: P stays below 2^8
+// The maximum over light tiles starts here, not at minus infinity: where it is a row's first maximum and no light pair counts
+// (every score minus infinity), each factor is then 2^-inf = 0 and the first dense tile's maximum takes its place.
+constexpr float kLowest = -3.4028234663852886e38f;
 
 struct TcMaps {
   CUtensorMap q, k, v, rt, rc;
@@ -679,7 +682,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
     }
     if (ok && n_light > 0) {
       const int col1 = col0 + n_light * TPB;
-      float m_light = -INFINITY;
+      float m_light = kLowest;
 #pragma unroll 1
       for (int c = col0 & ~15; c < col1; c += 16) {  // (warp-uniform; a short loop, as everything that runs once per CTA)
         uint32_t v[16];
@@ -702,7 +705,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         if (need) m_used = m_light;
       }
     }
-    const float m_ref = m_used == -INFINITY ? 0.f : m_used;  // (light tiles first, and no light pair counts: every factor is 0)
     // Two tiles per turn: one round trip for the temporal scores and one look at the barriers serve both,
     // and the second tile's products are formed while the first tile's stores are in flight.  (The scores
     // of the next pair are fetched meanwhile; with an odd count the last fetch reads the column after the
@@ -741,7 +743,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           for (int q = 0; q < TPB; ++q)
             if (q == tt) raw = tb_next[u * TPB + q];
           const float tb = p.c2 * (__uint_as_float(raw) + s_vr[col0 + (l + u) * TPB + tt]) + mc;
-          a_t[u][tl] = ex2(tb - m_ref);
+          a_t[u][tl] = ex2(tb - m_used);
         }
       }
       if (l + 2 < n_light) tb_fetch(l + 2);
@@ -820,7 +822,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           const bool need = m_tile > m_used + kRescaleThreshold;
           const float alpha = need ? ex2(m_used - m_tile) : 1.f;
           if (need) m_used = m_tile;
-          if (s == 0 && m_used == -INFINITY) m_used = 0.f;  // (nothing counted so far)
           s_merge[wg * 128 + row] = m_used;
           mbar_arrive(&bars[kBarMax + wg]);
           if (__any_sync(0xffffffffu, need)) {

@@ -304,6 +304,7 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) s_td[(c + jj) * 128 + row] = score(v[jj], j0 + jj);  // (t_k > t_i: not used)
       }
+      m_used = kLowest;
 #pragma unroll 1
       for (int c = 0; c < light_steps; c += 16) {
         uint32_t v[2][8];
@@ -314,7 +315,6 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         for (int jj = 0; jj < 16; ++jj)
           if (c + jj < light_steps) m_used = fmaxf(m_used, score(v[jj / 8][jj % 8], col0 + c + jj));
       }
-      const float m_ref = m_used == -INFINITY ? 0.f : m_used;  // (no light pair counts: every factor is 0)
 #pragma unroll 1
       for (int c = 0; c < light_steps; c += 16) {
         uint32_t v[2][8], w[8];
@@ -323,8 +323,8 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
         tmem_ld_wait();
 #pragma unroll
         for (int jj = 0; jj < 16; jj += 2)
-          w[jj / 2] = pack_bf16(ex2(score(v[jj / 8][jj % 8], col0 + c + jj) - m_ref),
-                                ex2(score(v[jj / 8][jj % 8 + 1], col0 + c + jj + 1) - m_ref));
+          w[jj / 2] = pack_bf16(ex2(score(v[jj / 8][jj % 8], col0 + c + jj) - m_used),
+                                ex2(score(v[jj / 8][jj % 8 + 1], col0 + c + jj + 1) - m_used));
         tmem_st8(lane_base + kX + c / 2, w);
       }
     }
@@ -407,7 +407,7 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
       uint32_t va[32];
       const float m_tile = dense_max<CP>(s_addr, t, cbf, va);
       if (e == 0 && n_light == 0) {
-        m_used = m_tile;
+        m_used = (m_tile == -INFINITY) ? 0.f : m_tile;
       } else {
         // O and l follow the maximum only when it moved by more than 2^8 (every PV product so far is complete: the
         // score product that has just been waited for was issued behind them)
@@ -420,7 +420,6 @@ tc_fwd_two_kernel(const __grid_constant__ TcMaps maps, const TcArgs p) {
           if (need) m_used = m_tile;
         }
       }
-      if (e == 0 && m_used == -INFINITY) m_used = 0.f;  // (nothing counted so far)
       const float psum = dense_exp<CP>(s_addr, t, cbf, m_used, va);
       if (e & 1) l_sum[1] += psum;
       else l_sum[0] += psum;
