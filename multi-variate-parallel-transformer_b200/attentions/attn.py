@@ -116,15 +116,20 @@ def _lay_out(q, u, vt, z, k, r_time, r_chan, v, q_time):
     """The operands as the kernels read them, copied only where their layout asks for it.  (They read through pointers: what
     does not go together is refused here.)"""
     _need_cuda(q)
-    Hkv, N, D = k.shape[1:]
+    B, Hkv, N, D = shape = k.shape
+    Bq, _, Nq, Dq = q.shape
     T, C = r_time.shape[-2], r_chan.shape[-2]
-    if (k.shape != v.shape or k.shape[0] != q.shape[0] or q.shape[3] != D or T * C != N or q.shape[2] != (q_time[1] or T) * C
-            or any(t.numel() != Hkv * n * D for t, n in ((u, 1), (vt, 1), (z, 1), (r_time, T), (r_chan, C)))):
+    row = Hkv * D
+    if (v.shape != shape or Bq != B or Dq != D or T * C != N or Nq != (q_time[1] or T) * C or u.numel() != row or vt.numel() != row
+            or z.numel() != row or r_time.numel() != row * T or r_chan.numel() != row * C):
         raise RuntimeError("flash_mvpa: the operands' shapes do not go together: "
                            + ", ".join(str(tuple(t.shape)) for t in (q, u, vt, z, k, r_time, r_chan, v)))
-    for t in (u, vt, z, k, r_time, r_chan, v):
-        if t.dtype != q.dtype or t.device != q.device:
-            raise RuntimeError(f"flash_mvpa: an operand is {t.dtype} on {t.device}, q is {q.dtype} on {q.device}")
+    dtype, device = q.dtype, q.get_device()
+    if not (u.dtype is vt.dtype is z.dtype is k.dtype is r_time.dtype is r_chan.dtype is v.dtype is dtype
+            and u.get_device() == vt.get_device() == z.get_device() == k.get_device() == r_time.get_device()
+            == r_chan.get_device() == v.get_device() == device):
+        raise RuntimeError("flash_mvpa: the operands are of different types or on different devices: "
+                           + ", ".join(f"{t.dtype} {t.device}" for t in (q, u, vt, z, k, r_time, r_chan, v)))
     return (_rows(q), u.contiguous(), vt.contiguous(), z.contiguous(), _rows(k), r_time.contiguous(), r_chan.contiguous(),
             _rows(v))
 
