@@ -744,7 +744,7 @@ def triton_point(args, device_index):
 def kernels_of_a_call(torch, attentions, t, w, flush, gout) -> str:
     """The library's kernels of one timed call, as the profiler names them (after everything that is timed)."""
     from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
         time_kernel(torch, attentions, t, w, 1, 0, flush, gout)
         torch.cuda.synchronize()
     names = [n for e in prof.events() for n in re.findall(r"\b(?:tc|simt|rel)_\w+_kernel(?:<[\w, ]*>)?", e.name)]
